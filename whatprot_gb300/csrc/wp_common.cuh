@@ -592,6 +592,43 @@ struct KBArgs {
                                 // the final top's distance, 4 scratch too small
 };
 
+// The k-hit set by levels (wp_khits.cu): the same inputs and results for
+// non-interacting models with counts of at most 15; per warp a list of `cap`
+// entries and the bins' scratch.
+struct KHArgs {
+    int R;                      // query slots
+    int* next;                  // work counter, zero on entry
+    const int* qperm;           // read index of each slot
+    const double* rads;         // [reads][TC] FP64 queries
+    int TC, C, DP, N;
+    long long k;                // < 2^31, at most the hits of all entries (< 2^31)
+    const uint8_t* cnt;         // [N][DP] counts (tree order)
+    const uint4* nib;           // [N / 128 up][DP / 8][32]: 8 counts each of a lane's four entries
+                                // (32 apart), four bits a count (byte u: coordinate 8j + u low,
+                                // 8j + 4 + u high)
+    const float* enorm;         // squared norms, padded to whole 128s
+    const double* ctab;         // [C][NC] coordinate of count n
+    int NC;                     // 2 .. 16
+    const float* llo;           // [nodes][DP] per leaf: box
+    const float* lhi;
+    const int* hits;            // [N]
+    const KDNode* nodes;
+    int stack_cap;
+    int cap;
+    int2* ent;                  // [warps][cap]
+    float* d;                   // [warps][cap]
+    uint16_t* bin;              // [warps][cap]
+    int2* order;                // [warps][cap]
+    uint16_t* rank;             // [warps][cap]
+    int4* state;                // [warps][2][groups]
+    long long* mem_d;           // [warps][rank limit]
+    unsigned* mem_k;            // [warps][rank limit]
+    int2* sorted;               // [warps][rank limit]
+    double* tf_d;               // per slot, as KBArgs; flag 4: left to the replay
+    int* tf_pos;
+    int* tf_flag;
+};
+
 // FP64 squared distance from a query to entry p as LeafNode::consider sums
 // it (kd-tree/leaf-node.h:31-62): per coordinate x = q - e, x * x, summed in
 // groups of four while i < D - 3, then singly.  Coordinates from the count
