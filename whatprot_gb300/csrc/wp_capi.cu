@@ -57,6 +57,8 @@ cudaError_t wp_launch_nn_select(int grid, cudaStream_t s, const NNSelectArgs& a)
 cudaError_t wp_launch_nn_threshold(cudaStream_t s, const NNArgs& a);
 cudaError_t wp_launch_nn_estimate(int DP, cudaStream_t s, const NNArgs& a);
 size_t wp_nn_sort_temp_bytes(int R);
+cudaError_t wp_launch_nn_subset(const float* rows, const int* list, int n, int DP, float* out, cudaStream_t s);
+cudaError_t wp_launch_nn_remap(int* perm, const int* list, int n, cudaStream_t s);
 cudaError_t wp_launch_nn_redo(const NNArgs& a, int* list, int* count, int shift, cudaStream_t s);
 cudaError_t wp_launch_nn_zero_hist(const NNArgs& a, cudaStream_t s);
 cudaError_t wp_launch_nn_sort_queries(const float* rows, int R, int DP, int TC, float* sorted, int* perm,
@@ -290,7 +292,8 @@ struct wp_ctx {
     DevBuf d_kb_reg, d_kb_prev, d_kb_stage, d_kb_next, d_kb_work, d_kb_tfd, d_kb_tfpos, d_kb_tfflag;
     // the k-hit sets by levels (wp_khits.cu): counts as nibbles, scratch
     bool nn_nib_packed = false;
-    DevBuf d_nn_nib, d_kh_ent, d_kh_d, d_kh_bin, d_kh_order, d_kh_rank, d_kh_state, d_kh_memd, d_kh_memk, d_kh_sorted;
+    DevBuf d_nn_nib, d_kh_ent, d_kh_d, d_kh_bin, d_kh_order, d_kh_rank, d_kh_state, d_kh_memd, d_kh_memk, d_kh_sorted, d_kh_seg, d_kh_kpos, d_kh_kd2,
+            d_kh_kn, d_nn_subset, d_nn_subq;
 
     // Per-batch scratch.
     DevBuf d_rads, d_lo, d_hi, d_Ls, d_Up, d_Lpk, d_Upk, d_allow, d_flags, d_table, d_gtab, d_gdelta, d_gK,
@@ -1014,13 +1017,24 @@ wp_status nn_prepare_peptides(wp_ctx* ctx) {
     return WP_OK;
 }
 
-// The reference's k-hit sets by levels (wp_khits.cu) for every query slot;
-// slots that it leaves to the replay are flagged.
-wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int R, long long k) {
+// Whether the reference's k-hit sets can be found by levels (wp_khits.cu):
+// coordinates that are a channel's mean times the count, counts of at most 15,
+// hits that reach k and whose sums fit 31 bits.
+bool nn_by_levels(const wp_ctx* ctx, long long k) {
+    return ctx->nn_selection == WP_NN_KDTREE && !ctx->nn_inter && ctx->nn_NC >= 2 && ctx->nn_NC <= 16 &&
+           k <= ctx->nn_hits_total && ctx->nn_hits_total < (1ll << 31);
+}
+
+// The k-hit sets by levels of the query slots q0 .. q0 + n: their entries in
+// d_kh_kpos / d_kh_kd2 (`stride` places each), their numbers in d_kh_kn (-1:
+// left to the replay).
+wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int q0, int n, long stride, long long k) {
     const int TC = ctx->nn_T * ctx->nn_C;
     KHArgs a;
     memset(&a, 0, sizeof(a));
-    a.R = R;
+    a.q0 = q0;
+    a.Rc = n;
+    a.stride = stride;
     a.next = ctx->d_kb_next.as<int>();
     a.qperm = ctx->d_nn_qperm.as<int>();
     a.rads = d_rads;
@@ -1030,6 +1044,7 @@ wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int R, long long k) {
     a.N = ctx->nn_N;
     a.k = k;
     a.cnt = ctx->d_nn_cnt8.as<uint8_t>();
+    a.coords = ctx->d_nn_coords.as<float>();
     a.enorm = ctx->d_nn_enorm.as<float>();
     a.ctab = ctx->d_nn_ctab.as<double>();
     a.NC = ctx->nn_NC;
@@ -1038,9 +1053,9 @@ wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int R, long long k) {
     a.hits = ctx->d_nn_hits.as<int>();
     a.nodes = ctx->d_nn_nodes.as<KDNode>();
     a.stack_cap = ctx->nn_depth + 2;
-    a.tf_d = ctx->d_kb_tfd.as<double>();
-    a.tf_pos = ctx->d_kb_tfpos.as<int>();
-    a.tf_flag = ctx->d_kb_tfflag.as<int>();
+    a.kept_pos = ctx->d_kh_kpos.as<int>();
+    a.kept_d2 = ctx->d_kh_kd2.as<float>();
+    a.kept_n = ctx->d_kh_kn.as<int>();
     if (!ctx->nn_nib_packed) {  // once per training set
         WP_CUDA(ctx->d_nn_nib.ensure(((size_t)a.N + 127) / 128 * 128 * (a.DP / 2)), "alloc kNN counts");
         WP_CUDA(wp_launch_khits_pack(a.cnt, a.N, a.DP, ctx->d_nn_nib.as<uint4>(), ctx->stream), "pack kNN counts");
@@ -1058,8 +1073,8 @@ wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int R, long long k) {
     if (smem > (size_t)dev_smem) return fail(ctx, WP_ERR_UNSUPPORTED, "kd-tree kNN: per-read tables exceed shared memory");
     const int wpc = wp_khits_warps_per_cta();
     const int per_sm = std::max(1, std::min(4, (int)((size_t)(228 * 1024) / (smem + 1024))));
-    long long grid = std::min<long long>((long long)sms * per_sm, (R + wpc - 1) / wpc);
-    const size_t per_warp = (size_t)a.cap * 24 + (size_t)wp_khits_groups() * 32 + (size_t)wp_khits_rank() * 20;
+    long long grid = std::min<long long>((long long)sms * per_sm, (n + wpc - 1) / wpc);
+    const size_t per_warp = (size_t)a.cap * 24 + (size_t)wp_khits_groups() * 40 + (size_t)wp_khits_rank() * 20;
     grid = std::max<long long>(1, std::min<long long>(grid, (long long)((6ull << 30) / (per_warp * wpc))));
     const size_t warps = (size_t)grid * wpc, list = a.cap * warps;
     WP_CUDA(ctx->d_kh_ent.ensure(sizeof(int2) * list), "alloc kNN lists");
@@ -1068,6 +1083,7 @@ wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int R, long long k) {
     WP_CUDA(ctx->d_kh_order.ensure(sizeof(int2) * list), "alloc kNN lists");
     WP_CUDA(ctx->d_kh_rank.ensure(sizeof(uint16_t) * list), "alloc kNN lists");
     WP_CUDA(ctx->d_kh_state.ensure(sizeof(int4) * 2 * wp_khits_groups() * warps), "alloc kNN lists");
+    WP_CUDA(ctx->d_kh_seg.ensure(sizeof(int2) * wp_khits_groups() * warps), "alloc kNN lists");
     WP_CUDA(ctx->d_kh_memd.ensure(sizeof(long long) * wp_khits_rank() * warps), "alloc kNN lists");
     WP_CUDA(ctx->d_kh_memk.ensure(sizeof(unsigned) * wp_khits_rank() * warps), "alloc kNN lists");
     WP_CUDA(ctx->d_kh_sorted.ensure(sizeof(int2) * wp_khits_rank() * warps), "alloc kNN lists");
@@ -1077,6 +1093,7 @@ wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int R, long long k) {
     a.order = ctx->d_kh_order.as<int2>();
     a.rank = ctx->d_kh_rank.as<uint16_t>();
     a.state = ctx->d_kh_state.as<int4>();
+    a.seg = ctx->d_kh_seg.as<int2>();
     a.mem_d = ctx->d_kh_memd.as<long long>();
     a.mem_k = ctx->d_kh_memk.as<unsigned>();
     a.sorted = ctx->d_kh_sorted.as<int2>();
@@ -1088,11 +1105,8 @@ wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int R, long long k) {
 }
 
 // The reference's k-hit set for R query slots (wp_kbest.cu): per slot the
-// final top of KBest.  Where the model and the counts allow it the sets are
-// found by levels (wp_khits.cu, 4.6 times as fast at 946,000 tracks and
-// k = 10,000), and the replay takes only the slots left over.  Slots whose scratch
-// ran out are replayed again by fewer warps with four times the scratch, then
-// sixteen times.
+// final top of KBest.  Slots whose scratch ran out are replayed again by
+// fewer warps with four times the scratch, then sixteen times.
 wp_status nn_replay(wp_ctx* ctx, const double* d_rads, int R, long long k) {
     const int T = ctx->nn_T, C = ctx->nn_C, TC = T * C;
     if (ctx->nn_NC == 0) return fail(ctx, WP_ERR_UNSUPPORTED, "kd-tree kNN needs dye counts in 0..255");
@@ -1137,23 +1151,7 @@ wp_status nn_replay(wp_ctx* ctx, const double* d_rads, int R, long long k) {
     // at a time, latency-bound: residency is what speeds it up)
     const int per_sm = std::max(1, std::min(8, (int)((size_t)(228 * 1024) / (smem + 1024))));
     const int ch = wp_kbest_chunk();
-    std::vector<int> redo, flags(R);
-    auto read_flags = [&]() -> wp_status {
-        WP_CUDA(cudaMemcpyAsync(flags.data(), a.tf_flag, sizeof(int) * R, cudaMemcpyDeviceToHost, ctx->stream), "copy");
-        WP_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
-        redo.clear();
-        for (int r = 0; r < R; r++)
-            if (flags[r] & 4) redo.push_back(r);
-        return WP_OK;
-    };
-    const bool by_levels = !ctx->nn_inter && ctx->nn_NC >= 2 && ctx->nn_NC <= 16 && k <= ctx->nn_hits_total &&
-                           ctx->nn_hits_total < (1ll << 31);
-    if (by_levels) {
-        wp_status st = nn_khits(ctx, d_rads, R, k);
-        if (st == WP_OK) st = read_flags();
-        if (st != WP_OK) return st;
-        if (redo.empty()) return WP_OK;
-    }
+    std::vector<int> redo;
     for (int round = 0; round < 3; round++) {
         // live entries stay below about k plus the extras KBest keeps
         const long long grow = 1ll << (2 * round);
@@ -1162,7 +1160,7 @@ wp_status nn_replay(wp_ctx* ctx, const double* d_rads, int R, long long k) {
         a.regcap = (int)(((2 * stage + 2048ll * ch) + ch - 1) / ch * ch);
         if (a.regcap / ch > 65535) a.regcap = 65535 * ch;
         int grid = sms * per_sm;
-        if (!redo.empty()) {
+        if (round > 0) {
             const int wpc = wp_kbest_warps_per_cta();
             grid = std::max(1, std::min(grid, ((int)redo.size() + wpc - 1) / wpc));
         }
@@ -1173,7 +1171,7 @@ wp_status nn_replay(wp_ctx* ctx, const double* d_rads, int R, long long k) {
         a.reg = ctx->d_kb_reg.as<KBItem>();
         a.prev = ctx->d_kb_prev.as<int>();
         a.stage = ctx->d_kb_stage.as<KBItem>();
-        if (redo.empty()) {
+        if (round == 0) {
             a.nwork = R;
             a.work = nullptr;
         } else {
@@ -1189,64 +1187,98 @@ wp_status nn_replay(wp_ctx* ctx, const double* d_rads, int R, long long k) {
             WP_CUDA(wp_launch_kbest(grid, ctx->stream, a), "kNN kd-tree replay");
             ctx->launches++;
         }
-        const wp_status st = read_flags();
-        if (st != WP_OK) return st;
+        std::vector<int> flags(R);
+        WP_CUDA(cudaMemcpyAsync(flags.data(), a.tf_flag, sizeof(int) * R, cudaMemcpyDeviceToHost, ctx->stream), "copy");
+        WP_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
+        redo.clear();
+        for (int r = 0; r < R; r++)
+            if (flags[r] & 4) redo.push_back(r);
         if (redo.empty()) return WP_OK;
     }
     return fail(ctx, WP_ERR_UNSUPPORTED, "kd-tree kNN: replay scratch exhausted");
 }
 
-// The kNN stage for R reads already on the device (FP64 [R][T][C]):
-// per read the top-h candidates in ascending (score, id) order, the total
-// and, when hybrid, candidate peptide indices and the subfraction.
-wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, int h, bool hybrid) {
+// The select kernel's arguments that do not depend on the reads' route, and
+// its per-warp accumulators.
+wp_status nn_select_args(wp_ctx* ctx, const double* d_rads, int k, double sig, int h, bool hybrid, int sel_grid,
+                         NNSelectArgs* out) {
+    const int T = ctx->nn_T, C = ctx->nn_C, DP = nn_padded_dim(T * C);
+    const long nwarps = (long)sel_grid * wp_nn_select_warps();
+    const int U = std::max(ctx->nn_U, 1);
+    WP_CUDA(ctx->d_nn_acc.ensure(sizeof(double) * nwarps * U), "alloc kNN accumulators");
+    WP_CUDA(ctx->d_nn_mark.ensure(sizeof(int) * nwarps * U), "alloc kNN accumulators");
+    WP_CUDA(ctx->d_nn_touched.ensure(sizeof(int) * nwarps * U), "alloc kNN accumulators");
+    // The select kernel leaves every accumulator it touched at zero again,
+    // so memory is cleared once, when first used.
+    if (sizeof(double) * nwarps * U > ctx->nn_acc_cleared) {
+        WP_CUDA(cudaMemsetAsync(ctx->d_nn_acc.p, 0, sizeof(double) * nwarps * U, ctx->stream), "clear");
+        WP_CUDA(cudaMemsetAsync(ctx->d_nn_mark.p, 0, sizeof(int) * nwarps * U, ctx->stream), "clear");
+        ctx->nn_acc_cleared = sizeof(double) * nwarps * U;
+    }
+    NNSelectArgs& b = *out;
+    memset(&b, 0, sizeof(b));
+    b.qperm = ctx->d_nn_qperm.as<int>();
+    b.hits = ctx->d_nn_hits.as<int>();
+    b.src_off = ctx->d_nn_src_off.as<int>();
+    b.src_dense = ctx->d_nn_src_dense.as<int>();
+    b.src_ratio = ctx->d_nn_src_ratio.as<double>();
+    b.src_hits = ctx->d_nn_src_hits.as<int>();
+    b.dense_id = ctx->d_nn_dense_id.as<int>();
+    b.dense_pep = hybrid ? ctx->d_nn_dense_pep.as<int>() : nullptr;
+    b.dense_count = hybrid ? ctx->d_nn_dense_count.as<int>() : nullptr;
+    b.U = U;
+    b.k = k;
+    b.inv_two_sig_sq = (float)(1.0 / (2.0 * sig * sig));
+    b.h = h;
+    b.acc = ctx->d_nn_acc.as<double>();
+    b.mark = ctx->d_nn_mark.as<int>();
+    b.touched = ctx->d_nn_touched.as<int>();
+    b.out_ncand = ctx->d_nn_ncand.as<int>();
+    b.out_cand_id = ctx->d_nn_cand_id.as<int>();
+    b.out_cand_pep = hybrid ? ctx->d_nn_cand_pep.as<int>() : nullptr;
+    b.out_cand_score = ctx->d_nn_cand_score.as<double>();
+    b.out_total = ctx->d_nn_total.as<double>();
+    b.out_subfrac = hybrid ? ctx->d_nn_subfrac.as<double>() : nullptr;
+    b.two_sig_sq = 2.0 * sig * sig;
+    if (ctx->nn_NC > 0) {
+        b.rads = d_rads;
+        b.TC = T * C;
+        b.C = C;
+        b.DP = DP;
+        b.NC = ctx->nn_NC;
+        b.cnt = ctx->d_nn_cnt8.as<uint8_t>();
+        b.ctab = ctx->d_nn_ctab.as<double>();
+        b.ecoord = ctx->nn_inter ? ctx->d_nn_ecoord.as<double>() : nullptr;
+    }
+    return WP_OK;
+}
+
+// n query rows in an order that groups alike ones: d_nn_qsorted, and each
+// slot's row in d_nn_qperm (results go back by it).
+wp_status nn_sort_rows(wp_ctx* ctx, const float* rows, int n, int DP, int TC) {
+    const size_t Rz = (size_t)std::max(n, 1);
+    WP_CUDA(ctx->d_nn_qsorted.ensure(sizeof(float) * Rz * DP), "alloc");
+    WP_CUDA(ctx->d_nn_qperm.ensure(sizeof(int) * Rz), "alloc");
+    WP_CUDA(ctx->d_nn_qkeys.ensure(sizeof(unsigned long long) * 2 * Rz), "alloc");
+    WP_CUDA(ctx->d_nn_qidx.ensure(sizeof(int) * 2 * Rz), "alloc");
+    const size_t tb = wp_nn_sort_temp_bytes(n);
+    WP_CUDA(ctx->d_nn_qtemp.ensure(std::max<size_t>(tb, 1)), "alloc");
+    WP_CUDA(wp_launch_nn_sort_queries(rows, n, DP, TC, ctx->d_nn_qsorted.as<float>(), ctx->d_nn_qperm.as<int>(),
+                                      ctx->d_nn_qkeys.as<unsigned long long>(), ctx->d_nn_qidx.as<int>(),
+                                      ctx->d_nn_qtemp.p, tb, ctx->stream),
+            "sort queries");
+    ctx->launches += 3;
+    return WP_OK;
+}
+
+// The kNN stage by brute force over the sorted query slots 0 .. R (d_nn_qsorted,
+// d_nn_qperm): the distance-ordered k-hit sets, or the replayed search's.
+wp_status nn_run_slots(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, int h, bool hybrid) {
     const int T = ctx->nn_T, C = ctx->nn_C, N = ctx->nn_N;
     const int DP = nn_padded_dim(T * C);
-    wp_status st = nn_prepare(ctx, k);
-    if (st != WP_OK) return st;
-    const bool exact = ctx->nn_selection == WP_NN_KDTREE;
-    if (hybrid) {
-        st = nn_prepare_peptides(ctx);
-        if (st != WP_OK) return st;
-    }
     const size_t Rz = (size_t)std::max(R, 1);
-    WP_CUDA(ctx->d_nn_queries.ensure(sizeof(float) * Rz * DP), "alloc queries");
-    WP_CUDA(ctx->d_nn_qbin.ensure(sizeof(int) * Rz), "alloc");
-    WP_CUDA(ctx->d_nn_qbase.ensure(sizeof(int) * Rz), "alloc");
-    WP_CUDA(ctx->d_nn_qbelow.ensure(sizeof(int) * Rz), "alloc");
-    WP_CUDA(ctx->d_nn_qcap.ensure(sizeof(long long) * Rz), "alloc");
-    WP_CUDA(ctx->d_nn_qoff.ensure(sizeof(long long) * Rz), "alloc");
-    WP_CUDA(ctx->d_nn_ncand.ensure(sizeof(int) * Rz), "alloc");
-    WP_CUDA(ctx->d_nn_cand_id.ensure(sizeof(int) * Rz * h), "alloc");
-    WP_CUDA(ctx->d_nn_cand_pep.ensure(sizeof(int) * Rz * h), "alloc");
-    WP_CUDA(ctx->d_nn_cand_score.ensure(sizeof(double) * Rz * h), "alloc");
-    WP_CUDA(ctx->d_nn_total.ensure(sizeof(double) * Rz), "alloc");
-    WP_CUDA(ctx->d_nn_subfrac.ensure(sizeof(double) * Rz), "alloc");
-    WP_CUDA(ctx->d_nn_err.ensure(sizeof(int)), "alloc");
-    WP_CUDA(cudaMemsetAsync(ctx->d_nn_err.p, 0, sizeof(int), ctx->stream), "clear");
-    if (R == 0) return WP_OK;
-    if (N == 0) {
-        WP_CUDA(cudaMemsetAsync(ctx->d_nn_ncand.p, 0, sizeof(int) * R, ctx->stream), "clear");
-        WP_CUDA(cudaMemsetAsync(ctx->d_nn_total.p, 0, sizeof(double) * R, ctx->stream), "clear");
-        WP_CUDA(cudaMemsetAsync(ctx->d_nn_subfrac.p, 0, sizeof(double) * R, ctx->stream), "clear");
-        return WP_OK;
-    }
-    WP_CUDA(wp_launch_nn_queries(d_rads, R, T * C, DP, ctx->d_nn_queries.as<float>(), ctx->stream), "queries");
-    ctx->launches++;
-    // reads in an order that groups alike ones (results go back by perm)
-    {
-        WP_CUDA(ctx->d_nn_qsorted.ensure(sizeof(float) * Rz * DP), "alloc");
-        WP_CUDA(ctx->d_nn_qperm.ensure(sizeof(int) * Rz), "alloc");
-        WP_CUDA(ctx->d_nn_qkeys.ensure(sizeof(unsigned long long) * 2 * Rz), "alloc");
-        WP_CUDA(ctx->d_nn_qidx.ensure(sizeof(int) * 2 * Rz), "alloc");
-        const size_t tb = wp_nn_sort_temp_bytes(R);
-        WP_CUDA(ctx->d_nn_qtemp.ensure(std::max<size_t>(tb, 1)), "alloc");
-        WP_CUDA(wp_launch_nn_sort_queries(ctx->d_nn_queries.as<float>(), R, DP, T * C, ctx->d_nn_qsorted.as<float>(),
-                                          ctx->d_nn_qperm.as<int>(), ctx->d_nn_qkeys.as<unsigned long long>(),
-                                          ctx->d_nn_qidx.as<int>(), ctx->d_nn_qtemp.p, tb, ctx->stream),
-                "sort queries");
-        ctx->launches += 3;
-    }
+    const bool exact = ctx->nn_selection == WP_NN_KDTREE;
+    wp_status st = WP_OK;
     if (exact) {
         st = nn_replay(ctx, d_rads, R, k);
         if (st != WP_OK) return st;
@@ -1348,20 +1380,10 @@ wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, in
     WP_CUDA(cudaMemcpyAsync(cap.data(), a.qcap, sizeof(long long) * R, cudaMemcpyDeviceToHost, ctx->stream),
             "copy caps");
     WP_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
-    // per-warp accumulators of the select kernel
     const int sel_grid = sms * 4;
-    const long nwarps = (long)sel_grid * wp_nn_select_warps();
-    const int U = std::max(ctx->nn_U, 1);
-    WP_CUDA(ctx->d_nn_acc.ensure(sizeof(double) * nwarps * U), "alloc kNN accumulators");
-    WP_CUDA(ctx->d_nn_mark.ensure(sizeof(int) * nwarps * U), "alloc kNN accumulators");
-    WP_CUDA(ctx->d_nn_touched.ensure(sizeof(int) * nwarps * U), "alloc kNN accumulators");
-    // The select kernel leaves every accumulator it touched at zero again,
-    // so memory is cleared once, when first used.
-    if (sizeof(double) * nwarps * U > ctx->nn_acc_cleared) {
-        WP_CUDA(cudaMemsetAsync(ctx->d_nn_acc.p, 0, sizeof(double) * nwarps * U, ctx->stream), "clear");
-        WP_CUDA(cudaMemsetAsync(ctx->d_nn_mark.p, 0, sizeof(int) * nwarps * U, ctx->stream), "clear");
-        ctx->nn_acc_cleared = sizeof(double) * nwarps * U;
-    }
+    NNSelectArgs b;
+    st = nn_select_args(ctx, d_rads, k, sig, h, hybrid, sel_grid, &b);
+    if (st != WP_OK) return st;
     // chunks of reads whose candidate lists fit the budget
     const long long budget = 256ll << 20;  // candidates per chunk (2 GiB of lists)
     int r0 = 0;
@@ -1395,12 +1417,9 @@ wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, in
             WP_CUDA(wp_launch_nn_dist(DP, false, ctx->stream, a), "kNN collect");
             ctx->launches++;
         }
-        NNSelectArgs b;
-        memset(&b, 0, sizeof(b));
         b.R = nq;
         b.q0 = r0;
         b.qbin = a.qbin;
-        b.qperm = ctx->d_nn_qperm.as<int>();
         b.qbase = a.qbase;
         b.qbelow = a.qbelow;
         b.slices = a.slices;
@@ -1413,50 +1432,10 @@ wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, in
         b.cand_d2 = a.cand_d2;
         b.cand_hits = a.cand_hits;
         b.cand_bin = a.cand_bin;
-        b.hits = a.hits;
-        b.src_off = ctx->d_nn_src_off.as<int>();
-        b.src_dense = ctx->d_nn_src_dense.as<int>();
-        b.src_ratio = ctx->d_nn_src_ratio.as<double>();
-        b.src_hits = ctx->d_nn_src_hits.as<int>();
-        b.dense_id = ctx->d_nn_dense_id.as<int>();
-        b.dense_pep = hybrid ? ctx->d_nn_dense_pep.as<int>() : nullptr;
-        b.dense_count = hybrid ? ctx->d_nn_dense_count.as<int>() : nullptr;
-        b.U = U;
-        b.k = k;
-        b.inv_two_sig_sq = (float)(1.0 / (2.0 * sig * sig));
-        b.h = h;
-        b.acc = ctx->d_nn_acc.as<double>();
-        b.mark = ctx->d_nn_mark.as<int>();
-        b.touched = ctx->d_nn_touched.as<int>();
-        b.out_ncand = ctx->d_nn_ncand.as<int>();
-        b.out_cand_id = ctx->d_nn_cand_id.as<int>();
-        b.out_cand_pep = hybrid ? ctx->d_nn_cand_pep.as<int>() : nullptr;
-        b.out_cand_score = ctx->d_nn_cand_score.as<double>();
-        b.out_total = ctx->d_nn_total.as<double>();
-        b.out_subfrac = hybrid ? ctx->d_nn_subfrac.as<double>() : nullptr;
-        b.two_sig_sq = 2.0 * sig * sig;
-        if (ctx->nn_NC > 0) {
-            b.rads = d_rads;
-            b.TC = T * C;
-            b.C = C;
-            b.DP = DP;
-            b.NC = ctx->nn_NC;
-            b.cnt = ctx->d_nn_cnt8.as<uint8_t>();
-            b.ctab = ctx->d_nn_ctab.as<double>();
-            b.ecoord = ctx->nn_inter ? ctx->d_nn_ecoord.as<double>() : nullptr;
-        }
         if (exact) {
             b.tf_d = ctx->d_kb_tfd.as<double>();
             b.tf_pos = ctx->d_kb_tfpos.as<int>();
             b.tf_flag = ctx->d_kb_tfflag.as<int>();
-            b.rads = d_rads;
-            b.TC = T * C;
-            b.C = C;
-            b.DP = DP;
-            b.NC = ctx->nn_NC;
-            b.cnt = ctx->d_nn_cnt8.as<uint8_t>();
-            b.ctab = ctx->d_nn_ctab.as<double>();
-            b.ecoord = ctx->nn_inter ? ctx->d_nn_ecoord.as<double>() : nullptr;
         }
         {
             TimedLaunch tl(ctx, 5);
@@ -1465,6 +1444,104 @@ wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, in
         }
         WP_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
         r0 = r1;
+    }
+    return WP_OK;
+}
+
+// The kNN stage for R reads already on the device (FP64 [R][T][C]):
+// per read the top-h candidates in ascending (score, id) order, the total
+// and, when hybrid, candidate peptide indices and the subfraction.
+wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, int h, bool hybrid) {
+    const int T = ctx->nn_T, C = ctx->nn_C, N = ctx->nn_N;
+    const int DP = nn_padded_dim(T * C);
+    wp_status st = nn_prepare(ctx, k);
+    if (st != WP_OK) return st;
+    if (hybrid) {
+        st = nn_prepare_peptides(ctx);
+        if (st != WP_OK) return st;
+    }
+    const size_t Rz = (size_t)std::max(R, 1);
+    WP_CUDA(ctx->d_nn_queries.ensure(sizeof(float) * Rz * DP), "alloc queries");
+    WP_CUDA(ctx->d_nn_qbin.ensure(sizeof(int) * Rz), "alloc");
+    WP_CUDA(ctx->d_nn_qbase.ensure(sizeof(int) * Rz), "alloc");
+    WP_CUDA(ctx->d_nn_qbelow.ensure(sizeof(int) * Rz), "alloc");
+    WP_CUDA(ctx->d_nn_qcap.ensure(sizeof(long long) * Rz), "alloc");
+    WP_CUDA(ctx->d_nn_qoff.ensure(sizeof(long long) * Rz), "alloc");
+    WP_CUDA(ctx->d_nn_ncand.ensure(sizeof(int) * Rz), "alloc");
+    WP_CUDA(ctx->d_nn_cand_id.ensure(sizeof(int) * Rz * h), "alloc");
+    WP_CUDA(ctx->d_nn_cand_pep.ensure(sizeof(int) * Rz * h), "alloc");
+    WP_CUDA(ctx->d_nn_cand_score.ensure(sizeof(double) * Rz * h), "alloc");
+    WP_CUDA(ctx->d_nn_total.ensure(sizeof(double) * Rz), "alloc");
+    WP_CUDA(ctx->d_nn_subfrac.ensure(sizeof(double) * Rz), "alloc");
+    WP_CUDA(ctx->d_nn_err.ensure(sizeof(int)), "alloc");
+    WP_CUDA(cudaMemsetAsync(ctx->d_nn_err.p, 0, sizeof(int), ctx->stream), "clear");
+    if (R == 0) return WP_OK;
+    if (N == 0) {
+        WP_CUDA(cudaMemsetAsync(ctx->d_nn_ncand.p, 0, sizeof(int) * R, ctx->stream), "clear");
+        WP_CUDA(cudaMemsetAsync(ctx->d_nn_total.p, 0, sizeof(double) * R, ctx->stream), "clear");
+        WP_CUDA(cudaMemsetAsync(ctx->d_nn_subfrac.p, 0, sizeof(double) * R, ctx->stream), "clear");
+        return WP_OK;
+    }
+    WP_CUDA(wp_launch_nn_queries(d_rads, R, T * C, DP, ctx->d_nn_queries.as<float>(), ctx->stream), "queries");
+    ctx->launches++;
+    st = nn_sort_rows(ctx, ctx->d_nn_queries.as<float>(), R, DP, T * C);
+    if (st != WP_OK) return st;
+    int left = R;
+    if (nn_by_levels(ctx, k)) {
+        // the kept entries of a chunk of reads, then their weights and scores;
+        // a set has at most min(N, k) entries: 2 GiB of lists per chunk
+        const long stride = (long)std::min<long long>(N, k);
+        const int chunk = (int)std::max<long long>(1, std::min<long long>(R, (256ll << 20) / stride));
+        WP_CUDA(ctx->d_kb_next.ensure(sizeof(int)), "alloc");
+        WP_CUDA(ctx->d_kh_kn.ensure(sizeof(int) * Rz), "alloc");
+        WP_CUDA(ctx->d_kh_kpos.ensure(sizeof(int) * (size_t)chunk * stride), "alloc kNN kept sets");
+        WP_CUDA(ctx->d_kh_kd2.ensure(sizeof(float) * (size_t)chunk * stride), "alloc kNN kept sets");
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+        NNSelectArgs b;
+        st = nn_select_args(ctx, d_rads, k, sig, h, hybrid, sms * 4, &b);
+        if (st != WP_OK) return st;
+        b.R_all = R;
+        b.cand_idx = ctx->d_kh_kpos.as<int>();
+        b.cand_d2 = ctx->d_kh_kd2.as<float>();
+        b.kept_n = ctx->d_kh_kn.as<int>();
+        b.stride = stride;
+        for (int r0 = 0; r0 < R; r0 += chunk) {
+            const int n = std::min(chunk, R - r0);
+            st = nn_khits(ctx, d_rads, r0, n, stride, k);
+            if (st != WP_OK) return st;
+            b.R = n;
+            b.q0 = r0;
+            TimedLaunch tl(ctx, 5);
+            WP_CUDA(wp_launch_nn_select(sms * 4, ctx->stream, b), "kNN select");
+            ctx->launches++;
+        }
+        // the slots left to the replay, as a batch of their own
+        std::vector<int> kept(R), perm(R), rest;
+        WP_CUDA(cudaMemcpyAsync(kept.data(), ctx->d_kh_kn.p, sizeof(int) * R, cudaMemcpyDeviceToHost, ctx->stream), "copy");
+        WP_CUDA(cudaMemcpyAsync(perm.data(), ctx->d_nn_qperm.p, sizeof(int) * R, cudaMemcpyDeviceToHost, ctx->stream), "copy");
+        WP_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
+        for (int r = 0; r < R; r++)
+            if (kept[r] < 0) rest.push_back(perm[r]);
+        left = (int)rest.size();
+        if (left > 0) {
+            WP_CUDA(ctx->d_nn_subset.ensure(sizeof(int) * left), "alloc");
+            WP_CUDA(ctx->d_nn_subq.ensure(sizeof(float) * (size_t)left * DP), "alloc");
+            WP_CUDA(cudaMemcpyAsync(ctx->d_nn_subset.p, rest.data(), sizeof(int) * left, cudaMemcpyHostToDevice,
+                                    ctx->stream), "copy");
+            WP_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
+            WP_CUDA(wp_launch_nn_subset(ctx->d_nn_queries.as<float>(), ctx->d_nn_subset.as<int>(), left, DP,
+                                        ctx->d_nn_subq.as<float>(), ctx->stream), "kNN subset");
+            st = nn_sort_rows(ctx, ctx->d_nn_subq.as<float>(), left, DP, T * C);
+            if (st != WP_OK) return st;
+            WP_CUDA(wp_launch_nn_remap(ctx->d_nn_qperm.as<int>(), ctx->d_nn_subset.as<int>(), left, ctx->stream),
+                    "kNN subset");
+            ctx->launches += 2;
+        }
+    }
+    if (left > 0) {
+        st = nn_run_slots(ctx, d_rads, left, k, sig, h, hybrid);
+        if (st != WP_OK) return st;
     }
     int err = 0;
     WP_CUDA(cudaMemcpy(&err, ctx->d_nn_err.p, sizeof(int), cudaMemcpyDeviceToHost), "read err");

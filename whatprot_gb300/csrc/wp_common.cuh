@@ -542,6 +542,10 @@ struct NNSelectArgs {
     const double* tf_d;         // [R_all]
     const int* tf_pos;
     const int* tf_flag;         // bit 0: every entry kept
+    // The kept entries themselves (KHArgs; then cand_idx and cand_d2 have
+    // `stride` places per query): their number, -1 for a query of another route.
+    const int* kept_n;          // [R_all] or null
+    long stride;
     const double* rads;         // [reads][TC] FP64 queries (read order); with
                                 // them the near entries' weights use FP64
                                 // distances
@@ -596,7 +600,6 @@ struct KBArgs {
 // non-interacting models with counts of at most 15; per warp a list of `cap`
 // entries and the bins' scratch.
 struct KHArgs {
-    int R;                      // query slots
     int* next;                  // work counter, zero on entry
     const int* qperm;           // read index of each slot
     const double* rads;         // [reads][TC] FP64 queries
@@ -624,9 +627,16 @@ struct KHArgs {
     long long* mem_d;           // [warps][rank limit]
     unsigned* mem_k;            // [warps][rank limit]
     int2* sorted;               // [warps][rank limit]
-    double* tf_d;               // per slot, as KBArgs; flag 4: left to the replay
-    int* tf_pos;
-    int* tf_flag;
+    int2* seg;                  // [warps][groups]
+    const float* coords;        // [N][DP] FP32 coordinates
+    // per slot: the kept entries in tree order, at most min(N, k) (each has a
+    // hit, and the set is some walk prefix's shortest one), and their number;
+    // -1: left to the replay
+    int q0, Rc;                 // the slots q0 .. q0 + Rc of this launch
+    long stride;                // min(N, k)
+    int* kept_pos;              // [Rc][stride]
+    float* kept_d2;             // [Rc][stride] FP32 squared distances as the collect pass forms them
+    int* kept_n;                // [R]
 };
 
 // FP64 squared distance from a query to entry p as LeafNode::consider sums

@@ -30,7 +30,8 @@
 //      the groups and, per group, an upper bound for the levels inside it,
 //   3. looks inside the few groups whose bound exceeds the maximum found
 //      (their entries ranked by FP64 distance), and
-//   4. ranks the bin that holds the M-th nearest entry: KBest's final top.
+//   4. ranks the bin that holds the M-th nearest entry, KBest's final top, and
+//      writes the M nearest in tree order (the walk's leaves put in order).
 //
 // Exactness.  Only ranks inside the groups of 3 and 4 need FP64 distances; an
 // entry whose FP32 distance lies within its rounding error of a bin edge is
@@ -51,6 +52,9 @@
 // against 132 ms for the replay (20,000 pushes per read, one at a time, and
 // its table look-ups of 48 coordinates for every entry met); 2,000 reads
 // against 70,000 tracks, k = 1,000: 1.1 ms against 4.1 ms.
+// Writing the kept entries here (the list holds them all) spares these reads
+// the brute-force passes that collected them (wp_nn.cu): another 41 of 99 ms
+// and 4.0 of 6.3 ms in the two cases.
 #include <cuda_runtime.h>
 #include <float.h>
 #include <math.h>
@@ -70,6 +74,7 @@ struct KHSmem {
     unsigned cnt[KH_NB];   // entries per bin
     unsigned hit[KH_NB];   // hits per bin; after the walk, the end of each bin in `order`
     int qpos[64];          // screened entries waiting for their distances
+    float4 q32[16];        // the read
 };
 
 // The list of one read and the state of the two moving pointers.
@@ -277,24 +282,27 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
     L.mem_d = a.mem_d + gw * KH_RANK;
     L.mem_k = a.mem_k + gw * KH_RANK;
     L.sorted = a.sorted + gw * KH_RANK;
+    int2* seg = a.seg + gw * KH_MAXG;
     const int k = (int)a.k;
 
     for (;;) {
         int slot = 0;
         if (lane == 0) slot = atomicAdd(a.next, 1);
         slot = __shfl_sync(0xffffffffu, slot, 0);
-        if (slot >= a.R) break;
+        if (slot >= a.Rc) break;
         // from the last (the reads are sorted, those with the most dyes, whose walks
         // are the longest, last) to the first
-        slot = a.R - 1 - slot;
+        slot = a.q0 + a.Rc - 1 - slot;
         const int r = a.qperm ? a.qperm[slot] : slot;
         const double* q64 = a.rads + (long)r * a.TC;
         // ---- the read: distance table, 16-bit rounding for the screen
+        for (int i = a.TC + lane; i < DP; i += 32) reinterpret_cast<float*>(sm->q32)[i] = 0.f;
         float amax = 0.f, qn = 0.f;
         bool finite = true;
         for (int i = lane; i < a.TC; i += 32) {
             const float v = (float)q64[i];
             const float w = (float)(q64[i] * a.ctab[(i % a.C) * a.NC + 1]);
+            reinterpret_cast<float*>(sm->q32)[i] = v;
             finite = finite && isfinite(v) && isfinite(w) && fabsf(v) < 1e6f && fabsf(w) < 1e6f;
             amax = fmaxf(amax, fabsf(w));
             qn = fmaf(v, v, qn);
@@ -337,7 +345,7 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
         __syncwarp();
 
         // ---- 1. the walk: depth first, nearer child first
-        int sp = 1, n = 0, tf = 0, base = 0;
+        int sp = 1, n = 0, tf = 0, base = 0, nseg = 0;
         bool fill = true, have_base = false;
         unsigned S = 0;                      // hits listed (until the fill ends)
         int Htf = 0;                         // hits of the first t_f entries
@@ -399,6 +407,7 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
                 }
                 if (!fill && g2 > ub_edge * (1.f + 1e-4f) + 1e-3f) continue;
             }
+            const int n_leaf = n;
             const int g_lo = nd.begin >> 7, g_hi = (nd.end - 1) >> 7;
             int qn_ = 0;
             uint4 w[DP / 8];
@@ -543,12 +552,16 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
                 if (fatal) break;
               }
             }
+            if (n > n_leaf) {
+                // the leaf's part of the list
+                if (nseg == KH_MAXG) fatal = fatal ? fatal : 10;
+                else if (lane == 0) seg[nseg] = make_int2(nd.begin, n_leaf);
+                nseg++;
+            }
         }
         if (!fatal && fill) fatal = 4;  // the hits never reached k: not for this kernel
 
         int M = 0;
-        double top_d = 0.0;
-        int top_pos = -1;
         if (!fatal) {
             L.n = n;
             // ---- 2. the list by finer bins: the coarse bins from bh (where the
@@ -771,26 +784,61 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
                 } else {
                     kh_bin_d64<DP>(a, L, lane, start, m, sq64);
                     const int want = start + m - M;  // its place, farthest first
-                    int at = -1;
-                    const bool distinct = kh_rank(L, lane, m, [&](int j, int place) {
-                        if (place == want) at = j;
-                    });
-                    const unsigned hit = __ballot_sync(0xffffffffu, at >= 0);
-                    if (hit && distinct) {
-                        at = __shfl_sync(0xffffffffu, at, __ffs(hit) - 1);
-                        top_d = __longlong_as_double(L.mem_d[at]);
-                        top_pos = L.ent[L.order[start + at].x].x;
-                    } else {
-                        fatal = 8;
+                    const bool distinct = kh_rank(
+                        L, lane, m, [&](int j, int place) { L.rank[L.order[start + j].x] = (uint16_t)place; });
+                    if (!distinct) fatal = 8;
+                    __syncwarp();
+                    if (!fatal) {
+                        // the leaves' parts in tree order, the kept entries of each
+                        for (int j = lane; j < nseg; j += 32) {
+                            const int2 s = seg[j];
+                            int place = 0;
+                            for (int v = 0; v < nseg; v++) place += seg[v].x < s.x ? 1 : 0;
+                            L.sorted[place] = make_int2(s.y, j + 1 < nseg ? seg[j + 1].y : n);
+                        }
+                        __syncwarp();
+                        const long out = (long)(slot - a.q0) * a.stride;
+                        int wrote = 0;
+                        for (int s = 0; s < nseg; s++) {
+                            const int2 part = L.sorted[s];
+                            for (int i0 = part.x; i0 < part.y; i0 += 32) {
+                                const int i = i0 + lane;
+                                bool kept = false;
+                                int pos = 0;
+                                if (i < part.y) {
+                                    const int bi = L.bin[i];
+                                    kept = bi < b || (bi == b && (int)L.rank[i] >= want);
+                                    pos = L.ent[i].x;
+                                }
+                                const unsigned km = __ballot_sync(0xffffffffu, kept);
+                                if (kept) {
+                                    // as wp_nn.cu's nn_d2
+                                    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+                                    const float4* e = reinterpret_cast<const float4*>(a.coords + (long)pos * DP);
+#pragma unroll
+                                    for (int u = 0; u < DP / 4; u++) {
+                                        const float4 v = __ldg(e + u), q = sm->q32[u];
+                                        const float x0 = q.x - v.x, x1 = q.y - v.y, x2 = q.z - v.z, x3 = q.w - v.w;
+                                        a0 = fmaf(x0, x0, a0);
+                                        a1 = fmaf(x1, x1, a1);
+                                        a2 = fmaf(x2, x2, a2);
+                                        a3 = fmaf(x3, x3, a3);
+                                    }
+                                    const int at = wrote + __popc(km & below);
+                                    if (at < a.stride) {
+                                        a.kept_pos[out + at] = pos;
+                                        a.kept_d2[out + at] = (a0 + a1) + (a2 + a3);
+                                    }
+                                }
+                                wrote += __popc(km);
+                            }
+                        }
+                        if (wrote != M || wrote > a.stride) fatal = 11;
                     }
                 }
             }
         }
-        if (lane == 0) {
-            a.tf_d[slot] = fatal ? 0.0 : top_d;
-            a.tf_pos[slot] = fatal ? -1 : top_pos;
-            a.tf_flag[slot] = fatal ? 4 | (fatal << 8) : 0;
-        }
+        if (lane == 0) a.kept_n[slot] = fatal ? -1 : M;
         __syncwarp();
     }
 }
@@ -842,7 +890,7 @@ static cudaError_t kh_launch(int grid, size_t smem, cudaStream_t s, const KHArgs
 
 cudaError_t wp_launch_khits(int grid, cudaStream_t s, const KHArgs& a) {
     const size_t smem = wp_khits_smem_bytes(a.TC, a.NC, a.stack_cap);
-    if (grid <= 0 || a.R == 0) return cudaSuccess;
+    if (grid <= 0 || a.Rc == 0) return cudaSuccess;
     switch (a.DP) {
         case 16: return kh_launch<16>(grid, smem, s, a);
         case 32: return kh_launch<32>(grid, smem, s, a);

@@ -598,20 +598,30 @@ __global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelec
 
     for (long lq = gw; lq < a.R; lq += nw) {
         const int gq = a.q0 + (int)lq;
-        const int bstar = a.qbin[gq];
-        long long need = a.k - a.qbelow[gq];  // hits still needed from bin b*
+        // the kept entries are given: one list of kept_n
+        const int kept = a.kept_n ? a.kept_n[gq] : 0;
+        if (kept < 0) continue;
+        const int slices = a.kept_n ? 1 : a.slices;
+        auto seg_begin = [&](int sl) -> long long {
+            return a.kept_n ? lq * a.stride : a.qoff[lq] + a.sliceoff[(long)sl * a.R_all + gq];
+        };
+        auto seg_count = [&](int sl) -> long long {
+            return a.kept_n ? kept : min(a.slicecnt[(long)sl * a.R_all + gq], a.slicecap[(long)sl * a.R_all + gq]);
+        };
+        const int bstar = a.kept_n ? 0 : a.qbin[gq];
+        long long need = a.kept_n ? 0 : a.k - a.qbelow[gq];  // hits still needed from bin b*
         // the reference's k-hit set: entries at or below the replayed final
         // top (FP64 distance, tree position); FP32 distances decide unless
         // they lie within their rounding margin of the top's
         const bool exact = a.tf_d != nullptr;
         const double tf_d = exact ? a.tf_d[gq] : 0.0;
         const int tf_pos = exact ? a.tf_pos[gq] : 0;
-        const bool tf_all = exact && (a.tf_flag[gq] & 1);
+        const bool tf_all = a.kept_n || (exact && (a.tf_flag[gq] & 1));
         const double tf_m = 2e-5 * tf_d + 1e-3;
         const double* q64 = exact ? a.rads + (long)(a.qperm ? a.qperm[gq] : gq) * a.TC : nullptr;
         unsigned kstar_out = 0u;
         bool take_all_out = false;
-        if (!exact) {
+        if (!exact && !a.kept_n) {
         // The query's candidates: one segment per entry slice, in slice
         // order (so in ascending entry index overall).
 
@@ -690,7 +700,7 @@ __global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelec
         kstar_out = prefix;
         take_all_out = take_all;
         }
-        const bool take_all = exact ? tf_all : take_all_out;
+        const bool take_all = exact || a.kept_n ? tf_all : take_all_out;
         const unsigned kstar = kstar_out;  // with take_all: unused
         // Weights of the entries near the read (within 18.5 x 2 sig^2 of the
         // nearest, i.e. above 1e-8 of the largest weight) from FP64
@@ -698,9 +708,9 @@ __global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelec
         // (their error is below 1e-8 of the largest weight).
         float dmin = INFINITY;
         if (a.rads) {
-            for (int sl = 0; sl < a.slices; sl++) {
-                const long long sb = a.qoff[lq] + a.sliceoff[(long)sl * a.R_all + gq];
-                const long long sn = min(a.slicecnt[(long)sl * a.R_all + gq], a.slicecap[(long)sl * a.R_all + gq]);
+            for (int sl = 0; sl < slices; sl++) {
+                const long long sb = seg_begin(sl);
+                const long long sn = seg_count(sl);
                 for (long long i = lane; i < sn; i += 32) dmin = fminf(dmin, a.cand_d2[sb + i]);
             }
             for (int o = 16; o > 0; o >>= 1) dmin = fminf(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
@@ -711,9 +721,9 @@ __global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelec
         double total_part = 0.0;
         int ntouched = 0;
         long long tie_cum = 0;  // hits of key == kstar entries seen so far
-        for (int sl = 0; sl < a.slices; sl++) {
-          const long long sb = a.qoff[lq] + a.sliceoff[(long)sl * a.R_all + gq];
-          const long long sn = min(a.slicecnt[(long)sl * a.R_all + gq], a.slicecap[(long)sl * a.R_all + gq]);
+        for (int sl = 0; sl < slices; sl++) {
+          const long long sb = seg_begin(sl);
+          const long long sn = seg_count(sl);
           for (long long i0 = 0; i0 < sn; i0 += 32) {
             const long long i = i0 + lane;
             bool keep = false;
@@ -723,8 +733,8 @@ __global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelec
             if (i < sn) {
                 e = a.cand_idx[sb + i];
                 d2 = a.cand_d2[sb + i];
-                const int b = a.cand_bin[sb + i];
                 const unsigned key = __float_as_uint(d2);
+                const int b = a.kept_n ? 0 : a.cand_bin[sb + i];
                 if (take_all) keep = true;
                 else if (exact) {
                     if ((double)d2 < tf_d - tf_m) keep = true;
@@ -1158,6 +1168,26 @@ __global__ void wp_nn_qgather_kernel(const float* __restrict__ rows, const int* 
     if (i >= (long)R * DP) return;
     const long r = i / DP;
     out[i] = rows[(long)perm[r] * DP + i % DP];
+}
+
+// Reads list[0 .. n) of rows [R][DP], in that order.
+cudaError_t wp_launch_nn_subset(const float* rows, const int* list, int n, int DP, float* out, cudaStream_t s) {
+    const long m = (long)n * DP;
+    if (m == 0) return cudaSuccess;
+    wp_nn_qgather_kernel<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(rows, list, n, DP, out);
+    return cudaGetLastError();
+}
+
+// perm[i] = list[perm[i]]: slots of a subset back to the reads' own indices.
+__global__ void wp_nn_remap_kernel(int* perm, const int* __restrict__ list, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) perm[i] = list[perm[i]];
+}
+
+cudaError_t wp_launch_nn_remap(int* perm, const int* list, int n, cudaStream_t s) {
+    if (n == 0) return cudaSuccess;
+    wp_nn_remap_kernel<<<(n + 255) / 256, 256, 0, s>>>(perm, list, n);
+    return cudaGetLastError();
 }
 
 size_t wp_nn_sort_temp_bytes(int R) {
