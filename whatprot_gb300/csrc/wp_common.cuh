@@ -675,6 +675,10 @@ __device__ __forceinline__ double wp_nn_exact_d2(const double* q64, long p, int 
 struct SimParams {
     int T, C, P, R;
     unsigned long long seed;
+    // several batches of `batch` reads in one launch: batch g as R = batch reads
+    // with seed + g * seed_step would come out (0: one batch of R)
+    int batch;
+    unsigned long long seed_step;
     unsigned long long thr_fail, thr_initial_block, thr_cyclic_block;
     unsigned long long thr_detach[WP_MAX_TIMESTEPS];
     unsigned long long thr_dud[WP_MAX_CHANNELS], thr_bleach[WP_MAX_CHANNELS];

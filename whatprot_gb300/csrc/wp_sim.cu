@@ -131,7 +131,10 @@ __global__ void wp_sim_reads_kernel(SimParams p) {
     const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= p.R) return;
     curandStatePhilox4_32_10_t st;
-    curand_init(p.seed, (unsigned long long)r, 0ull, &st);
+    if (p.batch > 0)
+        curand_init(p.seed + (unsigned long long)(r / p.batch) * p.seed_step, (unsigned long long)(r % p.batch), 0ull, &st);
+    else
+        curand_init(p.seed, (unsigned long long)r, 0ull, &st);
     // peptide by count weight (upper bound of u * total in the prefix sums),
     // or the peptide of copy r / per_peptide: generate_dye_tracks
     // (generate-dye-tracks.cc:40-47) makes per_peptide tracks for each of
