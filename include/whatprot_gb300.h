@@ -192,9 +192,10 @@ wp_status wp_fit_estep_batch(wp_ctx* ctx, const wp_seq_model* models, int B,
                              const int32_t* read_idx, int num_reads,
                              wp_fit_sums* out, double* sum_logp, int* num_zero);
 
-/* E-step kernel choice: 0 (default) one CTA per read with its vectors in
- * shared memory when they fit, else one thread per read; 1 always one
- * thread per read (tests compare the two).  No reference counterpart. */
+/* E-step kernel choice: 0 (default) by the shape: one warp per read with its
+ * vectors in shared memory where enough of them fit, one CTA per read where
+ * one fits, else one thread per read; 1 always one thread per read (tests
+ * compare them).  No reference counterpart. */
 wp_status wp_fit_set_kernel(wp_ctx* ctx, int kind);
 
 /* Which parameters a fit holds at their starting values: FitSettings and

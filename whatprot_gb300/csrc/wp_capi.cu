@@ -112,6 +112,12 @@ long wp_fit_cta_ckpt_floats(int T, int S, bool has_block);
 cudaError_t wp_launch_fit_cta(bool has_block, int grid, size_t smem, cudaStream_t s, const FitArgs& a, float* ckpt,
                               long ck_stride);
 int wp_fit_cta_ctas_per_sm(bool has_block, size_t smem);
+int wp_fit_warp_max_warps();
+size_t wp_fit_warp_smem_bytes(int T, int C, const int* D, bool hb, bool emission, int nslots, int warps);
+long wp_fit_warp_slab_floats(int T, int S, bool hb);
+int wp_fit_warp_ctas_per_sm(int C, bool hb, size_t smem, int warps);
+cudaError_t wp_launch_fit_warp(int C, bool hb, int grid, int warps, size_t smem, cudaStream_t s, const FitArgs& a,
+                               float* slab, long slab_stride);
 long wp_fit_floats_per_thread(int T, int C, int S, bool has_block);
 
 namespace {
@@ -2209,6 +2215,47 @@ wp_status wp_fit_begin(wp_ctx* ctx, const int16_t* dye_seq, int length, const do
     return WP_OK;
 }
 
+// Which E-step kernel takes a shape: a warp per read where at least eight
+// warps' vectors fit an SM's shared memory (60.3 against 5.6 ms for 50,000 reads
+// of 80 states and 16 timesteps; with fewer warps their latency shows and a
+// CTA per read is no slower), else a CTA per read where one read fits, else
+// none (the thread-per-read kernel).
+struct FitShape {
+    int warps = 0;   // warps (reads at a time) per CTA of the warp kernel, 0: the CTA kernel
+    int per_sm = 0;  // resident CTAs per SM
+    size_t smem = 0;
+    long stride = 0;  // scratch floats per CTA
+};
+static FitShape fit_shape(const wp_ctx* ctx, int T, int C, const int* D, int S, bool hb, bool emis) {
+    FitShape f;
+    // the CTA size with the most resident warps
+    for (int w = wp_fit_warp_max_warps(); w >= 1; w--) {
+        const size_t smem = wp_fit_warp_smem_bytes(T, C, D, hb, emis, wp_fit_nslots(T, C, emis), w);
+        const int n = smem <= (size_t)ctx->smem_optin ? wp_fit_warp_ctas_per_sm(C, hb, smem, w) : 0;
+        if (n * w > f.per_sm * f.warps) {
+            f.warps = w;
+            f.per_sm = n;
+            f.smem = smem;
+        }
+    }
+    if (f.per_sm * f.warps >= 8) {
+        f.stride = wp_fit_warp_slab_floats(T, S, hb) * f.warps;
+        return f;
+    }
+    f.warps = 0;
+    f.smem = wp_fit_cta_smem_bytes(T, C, S, hb, emis);
+    // (the kernel also holds the binomial tables in static shared memory)
+    f.per_sm = (long)f.smem + (long)sizeof(SmemModel) <= (long)ctx->smem_optin ? wp_fit_cta_ctas_per_sm(hb, f.smem) : 0;
+    f.stride = wp_fit_cta_ckpt_floats(T, S, hb);
+    return f;
+}
+
+static cudaError_t fit_launch(const wp_ctx* ctx, const FitShape& f, int C, bool hb, int grid, const FitArgs& a) {
+    float* scratch = ctx->d_fit_scratch.as<float>();
+    return f.warps ? wp_launch_fit_warp(C, hb, grid, f.warps, f.smem, ctx->stream, a, scratch, f.stride / f.warps)
+                   : wp_launch_fit_cta(hb, grid, f.smem, ctx->stream, a, scratch, f.stride);
+}
+
 wp_status wp_fit_estep(wp_ctx* ctx, wp_fit_sums* out, double* sum_logp, int* num_zero) {
     if (!ctx || !out) return WP_ERR_INVALID;
     std::lock_guard<std::mutex> lk(ctx->mu);
@@ -2246,22 +2293,17 @@ wp_status wp_fit_estep(wp_ctx* ctx, wp_fit_sums* out, double* sum_logp, int* num
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     const bool emis = ctx->fit_emission;
     const int nslots = wp_fit_nslots(T, C, emis);
-    // CTA-per-read kernel when a read's vectors fit shared memory, else the
-    // thread-per-read kernel over a global slab.
-    const size_t cta_smem = wp_fit_cta_smem_bytes(T, C, S, hb, emis);
-    // (the kernel also holds the binomial tables in static shared memory)
-    const int cta_per_sm = (long)cta_smem + (long)sizeof(SmemModel) <= (long)ctx->smem_optin
-                                   ? wp_fit_cta_ctas_per_sm(hb, cta_smem)
-                                   : 0;
-    const bool use_cta = cta_per_sm > 0 && !ctx->fit_force_thread;
+    const FitShape shape = fit_shape(ctx, T, C, ctx->fit_D, S, hb, emis);
+    const bool use_cta = shape.per_sm > 0 && !ctx->fit_force_thread;
     const int threads = 128;
     int grid = 0;
-    long nth = 0, per = 0, ck_stride = 0;
+    long nth = 0, per = 0;
     if (use_cta) {
-        grid = (int)std::min<long>((long)R, (long)sms * cta_per_sm);
+        const long reads_per_cta = std::max(1, shape.warps);
+        grid = (int)std::min<long>((R + reads_per_cta - 1) / reads_per_cta, (long)sms * shape.per_sm);
         nth = grid;
-        ck_stride = wp_fit_cta_ckpt_floats(T, S, hb);
-        WP_CUDA(ctx->d_fit_scratch.ensure(sizeof(float) * (size_t)grid * ck_stride), "alloc fit checkpoints");
+        WP_CUDA(ctx->d_fit_scratch.ensure(std::max<size_t>(sizeof(float) * (size_t)grid * shape.stride, 16)),
+                "alloc fit checkpoints");
     } else {
         long want = std::min<long>((long)R, (long)sms * 4 * threads);
         per = wp_fit_floats_per_thread(T, C, S, hb);
@@ -2302,13 +2344,12 @@ wp_status wp_fit_estep(wp_ctx* ctx, wp_fit_sums* out, double* sum_logp, int* num
     {
         TimedLaunch tl(ctx, 0);
         if (use_cta)
-            WP_CUDA(wp_launch_fit_cta(hb, grid, cta_smem, ctx->stream, fa, ctx->d_fit_scratch.as<float>(), ck_stride),
-                    "fit E-step launch");
+            WP_CUDA(fit_launch(ctx, shape, C, hb, grid, fa), "fit E-step launch");
         else
             WP_CUDA(wp_launch_fit_estep(hb, grid, threads, ctx->stream, fa), "fit E-step launch");
         ctx->launches++;
     }
-    wp_fit_reduce_kernel<<<(nslots + 63) / 64, 64, 0, ctx->stream>>>(fa.sums, nth, nslots, ctx->d_fit_out.as<double>());
+    wp_fit_reduce_kernel<<<(nslots + 3) / 4, 128, 0, ctx->stream>>>(fa.sums, nth, nslots, ctx->d_fit_out.as<double>());
     ctx->launches++;
     WP_CUDA(cudaGetLastError(), "fit reduce launch");
     std::vector<double> sums(nslots), lp(R);
@@ -2392,18 +2433,17 @@ wp_status wp_fit_estep_batch(wp_ctx* ctx, const wp_seq_model* models, int B, con
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     const int nslots = wp_fit_nslots(T, C, false);
-    const size_t cta_smem = wp_fit_cta_smem_bytes(T, C, S, hb, false);
-    const int cta_per_sm = (long)cta_smem + (long)sizeof(SmemModel) <= (long)ctx->smem_optin
-                                   ? wp_fit_cta_ctas_per_sm(hb, cta_smem)
-                                   : 0;
-    if (cta_per_sm <= 0) return fail(ctx, WP_ERR_UNSUPPORTED, "batched E-steps need the CTA-per-read kernel");
+    const FitShape shape = fit_shape(ctx, T, C, ctx->fit_D, S, hb, false);
+    if (shape.per_sm <= 0) return fail(ctx, WP_ERR_UNSUPPORTED, "batched E-steps need the CTA-per-read kernel");
     // CTAs per instance: the device's resident CTAs shared out (rounded down,
     // so that all CTAs are resident in one wave), at most one per read
-    const int G = (int)std::max<long>(1, std::min<long>((long)Rb, ((long)sms * cta_per_sm) / B));
+    const long reads_per_cta = std::max(1, shape.warps);
+    const int G = (int)std::max<long>(
+        1, std::min<long>((Rb + reads_per_cta - 1) / reads_per_cta, ((long)sms * shape.per_sm) / B));
     const long grid = (long)G * B;
     if (grid > INT32_MAX) return fail(ctx, WP_ERR_UNSUPPORTED, "too many batched instances");
-    const long ck_stride = wp_fit_cta_ckpt_floats(T, S, hb);
-    WP_CUDA(ctx->d_fit_scratch.ensure(sizeof(float) * (size_t)grid * ck_stride), "alloc fit checkpoints");
+    WP_CUDA(ctx->d_fit_scratch.ensure(std::max<size_t>(sizeof(float) * (size_t)grid * shape.stride, 16)),
+            "alloc fit checkpoints");
     WP_CUDA(ctx->d_fit_sums.ensure(sizeof(double) * (size_t)grid * nslots), "alloc fit sums");
     WP_CUDA(ctx->d_fit_logp.ensure(sizeof(double) * (size_t)B * Rb), "alloc fit logp");
     WP_CUDA(ctx->d_boot_models.ensure(sizeof(DevModel) * B), "alloc models");
@@ -2440,8 +2480,7 @@ wp_status wp_fit_estep_batch(wp_ctx* ctx, const wp_seq_model* models, int B, con
     fa.read_idx = ctx->d_boot_idx.as<int>();
     {
         TimedLaunch tl(ctx, 0);
-        WP_CUDA(wp_launch_fit_cta(hb, (int)grid, cta_smem, ctx->stream, fa, ctx->d_fit_scratch.as<float>(), ck_stride),
-                "fit E-step launch");
+        WP_CUDA(fit_launch(ctx, shape, C, hb, (int)grid, fa), "fit E-step launch");
         ctx->launches++;
     }
     // per-CTA sums [nslots][grid]; each instance's CTAs summed in CTA order
