@@ -53,9 +53,13 @@ size_t wp_dense_smem_bytes(int T, int S_cap, int C, bool has_block, int warps);
 cudaError_t wp_launch_fma_probe(int blocks, int threads, int iters, cudaStream_t stream, float* sink);
 cudaError_t wp_launch_fit_estep(bool has_block, int grid, int threads, cudaStream_t s, const FitArgs& a);
 cudaError_t wp_launch_nn_dist(int DP, bool hist, cudaStream_t s, const NNArgs& a);
+cudaError_t wp_launch_nn_pick(int grid, cudaStream_t s, const NNSelectArgs& a);
+size_t wp_nn_score_smem_bytes(int U, int table_entries);
+int wp_nn_score_ctas_per_sm(size_t smem);
+cudaError_t wp_launch_nn_score(int grid, size_t smem, cudaStream_t s, const NNScoreArgs& a);
 cudaError_t wp_launch_nn_select(int grid, cudaStream_t s, const NNSelectArgs& a);
 cudaError_t wp_launch_nn_threshold(cudaStream_t s, const NNArgs& a);
-cudaError_t wp_launch_nn_estimate(int DP, cudaStream_t s, const NNArgs& a);
+cudaError_t wp_launch_nn_estimate(int DP, int ctas, cudaStream_t s, const NNArgs& a);
 size_t wp_nn_sort_temp_bytes(int R);
 cudaError_t wp_launch_nn_subset(const float* rows, const int* list, int n, int DP, float* out, cudaStream_t s);
 cudaError_t wp_launch_nn_remap(int* perm, const int* list, int n, cudaStream_t s);
@@ -299,7 +303,7 @@ struct wp_ctx {
     // the k-hit sets by levels (wp_khits.cu): counts as nibbles, scratch
     bool nn_nib_packed = false;
     DevBuf d_nn_nib, d_kh_ent, d_kh_d, d_kh_bin, d_kh_order, d_kh_rank, d_kh_state, d_kh_memd, d_kh_memk, d_kh_sorted, d_kh_seg, d_kh_kpos, d_kh_kd2,
-            d_kh_kn, d_nn_subset, d_nn_subq;
+            d_kh_kn, d_nn_subset, d_nn_subq, d_nn_coarse, d_nn_koff;
 
     // Per-batch scratch.
     DevBuf d_rads, d_lo, d_hi, d_Ls, d_Up, d_Lpk, d_Upk, d_allow, d_flags, d_table, d_gtab, d_gdelta, d_gK,
@@ -1031,16 +1035,18 @@ bool nn_by_levels(const wp_ctx* ctx, long long k) {
            k <= ctx->nn_hits_total && ctx->nn_hits_total < (1ll << 31);
 }
 
-// The k-hit sets by levels of the query slots q0 .. q0 + n: their entries in
-// d_kh_kpos / d_kh_kd2 (`stride` places each), their numbers in d_kh_kn (-1:
-// left to the replay).
-wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int q0, int n, long stride, long long k) {
+// The k-hit sets by levels of the query slots q0 .. q0 + n: their candidate
+// lists in d_kh_kpos / d_kh_kd2 (`stride` places each), the lists' lengths in
+// d_kh_kn (-1: left to the replay).
+wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int q0, int n, int slice_len, long stride, long long k) {
     const int TC = ctx->nn_T * ctx->nn_C;
     KHArgs a;
     memset(&a, 0, sizeof(a));
     a.q0 = q0;
     a.Rc = n;
     a.stride = stride;
+    a.slice_len = slice_len;
+    a.qbase = ctx->d_nn_qbase.as<int>();
     a.next = ctx->d_kb_next.as<int>();
     a.qperm = ctx->d_nn_qperm.as<int>();
     a.rads = d_rads;
@@ -1204,23 +1210,10 @@ wp_status nn_replay(wp_ctx* ctx, const double* d_rads, int R, long long k) {
     return fail(ctx, WP_ERR_UNSUPPORTED, "kd-tree kNN: replay scratch exhausted");
 }
 
-// The select kernel's arguments that do not depend on the reads' route, and
-// its per-warp accumulators.
-wp_status nn_select_args(wp_ctx* ctx, const double* d_rads, int k, double sig, int h, bool hybrid, int sel_grid,
-                         NNSelectArgs* out) {
+// The pick and select kernels' arguments that do not depend on the reads' route.
+wp_status nn_select_args(wp_ctx* ctx, const double* d_rads, int k, double sig, int h, bool hybrid, NNSelectArgs* out) {
     const int T = ctx->nn_T, C = ctx->nn_C, DP = nn_padded_dim(T * C);
-    const long nwarps = (long)sel_grid * wp_nn_select_warps();
     const int U = std::max(ctx->nn_U, 1);
-    WP_CUDA(ctx->d_nn_acc.ensure(sizeof(double) * nwarps * U), "alloc kNN accumulators");
-    WP_CUDA(ctx->d_nn_mark.ensure(sizeof(int) * nwarps * U), "alloc kNN accumulators");
-    WP_CUDA(ctx->d_nn_touched.ensure(sizeof(int) * nwarps * U), "alloc kNN accumulators");
-    // The select kernel leaves every accumulator it touched at zero again,
-    // so memory is cleared once, when first used.
-    if (sizeof(double) * nwarps * U > ctx->nn_acc_cleared) {
-        WP_CUDA(cudaMemsetAsync(ctx->d_nn_acc.p, 0, sizeof(double) * nwarps * U, ctx->stream), "clear");
-        WP_CUDA(cudaMemsetAsync(ctx->d_nn_mark.p, 0, sizeof(int) * nwarps * U, ctx->stream), "clear");
-        ctx->nn_acc_cleared = sizeof(double) * nwarps * U;
-    }
     NNSelectArgs& b = *out;
     memset(&b, 0, sizeof(b));
     b.qperm = ctx->d_nn_qperm.as<int>();
@@ -1236,9 +1229,6 @@ wp_status nn_select_args(wp_ctx* ctx, const double* d_rads, int k, double sig, i
     b.k = k;
     b.inv_two_sig_sq = (float)(1.0 / (2.0 * sig * sig));
     b.h = h;
-    b.acc = ctx->d_nn_acc.as<double>();
-    b.mark = ctx->d_nn_mark.as<int>();
-    b.touched = ctx->d_nn_touched.as<int>();
     b.out_ncand = ctx->d_nn_ncand.as<int>();
     b.out_cand_id = ctx->d_nn_cand_id.as<int>();
     b.out_cand_pep = hybrid ? ctx->d_nn_cand_pep.as<int>() : nullptr;
@@ -1256,6 +1246,75 @@ wp_status nn_select_args(wp_ctx* ctx, const double* d_rads, int k, double sig, i
         b.ctab = ctx->d_nn_ctab.as<double>();
         b.ecoord = ctx->nn_inter ? ctx->d_nn_ecoord.as<double>() : nullptr;
     }
+    return WP_OK;
+}
+
+// Votes, totals and the top h over the kept entries (b.kept_*): a CTA per read
+// where the scores of all ids fit shared memory, else a warp per read.
+wp_status nn_vote(wp_ctx* ctx, NNSelectArgs b, int sms) {
+    TimedLaunch tl(ctx, 5);
+    const int entries = b.rads && !b.ecoord ? b.TC * b.NC : 0;
+    const size_t smem = wp_nn_score_smem_bytes(b.U, entries);
+    const int per_sm = smem <= (size_t)ctx->smem_optin ? wp_nn_score_ctas_per_sm(smem) : 0;
+    if (per_sm > 0) {
+        WP_CUDA(ctx->d_kb_next.ensure(sizeof(int)), "alloc");
+        NNScoreArgs a;
+        memset(&a, 0, sizeof(a));
+        a.R = b.R;
+        a.q0 = b.q0;
+        a.next = ctx->d_kb_next.as<int>();
+        a.qperm = b.qperm;
+        a.kept_n = b.kept_n;
+        a.kept_pos = b.kept_pos;
+        a.kept_d2 = b.kept_d2;
+        a.koff = b.koff;
+        a.stride = b.stride;
+        a.src_off = b.src_off;
+        a.src_dense = b.src_dense;
+        a.src_ratio = b.src_ratio;
+        a.src_hits = b.src_hits;
+        a.dense_id = b.dense_id;
+        a.dense_pep = b.dense_pep;
+        a.dense_count = b.dense_count;
+        a.U = b.U;
+        a.inv_two_sig_sq = b.inv_two_sig_sq;
+        a.two_sig_sq = b.two_sig_sq;
+        a.h = b.h;
+        a.out_ncand = b.out_ncand;
+        a.out_cand_id = b.out_cand_id;
+        a.out_cand_pep = b.out_cand_pep;
+        a.out_cand_score = b.out_cand_score;
+        a.out_total = b.out_total;
+        a.out_subfrac = b.out_subfrac;
+        a.rads = b.rads;
+        a.TC = b.TC;
+        a.C = b.C;
+        a.DP = b.DP;
+        a.NC = b.NC;
+        a.cnt = b.cnt;
+        a.ctab = b.ctab;
+        a.ecoord = b.ecoord;
+        a.table = entries > 0 ? 1 : 0;
+        WP_CUDA(wp_launch_nn_score((int)std::min<long>(b.R, (long)sms * per_sm), smem, ctx->stream, a), "kNN votes");
+    } else {
+        const int grid = sms * 4, U = b.U;
+        const long nwarps = (long)grid * wp_nn_select_warps();
+        WP_CUDA(ctx->d_nn_acc.ensure(sizeof(double) * nwarps * U), "alloc kNN accumulators");
+        WP_CUDA(ctx->d_nn_mark.ensure(sizeof(int) * nwarps * U), "alloc kNN accumulators");
+        WP_CUDA(ctx->d_nn_touched.ensure(sizeof(int) * nwarps * U), "alloc kNN accumulators");
+        // The select kernel leaves every accumulator it touched at zero again,
+        // so memory is cleared once, when first used.
+        if (sizeof(double) * nwarps * U > ctx->nn_acc_cleared) {
+            WP_CUDA(cudaMemsetAsync(ctx->d_nn_acc.p, 0, sizeof(double) * nwarps * U, ctx->stream), "clear");
+            WP_CUDA(cudaMemsetAsync(ctx->d_nn_mark.p, 0, sizeof(int) * nwarps * U, ctx->stream), "clear");
+            ctx->nn_acc_cleared = sizeof(double) * nwarps * U;
+        }
+        b.acc = ctx->d_nn_acc.as<double>();
+        b.mark = ctx->d_nn_mark.as<int>();
+        b.touched = ctx->d_nn_touched.as<int>();
+        WP_CUDA(wp_launch_nn_select(grid, ctx->stream, b), "kNN select");
+    }
+    ctx->launches++;
     return WP_OK;
 }
 
@@ -1277,9 +1336,43 @@ wp_status nn_sort_rows(wp_ctx* ctx, const float* rows, int n, int DP, int TC) {
     return WP_OK;
 }
 
+// Entry slices of a batch of R reads: enough CTAs (query blocks x slices) for
+// two waves of three CTAs per SM, each slice at least 1024 entries.  Votes are
+// grouped by slices (wp_nnscore.cu), so a part of the batch keeps its slices.
+int nn_slice_len(const wp_ctx* ctx, int R, int sms) {
+    const int N = ctx->nn_N;
+    const int qblocks = (R + wp_nn_queries_per_block() - 1) / wp_nn_queries_per_block();
+    int slices = (6 * sms + qblocks - 1) / qblocks;
+    slices = std::max(1, std::min(slices, std::min(32, (N + 1023) / 1024)));
+    return ((N + slices - 1) / slices + 31) / 32 * 32;
+}
+
+// The bin origins (d_nn_qbase) of R sorted query slots.
+wp_status nn_estimate(wp_ctx* ctx, int R, long long k, int sms) {
+    const int DP = nn_padded_dim(ctx->nn_T * ctx->nn_C);
+    WP_CUDA(ctx->d_nn_coarse.ensure(sizeof(unsigned) * (size_t)R * wp_nn_bins()), "alloc kNN estimate");
+    NNArgs a;
+    memset(&a, 0, sizeof(a));
+    a.queries = ctx->d_nn_qsorted.as<float>();
+    a.R = R;
+    a.coords = ctx->d_nn_coords.as<float>();
+    a.enorm = ctx->d_nn_enorm.as<float>();
+    a.k = k;
+    a.qbase = ctx->d_nn_qbase.as<int>();
+    a.coarse = ctx->d_nn_coarse.as<unsigned>();
+    a.sample = ctx->d_nn_sample.as<int>();
+    a.sample_n = ctx->nn_sample_n;
+    a.hits_total = ctx->nn_hits_total;
+    TimedLaunch tl(ctx, 4);
+    WP_CUDA(wp_launch_nn_estimate(DP, 4 * sms, ctx->stream, a), "kNN estimate");
+    ctx->launches += 2;
+    return WP_OK;
+}
+
 // The kNN stage by brute force over the sorted query slots 0 .. R (d_nn_qsorted,
 // d_nn_qperm): the distance-ordered k-hit sets, or the replayed search's.
-wp_status nn_run_slots(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, int h, bool hybrid) {
+// R_batch: the reads of the whole batch.
+wp_status nn_run_slots(wp_ctx* ctx, const double* d_rads, int R, int R_batch, int k, double sig, int h, bool hybrid) {
     const int T = ctx->nn_T, C = ctx->nn_C, N = ctx->nn_N;
     const int DP = nn_padded_dim(T * C);
     const size_t Rz = (size_t)std::max(R, 1);
@@ -1309,18 +1402,10 @@ wp_status nn_run_slots(wp_ctx* ctx, const double* d_rads, int R, int k, double s
     a.hits_total = ctx->nn_hits_total;
     a.tf_d = exact ? ctx->d_kb_tfd.as<double>() : nullptr;
     a.tf_flag = exact ? ctx->d_kb_tfflag.as<int>() : nullptr;
-    // Entry slices: enough CTAs (query blocks x slices) for two waves of
-    // three CTAs per SM, each slice at least 1024 entries.
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    {
-        const int qblocks = (R + wp_nn_queries_per_block() - 1) / wp_nn_queries_per_block();
-        int slices = (6 * sms + qblocks - 1) / qblocks;
-        slices = std::max(1, std::min(slices, std::min(32, (N + 1023) / 1024)));
-        a.slices = slices;
-        a.slice_len = ((N + slices - 1) / slices + 31) / 32 * 32;
-        a.slices = (N + a.slice_len - 1) / a.slice_len;
-    }
+    a.slice_len = nn_slice_len(ctx, R_batch, sms);
+    a.slices = (N + a.slice_len - 1) / a.slice_len;
     a.R_all = R;
     WP_CUDA(ctx->d_nn_shist.ensure(sizeof(unsigned) * (size_t)a.slices * R * wp_nn_bins()), "alloc kNN histograms");
     WP_CUDA(ctx->d_nn_sliceoff.ensure(sizeof(long long) * (size_t)a.slices * R), "alloc");
@@ -1338,11 +1423,8 @@ wp_status nn_run_slots(wp_ctx* ctx, const double* d_rads, int R, int k, double s
     a.queries = ctx->d_nn_qsorted.as<float>();
     a.R = R;
     a.q0 = 0;
-    {
-        TimedLaunch tl(ctx, 4);
-        WP_CUDA(wp_launch_nn_estimate(DP, ctx->stream, a), "kNN estimate");
-        ctx->launches++;
-    }
+    st = nn_estimate(ctx, R, k, sms);
+    if (st != WP_OK) return st;
     {
         TimedLaunch tl(ctx, 4);
         WP_CUDA(wp_launch_nn_dist(DP, true, ctx->stream, a), "kNN histogram");
@@ -1356,7 +1438,7 @@ wp_status nn_run_slots(wp_ctx* ctx, const double* d_rads, int R, int k, double s
     WP_CUDA(ctx->d_nn_redo.ensure(sizeof(int) * (Rz + 1)), "alloc");
     for (int round = 0; round < 3; round++) {
         int* list = ctx->d_nn_redo.as<int>() + 1;
-        WP_CUDA(wp_launch_nn_redo(a, list, ctx->d_nn_redo.as<int>(), 40, ctx->stream), "kNN redo");
+        WP_CUDA(wp_launch_nn_redo(a, list, ctx->d_nn_redo.as<int>(), WP_NN_REDO_SHIFT, ctx->stream), "kNN redo");
         ctx->launches++;
         int nredo = 0;
         WP_CUDA(cudaMemcpyAsync(&nredo, ctx->d_nn_redo.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "copy");
@@ -1386,24 +1468,31 @@ wp_status nn_run_slots(wp_ctx* ctx, const double* d_rads, int R, int k, double s
     WP_CUDA(cudaMemcpyAsync(cap.data(), a.qcap, sizeof(long long) * R, cudaMemcpyDeviceToHost, ctx->stream),
             "copy caps");
     WP_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
-    const int sel_grid = sms * 4;
+    WP_CUDA(ctx->d_kh_kn.ensure(sizeof(int) * Rz), "alloc");
     NNSelectArgs b;
-    st = nn_select_args(ctx, d_rads, k, sig, h, hybrid, sel_grid, &b);
+    st = nn_select_args(ctx, d_rads, k, sig, h, hybrid, &b);
     if (st != WP_OK) return st;
     // chunks of reads whose candidate lists fit the budget
     const long long budget = 256ll << 20;  // candidates per chunk (2 GiB of lists)
     int r0 = 0;
-    std::vector<long long> off;
+    std::vector<long long> off, koff;
     while (r0 < R) {
-        long long tot = 0;
+        // lists of candidates, and the same with every slice from a multiple of 32
+        long long tot = 0, ktot = 0;
         int r1 = r0;
         off.clear();
+        koff.clear();
         while (r1 < R && (r1 == r0 || tot + cap[r1] <= budget)) {
             off.push_back(tot);
+            koff.push_back(ktot);
             tot += cap[r1];
+            ktot += cap[r1] + 32ll * a.slices;
             r1++;
         }
         const int nq = r1 - r0;
+        WP_CUDA(ctx->d_nn_koff.ensure(sizeof(long long) * nq), "alloc");
+        WP_CUDA(cudaMemcpyAsync(ctx->d_nn_koff.p, koff.data(), sizeof(long long) * nq, cudaMemcpyHostToDevice,
+                                ctx->stream), "copy offsets");
         WP_CUDA(ctx->d_nn_cidx.ensure(sizeof(int) * std::max<long long>(tot, 1)), "alloc kNN candidates");
         WP_CUDA(ctx->d_nn_cd2.ensure(sizeof(float) * std::max<long long>(tot, 1)), "alloc kNN candidates");
         WP_CUDA(ctx->d_nn_chits.ensure(sizeof(int) * std::max<long long>(tot, 1)), "alloc kNN candidates");
@@ -1443,11 +1532,19 @@ wp_status nn_run_slots(wp_ctx* ctx, const double* d_rads, int R, int k, double s
             b.tf_pos = ctx->d_kb_tfpos.as<int>();
             b.tf_flag = ctx->d_kb_tfflag.as<int>();
         }
+        WP_CUDA(ctx->d_kh_kpos.ensure(sizeof(int) * ktot), "alloc kNN kept sets");
+        WP_CUDA(ctx->d_kh_kd2.ensure(sizeof(float) * ktot), "alloc kNN kept sets");
+        b.koff = ctx->d_nn_koff.as<long long>();
+        b.kept_n = ctx->d_kh_kn.as<int>();
+        b.kept_pos = ctx->d_kh_kpos.as<int>();
+        b.kept_d2 = ctx->d_kh_kd2.as<float>();
         {
             TimedLaunch tl(ctx, 5);
-            WP_CUDA(wp_launch_nn_select(sel_grid, ctx->stream, b), "kNN select");
+            WP_CUDA(wp_launch_nn_pick(sms * 4, ctx->stream, b), "kNN pick");
             ctx->launches++;
         }
+        st = nn_vote(ctx, b, sms);
+        if (st != WP_OK) return st;
         WP_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
         r0 = r1;
     }
@@ -1494,33 +1591,38 @@ wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, in
     if (st != WP_OK) return st;
     int left = R;
     if (nn_by_levels(ctx, k)) {
-        // the kept entries of a chunk of reads, then their weights and scores;
-        // a set has at most min(N, k) entries: 2 GiB of lists per chunk
-        const long stride = (long)std::min<long long>(N, k);
+        // the candidate lists of a chunk of reads, then their weights and scores.
+        // A set has at most min(N, k) entries (each has a hit, and the set is some
+        // walk prefix's shortest one); its bin's rest and the slices' gaps come on
+        // top.  2 GiB of lists per chunk.
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+        const int slice_len = nn_slice_len(ctx, R, sms);
+        const long stride = ((long)std::min<long long>(N, k + (long long)k / 2 + 1024) + 31) / 32 * 32 +
+                            32l * ((N + slice_len - 1) / slice_len);
         const int chunk = (int)std::max<long long>(1, std::min<long long>(R, (256ll << 20) / stride));
+        st = nn_estimate(ctx, R, k, sms);
+        if (st != WP_OK) return st;
         WP_CUDA(ctx->d_kb_next.ensure(sizeof(int)), "alloc");
         WP_CUDA(ctx->d_kh_kn.ensure(sizeof(int) * Rz), "alloc");
         WP_CUDA(ctx->d_kh_kpos.ensure(sizeof(int) * (size_t)chunk * stride), "alloc kNN kept sets");
         WP_CUDA(ctx->d_kh_kd2.ensure(sizeof(float) * (size_t)chunk * stride), "alloc kNN kept sets");
-        int sms = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
         NNSelectArgs b;
-        st = nn_select_args(ctx, d_rads, k, sig, h, hybrid, sms * 4, &b);
+        st = nn_select_args(ctx, d_rads, k, sig, h, hybrid, &b);
         if (st != WP_OK) return st;
         b.R_all = R;
-        b.cand_idx = ctx->d_kh_kpos.as<int>();
-        b.cand_d2 = ctx->d_kh_kd2.as<float>();
         b.kept_n = ctx->d_kh_kn.as<int>();
+        b.kept_pos = ctx->d_kh_kpos.as<int>();
+        b.kept_d2 = ctx->d_kh_kd2.as<float>();
         b.stride = stride;
         for (int r0 = 0; r0 < R; r0 += chunk) {
             const int n = std::min(chunk, R - r0);
-            st = nn_khits(ctx, d_rads, r0, n, stride, k);
+            st = nn_khits(ctx, d_rads, r0, n, slice_len, stride, k);
             if (st != WP_OK) return st;
             b.R = n;
             b.q0 = r0;
-            TimedLaunch tl(ctx, 5);
-            WP_CUDA(wp_launch_nn_select(sms * 4, ctx->stream, b), "kNN select");
-            ctx->launches++;
+            st = nn_vote(ctx, b, sms);
+            if (st != WP_OK) return st;
         }
         // the slots left to the replay, as a batch of their own
         std::vector<int> kept(R), perm(R), rest;
@@ -1546,7 +1648,7 @@ wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, in
         }
     }
     if (left > 0) {
-        st = nn_run_slots(ctx, d_rads, left, k, sig, h, hybrid);
+        st = nn_run_slots(ctx, d_rads, left, R, k, sig, h, hybrid);
         if (st != WP_OK) return st;
     }
     int err = 0;

@@ -456,8 +456,31 @@ struct FitArgs {
 };
 
 // ---- kNN stage (wp_nn.cu) -------------------------------------------------
+#define WP_NN_BINS 64           // distance bins per query
+#define WP_NN_REDO_SHIFT 40     // by which a query's bins move up when they end too early
+
+// Fine bin of a squared distance for one query: sixteen bins per octave
+// (exponent and top four mantissa bits), bin 1 starting at the query's
+// origin `base` (in units of float bits >> 19), bin 0 below, bin NB-1
+// open-ended: 62 fine bins span almost four octaves around the query's
+// estimated k-hit radius.  Monotone in d2.
+__device__ __forceinline__ int wp_nn_bin(float d2, int base) {
+    const int b = (int)(__float_as_uint(d2) >> 19) - base + 1;
+    return b < 0 ? 0 : (b > WP_NN_BINS - 1 ? WP_NN_BINS - 1 : b);
+}
+
+// Float value where a query's fine bin b starts.
+__device__ __forceinline__ float wp_nn_bin_start(int base, int b) {
+    return __uint_as_float((unsigned)(base + b - 1) << 19);
+}
+
+// A final top's distance plus the binning distance's rounding: the candidate
+// list ends with the bin that holds it.
+__device__ __forceinline__ float wp_nn_bound(double top) { return (float)(top * (1.0 + 1e-4) + 1e-3) * (1.f + 1e-6f); }
+
 struct NNArgs {
     const float* queries;   // [R][DP]
+    unsigned* coarse;       // [R][bins] coarse histograms of the estimate
     int R;                  // queries in this launch (chunk)
     int q0;                 // first query index of the chunk (into per-query arrays)
     const float* coords;    // [N][DP]
@@ -546,9 +569,13 @@ struct NNSelectArgs {
     const double* tf_d;         // [R_all]
     const int* tf_pos;
     const int* tf_flag;         // bit 0: every entry kept
-    // The kept entries themselves (KHArgs; then cand_idx and cand_d2 have
-    // `stride` places per query): their number, -1 for a query of another route.
-    const int* kept_n;          // [R_all] or null
+    // The candidate list with the kept entries (as KHArgs; wp_nn_pick_kernel
+    // writes it), at koff or local * stride; its length, -1 for a query of
+    // another route.
+    const long long* koff;
+    int* kept_n;                // [R_all]
+    int* kept_pos;
+    float* kept_d2;
     long stride;
     const double* rads;         // [reads][TC] FP64 queries (read order); with
                                 // them the near entries' weights use FP64
@@ -558,6 +585,41 @@ struct NNSelectArgs {
     const uint8_t* cnt;         // [N][DP] counts per coordinate (tree order)
     const double* ctab;         // [C][NC] coordinate of count n on channel c
     const double* ecoord;       // [N][TC] FP64 coordinates (interacting models), or null
+};
+
+// ---- votes over the kept tracks (wp_nnscore.cu) ----------------------------
+struct NNScoreArgs {
+    int R, q0;                  // query slots q0 .. q0 + R
+    int* next;                  // work counter
+    const int* qperm;           // read index of each slot
+    const int* kept_n;          // as NNSelectArgs
+    const int* kept_pos;
+    const float* kept_d2;
+    const long long* koff;
+    long stride;
+    const int* src_off;         // as NNSelectArgs
+    const int* src_dense;
+    const double* src_ratio;
+    const int* src_hits;
+    const int* dense_id;
+    const int* dense_pep;
+    const int* dense_count;
+    int U;
+    float inv_two_sig_sq;
+    double two_sig_sq;
+    int h;                      // <= 1024
+    int* out_ncand;
+    int* out_cand_id;
+    int* out_cand_pep;
+    double* out_cand_score;
+    double* out_total;
+    double* out_subfrac;
+    const double* rads;         // [reads][TC] (null: all weights from FP32 distances)
+    int TC, C, DP, NC;
+    const uint8_t* cnt;
+    const double* ctab;
+    const double* ecoord;
+    int table;                  // FP64 distances from the per-read table of ctab
 };
 
 // ---- the reference's k-hit set (wp_kbest.cu) ------------------------------
@@ -633,11 +695,14 @@ struct KHArgs {
     int2* sorted;               // [warps][rank limit]
     int2* seg;                  // [warps][groups]
     const float* coords;        // [N][DP] FP32 coordinates
-    // per slot: the kept entries in tree order, at most min(N, k) (each has a
-    // hit, and the set is some walk prefix's shortest one), and their number;
-    // -1: left to the replay
+    // per slot: the candidate list that the brute-force passes would leave (tree
+    // order, every slice of slice_len entries from a multiple of 32; tree
+    // positions of the kept entries, -1 for the others and the gaps) and its
+    // length; -1: left to the replay
     int q0, Rc;                 // the slots q0 .. q0 + Rc of this launch
-    long stride;                // min(N, k)
+    long stride;
+    const int* qbase;           // [R] bin origins, as NNArgs
+    int slice_len;
     int* kept_pos;              // [Rc][stride]
     float* kept_d2;             // [Rc][stride] FP32 squared distances as the collect pass forms them
     int* kept_n;                // [R]

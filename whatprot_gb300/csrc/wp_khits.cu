@@ -31,7 +31,10 @@
 //   3. looks inside the few groups whose bound exceeds the maximum found
 //      (their entries ranked by FP64 distance), and
 //   4. ranks the bin that holds the M-th nearest entry, KBest's final top, and
-//      writes the M nearest in tree order (the walk's leaves put in order).
+//      writes the read's candidate list as the brute-force passes would (wp_nn.cu:
+//      the entries up to the end of the top's distance bin, in tree order, by
+//      slices), the M kept ones with their positions, the others as -1.  The votes
+//      are added in groups of that list, so both routes give the same bits.
 //
 // Exactness.  Only ranks inside the groups of 3 and 4 need FP64 distances; an
 // entry whose FP32 distance lies within its rounding error of a bin edge is
@@ -47,14 +50,13 @@
 // TC (NC - 1) steps.
 //
 // Bound by the latency of one read's walk and by L2 bandwidth (3.5 KB per 128
-// entries screened; 450,000 of 946,000 entries screened and 21,000 listed per
-// read at k = 10,000).  4,000 reads against 946,000 tracks, k = 10,000: 29 ms,
+// entries screened; 450,000 of 946,000 entries screened and 25,000 listed per
+// read at k = 10,000).  4,000 reads against 946,000 tracks, k = 10,000: 36 ms,
 // against 132 ms for the replay (20,000 pushes per read, one at a time, and
-// its table look-ups of 48 coordinates for every entry met); 2,000 reads
-// against 70,000 tracks, k = 1,000: 1.1 ms against 4.1 ms.
-// Writing the kept entries here (the list holds them all) spares these reads
-// the brute-force passes that collected them (wp_nn.cu): another 41 of 99 ms
-// and 4.0 of 6.3 ms in the two cases.
+// its table look-ups of 48 coordinates for every entry met) and 41 ms for the
+// brute-force passes that then collected the entries (the list holds them
+// all); 2,000 reads against 70,000 tracks, k = 1,000: 1.1 ms against 4.1 and
+// 4.0 ms.
 #include <cuda_runtime.h>
 #include <float.h>
 #include <math.h>
@@ -351,13 +353,16 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
         int Htf = 0;                         // hits of the first t_f entries
         int bh = KH_NB, Cb = 0, bc = KH_NB, Cc = 0, mub = 0, ub = KH_NB - 1;
         long long Sb = 0;                    // hits in bins below bh
-        float ub_edge = INFINITY, rhs = INFINITY;
+        // entries are listed up to `reach`: KBest's threshold is at most the upper
+        // edge of bin ub, and the candidate list ends within 1/16 octave and the
+        // binning distance's margins beyond its last value
+        float reach = INFINITY, rhs = INFINITY;
         while (sp > 0 && !fatal) {
             sp--;
             int node = s_node[sp];
             const double plane = s_plane[sp];
             __syncwarp();
-            if (plane > (double)ub_edge) continue;
+            if (plane > (double)reach) continue;
             KDNode nd = a.nodes[node];
             while (!nd.leaf) {
                 const double qv = q64[nd.s];
@@ -405,7 +410,7 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
                     have_base = true;
                     base = (int)(__float_as_uint(f2 * (1.f + 1e-4f)) >> KH_SH) - (KH_NB - 1);
                 }
-                if (!fill && g2 > ub_edge * (1.f + 1e-4f) + 1e-3f) continue;
+                if (!fill && g2 > reach * (1.f + 1e-4f) + 1e-3f) continue;
             }
             const int n_leaf = n;
             const int g_lo = nd.begin >> 7, g_hi = (nd.end - 1) >> 7;
@@ -480,7 +485,7 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
                     __syncwarp();
                     if (lane + cntb < qn_) sm->qpos[lane] = rest;
                     qn_ -= cntb;
-                    const bool keep = lane < cntb && b <= ub;
+                    const bool keep = lane < cntb && (fill || d <= reach);
                     const unsigned km = __ballot_sync(0xffffffffu, keep);
                     if (km == 0u) {
                         __syncwarp();
@@ -545,8 +550,9 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
                     const int nub = max(bh, bc);
                     if (nub != ub) {
                         ub = nub;
-                        ub_edge = ub == KH_NB - 1 ? INFINITY : kh_edge(base, ub + 1);
-                        rhs = ub_edge + slack;
+                        reach = ub == KH_NB - 1 ? INFINITY
+                                                : fmaf(1.05f, kh_edge(base, ub + 1), fmaf(2e-5f, qn, 2e-3f));
+                        rhs = reach + slack;
                     }
                 }
                 if (fatal) break;
@@ -784,10 +790,29 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
                 } else {
                     kh_bin_d64<DP>(a, L, lane, start, m, sq64);
                     const int want = start + m - M;  // its place, farthest first
-                    const bool distinct = kh_rank(
-                        L, lane, m, [&](int j, int place) { L.rank[L.order[start + j].x] = (uint16_t)place; });
-                    if (!distinct) fatal = 8;
+                    int at = -1;
+                    const bool distinct = kh_rank(L, lane, m, [&](int j, int place) {
+                        L.rank[L.order[start + j].x] = (uint16_t)place;
+                        if (place == want) at = j;
+                    });
+                    const unsigned hit = __ballot_sync(0xffffffffu, at >= 0);
+                    if (!distinct || !hit) fatal = 8;
                     __syncwarp();
+                    // the brute-force passes' last candidate bin for this top (they
+                    // move their bins up at most three times)
+                    int bstar = WP_NN_BINS - 1, qbase = a.qbase[slot];
+                    float lim = 0.f;
+                    if (!fatal) {
+                        const double td = __longlong_as_double(L.mem_d[__shfl_sync(0xffffffffu, at, __ffs(hit) - 1)]);
+                        const float v = wp_nn_bound(td);
+                        for (int u = 0; u < 4; u++) {
+                            bstar = wp_nn_bin(v, qbase);
+                            if (bstar < WP_NN_BINS - 1) break;
+                            qbase += WP_NN_REDO_SHIFT;
+                        }
+                        if (bstar == WP_NN_BINS - 1) fatal = 12;
+                        lim = wp_nn_bin_start(qbase, bstar + 1);
+                    }
                     if (!fatal) {
                         // the leaves' parts in tree order, the kept entries of each
                         for (int j = lane; j < nseg; j += 32) {
@@ -798,22 +823,34 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
                         }
                         __syncwarp();
                         const long out = (long)(slot - a.q0) * a.stride;
-                        int wrote = 0;
-                        for (int s = 0; s < nseg; s++) {
+                        float qd = 0.f;
+                        {
+                            float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;  // as wp_nn.cu's nn_norm2
+#pragma unroll
+                            for (int u = 0; u < DP / 4; u++) {
+                                const float4 q = sm->q32[u];
+                                a0 = fmaf(q.x, q.x, a0);
+                                a1 = fmaf(q.y, q.y, a1);
+                                a2 = fmaf(q.z, q.z, a2);
+                                a3 = fmaf(q.w, q.w, a3);
+                            }
+                            qd = (a0 + a1) + (a2 + a3);
+                        }
+                        const float near = fmaf(1.001f, lim, fmaf(2e-5f, qn, 1e-4f));
+                        int kept = 0, slice = -1, wrote = 0;
+                        for (int s = 0; s < nseg && !fatal; s++) {
                             const int2 part = L.sorted[s];
-                            for (int i0 = part.x; i0 < part.y; i0 += 32) {
+                            for (int i0 = part.x; i0 < part.y && !fatal; i0 += 32) {
                                 const int i = i0 + lane;
-                                bool kept = false;
+                                bool cand = false, keep = false;
                                 int pos = 0;
-                                if (i < part.y) {
+                                float d2 = 0.f;
+                                if (i < part.y && L.d[i] <= near) {
                                     const int bi = L.bin[i];
-                                    kept = bi < b || (bi == b && (int)L.rank[i] >= want);
+                                    keep = bi < b || (bi == b && (int)L.rank[i] >= want);
                                     pos = L.ent[i].x;
-                                }
-                                const unsigned km = __ballot_sync(0xffffffffu, kept);
-                                if (kept) {
-                                    // as wp_nn.cu's nn_d2
-                                    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+                                    // as wp_nn.cu's nn_d2_dot (the bin) and nn_d2
+                                    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
                                     const float4* e = reinterpret_cast<const float4*>(a.coords + (long)pos * DP);
 #pragma unroll
                                     for (int u = 0; u < DP / 4; u++) {
@@ -823,17 +860,44 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
                                         a1 = fmaf(x1, x1, a1);
                                         a2 = fmaf(x2, x2, a2);
                                         a3 = fmaf(x3, x3, a3);
+                                        p0 = fmaf(q.x, v.x, p0);
+                                        p1 = fmaf(q.y, v.y, p1);
+                                        p2 = fmaf(q.z, v.z, p2);
+                                        p3 = fmaf(q.w, v.w, p3);
                                     }
-                                    const int at = wrote + __popc(km & below);
-                                    if (at < a.stride) {
-                                        a.kept_pos[out + at] = pos;
-                                        a.kept_d2[out + at] = (a0 + a1) + (a2 + a3);
-                                    }
+                                    d2 = (a0 + a1) + (a2 + a3);
+                                    const float dot = fmaxf(fmaf(-2.f, (p0 + p1) + (p2 + p3), qd + a.enorm[pos]), 0.f);
+                                    cand = wp_nn_bin(dot, qbase) <= bstar;
                                 }
-                                wrote += __popc(km);
+                                kept += __popc(__ballot_sync(0xffffffffu, keep));
+                                // slice by slice, each from a multiple of 32
+                                const int sl = pos / a.slice_len;
+                                unsigned left = __ballot_sync(0xffffffffu, cand);
+                                while (left) {
+                                    const int now = __shfl_sync(0xffffffffu, sl, __ffs(left) - 1);
+                                    if (now != slice) {
+                                        const int up = (wrote + 31) / 32 * 32;
+                                        if (wrote + lane < up && up <= a.stride) a.kept_pos[out + wrote + lane] = -1;
+                                        wrote = up;
+                                        slice = now;
+                                    }
+                                    const unsigned cm = __ballot_sync(0xffffffffu, cand && sl == now);
+                                    if (wrote + __popc(cm) > a.stride) {
+                                        fatal = 11;
+                                        break;
+                                    }
+                                    if (cand && sl == now) {
+                                        const long p = out + wrote + __popc(cm & below);
+                                        a.kept_pos[p] = keep ? pos : -1;
+                                        a.kept_d2[p] = d2;
+                                    }
+                                    wrote += __popc(cm);
+                                    left &= ~cm;
+                                }
                             }
                         }
-                        if (wrote != M || wrote > a.stride) fatal = 11;
+                        if (kept != M && !fatal) fatal = 13;
+                        M = wrote;
                     }
                 }
             }

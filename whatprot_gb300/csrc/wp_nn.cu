@@ -16,12 +16,13 @@
 //   wp_nn_collect_kernel  the same distances again; each query (one thread)
 //                         appends the entries in bins <= b* to its candidate
 //                         list, in entry order (deterministic).
-//   wp_nn_select_kernel   one warp per query: the exact k-hit set (entries in
+//   wp_nn_pick_kernel     one warp per query: the exact k-hit set (entries in
 //                         bins < b*, then those of bin b* by a hits-weighted
 //                         radix select on the distance bits, ties by entry
-//                         index), the weighted scores per peptide (per-id sums
-//                         formed in a fixed order), the total, and the top h
-//                         ids in ascending (score, id) order.
+//                         index).
+//
+// Votes, total and the top h ids over the kept entries: wp_nnscore.cu, or
+// wp_nn_select_kernel for very large sets.
 //
 // The set is the shortest prefix of the entries sorted by (squared
 // distance, entry index) whose hits reach k: what KBest (k-best.h:26-42)
@@ -31,11 +32,12 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <cub/cub.cuh>
 
 #include "wp_common.cuh"
 
-#define NN_NB 64           // distance bins per query
+#define NN_NB WP_NN_BINS    // distance bins per query
 #define NN_TE 32           // entries per shared-memory tile
 #define NN_THREADS 256     // threads per CTA in the distance kernels
 #define NN_QPT 1           // queries per thread (one: a warp's 32 sorted reads share
@@ -49,16 +51,6 @@
 // mantissa bits of the float), bin 0 below, bin NB-1 open-ended.
 __device__ __forceinline__ int nn_coarse_bin(float d2) {
     const int b = (int)(__float_as_uint(d2) >> 21) - ((127 - 6) << 2) + 1;
-    return b < 0 ? 0 : (b > NN_NB - 1 ? NN_NB - 1 : b);
-}
-
-// Fine bin of a squared distance for one query: sixteen bins per octave
-// (exponent and top four mantissa bits), bin 1 starting at the query's
-// origin `base` (in units of float bits >> 19), bin 0 below, bin NB-1
-// open-ended: 62 fine bins span almost four octaves around the query's
-// estimated k-hit radius.  Monotone in d2.
-__device__ __forceinline__ int nn_bin(float d2, int base) {
-    const int b = (int)(__float_as_uint(d2) >> 19) - base + 1;
     return b < 0 ? 0 : (b > NN_NB - 1 ? NN_NB - 1 : b);
 }
 
@@ -159,9 +151,6 @@ __device__ __forceinline__ bool nn_clears(float lb, float limit) {
     return lb > limit + 1e-3f + 1e-4f * limit;
 }
 
-// Float value where a query's fine bin b starts.
-__device__ __forceinline__ float nn_bin_start(int base, int b) { return __uint_as_float((unsigned)(base + b - 1) << 19); }
-
 // Load a tile of entries (coords, squared norms and hits) into shared memory.
 template <int DP>
 __device__ __forceinline__ void nn_load_tile(const NNArgs& a, int e0, int e_end, float* tile, int* thits,
@@ -220,7 +209,7 @@ __global__ void __launch_bounds__(NN_THREADS) wp_nn_hist_kernel(NNArgs a) {
 #pragma unroll
         for (int i = 0; i < DP; i++) q[j][i] = valid[j] ? src[i] : 0.f;
         base[j] = valid[j] ? a.qbase[a.q0 + slot] : 0;
-        far[j] = valid[j] ? nn_bin_start(base[j], NN_NB - 1) : INFINITY;
+        far[j] = valid[j] ? wp_nn_bin_start(base[j], NN_NB - 1) : INFINITY;
     }
     float qn[NN_QPT];
 #pragma unroll
@@ -275,7 +264,7 @@ __global__ void __launch_bounds__(NN_THREADS) wp_nn_hist_kernel(NNArgs a) {
                 for (int j = 0; j < NN_QPT; j++) {
                     const float d2 = nn_d2_dot<DP>(q[j], qn[j], tile + e * DP, ten[e]);
                     if (need[j]) {
-                        const int bin = nn_bin(d2, base[j]);
+                        const int bin = wp_nn_bin(d2, base[j]);
                         mb[j] = min(mb[j], bin);
                         atomicAdd(&hist[(j * NN_THREADS + threadIdx.x) * (NN_NB + 1) + bin], (unsigned)thits[e]);
                     }
@@ -320,7 +309,8 @@ __global__ void __launch_bounds__(NN_THREADS) wp_nn_hist_kernel(NNArgs a) {
 // octaves below that coarse bin and end, with the open last bin, half an
 // octave above it.  Only the bins move with the estimate; the
 // selection stays exact whatever it says (a poor estimate only leaves more
-// candidates).
+// candidates).  The sample is split over blockIdx.y so that small batches fill
+// the GPU (4,000 reads: 0.34 ms, against 3.6 ms with a CTA per 256 reads).
 template <int DP>
 __global__ void __launch_bounds__(NN_THREADS) wp_nn_estimate_kernel(NNArgs a) {
     extern __shared__ __align__(16) unsigned char nn_smem[];
@@ -343,9 +333,11 @@ __global__ void __launch_bounds__(NN_THREADS) wp_nn_estimate_kernel(NNArgs a) {
     float qn[NN_QPT];
 #pragma unroll
     for (int j = 0; j < NN_QPT; j++) qn[j] = nn_norm2<DP>(q[j]);
-    for (int s0 = 0; s0 < a.sample_n; s0 += NN_TE) {
+    // blockIdx.y takes a part of the sample
+    const int s_lo = (int)((long)a.sample_n * blockIdx.y / gridDim.y), s_hi = (int)((long)a.sample_n * (blockIdx.y + 1) / gridDim.y);
+    for (int s0 = s_lo; s0 < s_hi; s0 += NN_TE) {
         __syncthreads();
-        const int n = min(NN_TE, a.sample_n - s0);
+        const int n = min(NN_TE, s_hi - s0);
         for (int i = threadIdx.x; i < NN_TE * DP / 4; i += blockDim.x) {
             const int e = i / (DP / 4), part = i % (DP / 4);
             reinterpret_cast<float4*>(tile)[i] =
@@ -363,29 +355,36 @@ __global__ void __launch_bounds__(NN_THREADS) wp_nn_estimate_kernel(NNArgs a) {
         }
     }
     __syncthreads();
+    for (int i = threadIdx.x; i < NN_QPB * NN_NB; i += blockDim.x) {
+        const int lq = i / NN_NB, b = i % NN_NB;
+        const unsigned v = hist[((lq % NN_QPT) * NN_THREADS + lq / NN_QPT) * (NN_NB + 1) + b];
+        if (qb + lq < a.R && v) atomicAdd(&a.coarse[(long)(a.q0 + qb + lq) * NN_NB + b], v);
+    }
+}
+
+// The bins' origins from the parts' histograms, one thread per query.
+__global__ void wp_nn_origin_kernel(NNArgs a) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= a.R) return;
     // the sample point that stands for the k-th hit
     const long long kth = (a.k * a.sample_n + a.hits_total - 1) / a.hits_total;
-#pragma unroll
-    for (int j = 0; j < NN_QPT; j++) {
-        if (!valid[j]) continue;
-        const unsigned* h = hist + (threadIdx.x + j * NN_THREADS) * (NN_NB + 1);
-        long long run = 0;
-        int b = NN_NB - 1;
-        for (int i = 0; i < NN_NB; i++) {
-            run += h[i];
-            if (run >= kth) {
-                b = i;
-                break;
-            }
+    const unsigned* h = a.coarse + (long)(a.q0 + q) * NN_NB;
+    long long run = 0;
+    int b = NN_NB - 1;
+    for (int i = 0; i < NN_NB; i++) {
+        run += h[i];
+        if (run >= kth) {
+            b = i;
+            break;
         }
-        // coarse bin b starts at float bits >> 21 == b - 1 + ((127 - 6) << 2);
-        // the fine bins start 54 sixteenths of an octave below it, so the
-        // last (open) fine bin starts half an octave above it (a read whose
-        // radius lies beyond is counted again with its bins moved up,
-        // wp_nn_redo_kernel)
-        const int ck = b - 1 + ((127 - 6) << 2);
-        a.qbase[a.q0 + qb + threadIdx.x * NN_QPT + j] = 4 * ck - 54;
     }
+    // coarse bin b starts at float bits >> 21 == b - 1 + ((127 - 6) << 2);
+    // the fine bins start 54 sixteenths of an octave below it, so the
+    // last (open) fine bin starts half an octave above it (a read whose
+    // radius lies beyond is counted again with its bins moved up,
+    // wp_nn_redo_kernel)
+    const int ck = b - 1 + ((127 - 6) << 2);
+    a.qbase[a.q0 + q] = 4 * ck - 54;
 }
 
 // Per query: the slices' histograms summed, the bin b* where the running
@@ -404,8 +403,7 @@ __global__ void wp_nn_threshold_kernel(NNArgs a) {
     int bound_bin = -1;
     if (a.tf_d) {
         const double td = a.tf_d[gq];
-        bound_bin = (a.tf_flag[gq] & 1) ? NN_NB - 1
-                                         : nn_bin((float)(td * (1.0 + 1e-4) + 1e-3) * (1.f + 1e-6f), a.qbase[gq]);
+        bound_bin = (a.tf_flag[gq] & 1) ? NN_NB - 1 : wp_nn_bin(wp_nn_bound(td), a.qbase[gq]);
     }
     for (int i = 0; i < NN_NB; i++) {
         long long hi = 0;
@@ -469,7 +467,7 @@ __global__ void __launch_bounds__(NN_THREADS) wp_nn_collect_kernel(NNArgs a) {
         cap[j] = valid[j] ? a.slicecap[(long)s * a.R_all + gq] : 0;
         cnt[j] = 0;
         // candidates lie below the start of bin b* + 1 (none beyond the open last bin)
-        lim[j] = !valid[j] ? -1.f : (bstar[j] >= NN_NB - 1 ? INFINITY : nn_bin_start(base[j], bstar[j] + 1));
+        lim[j] = !valid[j] ? -1.f : (bstar[j] >= NN_NB - 1 ? INFINITY : wp_nn_bin_start(base[j], bstar[j] + 1));
     }
     float qn[NN_QPT];
 #pragma unroll
@@ -514,7 +512,7 @@ __global__ void __launch_bounds__(NN_THREADS) wp_nn_collect_kernel(NNArgs a) {
         for (int e = 0; e < n; e++) {
 #pragma unroll
             for (int j = 0; j < NN_QPT; j++) {
-                const int bin = nn_bin(nn_d2_dot<DP>(q[j], qn[j], tile + e * DP, ten[e]), base[j]);
+                const int bin = wp_nn_bin(nn_d2_dot<DP>(q[j], qn[j], tile + e * DP, ten[e]), base[j]);
                 if (bin <= bstar[j]) {
                     if (cnt[j] < cap[j]) {
                         a.cand_idx[off[j] + cnt[j]] = e0 + e;
@@ -581,47 +579,34 @@ __device__ int nn_digit_from_top(const unsigned long long* hist, long long want,
     return __shfl_sync(0xffffffffu, digit, L);
 }
 
-__global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelectArgs a) {
-    extern __shared__ __align__(16) unsigned char nn_sel_smem[];
-    unsigned long long(*s_hist)[256] = reinterpret_cast<unsigned long long(*)[256]>(nn_sel_smem);
-    double(*s_key)[NN_HMAX] = reinterpret_cast<double(*)[NN_HMAX]>(nn_sel_smem + sizeof(unsigned long long) * 256 * NN_SEL_WARPS);
-    int(*s_id)[NN_HMAX] = reinterpret_cast<int(*)[NN_HMAX]>(nn_sel_smem + sizeof(unsigned long long) * 256 * NN_SEL_WARPS
-                                                              + sizeof(double) * NN_HMAX * NN_SEL_WARPS);
+// The kept entries of a read's candidate list, one warp per read: for the
+// replayed search those at or below its final top, else the shortest prefix by
+// (squared distance, entry) whose hits reach k.  Writes the list with every slice
+// from a multiple of 32, -1 in the places of the others.
+__global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_pick_kernel(NNSelectArgs a) {
+    __shared__ unsigned long long s_hist[NN_SEL_WARPS][256];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     const long gw = (long)blockIdx.x * NN_SEL_WARPS + wib;
     const long nw = (long)gridDim.x * NN_SEL_WARPS;
-    double* acc = a.acc + gw * a.U;
-    int* mark = a.mark + gw * a.U;
-    int* touched = a.touched + gw * a.U;
     unsigned long long* hist = s_hist[wib];
 
     for (long lq = gw; lq < a.R; lq += nw) {
         const int gq = a.q0 + (int)lq;
-        // the kept entries are given: one list of kept_n
-        const int kept = a.kept_n ? a.kept_n[gq] : 0;
-        if (kept < 0) continue;
-        const int slices = a.kept_n ? 1 : a.slices;
-        auto seg_begin = [&](int sl) -> long long {
-            return a.kept_n ? lq * a.stride : a.qoff[lq] + a.sliceoff[(long)sl * a.R_all + gq];
-        };
-        auto seg_count = [&](int sl) -> long long {
-            return a.kept_n ? kept : min(a.slicecnt[(long)sl * a.R_all + gq], a.slicecap[(long)sl * a.R_all + gq]);
-        };
-        const int bstar = a.kept_n ? 0 : a.qbin[gq];
-        long long need = a.kept_n ? 0 : a.k - a.qbelow[gq];  // hits still needed from bin b*
+        const int bstar = a.qbin[gq];
+        long long need = a.k - a.qbelow[gq];  // hits still needed from bin b*
         // the reference's k-hit set: entries at or below the replayed final
         // top (FP64 distance, tree position); FP32 distances decide unless
         // they lie within their rounding margin of the top's
         const bool exact = a.tf_d != nullptr;
         const double tf_d = exact ? a.tf_d[gq] : 0.0;
         const int tf_pos = exact ? a.tf_pos[gq] : 0;
-        const bool tf_all = a.kept_n || (exact && (a.tf_flag[gq] & 1));
+        const bool tf_all = exact && (a.tf_flag[gq] & 1);
         const double tf_m = 2e-5 * tf_d + 1e-3;
         const double* q64 = exact ? a.rads + (long)(a.qperm ? a.qperm[gq] : gq) * a.TC : nullptr;
         unsigned kstar_out = 0u;
         bool take_all_out = false;
-        if (!exact && !a.kept_n) {
+        if (!exact) {
         // The query's candidates: one segment per entry slice, in slice
         // order (so in ascending entry index overall).
 
@@ -700,19 +685,84 @@ __global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelec
         kstar_out = prefix;
         take_all_out = take_all;
         }
-        const bool take_all = exact || a.kept_n ? tf_all : take_all_out;
+        const bool take_all = exact ? tf_all : take_all_out;
         const unsigned kstar = kstar_out;  // with take_all: unused
+        // ---- the kept entries
+        const long long out = a.koff[lq];
+        int wrote = 0;
+        long long tie_cum = 0;  // hits of key == kstar entries seen so far
+        for (int sl = 0; sl < a.slices; sl++) {
+            const long long sb = a.qoff[lq] + a.sliceoff[(long)sl * a.R_all + gq];
+            const long long sn = min(a.slicecnt[(long)sl * a.R_all + gq], a.slicecap[(long)sl * a.R_all + gq]);
+            for (long long i0 = 0; i0 < sn; i0 += 32) {
+                const long long i = i0 + lane;
+                bool keep = false;
+                int e = -1;
+                float d2 = 0.f;
+                bool tie = false;
+                if (i < sn) {
+                    e = a.cand_idx[sb + i];
+                    d2 = a.cand_d2[sb + i];
+                    const int b = a.cand_bin[sb + i];
+                    const unsigned key = __float_as_uint(d2);
+                    if (take_all) keep = true;
+                    else if (exact) {
+                        if ((double)d2 < tf_d - tf_m) keep = true;
+                        else if ((double)d2 <= tf_d + tf_m) {
+                            const double d64 = wp_nn_exact_d2(q64, e, a.TC, a.C, a.DP, a.cnt, a.ctab, a.NC, a.ecoord);
+                            keep = d64 < tf_d || (d64 == tf_d && e <= tf_pos);
+                        }
+                    } else if (b < bstar) keep = true;
+                    else if (key < kstar) keep = true;
+                    else if (key == kstar) tie = true;
+                }
+                // ties at kstar: keep in entry order while the tie hits before
+                // this one are below `need`
+                const long long th = tie ? (long long)a.cand_hits[sb + i] : 0;
+                const long long incl = warp_incl_scan(th);
+                if (tie && tie_cum + incl - th < need) keep = true;
+                tie_cum += __shfl_sync(0xffffffffu, incl, 31);
+                a.kept_pos[out + wrote + lane] = keep ? e : -1;
+                a.kept_d2[out + wrote + lane] = d2;
+                wrote += 32;
+            }
+        }
+        if (lane == 0) a.kept_n[gq] = wrote;
+        __syncwarp();
+    }
+}
+
+// NNClassifier's votes over the kept entries, one warp per read with its scores
+// in global memory: for sets of more source ids than wp_nnscore.cu's kernel
+// keeps in shared memory.
+__global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelectArgs a) {
+    extern __shared__ __align__(16) unsigned char nn_sel_smem[];
+    unsigned long long(*s_hist)[256] = reinterpret_cast<unsigned long long(*)[256]>(nn_sel_smem);
+    double(*s_key)[NN_HMAX] = reinterpret_cast<double(*)[NN_HMAX]>(nn_sel_smem + sizeof(unsigned long long) * 256 * NN_SEL_WARPS);
+    int(*s_id)[NN_HMAX] = reinterpret_cast<int(*)[NN_HMAX]>(nn_sel_smem + sizeof(unsigned long long) * 256 * NN_SEL_WARPS
+                                                              + sizeof(double) * NN_HMAX * NN_SEL_WARPS);
+    const int lane = threadIdx.x & 31;
+    const int wib = threadIdx.x >> 5;
+    const long gw = (long)blockIdx.x * NN_SEL_WARPS + wib;
+    const long nw = (long)gridDim.x * NN_SEL_WARPS;
+    double* acc = a.acc + gw * a.U;
+    int* mark = a.mark + gw * a.U;
+    int* touched = a.touched + gw * a.U;
+    unsigned long long* hist = s_hist[wib];
+
+    for (long lq = gw; lq < a.R; lq += nw) {
+        const int gq = a.q0 + (int)lq;
+        const int kept = a.kept_n[gq];
+        if (kept < 0) continue;
+        const long long sb = a.koff ? a.koff[lq] : lq * a.stride;
         // Weights of the entries near the read (within 18.5 x 2 sig^2 of the
         // nearest, i.e. above 1e-8 of the largest weight) from FP64
         // distances, as the reference forms them; the far ones from FP32
         // (their error is below 1e-8 of the largest weight).
         float dmin = INFINITY;
         if (a.rads) {
-            for (int sl = 0; sl < slices; sl++) {
-                const long long sb = seg_begin(sl);
-                const long long sn = seg_count(sl);
-                for (long long i = lane; i < sn; i += 32) dmin = fminf(dmin, a.cand_d2[sb + i]);
-            }
+            for (int i = lane; i < kept; i += 32)
+                if (a.kept_pos[sb + i] >= 0) dmin = fminf(dmin, a.kept_d2[sb + i]);
             for (int o = 16; o > 0; o >>= 1) dmin = fminf(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
         }
         const double wlim = (double)dmin + 18.5 * a.two_sig_sq + 1e-3;
@@ -720,38 +770,10 @@ __global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelec
         // ---- contributions of the kept entries, in candidate (entry) order.
         double total_part = 0.0;
         int ntouched = 0;
-        long long tie_cum = 0;  // hits of key == kstar entries seen so far
-        for (int sl = 0; sl < slices; sl++) {
-          const long long sb = seg_begin(sl);
-          const long long sn = seg_count(sl);
-          for (long long i0 = 0; i0 < sn; i0 += 32) {
-            const long long i = i0 + lane;
-            bool keep = false;
-            int e = -1;
-            float d2 = 0.f;
-            bool tie = false;
-            if (i < sn) {
-                e = a.cand_idx[sb + i];
-                d2 = a.cand_d2[sb + i];
-                const unsigned key = __float_as_uint(d2);
-                const int b = a.kept_n ? 0 : a.cand_bin[sb + i];
-                if (take_all) keep = true;
-                else if (exact) {
-                    if ((double)d2 < tf_d - tf_m) keep = true;
-                    else if ((double)d2 <= tf_d + tf_m) {
-                        const double d64 = wp_nn_exact_d2(q64, e, a.TC, a.C, a.DP, a.cnt, a.ctab, a.NC, a.ecoord);
-                        keep = d64 < tf_d || (d64 == tf_d && e <= tf_pos);
-                    }
-                } else if (b < bstar) keep = true;
-                else if (key < kstar) keep = true;
-                else if (key == kstar) tie = true;
-            }
-            // ties at kstar: keep in entry order while the tie hits before
-            // this one are below `need`
-            const long long th = tie ? (long long)a.cand_hits[sb + i] : 0;
-            const long long incl = warp_incl_scan(th);
-            if (tie && tie_cum + incl - th < need) keep = true;
-            tie_cum += __shfl_sync(0xffffffffu, incl, 31);
+        for (int i0 = 0; i0 < kept; i0 += 32) {
+            const int e = i0 + lane < kept ? a.kept_pos[sb + i0 + lane] : -1;
+            const bool keep = e >= 0;
+            const float d2 = keep ? a.kept_d2[sb + i0 + lane] : 0.f;
             // exp(-d2 / 2 sig^2) as 2^x: exp2f of the fraction, the integer
             // part applied in FP64 so far entries keep a non-zero weight
             double w = 0.0;
@@ -818,7 +840,6 @@ __global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelec
                 ntouched += __popc(fm);
                 __syncwarp();
             }
-          }
         }
         // total, summed in a fixed tree order and broadcast from lane 0
         double tot = total_part;
@@ -1059,23 +1080,31 @@ cudaError_t wp_launch_nn_dist(int DP, bool hist, cudaStream_t s, const NNArgs& a
 template <int DP>
 static cudaError_t launch_estimate(dim3 grid, cudaStream_t s, const NNArgs& a) {
     const size_t smem = wp_nn_dist_smem_bytes(DP, true);
-    cudaFuncSetAttribute(wp_nn_estimate_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(wp_nn_estimate_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
     wp_nn_estimate_kernel<DP><<<grid, NN_THREADS, smem, s>>>(a);
     return cudaGetLastError();
 }
 
-// The per-query bin origins (a.qbase) from a.sample_n sampled entries.
-cudaError_t wp_launch_nn_estimate(int DP, cudaStream_t s, const NNArgs& a) {
+// The per-query bin origins (a.qbase) from a.sample_n sampled entries;
+// a.coarse: [R][bins] scratch.  `ctas`: CTAs to spread the work over.
+cudaError_t wp_launch_nn_estimate(int DP, int ctas, cudaStream_t s, const NNArgs& a) {
     const int qblocks = (a.R + NN_QPB - 1) / NN_QPB;
     if (qblocks == 0) return cudaSuccess;
-    const dim3 grid(qblocks);
+    cudaError_t e = cudaMemsetAsync(a.coarse + (long)a.q0 * NN_NB, 0, sizeof(unsigned) * (size_t)a.R * NN_NB, s);
+    if (e != cudaSuccess) return e;
+    // at least 256 sample points per part (the read's own set-up costs as much as some tens)
+    const dim3 grid(qblocks, std::max(1, std::min((ctas + qblocks - 1) / qblocks, a.sample_n / 256)));
     switch (DP) {
-        case 16: return launch_estimate<16>(grid, s, a);
-        case 32: return launch_estimate<32>(grid, s, a);
-        case 48: return launch_estimate<48>(grid, s, a);
-        case 64: return launch_estimate<64>(grid, s, a);
+        case 16: e = launch_estimate<16>(grid, s, a); break;
+        case 32: e = launch_estimate<32>(grid, s, a); break;
+        case 48: e = launch_estimate<48>(grid, s, a); break;
+        case 64: e = launch_estimate<64>(grid, s, a); break;
         default: return cudaErrorInvalidValue;
     }
+    if (e != cudaSuccess) return e;
+    wp_nn_origin_kernel<<<(a.R + 127) / 128, 128, 0, s>>>(a);
+    return cudaGetLastError();
 }
 
 // Reads whose k-th hit fell in the open last bin (the estimate was low):
@@ -1121,6 +1150,12 @@ cudaError_t wp_launch_nn_redo(const NNArgs& a, int* list, int* count, int shift,
 cudaError_t wp_launch_nn_threshold(cudaStream_t s, const NNArgs& a) {
     if (a.R == 0) return cudaSuccess;
     wp_nn_threshold_kernel<<<(a.R + 127) / 128, 128, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t wp_launch_nn_pick(int grid, cudaStream_t s, const NNSelectArgs& a) {
+    if (a.R == 0) return cudaSuccess;
+    wp_nn_pick_kernel<<<grid, NN_SEL_WARPS * 32, 0, s>>>(a);
     return cudaGetLastError();
 }
 
