@@ -47,9 +47,12 @@ cudaError_t wp_launch_engine(int C, bool has_block, int threads, size_t smem, cu
                              int2* out, int* out_count, int slab_half, int scr_floats,
                              int spill_error, int* grid_out);
 size_t wp_engine_smem_bytes(int slab_half, int scr_floats, bool has_block, int threads);
-cudaError_t wp_launch_dense(bool has_block, int threads, size_t smem, cudaStream_t stream,
+cudaError_t wp_launch_coop(int C, bool has_block, int lanes, cudaStream_t s, const BatchArgs& a, const int2* in,
+                           const int* in_count, int* in_head, int2* out, int* out_count, int slab_half,
+                           int spill_error);
+cudaError_t wp_launch_dense(bool has_block, int T, int C, size_t smem_optin, cudaStream_t stream,
                             const BatchArgs& a);
-size_t wp_dense_smem_bytes(int T, int S_cap, int C, bool has_block, int warps);
+bool wp_dense_fits(int T, int S_cap, int C, bool has_block, size_t smem_optin);
 cudaError_t wp_launch_fma_probe(int blocks, int threads, int iters, cudaStream_t stream, float* sink);
 cudaError_t wp_launch_fit_estep(bool has_block, int grid, int threads, cudaStream_t s, const FitArgs& a);
 cudaError_t wp_launch_nn_dist(int DP, bool hist, cudaStream_t s, const NNArgs& a);
@@ -188,9 +191,9 @@ struct EngineReplay {
     bool valid = false;
     long long epoch = -1;  // g_alloc_epoch when recorded
     BatchArgs a;
-    int C = 0, T = 0, nt = 0, dense_warps = 0;
-    bool hb = false;
-    int threads[WP_MAX_TIERS], half[WP_MAX_TIERS];
+    int C = 0, T = 0, nt = 0;
+    bool hb = false, dense = false;
+    int threads[WP_MAX_TIERS], half[WP_MAX_TIERS], lanes[WP_MAX_TIERS];
     int2* list[WP_MAX_TIERS];
     int* cnt = nullptr;
 };
@@ -674,15 +677,10 @@ wp_status run_batch(wp_ctx* ctx, const double* d_rads, int R, double dist_cutoff
     a.ovf = ctx->d_ovf2.as<int2>();
     a.ovf_count = cnt + WP_CNT_DENSE;
     a.ovf_head = cnt + WP_CNT_DENSE + 1;
+    a.ovf_head2 = cnt + WP_CNT_DENSE + 2;
     a.dense_S_cap = ((ctx->S_max + 31) / 32) * 32;
     if (n_slots > 0) {
-        // Dense fallback shape: as many warps as fit (0: unavailable).
-        int dense_warps = 0;
-        for (int w = 16; w >= 1; w--)
-            if (wp_dense_smem_bytes(T, a.dense_S_cap, C, hb, w) <= (size_t)ctx->smem_optin) {
-                dense_warps = w;
-                break;
-            }
+        const bool dense = wp_dense_fits(T, a.dense_S_cap, C, hb, (size_t)ctx->smem_optin);
         // Pass 1 and pass 2 launch shapes (default: 2 CTAs of 256 threads
         // per SM, then 1 CTA of 256 with twice the slab); the dense kernel
         // takes what is left.
@@ -693,23 +691,30 @@ wp_status run_batch(wp_ctx* ctx, const double* d_rads, int R, double dist_cutoff
             return fail(ctx, WP_ERR_UNSUPPORTED, "shared memory too small for the pair engine");
         // Engine passes ("tiers") in order of growing slab: pass 1, a middle
         // pass of 3 CTAs of 128 threads per SM for the pairs just too large
-        // for pass 1, the last configured pass, and passes of one CTA of 128
-        // and of 64 threads per SM for what is left short of the dense
-        // kernel (one thread per pair stays faster than the dense kernel's
-        // warp over every state while the box fits).
+        // for pass 1 and the last configured pass, a thread per pair; then
+        // two passes with several lanes per pair (wp_coop.cu) for the pairs
+        // whose slabs leave an SM fewer than 256 and fewer than 128 threads
+        // (the slabs of 128 and of 64 threads per SM), short of the dense
+        // kernel.  There a thread per pair is bound by its chain of
+        // shared-memory loads: 48,400 pairs past pass 1 took 7.9 ms in these
+        // two passes and take 1.06 (8 and 16 lanes; 8 and 8: 1.17,
+        // 16 and 16: 1.10); one pass earlier a thread per
+        // pair is the cheaper where pairs are many (learned proposal, 4e6
+        // pairs: 6.43 ms, against 7.33 with lanes there too), as lanes issue
+        // about 3 times the instructions per pair.
         struct Tier {
-            int threads, per_sm, half;
+            int threads, per_sm, half, lanes;
         };
         Tier tiers[WP_MAX_TIERS];
         int nt = 0;
-        tiers[nt++] = {cfg.t1, cfg.s1, half1};
+        tiers[nt++] = {cfg.t1, cfg.s1, half1, 0};
         const int hmid = slab_half_for(ctx, 128, 3, hb);
-        if (hmid > half1 && hmid < half2) tiers[nt++] = {128, 3, hmid};
-        if (half2 > tiers[nt - 1].half) tiers[nt++] = {cfg.t2, cfg.s2, half2};
+        if (hmid > half1 && hmid < half2) tiers[nt++] = {128, 3, hmid, 0};
+        if (half2 > tiers[nt - 1].half) tiers[nt++] = {cfg.t2, cfg.s2, half2, 0};
         const int hbig = slab_half_for(ctx, 128, 1, hb);
-        if (hbig > tiers[nt - 1].half) tiers[nt++] = {128, 1, hbig};
+        if (hbig > tiers[nt - 1].half) tiers[nt++] = {128, 1, hbig, 8};
         const int hhuge = slab_half_for(ctx, 64, 1, hb);
-        if (hhuge > tiers[nt - 1].half) tiers[nt++] = {64, 1, hhuge};
+        if (hhuge > tiers[nt - 1].half) tiers[nt++] = {64, 1, hhuge, 16};
         DevBuf* lists[WP_MAX_TIERS] = {&ctx->d_work, &ctx->d_ovf1, &ctx->d_ovf3, &ctx->d_ovf4, &ctx->d_ovf5};
         // the compaction sends each pair to the first pass whose slab holds it
         a.n_tiers = nt;
@@ -718,7 +723,7 @@ wp_status run_batch(wp_ctx* ctx, const double* d_rads, int R, double dist_cutoff
             a.tier_list[k] = lists[k]->as<int2>();
             a.tier_count[k] = cnt + 2 * k;
         }
-        a.route_dense = dense_warps > 0 ? 1 : 0;
+        a.route_dense = dense ? 1 : 0;
         a.live_count = cnt + WP_CNT_LIVE;
         {
             TimedLaunch tl(ctx, 1);
@@ -744,19 +749,23 @@ wp_status run_batch(wp_ctx* ctx, const double* d_rads, int R, double dist_cutoff
         for (int k = 0; k < nt; k++) {
             TimedLaunch tl(ctx, 0);
             const bool last = k + 1 == nt;
-            size_t smem = wp_engine_smem_bytes(tiers[k].half, 0, hb, tiers[k].threads);
-            WP_CUDA(wp_launch_engine(C, hb, tiers[k].threads, smem, ctx->stream, a, lists[k]->as<int2>(),
-                                     cnt + 2 * k, cnt + 2 * k + 1,
-                                     last ? ctx->d_ovf2.as<int2>() : lists[k + 1]->as<int2>(),
-                                     last ? cnt + WP_CNT_DENSE : cnt + 2 * (k + 1), tiers[k].half, 0,
-                                     last && dense_warps == 0 ? 1 : 0, k == 0 ? &ctx->last_engine_grid : nullptr),
+            int2* next = last ? ctx->d_ovf2.as<int2>() : lists[k + 1]->as<int2>();
+            int* next_count = last ? cnt + WP_CNT_DENSE : cnt + 2 * (k + 1);
+            const int spill_error = last && !dense ? 1 : 0;
+            WP_CUDA(tiers[k].lanes > 0
+                            ? wp_launch_coop(C, hb, tiers[k].lanes, ctx->stream, a, lists[k]->as<int2>(), cnt + 2 * k,
+                                             cnt + 2 * k + 1, next, next_count, tiers[k].half, spill_error)
+                            : wp_launch_engine(C, hb, tiers[k].threads,
+                                               wp_engine_smem_bytes(tiers[k].half, 0, hb, tiers[k].threads),
+                                               ctx->stream, a, lists[k]->as<int2>(), cnt + 2 * k, cnt + 2 * k + 1,
+                                               next, next_count, tiers[k].half, 0, spill_error,
+                                               k == 0 ? &ctx->last_engine_grid : nullptr),
                     "engine pass");
             ctx->launches++;
         }
-        if (dense_warps > 0) {
+        if (dense) {
             TimedLaunch tl(ctx, 0);
-            size_t smem = wp_dense_smem_bytes(T, a.dense_S_cap, C, hb, dense_warps);
-            WP_CUDA(wp_launch_dense(hb, dense_warps * 32, smem, ctx->stream, a), "dense launch");
+            WP_CUDA(wp_launch_dense(hb, T, C, (size_t)ctx->smem_optin, ctx->stream, a), "dense launch");
             ctx->launches++;
         }
         if (mode == MODE_CLASSIFY) {
@@ -766,10 +775,11 @@ wp_status run_batch(wp_ctx* ctx, const double* d_rads, int R, double dist_cutoff
             rp.T = T;
             rp.hb = hb;
             rp.nt = nt;
-            rp.dense_warps = dense_warps;
+            rp.dense = dense;
             for (int k = 0; k < nt; k++) {
                 rp.threads[k] = tiers[k].threads;
                 rp.half[k] = tiers[k].half;
+                rp.lanes[k] = tiers[k].lanes;
                 rp.list[k] = lists[k]->as<int2>();
             }
             rp.cnt = cnt;
@@ -1886,19 +1896,23 @@ wp_status wp_engine_replay(wp_ctx* ctx, int reps, double* ms) {
         // heads go back to the start
         for (int k = 0; k < rp.nt; k++)
             WP_CUDA(cudaMemsetAsync(rp.cnt + 2 * k + 1, 0, sizeof(int), ctx->stream), "reset head");
-        WP_CUDA(cudaMemsetAsync(rp.cnt + WP_CNT_DENSE + 1, 0, sizeof(int), ctx->stream), "reset head");
+        WP_CUDA(cudaMemsetAsync(rp.cnt + WP_CNT_DENSE + 1, 0, 2 * sizeof(int), ctx->stream), "reset heads");
         for (int k = 0; k < rp.nt; k++) {
             const bool last = k + 1 == rp.nt;
-            size_t smem = wp_engine_smem_bytes(rp.half[k], 0, rp.hb, rp.threads[k]);
-            WP_CUDA(wp_launch_engine(rp.C, rp.hb, rp.threads[k], smem, ctx->stream, a, rp.list[k], rp.cnt + 2 * k,
-                                     rp.cnt + 2 * k + 1, last ? rp.a.ovf : rp.list[k + 1],
-                                     last ? rp.cnt + WP_CNT_DENSE : rp.cnt + 2 * (k + 1), rp.half[k], 0, 1, nullptr),
+            int2* next = last ? rp.a.ovf : rp.list[k + 1];
+            int* next_count = last ? rp.cnt + WP_CNT_DENSE : rp.cnt + 2 * (k + 1);
+            WP_CUDA(rp.lanes[k] > 0
+                            ? wp_launch_coop(rp.C, rp.hb, rp.lanes[k], ctx->stream, a, rp.list[k], rp.cnt + 2 * k,
+                                             rp.cnt + 2 * k + 1, next, next_count, rp.half[k], 1)
+                            : wp_launch_engine(rp.C, rp.hb, rp.threads[k],
+                                               wp_engine_smem_bytes(rp.half[k], 0, rp.hb, rp.threads[k]), ctx->stream,
+                                               a, rp.list[k], rp.cnt + 2 * k, rp.cnt + 2 * k + 1, next, next_count,
+                                               rp.half[k], 0, 1, nullptr),
                     "engine pass");
             ctx->launches++;
         }
-        if (rp.dense_warps > 0) {
-            size_t smem = wp_dense_smem_bytes(rp.T, rp.a.dense_S_cap, rp.C, rp.hb, rp.dense_warps);
-            WP_CUDA(wp_launch_dense(rp.hb, rp.dense_warps * 32, smem, ctx->stream, a), "dense launch");
+        if (rp.dense) {
+            WP_CUDA(wp_launch_dense(rp.hb, rp.T, rp.C, (size_t)ctx->smem_optin, ctx->stream, a), "dense launch");
             ctx->launches++;
         }
     }

@@ -15,9 +15,26 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "wp_common.cuh"
 
-#define WP_DENSE_WARPS_MAX 16
+#define WP_DENSE_WARPS 8
+
+// Edman success coefficients by (dye count n, remaining dyes tot) at
+// [n * 17 + tot], rounded as the kernel's own expression: the cut dye was
+// another one (x), the state one dye up lost the cut dye (y).
+struct DenseEdman {
+    float x[16 * 17], y[16 * 17];
+};
+
+#define WP_DENSE_NONE 31u  // in an Edman position's word: no dye there
+
+// Slab classes of a launch (see above).
+struct DensePass {
+    int S_small, S_cap;  // states per slice of a warp's slab in the two phases
+    int big_warps;       // warps of the second phase (0: no pair is larger than S_small)
+};
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -100,17 +117,16 @@ __device__ void binomial_step(float* X, int S, int W, int e_count, int stc,
 
 // Per-warp shared memory carve-up.
 struct WarpBufs {
+    uint32_t* code;  // [T - 1] Edman position: st << 16 | (D + 1) << 10 | tot << 5 | 4 c, WP_DENSE_NONE for no dye
     float* X;
-    float* Y;
     float* XB;
-    float* YB;
     float* em;
     uint16_t* coord;
     uint16_t* fib;  // [C][S_cap]
 };
 
 __host__ __device__ inline size_t wp_warp_bytes(int T, int S_cap, int C, bool has_block) {
-    size_t f = (size_t)(has_block ? 4 : 2) * T * S_cap + S_cap;
+    size_t f = (size_t)(has_block ? 2 : 1) * T * S_cap + S_cap;
     size_t h = (size_t)S_cap * (1 + C);
     size_t b = f * 4 + h * 2;
     return (b + 15) & ~(size_t)15;
@@ -118,26 +134,32 @@ __host__ __device__ inline size_t wp_warp_bytes(int T, int S_cap, int C, bool ha
 
 // Forward pass of one (read, peptide) pair by one warp.  Returns the
 // probability as mant * 2^expo (mant == 0: probability zero).
-template <bool HAS_BLOCK>
-__device__ void pair_forward(const BatchArgs& a, const SmemModel& H, int r,
+template <int C, bool HAS_BLOCK>
+__device__ void pair_forward(const BatchArgs& a, const SmemModel& H, const DenseEdman& ed, int r,
                              const DevModel& m, const PeptideRec& pep,
                              const WarpBufs& wb, int S_cap, int lane,
                              float* out_mant, int* out_expo, int* err) {
-    const int C = m.C, T = m.T;
+    const int T = m.T;
     const int W_read = a.W;
     const EmitEntry* __restrict__ rtab = a.tab + (long)r * a.entries;
     const uint8_t* blo = a.lo + (long)r * T * C;
     const uint8_t* bhi = a.hi + (long)r * T * C;
-    int Wc[WP_MAX_CHANNELS], st[WP_MAX_CHANNELS];
+    // widths D + 1 (one byte per channel) and strides (16 bits per channel)
+    uint32_t wpk = 0;
+    uint64_t spk = 0;
     int S = 1;
     bool empty = a.flags[r] != 0;
+#pragma unroll
     for (int c = 0; c < C; c++) {
-        Wc[c] = pep.D[c] + 1;
+        wpk |= (uint32_t)(pep.D[c] + 1) << (8 * c);
         if (pep.D[c] < a.Lsuf[(long)r * T * C + c]) empty = true;  // some L_t > D_c
     }
+    auto wid = [&](int c) { return (int)((wpk >> (8 * c)) & 255u); };
+    auto str = [&](int c) { return (int)((spk >> (16 * c)) & 65535u); };
+#pragma unroll
     for (int c = C - 1; c >= 0; c--) {
-        st[c] = S;
-        S *= Wc[c];
+        spk |= (uint64_t)S << (16 * c);
+        S *= wid(c);
     }
     if (empty) {
         *out_mant = 0.0f;
@@ -150,30 +172,35 @@ __device__ void pair_forward(const BatchArgs& a, const SmemModel& H, int r,
         *out_expo = 0;
         return;
     }
+    for (int e = lane; e < T - 1; e += 32) {
+        const int c = pep.dye[e];
+        wb.code[e] = c < 0 ? WP_DENSE_NONE
+                           : (uint32_t)str(c) << 16 | (uint32_t)wid(c) << 10 | (uint32_t)pep.tot[e] << 5 |
+                                     (uint32_t)(4 * c);
+    }
     // Coordinates of each state of an Edman slice, 4 bits per channel.
     for (int j = lane; j < S; j += 32) {
-        int code = 0;
-        for (int c = 0; c < C; c++) code |= ((j / st[c]) % Wc[c]) << (4 * c);
+        int code = 0, x = j;
+#pragma unroll
+        for (int c = C - 1; c >= 0; c--) {
+            const int q = x / wid(c);
+            code |= (x - q * wid(c)) << (4 * c);
+            x = q;
+        }
         wb.coord[j] = (uint16_t)code;
     }
     // Fiber base offsets per channel: the states with n_c == 0.
+#pragma unroll 1
     for (int c = 0; c < C; c++) {
-        if (Wc[c] == 1) continue;
-        int F = S / Wc[c];
+        if (wid(c) == 1) continue;
+        const int F = S / wid(c), sc = str(c);
         for (int rr = lane; rr < F; rr += 32) {
-            int rem = rr, j = 0;
-            for (int c2 = C - 1; c2 >= 0; c2--) {
-                if (c2 == c) continue;
-                j += (rem % Wc[c2]) * st[c2];
-                rem /= Wc[c2];
-            }
-            wb.fib[c * S_cap + rr] = (uint16_t)j;
+            const int q = rr / sc;
+            wb.fib[c * S_cap + rr] = (uint16_t)(q * sc * wid(c) + rr - q * sc);
         }
     }
-    float* X = wb.X;
-    float* Y = wb.Y;
-    float* XB = wb.XB;
-    float* YB = wb.YB;
+    float* const X = wb.X;
+    float* const XB = wb.XB;
     // t = 0: start state (0, D) (peptide-state-vector.cc:38-40), initial
     // block (block-transition.cc:33-62), then duds per channel.
     for (int j = lane; j < S; j += 32) {
@@ -185,10 +212,11 @@ __device__ void pair_forward(const BatchArgs& a, const SmemModel& H, int r,
         X[j] = a;
     }
     __syncwarp();
+#pragma unroll 1
     for (int c = 0; c < C; c++) {
-        if (Wc[c] == 1) continue;
-        binomial_step(X, S, Wc[c], 1, st[c], wb.fib + c * S_cap, H.dud[c], lane);
-        if (HAS_BLOCK) binomial_step(XB, S, Wc[c], 1, st[c], wb.fib + c * S_cap, H.dud[c], lane);
+        if (wid(c) == 1) continue;
+        binomial_step(X, S, wid(c), 1, str(c), wb.fib + c * S_cap, H.dud[c], lane);
+        if (HAS_BLOCK) binomial_step(XB, S, wid(c), 1, str(c), wb.fib + c * S_cap, H.dud[c], lane);
         __syncwarp();
     }
     int expo = 0;       // log2 of the factor the stored state is scaled by
@@ -210,54 +238,61 @@ __device__ void pair_forward(const BatchArgs& a, const SmemModel& H, int r,
             // Detach (detach-transition.cc:36-68) is folded into the
             // previous rescale (pd) and the pending factor fac_prev.
             // Bleach per channel.
+#pragma unroll 1
             for (int c = 0; c < C; c++) {
-                if (Wc[c] == 1) continue;
-                binomial_step(X, S, Wc[c], t, st[c], wb.fib + c * S_cap, H.bleach[c], lane);
-                if (HAS_BLOCK) binomial_step(XB, S, Wc[c], t, st[c], wb.fib + c * S_cap, H.bleach[c], lane);
+                if (wid(c) == 1) continue;
+                binomial_step(X, S, wid(c), t, str(c), wb.fib + c * S_cap, H.bleach[c], lane);
+                if (HAS_BLOCK) binomial_step(XB, S, wid(c), t, str(c), wb.fib + c * S_cap, H.bleach[c], lane);
                 __syncwarp();
             }
-            // Edman (edman-transition.cc:62-162) as a gather into Y.
+            // Edman (edman-transition.cc:62-162) as a gather, in place: state
+            // i of slice e reads i, i - S and i - S + st[c], all at most i, so
+            // the elements go from the last down, and those of one step are
+            // read before any of them is written.
             {
                 const float pf = m.pf, qf = 1.0f - m.pf;
-                int n = (t + 1) * S;
-                int e = lane / S, j = lane - (lane / S) * S;
+                const int n = (t + 1) * S;
                 const int de = 32 / S, dj = 32 - de * S;
-                for (int i = lane; i < n; i += 32) {
-                    float v = 0.0f;
-                    if (e < t) v = pf * X[i];
-                    if (e >= 1) {
-                        int c = pep.dye[e - 1];
-                        float xin = X[i - S];
-                        if (c < 0) {
-                            v = fmaf(qf, xin, v);
-                        } else {
-                            int nc = (wb.coord[j] >> (4 * c)) & 15;
-                            float tot = (float)pep.tot[e - 1];
-                            float ratio = (float)nc / tot;
-                            if (nc < pep.tot[e - 1]) v = fmaf(qf * (1.0f - ratio), xin, v);
-                            if (nc + 1 < Wc[c]) {
-                                float r1 = (float)(nc + 1) / tot;
-                                v = fmaf(qf * r1, X[i - S + st[c]], v);
+                const int top = ((n + 31) & ~31) - 32;
+                int e = (top + lane) / S, j = top + lane - e * S;
+                for (int i0 = top; i0 >= 0; i0 -= 64) {
+                    float v[2];
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        const int i = i0 - 32 * u + lane;
+                        v[u] = 0.0f;
+                        if (i >= 0 && i < n) {
+                            if (e < t) v[u] = pf * X[i];
+                            if (e >= 1) {
+                                const uint32_t code = wb.code[e - 1];
+                                const float xin = X[i - S];
+                                if (code == WP_DENSE_NONE) {
+                                    v[u] = fmaf(qf, xin, v[u]);
+                                } else {
+                                    const int nc = (wb.coord[j] >> (code & 31)) & 15, tot = (code >> 5) & 31;
+                                    if (nc < tot) v[u] = fmaf(ed.x[nc * 17 + tot], xin, v[u]);
+                                    if (nc + 1 < (int)((code >> 10) & 63))
+                                        v[u] = fmaf(ed.y[nc * 17 + tot], X[i - S + (int)(code >> 16)], v[u]);
+                                }
                             }
                         }
+                        j -= dj;
+                        e -= de;
+                        if (j < 0) {
+                            j += S;
+                            e--;
+                        }
                     }
-                    Y[i] = v;
-                    if (HAS_BLOCK) YB[i] = (e < t) ? XB[i] : 0.0f;
-                    j += dj;
-                    e += de;
-                    if (j >= S) {
-                        j -= S;
-                        e++;
+                    __syncwarp();
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        const int i = i0 - 32 * u + lane;
+                        if (i >= 0 && i < n) X[i] = v[u];
                     }
+                    __syncwarp();
                 }
-                float* tmp = X;
-                X = Y;
-                Y = tmp;
-                if (HAS_BLOCK) {
-                    tmp = XB;
-                    XB = YB;
-                    YB = tmp;
-                }
+                if (HAS_BLOCK)
+                    for (int j2 = lane; j2 < S; j2 += 32) XB[t * S + j2] = 0.0f;
                 __syncwarp();
             }
         }
@@ -266,14 +301,17 @@ __device__ void pair_forward(const BatchArgs& a, const SmemModel& H, int r,
         int kmax;
         if (!m.interacting) {
             kmax = 0;
+#pragma unroll
             for (int c = 0; c < C; c++) {
-                // largest exponent over [cmin, min(cmax, D + 1)) of channel c
+                // largest exponent over [cmin, min(cmax, D + 1)) of channel
+                // c (at most 16 counts: a lane each)
+                const int n1 = min((int)bhi[t * C + c], wid(c)), n = blo[t * C + c] + lane;
                 int km = WP_EXPO_ZERO;
-                int n1 = min((int)bhi[t * C + c], Wc[c]);
-                for (int n = blo[t * C + c]; n < n1; n++) {
-                    EmitEntry en = rtab[(t * C + c) * W_read + n];
-                    if (en.mant != 0.0f) km = max(km, en.expo);
+                if (n < n1) {
+                    const EmitEntry en = rtab[(t * C + c) * W_read + n];
+                    if (en.mant != 0.0f) km = en.expo;
                 }
+                km = warp_max_int(km);
                 if (km == WP_EXPO_ZERO) kmax = WP_EXPO_ZERO;
                 if (kmax != WP_EXPO_ZERO) kmax += km;
             }
@@ -298,6 +336,7 @@ __device__ void pair_forward(const BatchArgs& a, const SmemModel& H, int r,
             float mant = 1.0f;
             int ks = 0;
             if (!m.interacting) {
+#pragma unroll
                 for (int c = 0; c < C; c++) {
                     EmitEntry en = rtab[(t * C + c) * W_read + ((code >> (4 * c)) & 15)];
                     mant *= en.mant;
@@ -372,73 +411,131 @@ __device__ void pair_forward(const BatchArgs& a, const SmemModel& H, int r,
 }
 
 
-// Persistent: warps take overflow pairs one at a time.
-template <bool HAS_BLOCK>
-__global__ void __launch_bounds__(WP_DENSE_WARPS_MAX * 32) wp_dense_kernel(BatchArgs a) {
+// Persistent: warps take overflow pairs one at a time.  Both phases go
+// through the whole list, each taking the pairs of its class.
+template <int C, bool HAS_BLOCK>
+__global__ void __launch_bounds__(WP_DENSE_WARPS * 32, 4) wp_dense_kernel(BatchArgs a, DensePass ps) {
+    const int count = *a.ovf_count;
+    if (count == 0) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SmemModel& M = *reinterpret_cast<SmemModel*>(smem_raw);
+    DenseEdman& ed = *reinterpret_cast<DenseEdman*>(smem_raw + ((sizeof(SmemModel) + 15) & ~(size_t)15));
     const DevModel& m = *a.model;
     load_smem_model(M, m);
-    __syncthreads();
-    const int T = m.T, C = m.C;
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    unsigned char* wbase = smem_raw + ((sizeof(SmemModel) + 15) & ~(size_t)15);
-    size_t wbytes = wp_warp_bytes(T, a.dense_S_cap, C, HAS_BLOCK);
-    float* fb = reinterpret_cast<float*>(wbase + wbytes * warp);
-    WarpBufs wb;
-    size_t slab = (size_t)T * a.dense_S_cap;
-    wb.X = fb;
-    wb.Y = fb + slab;
-    float* after = fb + 2 * slab;
-    if (HAS_BLOCK) {
-        wb.XB = fb + 2 * slab;
-        wb.YB = fb + 3 * slab;
-        after = fb + 4 * slab;
-    } else {
-        wb.XB = wb.YB = nullptr;
-    }
-    wb.em = after;
-    wb.coord = reinterpret_cast<uint16_t*>(after + a.dense_S_cap);
-    wb.fib = wb.coord + a.dense_S_cap;
-    const int count = *a.ovf_count;
-    for (;;) {
-        int idx = 0;
-        if (lane == 0) idx = atomicAdd(a.ovf_head, 1);
-        idx = __shfl_sync(0xffffffffu, idx, 0);
-        if (idx >= count) break;
-        const int2 rg = a.ovf[idx];
-        int vmax;
-        const PeptideRec& pep = a.peps[slot_pep(a, rg.x, item_slot(a, rg, &vmax))];
-        float mant;
-        int ex;
-        pair_forward<HAS_BLOCK>(a, M, rg.x, m, pep, wb, a.dense_S_cap, lane, &mant, &ex, a.err);
-        if (lane == 0) {
-            a.res_mant[rg.y] = mant;
-            a.res_expo[rg.y] = ex;
+    {
+        const float qf = 1.0f - m.pf;
+        for (int i = threadIdx.x; i < 16 * 17; i += blockDim.x) {
+            const int n = i / 17;
+            const float tot = (float)max(i % 17, 1);
+            const float ratio = (float)n / tot, r1 = (float)(n + 1) / tot;
+            ed.x[i] = qf * (1.0f - ratio);
+            ed.y[i] = qf * r1;
         }
-        __syncwarp();
+    }
+    __syncthreads();
+    const int T = m.T;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    uint32_t* code = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(&ed) +
+                                                 ((sizeof(DenseEdman) + 15) & ~(size_t)15));
+    unsigned char* wbase = reinterpret_cast<unsigned char*>(code + WP_DENSE_WARPS * WP_MAX_TIMESTEPS);
+    for (int phase = 0; phase < 2; phase++) {
+        const int S_cap = phase == 0 ? ps.S_small : ps.S_cap;
+        if (phase == 1) {
+            if (ps.big_warps == 0) break;
+            __syncthreads();  // the small slabs are done with
+            if (warp >= ps.big_warps) break;
+        }
+        float* fb = reinterpret_cast<float*>(wbase + wp_warp_bytes(T, S_cap, C, HAS_BLOCK) * warp);
+        const size_t slab = (size_t)T * S_cap;
+        WarpBufs wb;
+        wb.code = code + warp * WP_MAX_TIMESTEPS;
+        wb.X = fb;
+        wb.XB = HAS_BLOCK ? fb + slab : nullptr;
+        wb.em = fb + (HAS_BLOCK ? 2 : 1) * slab;
+        wb.coord = reinterpret_cast<uint16_t*>(wb.em + S_cap);
+        wb.fib = wb.coord + S_cap;
+        int* head = phase == 0 ? a.ovf_head : a.ovf_head2;
+        for (;;) {
+            int idx = 0;
+            if (lane == 0) idx = atomicAdd(head, 1);
+            idx = __shfl_sync(0xffffffffu, idx, 0);
+            if (idx >= count) break;
+            const int2 rg = a.ovf[idx];
+            int vmax;
+            const PeptideRec& pep = a.peps[slot_pep(a, rg.x, item_slot(a, rg, &vmax))];
+            int S = 1;
+            for (int c = 0; c < C; c++) S *= pep.D[c] + 1;
+            if (ps.big_warps > 0 && (S > ps.S_small) != (phase == 1)) continue;
+            float mant;
+            int ex;
+            pair_forward<C, HAS_BLOCK>(a, M, ed, rg.x, m, pep, wb, S_cap, lane, &mant, &ex, a.err);
+            if (lane == 0) {
+                a.res_mant[rg.y] = mant;
+                a.res_expo[rg.y] = ex;
+            }
+            __syncwarp();
+        }
     }
 }
 
-size_t wp_dense_smem_bytes(int T, int S_cap, int C, bool has_block, int warps) {
-    return ((sizeof(SmemModel) + 15) & ~(size_t)15) + wp_warp_bytes(T, S_cap, C, has_block) * warps;
+static size_t dense_fixed_bytes() {
+    return ((sizeof(SmemModel) + 15) & ~(size_t)15) + ((sizeof(DenseEdman) + 15) & ~(size_t)15) +
+           sizeof(uint32_t) * WP_DENSE_WARPS * WP_MAX_TIMESTEPS;
 }
 
-// Persistent grid of one CTA per SM (overflow pairs are few).
-cudaError_t wp_launch_dense(bool has_block, int threads, size_t smem, cudaStream_t stream,
-                            const BatchArgs& a) {
-    int dev = 0, sms = 0;
+// Whether the dense kernel takes pairs of S_cap states per slice.  The limit
+// (two copies of the state beside the model) is a property of the framework,
+// not of this kernel's layout: larger pairs are refused.
+bool wp_dense_fits(int T, int S_cap, int C, bool has_block, size_t smem_optin) {
+    const size_t state = (size_t)(has_block ? 2 : 1) * T * S_cap * sizeof(float);
+    return ((sizeof(SmemModel) + 15) & ~(size_t)15) + wp_warp_bytes(T, S_cap, C, has_block) + state <= smem_optin &&
+           dense_fixed_bytes() + wp_warp_bytes(T, S_cap, C, has_block) <= smem_optin;
+}
+
+template <int C, bool HAS_BLOCK>
+static cudaError_t launch_dense(int T, size_t smem_optin, cudaStream_t stream, const BatchArgs& a) {
+    // Small class: as many states as let 4 CTAs share an SM (228 KB, 1 KB of
+    // it per CTA the system's).
+    const size_t fixed = dense_fixed_bytes();
+    const size_t quarter = (size_t)228 * 1024 / 4 - 1024 - fixed;
+    DensePass ps;
+    ps.S_cap = a.dense_S_cap;
+    ps.S_small = ps.S_cap;
+    while (ps.S_small > 4 && wp_warp_bytes(T, ps.S_small, C, HAS_BLOCK) * WP_DENSE_WARPS > quarter) ps.S_small -= 4;
+    size_t arena = wp_warp_bytes(T, ps.S_small, C, HAS_BLOCK) * WP_DENSE_WARPS;
+    ps.big_warps = 0;
+    if (ps.S_small < ps.S_cap) {
+        const size_t big = wp_warp_bytes(T, ps.S_cap, C, HAS_BLOCK);
+        arena = std::max(arena, big);
+        ps.big_warps = (int)std::min<size_t>(arena / big, WP_DENSE_WARPS);
+    }
+    const size_t smem = fixed + arena;
+    if (smem > smem_optin) return cudaErrorInvalidConfiguration;
+    cudaError_t e = cudaFuncSetAttribute(wp_dense_kernel<C, HAS_BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
+    if (e != cudaSuccess) return e;
+    int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e;
-    if (has_block) {
-        e = cudaFuncSetAttribute(wp_dense_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        wp_dense_kernel<true><<<sms, threads, smem, stream>>>(a);
-    } else {
-        e = cudaFuncSetAttribute(wp_dense_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        wp_dense_kernel<false><<<sms, threads, smem, stream>>>(a);
-    }
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wp_dense_kernel<C, HAS_BLOCK>, WP_DENSE_WARPS * 32, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    wp_dense_kernel<C, HAS_BLOCK><<<sms * per_sm, WP_DENSE_WARPS * 32, smem, stream>>>(a, ps);
     return cudaGetLastError();
+}
+
+// Persistent grid over the dense list (BatchArgs::ovf).
+cudaError_t wp_launch_dense(bool has_block, int T, int C, size_t smem_optin, cudaStream_t stream,
+                            const BatchArgs& a) {
+    switch (C * 2 + (has_block ? 1 : 0)) {
+        case 2: return launch_dense<1, false>(T, smem_optin, stream, a);
+        case 3: return launch_dense<1, true>(T, smem_optin, stream, a);
+        case 4: return launch_dense<2, false>(T, smem_optin, stream, a);
+        case 5: return launch_dense<2, true>(T, smem_optin, stream, a);
+        case 6: return launch_dense<3, false>(T, smem_optin, stream, a);
+        case 7: return launch_dense<3, true>(T, smem_optin, stream, a);
+        case 8: return launch_dense<4, false>(T, smem_optin, stream, a);
+        case 9: return launch_dense<4, true>(T, smem_optin, stream, a);
+        default: return cudaErrorInvalidValue;
+    }
 }

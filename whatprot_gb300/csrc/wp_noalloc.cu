@@ -42,9 +42,9 @@ cudaError_t wp_launch_engine(int C, bool has_block, int threads, size_t smem, cu
                              int2* out, int* out_count, int slab_half, int scr_floats,
                              int spill_error, int* grid_out);
 size_t wp_engine_smem_bytes(int slab_half, int scr_floats, bool has_block, int threads);
-cudaError_t wp_launch_dense(bool has_block, int threads, size_t smem, cudaStream_t stream,
+cudaError_t wp_launch_dense(bool has_block, int T, int C, size_t smem_optin, cudaStream_t stream,
                             const BatchArgs& a);
-size_t wp_dense_smem_bytes(int T, int S_cap, int C, bool has_block, int warps);
+bool wp_dense_fits(int T, int S_cap, int C, bool has_block, size_t smem_optin);
 
 namespace {
 
@@ -206,6 +206,7 @@ extern "C" wp_status wp_hmm_classify_noalloc(int device, const wp_seq_model* m, 
     a.ovf = reinterpret_cast<int2*>(base + o_ovf2);
     a.ovf_count = cnt + 4;
     a.ovf_head = cnt + 5;
+    a.ovf_head2 = cnt + 6;
     a.err = reinterpret_cast<int*>(base + o_err);
     a.dense_S_cap = ((S_max + 31) / 32) * 32;
     const bool hb = hm.has_block != 0;
@@ -228,12 +229,7 @@ extern "C" wp_status wp_hmm_classify_noalloc(int device, const wp_seq_model* m, 
     };
     const int half1 = half_for(256, 2), half2 = half_for(128, 1);
     if (half1 < 4 || half2 < 4) return WP_ERR_UNSUPPORTED;
-    int dense_warps = 0;
-    for (int w = 16; w >= 1; w--)
-        if (wp_dense_smem_bytes(T, a.dense_S_cap, C, hb, w) <= smem_optin) {
-            dense_warps = w;
-            break;
-        }
+    const bool dense = wp_dense_fits(T, a.dense_S_cap, C, hb, smem_optin);
     // the compaction sends each pair to the first pass whose slab holds it
     a.n_tiers = half2 > half1 ? 2 : 1;
     a.tier_half[0] = half1;
@@ -242,7 +238,7 @@ extern "C" wp_status wp_hmm_classify_noalloc(int device, const wp_seq_model* m, 
     a.tier_half[1] = half2;
     a.tier_list[1] = reinterpret_cast<int2*>(base + o_ovf1);
     a.tier_count[1] = cnt + 2;
-    a.route_dense = dense_warps > 0 ? 1 : 0;
+    a.route_dense = dense ? 1 : 0;
     wp_compact_kernel<<<R, 256, 0, s>>>(a);
     WP_NA(cudaGetLastError());
     WP_NA(wp_launch_engine(C, hb, 256, wp_engine_smem_bytes(half1, 0, hb, 256), s, a, a.work, cnt + 0,
@@ -250,9 +246,8 @@ extern "C" wp_status wp_hmm_classify_noalloc(int device, const wp_seq_model* m, 
     WP_NA(wp_launch_engine(C, hb, 128, wp_engine_smem_bytes(half2, 0, hb, 128), s, a,
                            reinterpret_cast<int2*>(base + o_ovf1), cnt + 2, cnt + 3,
                            reinterpret_cast<int2*>(base + o_ovf2), cnt + 4, half2, 0,
-                           dense_warps == 0 ? 1 : 0, nullptr));
-    if (dense_warps > 0)
-        WP_NA(wp_launch_dense(hb, dense_warps * 32, wp_dense_smem_bytes(T, a.dense_S_cap, C, hb, dense_warps), s, a));
+                           dense ? 0 : 1, nullptr));
+    if (dense) WP_NA(wp_launch_dense(hb, T, C, smem_optin, s, a));
     wp_reduce_kernel<<<(R + 3) / 4, 128, 0, s>>>(a, reinterpret_cast<int32_t*>(base + o_id),
                                                  reinterpret_cast<double*>(base + o_sc),
                                                  reinterpret_cast<double*>(base + o_tot), nullptr,
