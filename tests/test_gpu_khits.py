@@ -42,6 +42,7 @@ CASES = [
     (9, 3, 5, 2500, -1, 0.3),       # k = all hits
     (8, 2, 4, 2000, 150, 0.0),      # whole-number reads: equal distances
     (16, 3, 5, 20000, 4000, 0.02),  # reads almost on a track
+    (16, 3, 5, 40000, 15000, 0.4),  # many groups looked into, by several warps
     (4, 2, 15, 900, 60, 3.0),       # reads far from every track
 ]
 

@@ -1096,7 +1096,7 @@ wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int q0, int n, int slice_l
     const int wpc = wp_khits_warps_per_cta();
     const int per_sm = std::max(1, std::min(4, (int)((size_t)(228 * 1024) / (smem + 1024))));
     long long grid = std::min<long long>((long long)sms * per_sm, (n + wpc - 1) / wpc);
-    const size_t per_warp = (size_t)a.cap * 24 + (size_t)wp_khits_groups() * 40 + (size_t)wp_khits_rank() * 20;
+    const size_t per_warp = (size_t)a.cap * 24 + (size_t)wp_khits_groups() * 56 + (size_t)wp_khits_rank() * 20;
     grid = std::max<long long>(1, std::min<long long>(grid, (long long)((6ull << 30) / (per_warp * wpc))));
     const size_t warps = (size_t)grid * wpc, list = a.cap * warps;
     WP_CUDA(ctx->d_kh_ent.ensure(sizeof(int2) * list), "alloc kNN lists");
@@ -1104,7 +1104,7 @@ wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int q0, int n, int slice_l
     WP_CUDA(ctx->d_kh_bin.ensure(sizeof(uint16_t) * list), "alloc kNN lists");
     WP_CUDA(ctx->d_kh_order.ensure(sizeof(int2) * list), "alloc kNN lists");
     WP_CUDA(ctx->d_kh_rank.ensure(sizeof(uint16_t) * list), "alloc kNN lists");
-    WP_CUDA(ctx->d_kh_state.ensure(sizeof(int4) * 2 * wp_khits_groups() * warps), "alloc kNN lists");
+    WP_CUDA(ctx->d_kh_state.ensure(sizeof(int4) * 3 * wp_khits_groups() * warps), "alloc kNN lists");
     WP_CUDA(ctx->d_kh_seg.ensure(sizeof(int2) * wp_khits_groups() * warps), "alloc kNN lists");
     WP_CUDA(ctx->d_kh_memd.ensure(sizeof(long long) * wp_khits_rank() * warps), "alloc kNN lists");
     WP_CUDA(ctx->d_kh_memk.ensure(sizeof(unsigned) * wp_khits_rank() * warps), "alloc kNN lists");

@@ -28,8 +28,11 @@
 //      entries and moves one group down and some places up the list together
 //      (each step passes entries once, 32 at a time), which gives n between
 //      the groups and, per group, an upper bound for the levels inside it,
-//   3. looks inside the few groups whose bound exceeds the maximum found
-//      (their entries ranked by FP64 distance), and
+//   3. looks inside the groups whose bound exceeds the maximum found, those with
+//      the largest bounds first (their entries ranked by FP64 distance, a lane per
+//      level of a block of up to 64), the CTA's warps that are between reads
+//      helping: groups do not depend on one another, and one read can have 280 of
+//      them where the mean is 30, and
 //   4. ranks the bin that holds the M-th nearest entry, KBest's final top, and
 //      writes the read's candidate list as the brute-force passes would (wp_nn.cu:
 //      the entries up to the end of the top's distance bin, in tree order, by
@@ -49,14 +52,20 @@
 // 8-bit integer dot products (dp4a); the rounding is covered by a margin of
 // TC (NC - 1) steps.
 //
-// Bound by the latency of one read's walk and by L2 bandwidth (3.5 KB per 128
-// entries screened; 450,000 of 946,000 entries screened and 25,000 listed per
-// read at k = 10,000).  4,000 reads against 946,000 tracks, k = 10,000: 36 ms,
-// against 132 ms for the replay (20,000 pushes per read, one at a time, and
-// its table look-ups of 48 coordinates for every entry met) and 41 ms for the
-// brute-force passes that then collected the entries (the list holds them
-// all); 2,000 reads against 70,000 tracks, k = 1,000: 1.1 ms against 4.1 and
-// 4.0 ms.
+// Bound by the latency of a read's chain of instructions: 16 warps per SM (128
+// registers each) issue one every 7 to 9 cycles, with L2 at 4 % of its peak
+// (3,700 tiles of 128 entries screened, 25,000 of 470,000 entries listed per read
+// at k = 10,000: 57 % of the cycles in the walk, 10 % in the groups).  4,000 reads
+// against 946,000 tracks, k = 10,000: 27 ms, 36 with each group's levels followed
+// one by one by the read's own warp (the slowest read's groups alone took 27),
+// against 132 ms for the replay (20,000 pushes per read, one at a time, and its
+// table look-ups of 48 coordinates for every entry met) and 41 ms for the
+// brute-force passes that then collected the entries (the list holds them all);
+// 2,000 reads against 70,000 tracks, k = 1,000: 0.83 ms against 4.1 and 4.0 ms.
+// Tried and left out: integer sums in place of the FP64 ones in the groups, no
+// faster (39.9 against 41.4 ms for the whole call); warps that start from the
+// reads with the fewest dyes so as to help sooner, 1.55 against 1.67 ms in the
+// second case and 43.6 against 39.9 in the first.
 #include <cuda_runtime.h>
 #include <float.h>
 #include <math.h>
@@ -71,6 +80,7 @@
 #define KH_EPS 2e-6f   // bound of the FP32 distances' relative error (27 roundings, all terms >= 0)
 #define KH_GRP 96      // entries per group of bins, about
 #define KH_MAXG 1024   // groups
+#define KH_WAIT 4000000  // most turns of a wait (0.2 to 1 us each)
 
 struct KHSmem {
     unsigned cnt[KH_NB];   // entries per bin
@@ -88,6 +98,7 @@ struct KHList {
     uint16_t* rank;   // within a ranked group: the entry's place, farthest first
     int4* state;      // per group: pointer state above it, bound inside it
     int4* group;      // per group: lowest and highest bin, first place and end in `order`
+    int* pick;        // the groups to look into, those with the largest bounds first
     long long* mem_d; // a ranked group's FP64 distances (as bits: they order alike)
     unsigned* mem_k;  // the same relative to the nearest, in 32 bits
     int2* sorted;     // its (list index, hits), farthest first
@@ -259,8 +270,249 @@ __device__ __forceinline__ bool kh_rank(const KHList& L, int lane, int m, F f) {
     return false;
 }
 
+// The list of warp gw of the grid, with the scratch of warp own.
+__device__ __forceinline__ KHList kh_list(const KHArgs& a, long gw, long own) {
+    KHList L;
+    L.ent = a.ent + gw * a.cap;
+    L.d = a.d + gw * a.cap;
+    L.bin = a.bin + gw * a.cap;
+    L.order = a.order + gw * a.cap;
+    L.rank = a.rank + gw * a.cap;
+    L.state = a.state + gw * 3 * KH_MAXG;
+    L.group = L.state + KH_MAXG;
+    L.pick = reinterpret_cast<int*>(L.state + 2 * KH_MAXG);
+    L.mem_d = a.mem_d + own * KH_RANK;
+    L.mem_k = a.mem_k + own * KH_RANK;
+    L.sorted = a.sorted + own * KH_RANK;
+    L.n = 0;
+    return L;
+}
+
+// Looks inside group g of warp gw's list of n (its levels' n, from the state
+// above it): the larger of M and the largest found, or minus a fatal code.
 template <int DP>
-__global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
+__device__ __noinline__ int kh_group(const KHArgs& a, long gw, long own, int n, int lane, int g, int tf, int k,
+                                     const double* sq64, int M) {
+    KHList L = kh_list(a, gw, own);
+    L.n = n;
+    const int4 st = L.state[g];
+    int fatal = 0;
+    KHWindow win = {-64, 0, 0, 0};
+    const int4 gr = L.group[g];
+    const int m = gr.w - gr.z;
+    if (m > KH_RANK) return -5;
+    // the group by FP32 distance (equal ones in any order)
+    for (int j = lane; j < m; j += 32)
+        L.mem_d[j] = ((long long)__float_as_uint(L.d[L.order[gr.z + j].x]) << 11) | j;
+    __syncwarp();
+    kh_rank(L, lane, m, [&](int j, int place) {
+        const int2 x = L.order[gr.z + j];
+        L.sorted[place] = x;
+        L.rank[x.x] = (uint16_t)place;
+    });
+    __syncwarp();
+    int Tx = st.x, cx = st.y, Hx = st.z;
+    // blocks of up to 32 levels, cut where neighbours differ by more
+    // than the FP32 error: n between the blocks and a bound inside,
+    // as for the groups
+    for (int j0 = 0; j0 < m && !fatal;) {
+        int2 x[2];
+        int len = 0;
+        {
+            float d[2];
+            unsigned cut[2];
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int j = j0 + 32 * u + lane;
+                x[u] = j < m ? L.sorted[j] : make_int2(0x7fffffff, 0);
+                d[u] = j < m ? L.d[x[u].x] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                // the cut after this entry
+                const int j = j0 + 32 * u + lane;
+                const float next = u == 0 ? __shfl_sync(0xffffffffu, lane == 0 ? d[1] : d[0], (lane + 1) & 31)
+                                          : __shfl_down_sync(0xffffffffu, d[1], 1);
+                cut[u] = __ballot_sync(0xffffffffu, j == m - 1 || (j < m - 1 && (u == 0 || lane < 31) &&
+                                                                   d[u] * (1.f - KH_EPS) > next * (1.f + KH_EPS)));
+            }
+            len = cut[0] ? 32 - __clz(cut[0]) : (cut[1] ? 32 + __ffs(cut[1]) : 0);
+        }
+        if (len == 0) {
+            fatal = 9;
+            break;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+            if (32 * u + lane >= len) x[u] = make_int2(0x7fffffff, 0);
+        const unsigned gone = kh_sum((x[0].x < Tx ? 1u : 0u) + (x[1].x < Tx ? 1u : 0u));
+        int T1 = Tx, c1 = cx - (int)gone,
+            H1 = Hx - (int)kh_sum((x[0].x < Tx ? (unsigned)x[0].y : 0u) + (x[1].x < Tx ? (unsigned)x[1].y : 0u));
+        const bool reached = kh_advance(L, win, lane, gr.x, gr.y, j0 + len - 1, k, T1, c1, H1);
+        const int lim = reached ? T1 - 1 : n;
+        const int lt = (int)kh_sum((x[0].x < lim ? 1u : 0u) + (x[1].x < lim ? 1u : 0u));
+        const int bound = !reached ? c1 + lt + 1 : (T1 > tf ? c1 + lt : -1);
+        if (bound > M) {
+            // level by level, by FP64 distance, a lane per level (two of them if
+            // the block has more than 32).  A level's own entry and the farther
+            // ones of the block are out.  The distances as 31-bit keys (the bits
+            // below their common range, plus 1); only if two of those are equal
+            // are the full 64 bits ranked.
+            long long dd[2] = {0, 0};
+            unsigned key[2] = {0u, 0u};
+            {
+                long long lo = 0x7fffffffffffffffll, hi = 0;
+#pragma unroll
+                for (int u = 0; u < 2; u++)
+                    if (32 * u + lane < len) {
+                        dd[u] = __double_as_longlong(kh_d64<DP>(a.cnt, L.ent[x[u].x].x, sq64, a.NC, a.TC));
+                        lo = min(lo, dd[u]);
+                        hi = max(hi, dd[u]);
+                    }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+                }
+                const int sh = max(0, 33 - __clzll(hi - lo));
+#pragma unroll
+                for (int u = 0; u < 2; u++)
+                    if (32 * u + lane < len) key[u] = (unsigned)((dd[u] - lo) >> sh) + 1u;
+            }
+            // the state at each level's start: what the block loses to it taken out
+            int Hl[2], cl[2], Tl[2];
+            bool need[2];
+            for (int wide = 0; wide < 2; wide++) {
+                unsigned gone_h[2] = {0u, 0u}, gone_c[2] = {0u, 0u}, same = 0u;
+                const int in0 = x[0].x < Tx ? x[0].y : -1, in1 = x[1].x < Tx ? x[1].y : -1;
+                for (int v = 0; v < len; v++) {
+                    const unsigned kv = __shfl_sync(0xffffffffu, v < 32 ? key[0] : key[1], v & 31);
+                    const int hv = __shfl_sync(0xffffffffu, v < 32 ? in0 : in1, v & 31);
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        const bool out = kv >= key[u];
+                        same += kv == key[u] ? 1u : 0u;
+                        if (out && hv >= 0) {
+                            gone_h[u] += (unsigned)hv;
+                            gone_c[u]++;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    Hl[u] = Hx - (int)gone_h[u];
+                    cl[u] = cx - (int)gone_c[u];
+                    Tl[u] = Tx;
+                    need[u] = 32 * u + lane < len && Hl[u] < k;
+                }
+                // each key meets itself and no other (a lane without a level has key
+                // 0, no level has)
+                if (kh_sum(same) == (unsigned)len) break;
+                if (wide) {
+                    fatal = 6;
+                    break;
+                }
+                // equal keys: the ranks of the full distances in their place
+                unsigned nearer[2] = {0u, 0u};
+                for (int v = 0; v < len; v++) {
+                    const long long dv = __shfl_sync(0xffffffffu, v < 32 ? dd[0] : dd[1], v & 31);
+#pragma unroll
+                    for (int u = 0; u < 2; u++) nearer[u] += dv < dd[u] ? 1u : 0u;
+                }
+#pragma unroll
+                for (int u = 0; u < 2; u++)
+                    if (32 * u + lane < len) key[u] = nearer[u] + 1u;
+            }
+            if (fatal) break;
+            // the list from Tx until each level's hits reach k again, all levels
+            // together: an entry nearer than the block counts for all of them (key 0),
+            // one of the block for the levels farther than it
+            const int end = reached ? T1 : n;
+            for (int i0 = Tx & ~31; i0 < end; i0 += 32) {
+                const int i = i0 + lane;
+                int place = -1, h = 0;
+                if (i >= Tx && i < end) {
+                    const int bi = L.bin[i];
+                    if (bi < gr.x) {
+                        place = 64;
+                    } else if (bi <= gr.y) {
+                        const int rk = (int)L.rank[i] - j0;
+                        place = rk < 0 ? -1 : (rk < len ? rk : 64);
+                    }
+                    if (place >= 0) h = L.ent[i].y;
+                }
+                unsigned ke = __shfl_sync(0xffffffffu, key[0], place & 31);
+                const unsigned k1 = __shfl_sync(0xffffffffu, key[1], place & 31);
+                if (place >= 32) ke = place == 64 ? 0u : k1;
+                unsigned todo = __ballot_sync(0xffffffffu, place >= 0);
+                while (todo) {
+                    const int l = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    const unsigned kv = __shfl_sync(0xffffffffu, ke, l);
+                    const int hl = __shfl_sync(0xffffffffu, h, l);
+#pragma unroll
+                    for (int u = 0; u < 2; u++)
+                        if (need[u] && kv < key[u]) {
+                            Hl[u] += hl;
+                            cl[u]++;
+                            if (Hl[u] >= k) {
+                                need[u] = false;
+                                Tl[u] = i0 + l + 1;
+                            }
+                        }
+                }
+                if (!__any_sync(0xffffffffu, need[0] || need[1])) break;
+            }
+            int most = -1;
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+                if (32 * u + lane < len) most = max(most, need[u] ? cl[u] + 1 : (Tl[u] > tf ? cl[u] : -1));
+            M = max(M, __reduce_max_sync(0xffffffffu, most));
+        }
+        if (!reached) break;
+        if (T1 > tf) M = max(M, c1);
+        Tx = T1;
+        cx = c1;
+        Hx = H1;
+        j0 += len;
+    }
+    return fatal ? -fatal : M;
+}
+
+// One warp's groups, for the CTA's warps to take (kh_help).
+struct KHShare {
+    int open;   // groups can be taken
+    int busy;   // other warps looking or at work
+    int np, next, fatal, M, tf, n;
+};
+
+// Takes groups of the read that sh describes (its list is warp gw's) until none
+// is left; own: the calling warp, for its scratch.
+template <int DP>
+__device__ __forceinline__ void kh_help(const KHArgs& a, long own, int lane, KHShare* sh, long gw,
+                                        const double* sq64, int k) {
+    const int* pick = reinterpret_cast<const int*>(a.state + gw * 3 * KH_MAXG + 2 * KH_MAXG);
+    const int np = *(volatile int*)&sh->np, tf = *(volatile int*)&sh->tf, n = *(volatile int*)&sh->n;
+    for (;;) {
+        int g = 0;
+        if (lane == 0) g = atomicAdd(&sh->next, 1);
+        g = __shfl_sync(0xffffffffu, g, 0);
+        if (g >= np) break;
+        const int M = __shfl_sync(0xffffffffu, *(volatile int*)&sh->M, 0);
+        g = pick[g];
+        if (a.state[gw * 3 * KH_MAXG + g].w <= M) break;  // nor do the rest exceed it
+        const int found = kh_group<DP>(a, gw, own, n, lane, g, tf, k, sq64, M);
+        if (lane == 0) {
+            if (found > M) atomicMax(&sh->M, found);
+            if (found < 0) atomicMax(&sh->fatal, -found);
+        }
+        __syncwarp();
+        if (found < 0) break;
+    }
+}
+
+template <int DP>
+__global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(const __grid_constant__ KHArgs a) {
     extern __shared__ __align__(16) unsigned char kh_smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const unsigned below = (1u << lane) - 1u;
@@ -273,21 +525,44 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
     double* s_plane = reinterpret_cast<double*>(mine + sizeof(KHSmem) + tab_bytes);
     int* s_node = reinterpret_cast<int*>(s_plane + a.stack_cap);
     const long gw = (long)blockIdx.x * KH_WARPS + wib;
-    KHList L;
-    L.ent = a.ent + gw * a.cap;
-    L.d = a.d + gw * a.cap;
-    L.bin = a.bin + gw * a.cap;
-    L.order = a.order + gw * a.cap;
-    L.rank = a.rank + gw * a.cap;
-    L.state = a.state + gw * 2 * KH_MAXG;
-    L.group = L.state + KH_MAXG;
-    L.mem_d = a.mem_d + gw * KH_RANK;
-    L.mem_k = a.mem_k + gw * KH_RANK;
-    L.sorted = a.sorted + gw * KH_RANK;
+    KHList L = kh_list(a, gw, gw);
+    __shared__ KHShare share[KH_WARPS];
+    __shared__ int leaving;  // warps without further reads
+    KHShare* const sh = share + wib;
+    if (lane == 0) {
+        sh->open = sh->busy = 0;
+        if (wib == 0) leaving = 0;
+    }
+    __syncthreads();
     int2* seg = a.seg + gw * KH_MAXG;
     const int k = (int)a.k;
 
+    // helps the CTA's other warps with the groups they have left
+    auto help = [&]() {
+        for (int v = 1; v < KH_WARPS; v++) {
+            const int o = (wib + v) % KH_WARPS;
+            KHShare* const so = share + o;
+            int go = 0;
+            if (lane == 0 && *(volatile int*)&so->open) {
+                atomicAdd(&so->busy, 1);
+                __threadfence_block();
+                go = *(volatile int*)&so->open;
+                if (!go) atomicSub(&so->busy, 1);
+            }
+            if (!__shfl_sync(0xffffffffu, go, 0)) continue;
+            __threadfence_block();
+            kh_help<DP>(a, gw, lane, so, gw - wib + o,
+                        reinterpret_cast<const double*>(kh_smem + (sizeof(KHSmem) + tab_bytes + stack_bytes) * o +
+                                                        sizeof(KHSmem)),
+                        k);
+            __threadfence_block();
+            __syncwarp();
+            if (lane == 0) atomicSub(&so->busy, 1);
+        }
+    };
+
     for (;;) {
+        help();
         int slot = 0;
         if (lane == 0) slot = atomicAdd(a.next, 1);
         slot = __shfl_sync(0xffffffffu, slot, 0);
@@ -670,113 +945,59 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
                 e = start;
             }
             __syncwarp();
-            // ---- 3. the groups whose bound exceeds the maximum
-            for (int g = 0; g < ng && !fatal; g++) {
-                const int4 st = L.state[g];
-                if (st.w <= M) continue;
-                const int4 gr = L.group[g];
-                const int m = gr.w - gr.z;
-                if (m > KH_RANK) {
-                    fatal = 5;
-                    break;
+            // ---- 3. the groups whose bound exceeds the maximum, those with the
+            // largest bounds first (they raise the maximum past most others' bounds),
+            // with the CTA's other warps
+            int np = 0;
+            for (int g0 = 0; g0 < ng; g0 += 32) {
+                const int bound = g0 + lane < ng ? L.state[g0 + lane].w : -1;
+                const unsigned in = __ballot_sync(0xffffffffu, bound > M);
+                if (bound > M) {
+                    L.mem_k[np + __popc(in & below)] = (unsigned)bound;
+                    L.sorted[np + __popc(in & below)].x = g0 + lane;
                 }
-                // the group by FP32 distance (equal ones in any order)
-                for (int j = lane; j < m; j += 32)
-                    L.mem_d[j] = ((long long)__float_as_uint(L.d[L.order[gr.z + j].x]) << 11) | j;
-                __syncwarp();
-                kh_rank(L, lane, m, [&](int j, int place) {
-                    const int2 x = L.order[gr.z + j];
-                    L.sorted[place] = x;
-                    L.rank[x.x] = (uint16_t)place;
-                });
-                __syncwarp();
-                int Tx = st.x, cx = st.y, Hx = st.z;
-                win.base = -64;
-                // blocks of up to 32 levels, cut where neighbours differ by more
-                // than the FP32 error: n between the blocks and a bound inside,
-                // as for the groups
-                for (int j0 = 0; j0 < m && !fatal;) {
-                    int2 x[2];
-                    int len = 0;
-                    {
-                        float d[2];
-                        unsigned cut[2];
-#pragma unroll
-                        for (int u = 0; u < 2; u++) {
-                            const int j = j0 + 32 * u + lane;
-                            x[u] = j < m ? L.sorted[j] : make_int2(0x7fffffff, 0);
-                            d[u] = j < m ? L.d[x[u].x] : 0.f;
-                        }
-#pragma unroll
-                        for (int u = 0; u < 2; u++) {
-                            // the cut after this entry
-                            const int j = j0 + 32 * u + lane;
-                            const float next = u == 0 ? __shfl_sync(0xffffffffu, lane == 0 ? d[1] : d[0], (lane + 1) & 31)
-                                                      : __shfl_down_sync(0xffffffffu, d[1], 1);
-                            cut[u] = __ballot_sync(0xffffffffu, j == m - 1 || (j < m - 1 && (u == 0 || lane < 31) &&
-                                                                               d[u] * (1.f - KH_EPS) > next * (1.f + KH_EPS)));
-                        }
-                        len = cut[0] ? 32 - __clz(cut[0]) : (cut[1] ? 32 + __ffs(cut[1]) : 0);
-                    }
-                    if (len == 0) {
-                        fatal = 9;
-                        break;
-                    }
-#pragma unroll
-                    for (int u = 0; u < 2; u++)
-                        if (32 * u + lane >= len) x[u] = make_int2(0x7fffffff, 0);
-                    const unsigned gone = kh_sum((x[0].x < Tx ? 1u : 0u) + (x[1].x < Tx ? 1u : 0u));
-                    int T1 = Tx, c1 = cx - (int)gone,
-                        H1 = Hx - (int)kh_sum((x[0].x < Tx ? (unsigned)x[0].y : 0u) + (x[1].x < Tx ? (unsigned)x[1].y : 0u));
-                    const bool reached = kh_advance(L, win, lane, gr.x, gr.y, j0 + len - 1, k, T1, c1, H1);
-                    const int lim = reached ? T1 - 1 : n;
-                    const int lt = (int)kh_sum((x[0].x < lim ? 1u : 0u) + (x[1].x < lim ? 1u : 0u));
-                    const int bound = !reached ? c1 + lt + 1 : (T1 > tf ? c1 + lt : -1);
-                    if (bound > M) {
-                        // level by level, by FP64 distance; entries that T has not
-                        // passed change nothing
-#pragma unroll
-                        for (int u = 0; u < 2; u++)
-                            if (32 * u + lane < len)
-                                L.mem_d[32 * u + lane] =
-                                    __double_as_longlong(kh_d64<DP>(a.cnt, L.ent[x[u].x].x, sq64, a.NC, a.TC));
-                        __syncwarp();
-                        const bool distinct = kh_rank(L, lane, len, [&](int j, int place) {
-                            const int2 y = j < 32 ? x[0] : x[1];
-                            L.sorted[j0 + place] = y;
-                            L.rank[y.x] = (uint16_t)(j0 + place);
-                        });
-                        if (!distinct) {
-                            fatal = 6;
-                            break;
-                        }
-                        __syncwarp();
-#pragma unroll
-                        for (int u = 0; u < 2; u++)
-                            if (32 * u + lane < len) x[u] = L.sorted[j0 + 32 * u + lane];
-                        win.base = -64;
-                        bool on = true;
-                        for (int u = 0; u < len && on; u++) {
-                            const unsigned long long in =
-                                (unsigned long long)__ballot_sync(0xffffffffu, x[0].x < Tx) |
-                                ((unsigned long long)__ballot_sync(0xffffffffu, x[1].x < Tx) << 32);
-                            if ((in >> u) == 0ull) break;
-                            u += __ffsll((long long)(in >> u)) - 1;
-                            cx--;
-                            Hx -= __shfl_sync(0xffffffffu, u < 32 ? x[0].y : x[1].y, u & 31);
-                            on = kh_advance(L, win, lane, gr.x, gr.y, j0 + u, k, Tx, cx, Hx);
-                            if (!on) M = max(M, cx + 1);
-                            else if (Tx > tf) M = max(M, cx);
-                        }
-                    }
-                    if (!reached) break;
-                    if (T1 > tf) M = max(M, c1);
-                    Tx = T1;
-                    cx = c1;
-                    Hx = H1;
-                    j0 += len;
-                }
+                np += __popc(in);
             }
+            __syncwarp();
+            for (int j = lane; j < np; j += 32) {
+                const unsigned mine_ = L.mem_k[j];
+                int place = 0;
+#pragma unroll 8
+                for (int v = 0; v < np; v++) {
+                    const unsigned o = L.mem_k[v];
+                    place += o > mine_ || (o == mine_ && v < j) ? 1 : 0;
+                }
+                L.pick[place] = L.sorted[j].x;
+            }
+            __syncwarp();
+            if (lane == 0) {
+                sh->np = np;
+                sh->next = 0;
+                sh->fatal = 0;
+                sh->M = M;
+                sh->tf = tf;
+                sh->n = n;
+                __threadfence_block();
+                *(volatile int*)&sh->open = 1;
+            }
+            __syncwarp();
+            kh_help<DP>(a, gw, lane, sh, gw, sq64, k);
+            if (lane == 0) {
+                *(volatile int*)&sh->open = 0;
+                __threadfence_block();
+                // helpers still in a group (bounded: each ends its group and leaves)
+                int wait = 0;
+                while (*(volatile int*)&sh->busy > 0 && wait < KH_WAIT) {
+                    __nanosleep(200);
+                    wait++;
+                }
+                if (wait == KH_WAIT) sh->fatal = 14;
+                __threadfence_block();
+            }
+            __syncwarp();
+            M = *(volatile int*)&sh->M;
+            fatal = max(fatal, *(volatile int*)&sh->fatal);
+            __syncwarp();
             // ---- 4. the M-th nearest entry
             if (!fatal) {
                 int b = -1;
@@ -904,6 +1125,16 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(KHArgs a) {
         }
         if (lane == 0) a.kept_n[slot] = fatal ? -1 : M;
         __syncwarp();
+    }
+    // no reads left: help until the CTA's other warps are through (or, past the
+    // limit, leave the rest to them)
+    if (lane == 0) atomicAdd(&leaving, 1);
+    for (int i = 0; i < KH_WAIT; i++) {
+        int left = 0;
+        if (lane == 0) left = *(volatile int*)&leaving;
+        if (__shfl_sync(0xffffffffu, left, 0) == KH_WARPS) break;
+        help();
+        __nanosleep(1000);
     }
 }
 
