@@ -19,10 +19,20 @@
 //                        accumulator's `full` mbarrier after the last K
 //                        slice; warp 1 also owns the TMEM allocation;
 //   warps 2-5            epilogue: each reads its 32 TMEM lanes (rows) in
-//                        32-column chunks with tcgen05.ld, stages them in
-//                        shared memory, stores rows contiguously, and frees
-//                        the accumulator (its `empty` mbarrier) for the
-//                        tile after next.
+//                        32-column chunks with tcgen05.ld (the next chunk's
+//                        load in flight), adds the bias (the tile's biases
+//                        fetched to shared memory ahead), and stores from
+//                        registers, a 32-byte sector of its row per lane and
+//                        store; the accumulator is freed (its `empty`
+//                        mbarrier) for the tile after next as soon as its
+//                        last chunk is in registers.
+// A tile's products at K = 1024 take 11,300 cycles, and the epilogue's 32,768
+// outputs must take no longer or they set the time.  Shared memory is what
+// they must stay off: the products keep it busy, and outputs staged through
+// it for stores of whole rows took 24,000 cycles a tile.  4,096 x 20,000 x
+// 1,024: BF16 output 171 -> 119 us, FP32 output 212 -> 154 (its 328 MB of
+// stores bound it: 109 without them); 4,096 x 1,024 x 64 with GELU and
+// pre-activation, 34 -> 18 us.
 // Every mbarrier wait is bounded; on expiry the CTA records an error code,
 // stops issuing work, waits (bounded) for what it issued and frees its TMEM.
 #include <cuda.h>
@@ -42,7 +52,6 @@
 #define GEMM_A_STAGE (GEMM_BM * GEMM_BK * 2)  // 16 KB
 #define GEMM_B_STAGE (GEMM_BN * GEMM_BK * 2)  // 32 KB
 #define GEMM_WAIT_LIMIT (1L << 22)
-#define GEMM_SROW 36  // floats per row of the epilogue staging tile (32 + 4: conflict-free float4)
 
 typedef __nv_bfloat16 bf16_t;
 
@@ -136,7 +145,7 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                  : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
+__device__ __forceinline__ void tmem_ld32_start(uint32_t taddr, uint32_t* r) {
     asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
             "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -147,10 +156,74 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
               "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
               "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
             : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// Waits for the loads started; the registers pass through, so that nothing
+// reads them earlier.
+__device__ __forceinline__ void tmem_ld32_wait(uint32_t* r) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
+                   "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
+                   "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]),
+                   "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
+                   "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]),
+                   "+r"(r[30]), "+r"(r[31])
+                 :
+                 : "memory");
 }
 
 __device__ __forceinline__ float gelu_erf(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
+
+// 32 bytes to a 32-byte boundary in one store: a whole sector per lane.
+__device__ __forceinline__ void store_32b(void* p, const uint32_t* u) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(u[0]), "r"(u[1]), "r"(u[2]),
+                 "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7])
+                 : "memory");
+}
+
+// A lane's 32 columns (the first `cols` of them) of one row.
+__device__ __forceinline__ void store_f32(float* d, const float* v, int cols) {
+    const int align = (int)(reinterpret_cast<uintptr_t>(d) & 31);
+    if (cols == 32 && align == 0) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+            uint32_t u[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) u[i] = __float_as_uint(v[j + i]);
+            store_32b(d + j, u);
+        }
+    } else if (cols == 32 && (align & 15) == 0) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(d + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            if (j < cols) d[j] = v[j];
+    }
+}
+
+__device__ __forceinline__ void store_bf16(bf16_t* d, const float* v, int cols) {
+    const int align = (int)(reinterpret_cast<uintptr_t>(d) & 31);
+    uint32_t u[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+        u[j] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    if (cols == 32 && align == 0) {
+        store_32b(d, u);
+        store_32b(d + 16, u + 8);
+    } else if (cols == 32 && (align & 15) == 0) {
+#pragma unroll
+        for (int j = 0; j < 16; j += 4)
+            *reinterpret_cast<uint4*>(d + 2 * j) = make_uint4(u[j], u[j + 1], u[j + 2], u[j + 3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            if (j < cols) d[j] = __ushort_as_bfloat16((unsigned short)((j & 1) ? u[j >> 1] >> 16 : u[j >> 1] & 0xffffu));
+    }
+}
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -159,8 +232,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // Persistent: CTA b takes tiles b, b + gridDim.x, ... (M blocks fastest, so
 // the CTAs running at once share B tiles in L2).  Two TMEM accumulators
 // (2 x 256 columns): the MMA thread fills one while the epilogue warps drain
-// the other.  Epilogue stores go through a per-warp shared-memory tile so
-// that global stores are row-contiguous.
+// the other.
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
         wp_gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                           GemmParams p) {
@@ -168,8 +240,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* sA = smem;
     uint8_t* sB = smem + GEMM_STAGES * GEMM_A_STAGE;
-    float* stage_out = reinterpret_cast<float*>(sB + GEMM_STAGES * GEMM_B_STAGE);  // [4 warps][32][GEMM_SROW]
-    uint64_t* full = reinterpret_cast<uint64_t*>(stage_out + 4 * 32 * GEMM_SROW);
+    float* bias_tile = reinterpret_cast<float*>(sB + GEMM_STAGES * GEMM_B_STAGE);  // [4 warps][GEMM_BN]
+    uint64_t* full = reinterpret_cast<uint64_t*>(bias_tile + 4 * GEMM_BN);
     uint64_t* empty = full + GEMM_STAGES;
     uint64_t* acc_full = empty + GEMM_STAGES;  // [2]
     uint64_t* acc_empty = acc_full + 2;        // [2]
@@ -263,104 +335,76 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     } else {
         // epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31
         const int q = warp & 3;
-        float* st = stage_out + q * 32 * GEMM_SROW;
+        float* sb = bias_tile + q * GEMM_BN;
         int li = 0;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x, li++) {
             const int b = li & 1, use = li >> 1;
             const int m0 = (t % mblocks) * GEMM_BM, n0 = (t / mblocks) * GEMM_BN;
+            const int rbase = m0 + 32 * q;
+            if (p.bias) {
+                // this tile's biases, while its products are formed
+                __syncwarp();
+                for (int j = lane; j < GEMM_BN; j += 32) sb[j] = n0 + j < p.N ? p.bias[n0 + j] : 0.0f;
+                __syncwarp();
+            }
             if (*abort_flag || !mbar_wait(&acc_full[b], use & 1, p.err, 103)) {
                 *abort_flag = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int rbase = m0 + 32 * q;
-            for (int ch = 0; ch < GEMM_BN / 32; ch++) {
-                uint32_t r[32];
-                tmem_ld32(tmem + (uint32_t)(b * GEMM_TMEM_COLS) + ((uint32_t)(32 * q) << 16) + (uint32_t)(ch * 32), r);
+            const int nch = rbase < p.M ? (min(GEMM_BN, p.N - n0) + 31) / 32 : 0;
+            const uint32_t tacc = tmem + (uint32_t)(b * GEMM_TMEM_COLS) + ((uint32_t)(32 * q) << 16);
+            // this accumulator may be refilled (after the last chunk is in registers)
+            auto release = [&]() {
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[b]);
+            };
+            // one chunk: a lane's 32 columns of its row, straight from registers
+            const int row = rbase + lane;
+            const bool live = row < p.M;
+            auto chunk = [&](const uint32_t* r, int ch) {
                 const int c0 = n0 + ch * 32;
-                if (c0 >= p.N || rbase >= p.M) continue;  // warp-uniform
+                const int cols = min(32, p.N - c0);
                 float v[32];
 #pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    float x = __uint_as_float(r[j]);
-                    if (p.bias) x += (c0 + j < p.N) ? p.bias[c0 + j] : 0.0f;
-                    v[j] = x;
+                for (int j = 0; j < 32; j += 4) {
+                    float4 bv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (p.bias) bv = *reinterpret_cast<const float4*>(sb + ch * 32 + j);
+                    const float w[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        v[j + u] = __uint_as_float(r[j + u]);
+                        if (p.bias) v[j + u] += w[u];
+                    }
                 }
-                // two passes through the staging tile: pre-activation, output
-                for (int pass = p.Z ? 0 : 1; pass < 2; pass++) {
-                    float o[32];
+                const long at = (long)row * p.ldc + c0;
+                if (p.Z && live) store_bf16(p.Z + at, v, cols);
+                if (p.act == 1) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++) o[j] = (pass == 1 && p.act == 1) ? gelu_erf(v[j]) : v[j];
-                    const bool f32 = pass == 1 && p.c_fp32;
-                    __syncwarp();
-                    if (f32) {
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4)
-                            *reinterpret_cast<float4*>(st + lane * GEMM_SROW + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
-                    } else {
-                        uint32_t* su = reinterpret_cast<uint32_t*>(st + lane * GEMM_SROW);
-#pragma unroll
-                        for (int j = 0; j < 16; j += 4) {
-                            uint4 u;
-                            __nv_bfloat162 h0 = __floats2bfloat162_rn(o[2 * j], o[2 * j + 1]);
-                            __nv_bfloat162 h1 = __floats2bfloat162_rn(o[2 * j + 2], o[2 * j + 3]);
-                            __nv_bfloat162 h2 = __floats2bfloat162_rn(o[2 * j + 4], o[2 * j + 5]);
-                            __nv_bfloat162 h3 = __floats2bfloat162_rn(o[2 * j + 6], o[2 * j + 7]);
-                            u.x = *reinterpret_cast<uint32_t*>(&h0);
-                            u.y = *reinterpret_cast<uint32_t*>(&h1);
-                            u.z = *reinterpret_cast<uint32_t*>(&h2);
-                            u.w = *reinterpret_cast<uint32_t*>(&h3);
-                            *reinterpret_cast<uint4*>(su + j) = u;
-                        }
-                    }
-                    __syncwarp();
-                    // row-contiguous stores: FP32 rows are 8 x 16 B (8 lanes
-                    // per row, 4 rows per pass), BF16 rows 4 x 16 B
-                    const bool full_cols = c0 + 32 <= p.N;
-                    if (f32) {
-                        float* C = reinterpret_cast<float*>(p.C);
-                        for (int i = 0; i < 8; i++) {
-                            const int rr = i * 4 + (lane >> 3), cc = (lane & 7) * 4;
-                            const int row = rbase + rr;
-                            if (row >= p.M) continue;
-                            const float4 val = *reinterpret_cast<const float4*>(st + rr * GEMM_SROW + cc);
-                            float* dst = C + (long)row * p.ldc + c0 + cc;
-                            if (full_cols && (p.ldc & 3) == 0) {
-                                *reinterpret_cast<float4*>(dst) = val;
-                            } else {
-                                const float e4[4] = {val.x, val.y, val.z, val.w};
-                                for (int j = 0; j < 4; j++)
-                                    if (c0 + cc + j < p.N) dst[j] = e4[j];
-                            }
-                        }
-                    } else {
-                        bf16_t* D = pass == 0 ? p.Z : reinterpret_cast<bf16_t*>(p.C);
-                        const uint32_t* su = reinterpret_cast<const uint32_t*>(st);
-                        for (int i = 0; i < 4; i++) {
-                            const int rr = i * 8 + (lane >> 2), cw = (lane & 3) * 4;  // 4 words = 8 BF16
-                            const int row = rbase + rr;
-                            if (row >= p.M) continue;
-                            const uint4 val = *reinterpret_cast<const uint4*>(su + rr * GEMM_SROW + cw);
-                            bf16_t* dst = D + (long)row * p.ldc + c0 + 2 * cw;
-                            if (full_cols && (p.ldc & 7) == 0) {
-                                *reinterpret_cast<uint4*>(dst) = val;
-                            } else {
-                                const uint32_t w4[4] = {val.x, val.y, val.z, val.w};
-                                for (int j = 0; j < 8; j++)
-                                    if (c0 + 2 * cw + j < p.N) {
-                                        const uint32_t wv = w4[j >> 1];
-                                        const unsigned short hv = (j & 1) ? (unsigned short)(wv >> 16) : (unsigned short)(wv & 0xffffu);
-                                        dst[j] = __ushort_as_bfloat16(hv);
-                                    }
-                            }
-                        }
-                    }
+                    for (int j = 0; j < 32; j++) v[j] = gelu_erf(v[j]);
+                }
+                if (live) {
+                    if (p.c_fp32) store_f32(reinterpret_cast<float*>(p.C) + at, v, cols);
+                    else store_bf16(reinterpret_cast<bf16_t*>(p.C) + at, v, cols);
+                }
+            };
+            // two register buffers: the next chunk's load runs under this one's stores
+            uint32_t r0[32], r1[32];
+            if (nch > 0) tmem_ld32_start(tacc, r0);
+            for (int ch = 0; ch < nch; ch += 2) {
+                tmem_ld32_wait(r0);
+                if (ch + 1 < nch) tmem_ld32_start(tacc + (uint32_t)(32 * (ch + 1)), r1);
+                else release();
+                chunk(r0, ch);
+                if (ch + 1 < nch) {
+                    tmem_ld32_wait(r1);
+                    if (ch + 2 < nch) tmem_ld32_start(tacc + (uint32_t)(32 * (ch + 2)), r0);
+                    else release();
+                    chunk(r1, ch + 1);
                 }
             }
-            // this accumulator may be refilled
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[b]);
+            if (nch == 0) release();
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -406,7 +450,7 @@ static bool make_map(CUtensorMap* map, const void* ptr, int rows, int K, int ld,
 }
 
 size_t wp_gemm_smem_bytes() {
-    return 1024 + GEMM_STAGES * (GEMM_A_STAGE + GEMM_B_STAGE) + 4 * 32 * GEMM_SROW * 4 + (2 * GEMM_STAGES + 5) * 8 + 16;
+    return 1024 + GEMM_STAGES * (GEMM_A_STAGE + GEMM_B_STAGE) + 4 * GEMM_BN * 4 + (2 * GEMM_STAGES + 5) * 8 + 16;
 }
 
 // C = act(A . B^T + bias).  A: [M][K] (pitch lda), B: [N][K] (pitch ldb),
