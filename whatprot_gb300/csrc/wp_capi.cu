@@ -89,8 +89,6 @@ cudaError_t wp_launch_dedup_range(const int16_t* c, size_t total, int* minmax, c
 cudaError_t wp_launch_dedup(const DedupArgs& a, cudaStream_t s, int* launches);
 #include <cuda_bf16.h>
 cudaError_t wp_mlp_launch_input(const float* xf, const double* xd, int B, int TC, __nv_bfloat16* X, cudaStream_t s);
-cudaError_t wp_mlp_launch_transpose(const __nv_bfloat16* in, int rows, int cols, int ld_in, __nv_bfloat16* out,
-                                    int ld_out, cudaStream_t s);
 cudaError_t wp_mlp_launch_colsum(const __nv_bfloat16* M, int rows, int cols, int ld, float* out, cudaStream_t s);
 cudaError_t wp_mlp_launch_softmax_ce(const float* logits, int B, int P, int ld, const int* labels, float scale,
                                      __nv_bfloat16* dL, double* loss, cudaStream_t s);
@@ -102,6 +100,9 @@ cudaError_t wp_mlp_launch_init(float* w, long rows, long cols, long valid_rows, 
                                cudaStream_t s);
 cudaError_t wp_mlp_launch_topk(const float* logits, int R, int P, int ld, int h, const int* counts, int* idx,
                                float* prob, double* mass, int* fail, cudaStream_t s);
+cudaError_t wp_gemm_bf16(const void* A, int lda, bool a_mn, const void* B, int ldb, bool b_mn, int M, int N, int K,
+                         void* C, int ldc, int c_fp32, const float* bias, int act, void* Z, int* err,
+                         cudaStream_t s);
 cudaError_t wp_gemm_bf16_tn(const void* A, int lda, const void* B, int ldb, int M, int N, int K, void* C, int ldc,
                             int c_fp32, const float* bias, int act, void* Z, int accumulate, int* err,
                             cudaStream_t s);
@@ -3067,8 +3068,8 @@ struct wp_mlp {
     // FP32: W1 b1 W2 b2 W3 b3, each with grad, Adam m, v
     DevBuf w[6], g[6], m[6], v[6];
     long n[6] = {0, 0, 0, 0, 0, 0};
-    DevBuf W1b, W2b, W3b, W2T, W3T;  // BF16 copies
-    DevBuf X, XT, Z1, H1, H1T, Z2, H2, H2T, dL, dLT, dZ2, dZ2T, dZ1, dZ1T, L, dH2, dH1, loss, labels, xsim, err;
+    DevBuf W1b, W2b, W3b;  // BF16 copies
+    DevBuf X, Z1, H1, Z2, H2, dL, dZ2, dZ1, L, dH2, dH1, loss, labels, xsim, err;
     DevBuf topi, topp, mass, counts, loss_sum, tkfail;
 };
 
@@ -3082,10 +3083,11 @@ typedef __nv_bfloat16 bf16;
         if (_e != cudaSuccess) return cuda_fail(ctx, _e, what); \
     } while (0)
 
-wp_status mlp_gemm(wp_ctx* ctx, wp_mlp* m, const void* A, int lda, const void* B, int ldb, int M, int N, int K,
-                   void* C, int ldc, int c_fp32, const float* bias, int act, void* Z) {
-    cudaError_t e = wp_gemm_bf16_tn(A, lda, B, ldb, M, N, K, C, ldc, c_fp32, bias, act, Z, 0, m->err.as<int>(),
-                                    ctx->stream);
+// a_mn, b_mn: the operand is stored with K as its rows (wp_gemm_bf16).
+wp_status mlp_gemm(wp_ctx* ctx, wp_mlp* m, const void* A, int lda, bool a_mn, const void* B, int ldb, bool b_mn,
+                   int M, int N, int K, void* C, int ldc, int c_fp32, const float* bias, int act, void* Z) {
+    cudaError_t e = wp_gemm_bf16(A, lda, a_mn, B, ldb, b_mn, M, N, K, C, ldc, c_fp32, bias, act, Z,
+                                 m->err.as<int>(), ctx->stream);
     ctx->launches++;
     if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor-core GEMM launch");
     return WP_OK;
@@ -3095,11 +3097,9 @@ wp_status mlp_ensure(wp_ctx* ctx, wp_mlp* m, int B) {
     if (B <= m->cap) return WP_OK;
     const size_t b = (size_t)B, H = m->H, Pp = m->Ppad;
     MLP_CUDA(m->X.ensure(sizeof(bf16) * b * 64), "alloc");
-    MLP_CUDA(m->XT.ensure(sizeof(bf16) * b * 64), "alloc");
-    for (DevBuf* d : {&m->Z1, &m->H1, &m->H1T, &m->Z2, &m->H2, &m->H2T, &m->dZ2, &m->dZ2T, &m->dZ1, &m->dZ1T})
+    for (DevBuf* d : {&m->Z1, &m->H1, &m->Z2, &m->H2, &m->dZ2, &m->dZ1})
         MLP_CUDA(d->ensure(sizeof(bf16) * b * H), "alloc activations");
     MLP_CUDA(m->dL.ensure(sizeof(bf16) * b * Pp), "alloc logits gradient");
-    MLP_CUDA(m->dLT.ensure(sizeof(bf16) * b * Pp), "alloc logits gradient");
     MLP_CUDA(m->L.ensure(sizeof(float) * b * Pp), "alloc logits");
     MLP_CUDA(m->dH2.ensure(sizeof(float) * b * H), "alloc");
     MLP_CUDA(m->dH1.ensure(sizeof(float) * b * H), "alloc");
@@ -3110,26 +3110,23 @@ wp_status mlp_ensure(wp_ctx* ctx, wp_mlp* m, int B) {
     return WP_OK;
 }
 
-// BF16 copies (and transposes) of the master weights.
+// BF16 copies of the master weights.
 wp_status mlp_refresh(wp_ctx* ctx, wp_mlp* m) {
     MLP_CUDA(wp_mlp_launch_to_bf16(m->w[0].as<float>(), m->n[0], m->W1b.as<bf16>(), ctx->stream), "bf16");
     MLP_CUDA(wp_mlp_launch_to_bf16(m->w[2].as<float>(), m->n[2], m->W2b.as<bf16>(), ctx->stream), "bf16");
     MLP_CUDA(wp_mlp_launch_to_bf16(m->w[4].as<float>(), m->n[4], m->W3b.as<bf16>(), ctx->stream), "bf16");
-    MLP_CUDA(wp_mlp_launch_transpose(m->W2b.as<bf16>(), m->H, m->H, m->H, m->W2T.as<bf16>(), m->H, ctx->stream), "T");
-    MLP_CUDA(wp_mlp_launch_transpose(m->W3b.as<bf16>(), m->Ppad, m->H, m->H, m->W3T.as<bf16>(), m->Ppad, ctx->stream),
-             "T");
-    ctx->launches += 5;
+    ctx->launches += 3;
     return WP_OK;
 }
 
 // Logits of B inputs already in m->X.
 wp_status mlp_forward(wp_ctx* ctx, wp_mlp* m, int B) {
     const int H = m->H, Pp = m->Ppad;
-    wp_status st = mlp_gemm(ctx, m, m->X.p, 64, m->W1b.p, 64, B, H, 64, m->H1.p, H, 0, m->w[1].as<float>(), 1, m->Z1.p);
+    wp_status st = mlp_gemm(ctx, m, m->X.p, 64, false, m->W1b.p, 64, false, B, H, 64, m->H1.p, H, 0, m->w[1].as<float>(), 1, m->Z1.p);
     if (st != WP_OK) return st;
-    st = mlp_gemm(ctx, m, m->H1.p, H, m->W2b.p, H, B, H, H, m->H2.p, H, 0, m->w[3].as<float>(), 1, m->Z2.p);
+    st = mlp_gemm(ctx, m, m->H1.p, H, false, m->W2b.p, H, false, B, H, H, m->H2.p, H, 0, m->w[3].as<float>(), 1, m->Z2.p);
     if (st != WP_OK) return st;
-    return mlp_gemm(ctx, m, m->H2.p, H, m->W3b.p, H, B, Pp, H, m->L.p, Pp, 1, m->w[5].as<float>(), 0, nullptr);
+    return mlp_gemm(ctx, m, m->H2.p, H, false, m->W3b.p, H, false, B, Pp, H, m->L.p, Pp, 1, m->w[5].as<float>(), 0, nullptr);
 }
 
 // One optimiser step on B inputs in m->X with the given labels (lr 0:
@@ -3141,28 +3138,22 @@ wp_status mlp_step(wp_ctx* ctx, wp_mlp* m, const int* labels, int B, float lr) {
     if (st != WP_OK) return st;
     MLP_CUDA(wp_mlp_launch_softmax_ce(m->L.as<float>(), B, m->P, Pp, labels, 1.0f / (float)B,
                                       m->dL.as<bf16>(), m->loss.as<double>(), s), "softmax");
-    MLP_CUDA(wp_mlp_launch_transpose(m->dL.as<bf16>(), B, Pp, Pp, m->dLT.as<bf16>(), B, s), "T");
-    MLP_CUDA(wp_mlp_launch_transpose(m->H2.as<bf16>(), B, H, H, m->H2T.as<bf16>(), B, s), "T");
-    ctx->launches += 3;
-    st = mlp_gemm(ctx, m, m->dLT.p, B, m->H2T.p, B, Pp, H, B, m->g[4].p, H, 1, nullptr, 0, nullptr);  // dW3
+    ctx->launches++;
+    st = mlp_gemm(ctx, m, m->dL.p, Pp, true, m->H2.p, H, true, Pp, H, B, m->g[4].p, H, 1, nullptr, 0, nullptr);  // dW3
     if (st != WP_OK) return st;
     MLP_CUDA(wp_mlp_launch_colsum(m->dL.as<bf16>(), B, Pp, Pp, m->g[5].as<float>(), s), "colsum");
-    st = mlp_gemm(ctx, m, m->dL.p, Pp, m->W3T.p, Pp, B, H, Pp, m->dH2.p, H, 1, nullptr, 0, nullptr);  // dH2
+    st = mlp_gemm(ctx, m, m->dL.p, Pp, false, m->W3b.p, H, true, B, H, Pp, m->dH2.p, H, 1, nullptr, 0, nullptr);  // dH2
     if (st != WP_OK) return st;
     MLP_CUDA(wp_mlp_launch_gelu_bwd(m->dH2.as<float>(), m->Z2.as<bf16>(), (long)B * H, m->dZ2.as<bf16>(), s), "gelu'");
-    MLP_CUDA(wp_mlp_launch_transpose(m->dZ2.as<bf16>(), B, H, H, m->dZ2T.as<bf16>(), B, s), "T");
-    MLP_CUDA(wp_mlp_launch_transpose(m->H1.as<bf16>(), B, H, H, m->H1T.as<bf16>(), B, s), "T");
-    ctx->launches += 4;
-    st = mlp_gemm(ctx, m, m->dZ2T.p, B, m->H1T.p, B, H, H, B, m->g[2].p, H, 1, nullptr, 0, nullptr);  // dW2
+    ctx->launches += 2;
+    st = mlp_gemm(ctx, m, m->dZ2.p, H, true, m->H1.p, H, true, H, H, B, m->g[2].p, H, 1, nullptr, 0, nullptr);  // dW2
     if (st != WP_OK) return st;
     MLP_CUDA(wp_mlp_launch_colsum(m->dZ2.as<bf16>(), B, H, H, m->g[3].as<float>(), s), "colsum");
-    st = mlp_gemm(ctx, m, m->dZ2.p, H, m->W2T.p, H, B, H, H, m->dH1.p, H, 1, nullptr, 0, nullptr);  // dH1
+    st = mlp_gemm(ctx, m, m->dZ2.p, H, false, m->W2b.p, H, true, B, H, H, m->dH1.p, H, 1, nullptr, 0, nullptr);  // dH1
     if (st != WP_OK) return st;
     MLP_CUDA(wp_mlp_launch_gelu_bwd(m->dH1.as<float>(), m->Z1.as<bf16>(), (long)B * H, m->dZ1.as<bf16>(), s), "gelu'");
-    MLP_CUDA(wp_mlp_launch_transpose(m->dZ1.as<bf16>(), B, H, H, m->dZ1T.as<bf16>(), B, s), "T");
-    MLP_CUDA(wp_mlp_launch_transpose(m->X.as<bf16>(), B, 64, 64, m->XT.as<bf16>(), B, s), "T");
-    ctx->launches += 4;
-    st = mlp_gemm(ctx, m, m->dZ1T.p, B, m->XT.p, B, H, 64, B, m->g[0].p, 64, 1, nullptr, 0, nullptr);  // dW1
+    ctx->launches += 2;
+    st = mlp_gemm(ctx, m, m->dZ1.p, H, true, m->X.p, 64, true, H, 64, B, m->g[0].p, 64, 1, nullptr, 0, nullptr);  // dW1
     if (st != WP_OK) return st;
     MLP_CUDA(wp_mlp_launch_colsum(m->dZ1.as<bf16>(), B, H, H, m->g[1].as<float>(), s), "colsum");
     ctx->launches++;
@@ -3176,9 +3167,6 @@ wp_status mlp_step(wp_ctx* ctx, wp_mlp* m, const int* labels, int B, float lr) {
                                         m->v[i].as<float>(), m->n[i], lr, b1, b2, eps, bc1, bc2, wb[i], s), "adam");
             ctx->launches++;
         }
-        MLP_CUDA(wp_mlp_launch_transpose(m->W2b.as<bf16>(), H, H, H, m->W2T.as<bf16>(), H, s), "T");
-        MLP_CUDA(wp_mlp_launch_transpose(m->W3b.as<bf16>(), Pp, H, H, m->W3T.as<bf16>(), Pp, s), "T");
-        ctx->launches += 2;
     }
     return WP_OK;
 }
@@ -3261,8 +3249,7 @@ wp_status wp_mlp_create(wp_ctx* ctx, int hidden, unsigned long long seed, wp_mlp
         }
     }
     if (m->W1b.ensure(sizeof(bf16) * H * 64) || m->W2b.ensure(sizeof(bf16) * H * H) ||
-        m->W3b.ensure(sizeof(bf16) * Pp * H) || m->W2T.ensure(sizeof(bf16) * H * H) ||
-        m->W3T.ensure(sizeof(bf16) * Pp * H) || m->err.ensure(sizeof(int)) || m->loss_sum.ensure(sizeof(double))) {
+        m->W3b.ensure(sizeof(bf16) * Pp * H) || m->err.ensure(sizeof(int)) || m->loss_sum.ensure(sizeof(double))) {
         delete m;
         return fail(ctx, WP_ERR_OOM, "alloc network");
     }

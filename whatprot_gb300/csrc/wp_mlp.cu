@@ -10,14 +10,14 @@
 // The reference has no such network; this file has no reference
 // counterpart.
 //
-// All products are C = A . B^T with K-major operands (wp_gemm_bf16_tn), so
-// the backward pass keeps transposed BF16 copies where an operand's
-// reduction dimension would otherwise be strided:
-//     dH2 = dL . W3         uses W3^T  [1024][P]
-//     dW3 = dL^T . H2       uses dL^T [P][B] and H2^T [1024][B]
-//     dH1 = dZ2 . W2        uses W2^T
-//     dW2 = dZ2^T . H1      uses dZ2^T, H1^T
-//     dW1 = dZ1^T . X       uses dZ1^T, X^T
+// All products are C = A . B^T (wp_gemm_bf16); where an operand's reduction
+// dimension is the strided one the tensor cores read it as it is (MN-major),
+// so the backward pass needs no transposed copies:
+//     dH2 = dL . W3         W3 [P][1024] MN-major
+//     dW3 = dL^T . H2       both MN-major
+//     dH1 = dZ2 . W2        W2 MN-major
+//     dW2 = dZ2^T . H1      both
+//     dW1 = dZ1^T . X       both
 // Master weights, gradients and Adam moments are FP32.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -40,56 +40,6 @@ __global__ void wp_mlp_input_kernel(const float* __restrict__ xf, const double* 
     float v = 0.f;
     if (d < TC) v = xf ? xf[b * TC + d] : (float)xd[b * TC + d];
     X[i] = __float2bfloat16_rn(v);
-}
-
-// out[c][r] = in[r][c] for a rows x cols BF16 matrix, rows and cols multiples
-// of 64, pitches of 8 (every matrix of the network); blockIdx.y splits the
-// rows.  Tiles of 64 x 64, 16-byte loads and stores, eight lanes to 128 bytes of
-// an output row; a tile row of 33 words puts the eight rows that a lane gathers
-// two to a bank.  Bound by HBM.  Logit gradient of 4,096 x 20,032: 52 us,
-// against 150 us with 2-byte accesses.
-#define TR_ROW 66
-__global__ void __launch_bounds__(256) wp_transpose_bf16_kernel(const bf16* __restrict__ in, int rows, int ld_in,
-                                                                bf16* __restrict__ out, int ld_out) {
-    __shared__ __align__(16) unsigned short tile[64 * TR_ROW];
-    const int c0 = blockIdx.x * 64;
-    const int nt = rows / 64, t0 = (int)((long)nt * blockIdx.y / gridDim.y), t1 = (int)((long)nt * (blockIdx.y + 1) / gridDim.y);
-    const int lr = threadIdx.x >> 3, lc = (threadIdx.x & 7) * 8;  // load: rows lr, lr + 32, columns lc ..
-    const int sc = threadIdx.x >> 3, sr = (threadIdx.x & 7) * 8;  // store: columns sc, sc + 32, rows sr ..
-    uint4 v[2];
-#pragma unroll
-    for (int u = 0; u < 2; u++)
-        if (t0 < t1) v[u] = *reinterpret_cast<const uint4*>(in + (long)(t0 * 64 + lr + 32 * u) * ld_in + c0 + lc);
-    for (int t = t0; t < t1; t++) {
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            unsigned* dst = reinterpret_cast<unsigned*>(tile + (lr + 32 * u) * TR_ROW + lc);
-            dst[0] = v[u].x;
-            dst[1] = v[u].y;
-            dst[2] = v[u].z;
-            dst[3] = v[u].w;
-        }
-        __syncthreads();
-        if (t + 1 < t1) {
-#pragma unroll
-            for (int u = 0; u < 2; u++)
-                v[u] = *reinterpret_cast<const uint4*>(in + (long)((t + 1) * 64 + lr + 32 * u) * ld_in + c0 + lc);
-        }
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int c = sc + 32 * u;
-            unsigned short x[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) x[i] = tile[(sr + i) * TR_ROW + c];
-            uint4 o;
-            o.x = x[0] | ((unsigned)x[1] << 16);
-            o.y = x[2] | ((unsigned)x[3] << 16);
-            o.z = x[4] | ((unsigned)x[5] << 16);
-            o.w = x[6] | ((unsigned)x[7] << 16);
-            *reinterpret_cast<uint4*>(out + (long)(c0 + c) * ld_out + t * 64 + sr) = o;
-        }
-        __syncthreads();
-    }
 }
 
 // Block-wide reductions in a fixed order (warp trees, then warp 0).
@@ -127,9 +77,11 @@ __device__ float block_sum(float v, float* sh) {
 // the label (rows with label < 0 are skipped: loss 0, gradient 0), and the
 // logit gradient (softmax - onehot) * scale as BF16 (zero past P).  The row
 // (ld a multiple of 4, 16-byte aligned) stays in shared memory, so HBM sees
-// each logit once and each exponential is formed once; 4,096 rows of 20,032:
-// 158 us, against 365 us for three passes over global memory.  Rows beyond the
-// shared memory (`keep` 0) are read again for each pass.
+// each logit once and each exponential is formed once.  Bound by issue slots and
+// the phases' latency at two CTAs per SM.  4,096 rows of 20,032: 139 us, 158
+// with the label compared at every element of 4-byte stores, 365 for three
+// passes over global memory.  Rows beyond the shared memory (`keep` 0) are read
+// again for each pass.
 __global__ void __launch_bounds__(256) wp_softmax_ce_kernel(const float* __restrict__ logits, int P, int ld,
                                                             const int* __restrict__ labels, float scale,
                                                             bf16* __restrict__ dL, double* __restrict__ loss, int keep) {
@@ -170,75 +122,129 @@ __global__ void __launch_bounds__(256) wp_softmax_ce_kernel(const float* __restr
     s = block_sum(s, sh);
     const float inv = 1.0f / s;
     bf16* g = dL + row * ld;
-    for (int j = 2 * threadIdx.x; j < ld; j += 512) {
-        float v[2] = {0.f, 0.f};
-        if (y >= 0) {
-#pragma unroll
-            for (int u = 0; u < 2; u++)
-                if (j + u < P) {
-                    const float e = keep ? ce_row[j + u] : expf(l[j + u] - mx);
-                    v[u] = (e * inv - (j + u == y ? 1.f : 0.f)) * scale;
-                }
+    if (keep && y >= 0) {
+#pragma unroll 2
+        for (int j = 4 * threadIdx.x; j < ld; j += 1024) {
+            float4 e = *reinterpret_cast<const float4*>(ce_row + j);
+            if (j + 3 >= P) {
+                if (j >= P) e.x = 0.f;
+                if (j + 1 >= P) e.y = 0.f;
+                if (j + 2 >= P) e.z = 0.f;
+                e.w = 0.f;
+            }
+            const __nv_bfloat162 h0 = __floats2bfloat162_rn((e.x * inv) * scale, (e.y * inv) * scale);
+            const __nv_bfloat162 h1 = __floats2bfloat162_rn((e.z * inv) * scale, (e.w * inv) * scale);
+            uint2 u;
+            u.x = *reinterpret_cast<const unsigned*>(&h0);
+            u.y = *reinterpret_cast<const unsigned*>(&h1);
+            *reinterpret_cast<uint2*>(g + j) = u;
         }
-        *reinterpret_cast<__nv_bfloat162*>(g + j) = __floats2bfloat162_rn(v[0], v[1]);
+        // the label's element again, by the thread that wrote it
+        if ((int)threadIdx.x == (y >> 2) % 256) g[y] = __float2bfloat16_rn(fmaf(ce_row[y], inv, -1.f) * scale);
+    } else {
+        for (int j = 2 * threadIdx.x; j < ld; j += 512) {
+            float v[2] = {0.f, 0.f};
+            if (y >= 0) {
+#pragma unroll
+                for (int u = 0; u < 2; u++)
+                    if (j + u < P) v[u] = fmaf(expf(l[j + u] - mx), inv, j + u == y ? -1.f : 0.f) * scale;
+            }
+            *reinterpret_cast<__nv_bfloat162*>(g + j) = __floats2bfloat162_rn(v[0], v[1]);
+        }
     }
     if (threadIdx.x == 0) loss[row] = y >= 0 ? (double)(logf(s) + mx - l[y]) : 0.0;
 }
 
-// dZ = dH * GELU'(Z), GELU(z) = z Phi(z):  GELU'(z) = Phi(z) + z phi(z).
-__global__ void wp_gelu_bwd_kernel(const float* __restrict__ dH, const bf16* __restrict__ Z, long n,
-                                   bf16* __restrict__ dZ) {
+// dZ = dH * GELU'(Z), GELU(z) = z Phi(z):  GELU'(z) = Phi(z) + z phi(z).  Four
+// elements per thread (n a multiple of 4, 16-byte aligned).
+__global__ void wp_gelu_bwd_kernel(const float4* __restrict__ dH, const uint2* __restrict__ Z, long n4,
+                                   uint2* __restrict__ dZ) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float z = __bfloat162float(Z[i]);
-    const float d = 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
-    dZ[i] = __float2bfloat16_rn(dH[i] * d);
+    if (i >= n4) return;
+    const float4 h = dH[i];
+    const uint2 zz = Z[i];
+    const float hv[4] = {h.x, h.y, h.z, h.w};
+    const unsigned zw[4] = {zz.x << 16, zz.x & 0xffff0000u, zz.y << 16, zz.y & 0xffff0000u};
+    float o[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const float z = __uint_as_float(zw[u]);
+        const float d = 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
+        o[u] = hv[u] * d;
+    }
+    const __nv_bfloat162 h0 = __floats2bfloat162_rn(o[0], o[1]), h1 = __floats2bfloat162_rn(o[2], o[3]);
+    dZ[i] = make_uint2(*reinterpret_cast<const unsigned*>(&h0), *reinterpret_cast<const unsigned*>(&h1));
 }
 
 // Column sums of a BF16 [rows][ld] matrix, each column's rows added in order
-// (rows a multiple of 64, columns of 16).  A CTA takes 16 columns: all its
-// threads bring tiles of 128 rows into shared memory (the next tile's loads
-// under way), 16 of them add.  The chain of `rows` additions bounds a column (4
-// cycles each), HBM the wide matrix: 4,096 x 20,032 in 68 us, against 700 us
-// for a thread per column that loads its own elements.
-#define CS_COLS 16
-#define CS_ROWS 128
+// (rows and columns multiples of 64).  A CTA takes 64 columns: all its threads
+// bring tiles of 64 rows (128 bytes of each) into shared memory, four tiles in
+// flight, 64 of them add.  The chain of `rows` additions bounds a column (4
+// cycles each) and with it the narrow matrices, HBM the wide one.  4,096 x 20,032:
+// 30 us, 68 us with 16 columns per CTA and one tile in flight (32-byte pieces of
+// rows), 700 us for a thread per column that loads its own elements; 4,096 x
+// 1,024: 18 us, 24 before.
+#define CS_COLS 64
+#define CS_ROWS 64
+#define CS_STAGES 5
 __global__ void __launch_bounds__(256) wp_colsum_bf16_kernel(const bf16* __restrict__ M, int rows, int ld,
                                                              float* __restrict__ out) {
-    __shared__ __align__(16) bf16 tile[2][CS_ROWS * CS_COLS];
-    const int c0 = blockIdx.x * CS_COLS, r = threadIdx.x >> 1, half = (threadIdx.x & 1) * 8;
-    const bf16* src = M + c0 + half;
-    uint4 v = r < rows ? *reinterpret_cast<const uint4*>(src + (long)r * ld) : make_uint4(0, 0, 0, 0);
+    __shared__ __align__(16) bf16 tile[CS_STAGES][CS_ROWS * CS_COLS];
+    const int c0 = blockIdx.x * CS_COLS, nt = rows / CS_ROWS;
+    const int r = threadIdx.x >> 3, cc = (threadIdx.x & 7) * 8;  // rows r and r + 32, 8 columns from cc
+    const bf16* src = M + (long)r * ld + c0 + cc;
+    auto fetch = [&](int t) {
+        if (t < nt) {
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(
+                                     &tile[t % CS_STAGES][(r + 32 * u) * CS_COLS + cc])),
+                             "l"(src + (long)(t * CS_ROWS + 32 * u) * ld)
+                             : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int t = 0; t < CS_STAGES - 1; t++) fetch(t);
     float s = 0.f;
-    for (int r0 = 0, b = 0; r0 < rows; r0 += CS_ROWS, b ^= 1) {
-        *reinterpret_cast<uint4*>(&tile[b][r * CS_COLS + half]) = v;
-        __syncthreads();
-        const int rn = r0 + CS_ROWS + r;
-        if (rn < rows) v = *reinterpret_cast<const uint4*>(src + (long)rn * ld);
+    for (int t = 0; t < nt; t++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(CS_STAGES - 2) : "memory");
+        __syncthreads();  // tile t is there, tile t - 1 has been added
+        fetch(t + CS_STAGES - 1);
         if (threadIdx.x < CS_COLS) {
-            const bf16* t = &tile[b][threadIdx.x];
-            const int n = min(CS_ROWS, rows - r0);
-#pragma unroll 16
-            for (int i = 0; i < n; i++) s += __bfloat162float(t[i * CS_COLS]);
+            const bf16* x = &tile[t % CS_STAGES][threadIdx.x];
+#pragma unroll
+            for (int i = 0; i < CS_ROWS; i++) s += __bfloat162float(x[i * CS_COLS]);
         }
     }
     if (threadIdx.x < CS_COLS) out[c0 + threadIdx.x] = s;
 }
 
 // Adam (Kingma & Ba 2015) on FP32 master weights; refreshes the BF16 copy.
-__global__ void wp_adam_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                               float* __restrict__ v, long n, float lr, float b1, float b2, float eps, float bc1,
-                               float bc2, bf16* __restrict__ wb) {
+// Four weights per thread (n a multiple of 4, 16-byte aligned).  Bound by HBM (30
+// bytes per weight): 20.5 million in 84 us, 113 with one weight per thread.
+__global__ void wp_adam_kernel(float4* __restrict__ w, const float4* __restrict__ g, float4* __restrict__ m,
+                               float4* __restrict__ v, long n4, float lr, float b1, float b2, float eps, float bc1,
+                               float bc2, uint2* __restrict__ wb) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float wi = w[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-    w[i] = wi;
-    if (wb) wb[i] = __float2bfloat16_rn(wi);
+    if (i >= n4) return;
+    const float4 g4 = g[i], m4 = m[i], v4 = v[i], w4 = w[i];
+    const float gi[4] = {g4.x, g4.y, g4.z, g4.w};
+    float mi[4] = {m4.x, m4.y, m4.z, m4.w}, vi[4] = {v4.x, v4.y, v4.z, v4.w}, wi[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        // the rounding is spelled out: a weight's path must not depend on what the
+        // compiler makes of the sums
+        mi[u] = fmaf(1.f - b1, gi[u], __fmul_rn(b1, mi[u]));
+        vi[u] = fmaf(__fmul_rn(1.f - b2, gi[u]), gi[u], __fmul_rn(b2, vi[u]));
+        wi[u] = wi[u] - lr * (mi[u] / bc1) / (sqrtf(vi[u] / bc2) + eps);
+    }
+    m[i] = make_float4(mi[0], mi[1], mi[2], mi[3]);
+    v[i] = make_float4(vi[0], vi[1], vi[2], vi[3]);
+    w[i] = make_float4(wi[0], wi[1], wi[2], wi[3]);
+    if (wb) {
+        const __nv_bfloat162 h0 = __floats2bfloat162_rn(wi[0], wi[1]), h1 = __floats2bfloat162_rn(wi[2], wi[3]);
+        wb[i] = make_uint2(*reinterpret_cast<const unsigned*>(&h0), *reinterpret_cast<const unsigned*>(&h1));
+    }
 }
 
 __global__ void wp_f32_to_bf16_kernel(const float* __restrict__ in, long n, bf16* __restrict__ out) {
@@ -671,14 +677,6 @@ cudaError_t wp_mlp_launch_input(const float* xf, const double* xd, int B, int TC
 }
 
 // rows, cols multiples of 64; rows split so that every SM gets about eight CTAs.
-cudaError_t wp_mlp_launch_transpose(const bf16* in, int rows, int cols, int ld_in, bf16* out, int ld_out,
-                                    cudaStream_t s) {
-    if (rows % 64 || cols % 64) return cudaErrorInvalidValue;
-    const int splits = std::max(1, std::min(rows / 64, 1216 / std::max(1, cols / 64)));
-    wp_transpose_bf16_kernel<<<dim3(cols / 64, splits), 256, 0, s>>>(in, rows, ld_in, out, ld_out);
-    return cudaGetLastError();
-}
-
 cudaError_t wp_mlp_launch_colsum(const bf16* M, int rows, int cols, int ld, float* out, cudaStream_t s) {
     if (rows % 64 || cols % 64) return cudaErrorInvalidValue;
     wp_colsum_bf16_kernel<<<cols / CS_COLS, 256, 0, s>>>(M, rows, ld, out);
@@ -700,13 +698,21 @@ cudaError_t wp_mlp_launch_softmax_ce(const float* logits, int B, int P, int ld, 
 }
 
 cudaError_t wp_mlp_launch_gelu_bwd(const float* dH, const bf16* Z, long n, bf16* dZ, cudaStream_t s) {
-    wp_gelu_bwd_kernel<<<(int)((n + 255) / 256), 256, 0, s>>>(dH, Z, n, dZ);
+    if (n % 4) return cudaErrorInvalidValue;
+    const long n4 = n / 4;
+    wp_gelu_bwd_kernel<<<(int)((n4 + 255) / 256), 256, 0, s>>>(reinterpret_cast<const float4*>(dH),
+                                                               reinterpret_cast<const uint2*>(Z), n4,
+                                                               reinterpret_cast<uint2*>(dZ));
     return cudaGetLastError();
 }
 
 cudaError_t wp_mlp_launch_adam(float* w, const float* g, float* m, float* v, long n, float lr, float b1, float b2,
                                float eps, float bc1, float bc2, bf16* wb, cudaStream_t s) {
-    wp_adam_kernel<<<(int)((n + 255) / 256), 256, 0, s>>>(w, g, m, v, n, lr, b1, b2, eps, bc1, bc2, wb);
+    if (n % 4) return cudaErrorInvalidValue;
+    const long n4 = n / 4;
+    wp_adam_kernel<<<(int)((n4 + 255) / 256), 256, 0, s>>>(
+            reinterpret_cast<float4*>(w), reinterpret_cast<const float4*>(g), reinterpret_cast<float4*>(m),
+            reinterpret_cast<float4*>(v), n4, lr, b1, b2, eps, bc1, bc2, reinterpret_cast<uint2*>(wb));
     return cudaGetLastError();
 }
 
