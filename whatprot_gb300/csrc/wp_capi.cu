@@ -2710,6 +2710,23 @@ int field_bits(int most) {
     return b;
 }
 
+// Bits of the number of C channels' sequences of T counts that never rise from at
+// most `most` (wp_dedup.cu), 65 if more than 64.
+int track_rank_bits(int T, int C, int most) {
+    unsigned __int128 one = 1, all = 1;
+    for (int x = 1; x <= most; x++) {
+        one = one * (unsigned)(T + x) / (unsigned)x;
+        if (one >> 64) return 65;
+    }
+    for (int c = 0; c < C; c++) {
+        all *= one;
+        if (all >> 64) return 65;
+    }
+    int b = 0;
+    while (all >> b) b++;  // ranks are below it
+    return b;
+}
+
 // Runs the dedup of n instances already on the device (d_dd_in as int16, or
 // in_u8 with per-instance peptide indices) and keeps the result.
 wp_status dedup_run(wp_ctx* ctx, int n, int T, int C, int bits, const uint8_t* in_u8, const int* pep,
@@ -2720,8 +2737,13 @@ wp_status dedup_run(wp_ctx* ctx, int n, int T, int C, int bits, const uint8_t* i
     int id_bits = 0;
     while (id_bits < 33 && ((id_max - id_min) >> id_bits) != 0) id_bits++;
     const bool fold = last_bits + id_bits <= 64;
+    // One key per instance for the simulator's tracks (their counts never rise)
+    // where rank and id fit 64 bits: fewer digit passes than the words take.
+    const int most = ctx->sim_max_dyes;
+    const int rank_bits = in_u8 && pep && most >= 1 && most <= 15 ? track_rank_bits(T, C, most) : 65;
+    const bool ranked = rank_bits + id_bits <= 64;
     const size_t nn = (size_t)std::max(n, 1);
-    WP_CUDA(ctx->d_dd_words.ensure(sizeof(uint64_t) * W * nn), "alloc dedup");
+    if (!ranked) WP_CUDA(ctx->d_dd_words.ensure(sizeof(uint64_t) * W * nn), "alloc dedup");
     WP_CUDA(ctx->d_dd_k0.ensure(sizeof(uint64_t) * nn), "alloc dedup");
     WP_CUDA(ctx->d_dd_k1.ensure(sizeof(uint64_t) * nn), "alloc dedup");
     for (DevBuf* b : {&ctx->d_dd_p0, &ctx->d_dd_p1, &ctx->d_dd_id, &ctx->d_dd_cnt, &ctx->d_dd_ft, &ctx->d_dd_fs,
@@ -2747,6 +2769,11 @@ wp_status dedup_run(wp_ctx* ctx, int n, int T, int C, int bits, const uint8_t* i
         a.id_shift = 64 - last_bits - id_bits;
         a.id_min = id_min;
         a.last_mask = ~0ull << (64 - last_bits);
+        a.rank_bits = ranked ? rank_bits : 0;
+        a.rank_id_bits = id_bits;
+        a.T = T;
+        a.C = C;
+        a.most = most;
         a.in_u8 = in_u8;
         a.in_i16 = in_u8 ? nullptr : ctx->d_dd_in.as<int16_t>();
         a.pep = pep;

@@ -781,6 +781,9 @@ struct DedupArgs {
     int id_shift;              // the last word's spare low bits at id_shift
     long long id_min;          // (else a separate sort by id)
     uint64_t last_mask;        // the field bits of the last word
+    int rank_bits;             // > 0: one key per instance, the track's rank in
+    int rank_id_bits;          // rank_bits bits above the id's offset; T, C and
+    int T, C, most;            // the most dyes of a channel then apply
     const uint8_t* in_u8;      // [n][TC] instance tracks, or
     const int16_t* in_i16;     // [n][TC] (exactly one of the two)
     const int* pep;            // [n] peptide index (-1: none), or null when
