@@ -55,14 +55,14 @@ cudaError_t wp_launch_dense(bool has_block, int T, int C, size_t smem_optin, cud
 bool wp_dense_fits(int T, int S_cap, int C, bool has_block, size_t smem_optin);
 cudaError_t wp_launch_fma_probe(int blocks, int threads, int iters, cudaStream_t stream, float* sink);
 cudaError_t wp_launch_fit_estep(bool has_block, int grid, int threads, cudaStream_t s, const FitArgs& a);
-cudaError_t wp_launch_nn_dist(int DP, bool hist, cudaStream_t s, const NNArgs& a);
+cudaError_t wp_launch_nn_dist(int DP, int TC, bool hist, cudaStream_t s, const NNArgs& a);
 cudaError_t wp_launch_nn_pick(int grid, cudaStream_t s, const NNSelectArgs& a);
 size_t wp_nn_score_smem_bytes(int U, int table_entries);
 int wp_nn_score_ctas_per_sm(size_t smem);
 cudaError_t wp_launch_nn_score(int grid, size_t smem, cudaStream_t s, const NNScoreArgs& a);
 cudaError_t wp_launch_nn_select(int grid, cudaStream_t s, const NNSelectArgs& a);
 cudaError_t wp_launch_nn_threshold(cudaStream_t s, const NNArgs& a);
-cudaError_t wp_launch_nn_estimate(int DP, int ctas, cudaStream_t s, const NNArgs& a);
+cudaError_t wp_launch_nn_estimate(int DP, int TC, int ctas, cudaStream_t s, const NNArgs& a);
 size_t wp_nn_sort_temp_bytes(int R);
 cudaError_t wp_launch_nn_subset(const float* rows, const int* list, int n, int DP, float* out, cudaStream_t s);
 cudaError_t wp_launch_nn_remap(int* perm, const int* list, int n, cudaStream_t s);
@@ -1375,7 +1375,7 @@ wp_status nn_estimate(wp_ctx* ctx, int R, long long k, int sms) {
     a.sample_n = ctx->nn_sample_n;
     a.hits_total = ctx->nn_hits_total;
     TimedLaunch tl(ctx, 4);
-    WP_CUDA(wp_launch_nn_estimate(DP, 4 * sms, ctx->stream, a), "kNN estimate");
+    WP_CUDA(wp_launch_nn_estimate(DP, ctx->nn_T * ctx->nn_C, 4 * sms, ctx->stream, a), "kNN estimate");
     ctx->launches += 2;
     return WP_OK;
 }
@@ -1438,7 +1438,7 @@ wp_status nn_run_slots(wp_ctx* ctx, const double* d_rads, int R, int R_batch, in
     if (st != WP_OK) return st;
     {
         TimedLaunch tl(ctx, 4);
-        WP_CUDA(wp_launch_nn_dist(DP, true, ctx->stream, a), "kNN histogram");
+        WP_CUDA(wp_launch_nn_dist(DP, ctx->nn_T * ctx->nn_C, true, ctx->stream, a), "kNN histogram");
         ctx->launches++;
     }
     WP_CUDA(wp_launch_nn_threshold(ctx->stream, a), "kNN threshold");
@@ -1468,7 +1468,7 @@ wp_status nn_run_slots(wp_ctx* ctx, const double* d_rads, int R, int R_batch, in
         }
         {
             TimedLaunch tl(ctx, 4);
-            WP_CUDA(wp_launch_nn_dist(DP, true, ctx->stream, r), "kNN histogram");
+            WP_CUDA(wp_launch_nn_dist(DP, ctx->nn_T * ctx->nn_C, true, ctx->stream, r), "kNN histogram");
             ctx->launches++;
         }
         r.sub = 0;
@@ -1520,7 +1520,7 @@ wp_status nn_run_slots(wp_ctx* ctx, const double* d_rads, int R, int R_batch, in
         a.cand_bin = ctx->d_nn_cbin.as<unsigned char>();
         {
             TimedLaunch tl(ctx, 4);
-            WP_CUDA(wp_launch_nn_dist(DP, false, ctx->stream, a), "kNN collect");
+            WP_CUDA(wp_launch_nn_dist(DP, ctx->nn_T * ctx->nn_C, false, ctx->stream, a), "kNN collect");
             ctx->launches++;
         }
         b.R = nq;

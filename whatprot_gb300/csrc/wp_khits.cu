@@ -1046,7 +1046,7 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(const __grid
                         const long out = (long)(slot - a.q0) * a.stride;
                         float qd = 0.f;
                         {
-                            float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;  // as wp_nn.cu's nn_norm2
+                            float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;  // as wp_nn.cu's nn_norm2_x2
 #pragma unroll
                             for (int u = 0; u < DP / 4; u++) {
                                 const float4 q = sm->q32[u];
@@ -1070,7 +1070,7 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(const __grid
                                     const int bi = L.bin[i];
                                     keep = bi < b || (bi == b && (int)L.rank[i] >= want);
                                     pos = L.ent[i].x;
-                                    // as wp_nn.cu's nn_d2_dot (the bin) and nn_d2
+                                    // as wp_nn.cu's nn_d2_dot_x2 (the bin) and nn_d2_x2
                                     float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
                                     const float4* e = reinterpret_cast<const float4*>(a.coords + (long)pos * DP);
 #pragma unroll

@@ -40,9 +40,6 @@
 #define NN_NB WP_NN_BINS    // distance bins per query
 #define NN_TE 32           // entries per shared-memory tile
 #define NN_THREADS 256     // threads per CTA in the distance kernels
-#define NN_QPT 1           // queries per thread (one: a warp's 32 sorted reads share
-                           // fewer far tiles than 64 would)
-#define NN_QPB (NN_THREADS * NN_QPT)
 #define NN_SEL_WARPS 4     // warps per CTA in the select kernel
 #define NN_HMAX 1024       // largest h
 
@@ -54,101 +51,129 @@ __device__ __forceinline__ int nn_coarse_bin(float d2) {
     return b < 0 ? 0 : (b > NN_NB - 1 ? NN_NB - 1 : b);
 }
 
-// Squared distance of a query (registers) to an entry (shared memory); the
-// same code in both distance kernels, so both see the same float.
-template <int DP>
-__device__ __forceinline__ float nn_d2(const float* q, const float* e) {
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-#pragma unroll
-    for (int i = 0; i < DP; i += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(e + i);
-        const float x0 = q[i] - v.x, x1 = q[i + 1] - v.y, x2 = q[i + 2] - v.z, x3 = q[i + 3] - v.w;
-        a0 = fmaf(x0, x0, a0);
-        a1 = fmaf(x1, x1, a1);
-        a2 = fmaf(x2, x2, a2);
-        a3 = fmaf(x3, x3, a3);
-    }
-    return (a0 + a1) + (a2 + a3);
-}
-
-
-// Squared distance for binning, as |q|^2 + |e|^2 - 2 q.e: one multiply-add
-// per coordinate instead of a subtract and a multiply-add.  Its rounding
-// error (about 1e-7 of |q|^2 + |e|^2) only moves entries lying that close to
-// a bin edge into the neighbouring bin; the candidates' exact distances
-// (nn_d2) decide their order.
-template <int DP>
-__device__ __forceinline__ float nn_d2_dot(const float* q, float qn, const float* e, float en) {
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-#pragma unroll
-    for (int i = 0; i < DP; i += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(e + i);
-        a0 = fmaf(q[i], v.x, a0);
-        a1 = fmaf(q[i + 1], v.y, a1);
-        a2 = fmaf(q[i + 2], v.z, a2);
-        a3 = fmaf(q[i + 3], v.w, a3);
-    }
-    return fmaxf(fmaf(-2.f, (a0 + a1) + (a2 + a3), qn + en), 0.f);
-}
-
-// |q|^2 of a query held in registers (the same order in every kernel).
-template <int DP>
-__device__ __forceinline__ float nn_norm2(const float* q) {
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-#pragma unroll
-    for (int i = 0; i < DP; i += 4) {
-        a0 = fmaf(q[i], q[i], a0);
-        a1 = fmaf(q[i + 1], q[i + 1], a1);
-        a2 = fmaf(q[i + 2], q[i + 2], a2);
-        a3 = fmaf(q[i + 3], q[i + 3], a3);
-    }
-    return (a0 + a1) + (a2 + a3);
-}
-
-// Lower bound of the squared distance from a query to any entry of a tile:
-// the distance to the tile's bounding box.
-template <int DP>
-__device__ __forceinline__ float nn_box_d2(const float* q, const float* lo, const float* hi) {
-    float a0 = 0.f, a1 = 0.f;
-#pragma unroll
-    for (int i = 0; i < DP; i += 2) {
-        const float g0 = fmaxf(fmaxf(lo[i] - q[i], q[i] - hi[i]), 0.f);
-        const float g1 = fmaxf(fmaxf(lo[i + 1] - q[i + 1], q[i + 1] - hi[i + 1]), 0.f);
-        a0 = fmaf(g0, g0, a0);
-        a1 = fmaf(g1, g1, a1);
-    }
-    return a0 + a1;
-}
-
-// The same with the box read from global memory (every lane of a warp reads
-// the same box, so the loads are broadcasts from L1).
-template <int DP>
-__device__ __forceinline__ float nn_box_d2_global(const float* q, const float* __restrict__ lo,
-                                                  const float* __restrict__ hi) {
-    float a0 = 0.f, a1 = 0.f;
-#pragma unroll
-    for (int i = 0; i < DP; i += 4) {
-        const float4 l = __ldg(reinterpret_cast<const float4*>(lo + i));
-        const float4 h = __ldg(reinterpret_cast<const float4*>(hi + i));
-        const float g0 = fmaxf(fmaxf(l.x - q[i], q[i] - h.x), 0.f);
-        const float g1 = fmaxf(fmaxf(l.y - q[i + 1], q[i + 1] - h.y), 0.f);
-        const float g2 = fmaxf(fmaxf(l.z - q[i + 2], q[i + 2] - h.z), 0.f);
-        const float g3 = fmaxf(fmaxf(l.w - q[i + 3], q[i + 3] - h.w), 0.f);
-        a0 = fmaf(g0, g0, a0);
-        a1 = fmaf(g1, g1, a1);
-        a0 = fmaf(g2, g2, a0);
-        a1 = fmaf(g3, g3, a1);
-    }
-    return a0 + a1;
-}
-
 #define NN_SUPER 32  // tiles whose boxes a CTA checks between two votes
 
 // A tile whose box bound clears a distance limit by this margin holds no
-// entry that nn_d2_dot puts below the limit (its rounding error is some
+// entry that nn_d2_dot_x2 puts below the limit (its rounding error is some
 // 1e-7 of |q|^2 + |e|^2).
 __device__ __forceinline__ bool nn_clears(float lb, float limit) {
     return lb > limit + 1e-3f + 1e-4f * limit;
+}
+
+// ---- two queries per lane (the distance kernels).  A CTA's warp holds 32
+// queries: lane l and lane l + 16 both hold queries l and l + 16, lanes below 16
+// take the even entries of a tile, the others the odd ones.  An entry's
+// coordinates, read from shared memory, then serve two queries: with a query
+// per lane the 16-byte broadcasts (4 cycles each to fill 32 lanes' registers)
+// took four times as long as the multiply-adds they fed.  Coordinates are kept
+// in pairs for the packed FP32 multiply-add (two of a distance's four sums at a
+// time, the same roundings); DQ: groups of four coordinates that are in use (the
+// rest of a row is zero and adds nothing).
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ f32x2 fma_x2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float lo_of(f32x2 x) { return __uint_as_float((unsigned)x); }
+__device__ __forceinline__ float hi_of(f32x2 x) { return __uint_as_float((unsigned)(x >> 32)); }
+
+template <int DQ>
+__device__ __forceinline__ float nn_norm2_x2(const f32x2* q) {
+    f32x2 a = 0ull, b = 0ull;
+#pragma unroll
+    for (int i = 0; i < DQ; i++) {
+        a = fma_x2(q[2 * i], q[2 * i], a);
+        b = fma_x2(q[2 * i + 1], q[2 * i + 1], b);
+    }
+    return (lo_of(a) + hi_of(a)) + (lo_of(b) + hi_of(b));
+}
+
+// Squared distances for binning, as |q|^2 + |e|^2 - 2 q.e: one multiply-add per
+// coordinate instead of a subtract and a multiply-add.  The rounding error
+// (about 1e-7 of |q|^2 + |e|^2) only moves entries lying that close to a bin edge
+// into the neighbouring bin; the candidates' exact distances (nn_d2_x2) decide
+// their order.  The same code in every kernel, so all see the same float.
+template <int DQ>
+__device__ __forceinline__ void nn_d2_dot_x2(const f32x2 (&q)[2][2 * DQ], const float (&qn)[2], const float* e,
+                                             float en, float (&d2)[2]) {
+    f32x2 a[2] = {0ull, 0ull}, b[2] = {0ull, 0ull};
+#pragma unroll
+    for (int i = 0; i < DQ; i++) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(e + 4 * i);
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            a[j] = fma_x2(q[j][2 * i], v.x, a[j]);
+            b[j] = fma_x2(q[j][2 * i + 1], v.y, b[j]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+        d2[j] = fmaxf(fmaf(-2.f, (lo_of(a[j]) + hi_of(a[j])) + (lo_of(b[j]) + hi_of(b[j])), qn[j] + en), 0.f);
+}
+
+// Squared distances as sums of squared differences (the differences as
+// multiply-adds with -1: exact products, so one rounding each).
+template <int DQ>
+__device__ __forceinline__ void nn_d2_x2(const f32x2 (&q)[2][2 * DQ], const float* e, float (&d2)[2]) {
+    const f32x2 minus = 0xbf800000bf800000ull;
+    f32x2 a[2] = {0ull, 0ull}, b[2] = {0ull, 0ull};
+#pragma unroll
+    for (int i = 0; i < DQ; i++) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(e + 4 * i);
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const f32x2 x = fma_x2(v.x, minus, q[j][2 * i]), y = fma_x2(v.y, minus, q[j][2 * i + 1]);
+            a[j] = fma_x2(x, x, a[j]);
+            b[j] = fma_x2(y, y, b[j]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; j++) d2[j] = (lo_of(a[j]) + hi_of(a[j])) + (lo_of(b[j]) + hi_of(b[j]));
+}
+
+// Lower bound of both queries' squared distances to any entry of a tile: the
+// distance to the tile's bounding box, read from global memory (every lane of a
+// half warp reads the same box).
+template <int DQ>
+__device__ __forceinline__ void nn_box_d2_x2(const f32x2 (&q)[2][2 * DQ], const float* __restrict__ lo,
+                                             const float* __restrict__ hi, float (&d2)[2]) {
+    float a0[2] = {0.f, 0.f}, a1[2] = {0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < DQ; i++) {
+        const float4 l = __ldg(reinterpret_cast<const float4*>(lo + 4 * i));
+        const float4 h = __ldg(reinterpret_cast<const float4*>(hi + 4 * i));
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const float x = lo_of(q[j][2 * i]), y = hi_of(q[j][2 * i]), z = lo_of(q[j][2 * i + 1]),
+                        w = hi_of(q[j][2 * i + 1]);
+            const float g0 = fmaxf(fmaxf(l.x - x, x - h.x), 0.f), g1 = fmaxf(fmaxf(l.y - y, y - h.y), 0.f);
+            const float g2 = fmaxf(fmaxf(l.z - z, z - h.z), 0.f), g3 = fmaxf(fmaxf(l.w - w, w - h.w), 0.f);
+            a0[j] = fmaf(g0, g0, a0[j]);
+            a1[j] = fmaf(g1, g1, a1[j]);
+            a0[j] = fmaf(g2, g2, a0[j]);
+            a1[j] = fmaf(g3, g3, a1[j]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; j++) d2[j] = a0[j] + a1[j];
+}
+
+// Both queries' coordinates (zero where there is no query).
+template <int DQ>
+__device__ __forceinline__ void nn_load_queries(const float* __restrict__ queries, int DP, const int (&slot)[2],
+                                                const bool (&valid)[2], f32x2 (&q)[2][2 * DQ]) {
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const ulonglong2* src = reinterpret_cast<const ulonglong2*>(queries + (long)slot[j] * DP);
+#pragma unroll
+        for (int i = 0; i < DQ; i++) {
+            const ulonglong2 v = valid[j] ? src[i] : make_ulonglong2(0ull, 0ull);
+            q[j][2 * i] = v.x;
+            q[j][2 * i + 1] = v.y;
+        }
+    }
 }
 
 // Load a tile of entries (coords, squared norms and hits) into shared memory.
@@ -166,22 +191,27 @@ __device__ __forceinline__ void nn_load_tile(const NNArgs& a, int e0, int e_end,
     }
 }
 
-// A thread's queries are NN_QPT consecutive (sorted) slots, so a warp holds
-// 32 NN_QPT similar reads; its histogram rows sit at row j * NN_THREADS + tid
-// (bank-conflict free).  Per tile of 32 entries, each query first bounds
-// its distance to the tile's box: a tile beyond the start of the query's
-// last bin (open-ended, far beyond its k-hit radius) adds its hits to that
-// bin at once; the CTA loads the tile only if some query needs it, and a
-// warp whose queries all clear it skips the distances.
-template <int DP>
-__global__ void __launch_bounds__(NN_THREADS) wp_nn_hist_kernel(NNArgs a) {
+// A CTA's 256 queries are consecutive (sorted) slots, so a warp holds 32 similar
+// reads; query i's histogram is row i (bank-conflict free).  Per tile of 32
+// entries, each query first bounds its distance to the tile's box (its two
+// lanes take every other tile): a tile beyond the start of the query's last bin
+// (open-ended, far beyond its k-hit radius) adds its hits to that bin at once;
+// the CTA loads the tile only if some query needs it, and a warp whose queries
+// all clear it skips the distances.  Bound by the shared-memory loads of the
+// entries' coordinates and the histogram atomics.  10,007 reads against the
+// tracks of 5,000 peptides x 60, 36 coordinates: 3.5 ms, 6.0 with a query per
+// lane and all 48 padded coordinates.
+template <int DP, int DQ>
+__global__ void __launch_bounds__(NN_THREADS, DQ > 12 ? 1 : 2) wp_nn_hist_kernel(NNArgs a) {
     extern __shared__ __align__(16) unsigned char nn_smem[];
     float* tile = reinterpret_cast<float*>(nn_smem);
     int* thits = reinterpret_cast<int*>(tile + NN_TE * DP);
     float* ten = reinterpret_cast<float*>(thits + NN_TE);
     float* box = ten + NN_TE;                                    // [2][DP]
-    unsigned* hist = reinterpret_cast<unsigned*>(box + 2 * DP);  // [NN_QPB][NN_NB + 1]
-    const int qb = blockIdx.x * NN_QPB;
+    unsigned* hist = reinterpret_cast<unsigned*>(box + 2 * DP);  // [NN_THREADS][NN_NB + 1]
+    const int qb = blockIdx.x * NN_THREADS;
+    const int lane = threadIdx.x & 31, h = lane >> 4;
+    const int row[2] = {(int)(threadIdx.x & ~31u) + (lane & 15), (int)(threadIdx.x & ~31u) + (lane & 15) + 16};
     // entry slice s, or with sub-slices part p of it (whole super-tiles)
     const int sub = a.sub > 1 ? a.sub : 1;
     const int s = blockIdx.y / sub, part = blockIdx.y % sub;
@@ -195,56 +225,49 @@ __global__ void __launch_bounds__(NN_THREADS) wp_nn_hist_kernel(NNArgs a) {
         e_lo = min(e_hi, lo + a0 * NN_TE * NN_SUPER);
         e_hi = min(e_hi, lo + a1 * NN_TE * NN_SUPER);
     }
-    for (int i = threadIdx.x; i < NN_QPB * (NN_NB + 1); i += blockDim.x) hist[i] = 0u;
-    float q[NN_QPT][DP];
-    bool valid[NN_QPT];
-    int base[NN_QPT];
-    float far[NN_QPT];
+    for (int i = threadIdx.x; i < NN_THREADS * (NN_NB + 1); i += blockDim.x) hist[i] = 0u;
+    bool valid[2];
+    int slot[2], base[2];
+    float far[2], qn[2];
 #pragma unroll
-    for (int j = 0; j < NN_QPT; j++) {
-        const int lq = threadIdx.x * NN_QPT + j;
-        valid[j] = qb + lq < a.R;
-        const int slot = !valid[j] ? 0 : (a.slots ? a.slots[qb + lq] : qb + lq);
-        const float* src = a.queries + (long)slot * DP;
-#pragma unroll
-        for (int i = 0; i < DP; i++) q[j][i] = valid[j] ? src[i] : 0.f;
-        base[j] = valid[j] ? a.qbase[a.q0 + slot] : 0;
+    for (int j = 0; j < 2; j++) {
+        valid[j] = qb + row[j] < a.R;
+        slot[j] = !valid[j] ? 0 : (a.slots ? a.slots[qb + row[j]] : qb + row[j]);
+        base[j] = valid[j] ? a.qbase[a.q0 + slot[j]] : 0;
         far[j] = valid[j] ? wp_nn_bin_start(base[j], NN_NB - 1) : INFINITY;
     }
-    float qn[NN_QPT];
+    f32x2 q[2][2 * DQ];
+    nn_load_queries<DQ>(a.queries, DP, slot, valid, q);
 #pragma unroll
-    for (int j = 0; j < NN_QPT; j++) qn[j] = nn_norm2<DP>(q[j]);
+    for (int j = 0; j < 2; j++) qn[j] = nn_norm2_x2<DQ>(q[j]);
     unsigned* vote = reinterpret_cast<unsigned*>(box);
+    __syncthreads();
     for (int st0 = e_lo; st0 < e_hi; st0 += NN_TE * NN_SUPER) {
         // which of the next NN_SUPER tiles each read needs; the others add
         // their hits to the read's open last bin
         const int t0 = st0 / NN_TE, nt = min(NN_SUPER, (e_hi - st0 + NN_TE - 1) / NN_TE);
-        unsigned nm[NN_QPT];
-        int mb[NN_QPT];  // smallest bin of the read's entries in this super-tile
-#pragma unroll
-        for (int j = 0; j < NN_QPT; j++) {
-            nm[j] = 0u;
-            mb[j] = NN_NB - 1;
-        }
-        for (int tt = 0; tt < nt; tt++) {
+        unsigned nm[2] = {0u, 0u};
+        int mb[2] = {NN_NB - 1, NN_NB - 1};  // smallest bin of the read's entries in this super-tile
+        for (int tt = h; tt < nt; tt += 2) {
             const long t = t0 + tt;
+            float d2[2];
+            nn_box_d2_x2<DQ>(q, a.tlo + t * DP, a.thi + t * DP, d2);
 #pragma unroll
-            for (int j = 0; j < NN_QPT; j++) {
+            for (int j = 0; j < 2; j++) {
                 if (!valid[j]) continue;
-                if (!nn_clears(nn_box_d2_global<DP>(q[j], a.tlo + t * DP, a.thi + t * DP), far[j]))
+                if (!nn_clears(d2[j], far[j]))
                     nm[j] |= 1u << tt;
                 else
-                    atomicAdd(&hist[(j * NN_THREADS + threadIdx.x) * (NN_NB + 1) + NN_NB - 1], (unsigned)a.ttot[t]);
+                    atomicAdd(&hist[row[j] * (NN_NB + 1) + NN_NB - 1], (unsigned)a.ttot[t]);
             }
         }
-        unsigned wm = 0u;
 #pragma unroll
-        for (int j = 0; j < NN_QPT; j++) wm |= nm[j];
-        wm = __reduce_or_sync(0xffffffffu, wm);
+        for (int j = 0; j < 2; j++) nm[j] |= __shfl_xor_sync(0xffffffffu, nm[j], 16);
+        const unsigned wm = __reduce_or_sync(0xffffffffu, nm[0] | nm[1]);
         __syncthreads();
         if (threadIdx.x == 0) vote[0] = 0u;
         __syncthreads();
-        if ((threadIdx.x & 31) == 0 && wm) atomicOr(&vote[0], wm);
+        if (lane == 0 && wm) atomicOr(&vote[0], wm);
         __syncthreads();
         unsigned cm = vote[0];
         while (cm) {
@@ -255,18 +278,18 @@ __global__ void __launch_bounds__(NN_THREADS) wp_nn_hist_kernel(NNArgs a) {
             nn_load_tile<DP>(a, e0, e_hi, tile, thits, ten);
             __syncthreads();
             if (!((wm >> tt) & 1u)) continue;
-            bool need[NN_QPT];
-#pragma unroll
-            for (int j = 0; j < NN_QPT; j++) need[j] = (nm[j] >> tt) & 1u;
+            const bool need[2] = {((nm[0] >> tt) & 1u) != 0u, ((nm[1] >> tt) & 1u) != 0u};
             const int n = min(NN_TE, e_hi - e0);
-            for (int e = 0; e < n; e++) {
+            for (int e = h; e < n; e += 2) {
+                float d2[2];
+                nn_d2_dot_x2<DQ>(q, qn, tile + e * DP, ten[e], d2);
+                const unsigned hits = (unsigned)thits[e];
 #pragma unroll
-                for (int j = 0; j < NN_QPT; j++) {
-                    const float d2 = nn_d2_dot<DP>(q[j], qn[j], tile + e * DP, ten[e]);
+                for (int j = 0; j < 2; j++) {
+                    const int bin = wp_nn_bin(d2[j], base[j]);
                     if (need[j]) {
-                        const int bin = wp_nn_bin(d2, base[j]);
                         mb[j] = min(mb[j], bin);
-                        atomicAdd(&hist[(j * NN_THREADS + threadIdx.x) * (NN_NB + 1) + bin], (unsigned)thits[e]);
+                        atomicAdd(&hist[row[j] * (NN_NB + 1) + bin], hits);
                     }
                 }
             }
@@ -274,23 +297,20 @@ __global__ void __launch_bounds__(NN_THREADS) wp_nn_hist_kernel(NNArgs a) {
         if (a.stmin) {
             const int sti = s * nsps + (st0 - slice0) / (NN_TE * NN_SUPER);
 #pragma unroll
-            for (int j = 0; j < NN_QPT; j++) {
-                const int lq = threadIdx.x * NN_QPT + j;
-                if (!valid[j]) continue;
-                const int slot = a.slots ? a.slots[qb + lq] : qb + lq;
-                a.stmin[(long)(a.q0 + slot) * a.n_super + sti] = (unsigned char)mb[j];
+            for (int j = 0; j < 2; j++) {
+                mb[j] = min(mb[j], __shfl_xor_sync(0xffffffffu, mb[j], 16));
+                if (valid[j] && h == j) a.stmin[(long)(a.q0 + slot[j]) * a.n_super + sti] = (unsigned char)mb[j];
             }
         }
     }
     __syncthreads();
     // this slice's histograms, query-major within the slice
-    for (int i = threadIdx.x; i < NN_QPB * NN_NB; i += blockDim.x) {
+    for (int i = threadIdx.x; i < NN_THREADS * NN_NB; i += blockDim.x) {
         const int lq = i / NN_NB, b = i % NN_NB;
-        const int row = (lq % NN_QPT) * NN_THREADS + lq / NN_QPT;
         if (qb + lq < a.R) {
-            const int slot = a.slots ? a.slots[qb + lq] : qb + lq;
-            unsigned* dst = &a.shist[((long)s * a.R_all + a.q0 + slot) * NN_NB + b];
-            const unsigned v = hist[row * (NN_NB + 1) + b];
+            const int slot_q = a.slots ? a.slots[qb + lq] : qb + lq;
+            unsigned* dst = &a.shist[((long)s * a.R_all + a.q0 + slot_q) * NN_NB + b];
+            const unsigned v = hist[lq * (NN_NB + 1) + b];
             if (sub > 1) {
                 if (v) atomicAdd(dst, v);
             } else {
@@ -310,29 +330,24 @@ __global__ void __launch_bounds__(NN_THREADS) wp_nn_hist_kernel(NNArgs a) {
 // octave above it.  Only the bins move with the estimate; the
 // selection stays exact whatever it says (a poor estimate only leaves more
 // candidates).  The sample is split over blockIdx.y so that small batches fill
-// the GPU (4,000 reads: 0.34 ms, against 3.6 ms with a CTA per 256 reads).
-template <int DP>
-__global__ void __launch_bounds__(NN_THREADS) wp_nn_estimate_kernel(NNArgs a) {
+// the GPU (4,000 reads: 0.34 ms, against 3.6 ms with a CTA per 256 reads; two
+// queries per lane: 10,007 reads of 36 coordinates 0.75 -> 0.49 ms).
+template <int DP, int DQ>
+__global__ void __launch_bounds__(NN_THREADS, DQ > 12 ? 1 : 2) wp_nn_estimate_kernel(NNArgs a) {
     extern __shared__ __align__(16) unsigned char nn_smem[];
     float* tile = reinterpret_cast<float*>(nn_smem);
     int* thits = reinterpret_cast<int*>(tile + NN_TE * DP);
     float* ten = reinterpret_cast<float*>(thits + NN_TE);
-    unsigned* hist = reinterpret_cast<unsigned*>(ten + NN_TE);  // [NN_QPB][NN_NB + 1]
-    const int qb = blockIdx.x * NN_QPB;
-    for (int i = threadIdx.x; i < NN_QPB * (NN_NB + 1); i += blockDim.x) hist[i] = 0u;
-    float q[NN_QPT][DP];
-    bool valid[NN_QPT];
-#pragma unroll
-    for (int j = 0; j < NN_QPT; j++) {
-        const int lq = threadIdx.x * NN_QPT + j;
-        valid[j] = qb + lq < a.R;
-        const float* src = a.queries + (long)(valid[j] ? qb + lq : 0) * DP;
-#pragma unroll
-        for (int i = 0; i < DP; i++) q[j][i] = valid[j] ? src[i] : 0.f;
-    }
-    float qn[NN_QPT];
-#pragma unroll
-    for (int j = 0; j < NN_QPT; j++) qn[j] = nn_norm2<DP>(q[j]);
+    unsigned* hist = reinterpret_cast<unsigned*>(ten + NN_TE);  // [NN_THREADS][NN_NB + 1]
+    const int qb = blockIdx.x * NN_THREADS;
+    const int lane = threadIdx.x & 31, h = lane >> 4;
+    const int row[2] = {(int)(threadIdx.x & ~31u) + (lane & 15), (int)(threadIdx.x & ~31u) + (lane & 15) + 16};
+    for (int i = threadIdx.x; i < NN_THREADS * (NN_NB + 1); i += blockDim.x) hist[i] = 0u;
+    const bool valid[2] = {qb + row[0] < a.R, qb + row[1] < a.R};
+    const int slot[2] = {valid[0] ? qb + row[0] : 0, valid[1] ? qb + row[1] : 0};
+    f32x2 q[2][2 * DQ];
+    nn_load_queries<DQ>(a.queries, DP, slot, valid, q);
+    const float qn[2] = {nn_norm2_x2<DQ>(q[0]), nn_norm2_x2<DQ>(q[1])};
     // blockIdx.y takes a part of the sample
     const int s_lo = (int)((long)a.sample_n * blockIdx.y / gridDim.y), s_hi = (int)((long)a.sample_n * (blockIdx.y + 1) / gridDim.y);
     for (int s0 = s_lo; s0 < s_hi; s0 += NN_TE) {
@@ -346,18 +361,18 @@ __global__ void __launch_bounds__(NN_THREADS) wp_nn_estimate_kernel(NNArgs a) {
         }
         for (int i = threadIdx.x; i < NN_TE; i += blockDim.x) ten[i] = i < n ? a.enorm[a.sample[s0 + i]] : 0.f;
         __syncthreads();
-        for (int e = 0; e < n; e++) {
+        for (int e = h; e < n; e += 2) {
+            float d2[2];
+            nn_d2_dot_x2<DQ>(q, qn, tile + e * DP, ten[e], d2);
 #pragma unroll
-            for (int j = 0; j < NN_QPT; j++) {
-                const float d2 = nn_d2_dot<DP>(q[j], qn[j], tile + e * DP, ten[e]);
-                if (valid[j]) atomicAdd(&hist[(threadIdx.x + j * NN_THREADS) * (NN_NB + 1) + nn_coarse_bin(d2)], 1u);
-            }
+            for (int j = 0; j < 2; j++)
+                if (valid[j]) atomicAdd(&hist[row[j] * (NN_NB + 1) + nn_coarse_bin(d2[j])], 1u);
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < NN_QPB * NN_NB; i += blockDim.x) {
+    for (int i = threadIdx.x; i < NN_THREADS * NN_NB; i += blockDim.x) {
         const int lq = i / NN_NB, b = i % NN_NB;
-        const unsigned v = hist[((lq % NN_QPT) * NN_THREADS + lq / NN_QPT) * (NN_NB + 1) + b];
+        const unsigned v = hist[lq * (NN_NB + 1) + b];
         if (qb + lq < a.R && v) atomicAdd(&a.coarse[(long)(a.q0 + qb + lq) * NN_NB + b], v);
     }
 }
@@ -436,102 +451,111 @@ __global__ void wp_nn_threshold_kernel(NNArgs a) {
     }
 }
 
-template <int DP>
-__global__ void __launch_bounds__(NN_THREADS) wp_nn_collect_kernel(NNArgs a) {
+// The second pass, in the same shape: both lanes of a query count its candidates
+// alike and write them in entry order.  The reads above: 4.8 ms, 6.1 with a query
+// per lane (45 million candidates written one by one).
+template <int DP, int DQ>
+__global__ void __launch_bounds__(NN_THREADS, DQ > 12 ? 1 : 2) wp_nn_collect_kernel(NNArgs a) {
     extern __shared__ __align__(16) unsigned char nn_smem[];
     float* tile = reinterpret_cast<float*>(nn_smem);
     int* thits = reinterpret_cast<int*>(tile + NN_TE * DP);
     float* ten = reinterpret_cast<float*>(thits + NN_TE);
     float* box = ten + NN_TE;  // [2][DP]
-    const int qb = blockIdx.x * NN_QPB;
+    const int qb = blockIdx.x * NN_THREADS;
+    const int lane = threadIdx.x & 31, h = lane >> 4;
+    const int row[2] = {(int)(threadIdx.x & ~31u) + (lane & 15), (int)(threadIdx.x & ~31u) + (lane & 15) + 16};
     const int s = blockIdx.y;
     const int e_lo = s * a.slice_len, e_hi = min(a.N, e_lo + a.slice_len);
     const int nsps = (a.slice_len + NN_TE * NN_SUPER - 1) / (NN_TE * NN_SUPER);
-    float q[NN_QPT][DP];
-    bool valid[NN_QPT];
-    int bstar[NN_QPT], base[NN_QPT];
-    float lim[NN_QPT];
-    long long off[NN_QPT], cap[NN_QPT], cnt[NN_QPT];
+    bool valid[2];
+    int slot[2], bstar[2], base[2];
+    float lim[2], qn[2];
+    long long off[2], cap[2], cnt[2];  // cnt: both lanes of a query count alike
 #pragma unroll
-    for (int j = 0; j < NN_QPT; j++) {
-        const int lq = threadIdx.x * NN_QPT + j;
-        valid[j] = qb + lq < a.R;
-        const int l = valid[j] ? qb + lq : 0;
-        const int gq = a.q0 + l;
-        const float* src = a.queries + (long)l * DP;
-#pragma unroll
-        for (int i = 0; i < DP; i++) q[j][i] = valid[j] ? src[i] : 0.f;
+    for (int j = 0; j < 2; j++) {
+        valid[j] = qb + row[j] < a.R;
+        slot[j] = valid[j] ? qb + row[j] : 0;
+        const int gq = a.q0 + slot[j];
         bstar[j] = valid[j] ? a.qbin[gq] : -1;
         base[j] = valid[j] ? a.qbase[gq] : 0;
-        off[j] = valid[j] ? a.qoff[l] + a.sliceoff[(long)s * a.R_all + gq] : 0;
+        off[j] = valid[j] ? a.qoff[slot[j]] + a.sliceoff[(long)s * a.R_all + gq] : 0;
         cap[j] = valid[j] ? a.slicecap[(long)s * a.R_all + gq] : 0;
         cnt[j] = 0;
         // candidates lie below the start of bin b* + 1 (none beyond the open last bin)
         lim[j] = !valid[j] ? -1.f : (bstar[j] >= NN_NB - 1 ? INFINITY : wp_nn_bin_start(base[j], bstar[j] + 1));
     }
-    float qn[NN_QPT];
+    f32x2 q[2][2 * DQ];
+    nn_load_queries<DQ>(a.queries, DP, slot, valid, q);
 #pragma unroll
-    for (int j = 0; j < NN_QPT; j++) qn[j] = nn_norm2<DP>(q[j]);
+    for (int j = 0; j < 2; j++) qn[j] = nn_norm2_x2<DQ>(q[j]);
     unsigned* vote = reinterpret_cast<unsigned*>(box);
     for (int st0 = e_lo; st0 < e_hi; st0 += NN_TE * NN_SUPER) {
         const int t0 = st0 / NN_TE, nt = min(NN_SUPER, (e_hi - st0 + NN_TE - 1) / NN_TE);
         // reads with no entry at or below b* in this super-tile (the
         // histogram pass's smallest bin) need none of its tiles
-        bool sn[NN_QPT];
+        bool sn[2];
         const int sti = s * nsps + (st0 - e_lo) / (NN_TE * NN_SUPER);
 #pragma unroll
-        for (int j = 0; j < NN_QPT; j++) {
-            const int lq = threadIdx.x * NN_QPT + j;
-            sn[j] = valid[j] && (!a.stmin || (int)a.stmin[(long)(a.q0 + qb + lq) * a.n_super + sti] <= bstar[j]);
-        }
+        for (int j = 0; j < 2; j++)
+            sn[j] = valid[j] && (!a.stmin || (int)a.stmin[(long)(a.q0 + slot[j]) * a.n_super + sti] <= bstar[j]);
         unsigned wm = 0u;
-        for (int tt = 0; tt < nt; tt++) {
-            const long t = t0 + tt;
-            bool nd = false;
-#pragma unroll
-            for (int j = 0; j < NN_QPT; j++)
-                nd |= sn[j] && !nn_clears(nn_box_d2_global<DP>(q[j], a.tlo + t * DP, a.thi + t * DP), lim[j]);
-            if (nd) wm |= 1u << tt;
-        }
+        if (__any_sync(0xffffffffu, sn[0] || sn[1]))
+            for (int tt = h; tt < nt; tt += 2) {
+                const long t = t0 + tt;
+                float d2[2];
+                nn_box_d2_x2<DQ>(q, a.tlo + t * DP, a.thi + t * DP, d2);
+                if ((sn[0] && !nn_clears(d2[0], lim[0])) || (sn[1] && !nn_clears(d2[1], lim[1]))) wm |= 1u << tt;
+            }
         wm = __reduce_or_sync(0xffffffffu, wm);
         __syncthreads();
         if (threadIdx.x == 0) vote[0] = 0u;
         __syncthreads();
-        if ((threadIdx.x & 31) == 0 && wm) atomicOr(&vote[0], wm);
+        if (lane == 0 && wm) atomicOr(&vote[0], wm);
         __syncthreads();
         unsigned cm = vote[0];
         while (cm) {
-        const int tt = __ffs(cm) - 1;
-        cm &= cm - 1;
-        const int e0 = st0 + tt * NN_TE;
-        __syncthreads();
-        nn_load_tile<DP>(a, e0, e_hi, tile, thits, ten);
-        __syncthreads();
-        if (!((wm >> tt) & 1u)) continue;
-        const int n = min(NN_TE, e_hi - e0);
-        for (int e = 0; e < n; e++) {
+            const int tt = __ffs(cm) - 1;
+            cm &= cm - 1;
+            const int e0 = st0 + tt * NN_TE;
+            __syncthreads();
+            nn_load_tile<DP>(a, e0, e_hi, tile, thits, ten);
+            __syncthreads();
+            if (!((wm >> tt) & 1u)) continue;
+            const int n = min(NN_TE, e_hi - e0);
+            for (int ep = 0; ep < n; ep += 2) {
+                const int e = ep + h;
+                const bool there = e < n;  // the tile's rows past n are zero
+                float d2[2];
+                nn_d2_dot_x2<DQ>(q, qn, tile + e * DP, ten[e], d2);
+                const int bin[2] = {wp_nn_bin(d2[0], base[0]), wp_nn_bin(d2[1], base[1])};
+                const unsigned km[2] = {__ballot_sync(0xffffffffu, there && bin[0] <= bstar[0]),
+                                        __ballot_sync(0xffffffffu, there && bin[1] <= bstar[1])};
+                if ((km[0] | km[1]) == 0u) continue;
+                nn_d2_x2<DQ>(q, tile + e * DP, d2);
 #pragma unroll
-            for (int j = 0; j < NN_QPT; j++) {
-                const int bin = wp_nn_bin(nn_d2_dot<DP>(q[j], qn[j], tile + e * DP, ten[e]), base[j]);
-                if (bin <= bstar[j]) {
-                    if (cnt[j] < cap[j]) {
-                        a.cand_idx[off[j] + cnt[j]] = e0 + e;
-                        a.cand_d2[off[j] + cnt[j]] = nn_d2<DP>(q[j], tile + e * DP);
-                        a.cand_hits[off[j] + cnt[j]] = thits[e];
-                        a.cand_bin[off[j] + cnt[j]] = (unsigned char)bin;
-                    } else {
-                        atomicExch(a.err, 1);
+                for (int j = 0; j < 2; j++) {
+                    // in entry order: the even entry's lane first
+                    const int even = (int)((km[j] >> (lane & 15)) & 1u), odd = (int)((km[j] >> ((lane & 15) + 16)) & 1u);
+                    if (h ? odd : even) {
+                        const long long at = cnt[j] + (h ? even : 0);
+                        if (at < cap[j]) {
+                            a.cand_idx[off[j] + at] = e0 + e;
+                            a.cand_d2[off[j] + at] = d2[j];
+                            a.cand_hits[off[j] + at] = thits[e];
+                            a.cand_bin[off[j] + at] = (unsigned char)bin[j];
+                        } else {
+                            atomicExch(a.err, 1);
+                        }
                     }
-                    cnt[j]++;
+                    cnt[j] += even + odd;
                 }
             }
         }
-        }
     }
 #pragma unroll
-    for (int j = 0; j < NN_QPT; j++) {
-        if (!valid[j]) continue;
-        a.slicecnt[(long)s * a.R_all + a.q0 + qb + threadIdx.x * NN_QPT + j] = cnt[j];
+    for (int j = 0; j < 2; j++) {
+        if (!valid[j] || h != j) continue;
+        a.slicecnt[(long)s * a.R_all + a.q0 + slot[j]] = cnt[j];
         if (cnt[j] > cap[j]) atomicExch(a.err, 1);
     }
 }
@@ -1039,67 +1063,68 @@ cudaError_t wp_launch_hybrid_finish(const int* ncand, const double* subfrac, int
 
 size_t wp_nn_dist_smem_bytes(int DP, bool with_hist) {
     size_t b = sizeof(float) * NN_TE * DP + sizeof(int) * NN_TE + sizeof(float) * NN_TE + sizeof(float) * 2 * DP;
-    if (with_hist) b += sizeof(unsigned) * NN_QPB * (NN_NB + 1);
+    if (with_hist) b += sizeof(unsigned) * NN_THREADS * (NN_NB + 1);
     return b;
 }
 
 int wp_nn_bins() { return NN_NB; }
 
-int wp_nn_queries_per_block() { return NN_QPB; }
+int wp_nn_queries_per_block() { return NN_THREADS; }
 int wp_nn_select_warps() { return NN_SEL_WARPS; }
 int wp_nn_hmax() { return NN_HMAX; }
 
-template <int DP>
+template <int DP, int DQ>
 static cudaError_t launch_dist(bool hist, dim3 grid, cudaStream_t s, const NNArgs& a) {
     const size_t smem = wp_nn_dist_smem_bytes(DP, hist);
     if (hist) {
-        cudaFuncSetAttribute(wp_nn_hist_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        wp_nn_hist_kernel<DP><<<grid, NN_THREADS, smem, s>>>(a);
+        cudaFuncSetAttribute(wp_nn_hist_kernel<DP, DQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        wp_nn_hist_kernel<DP, DQ><<<grid, NN_THREADS, smem, s>>>(a);
     } else {
-        cudaFuncSetAttribute(wp_nn_collect_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        wp_nn_collect_kernel<DP><<<grid, NN_THREADS, smem, s>>>(a);
+        cudaFuncSetAttribute(wp_nn_collect_kernel<DP, DQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        wp_nn_collect_kernel<DP, DQ><<<grid, NN_THREADS, smem, s>>>(a);
     }
     return cudaGetLastError();
 }
 
-// DP: padded dimension, one of 16, 32, 48, 64.  Grid: query blocks x the
-// args' entry slices.
-cudaError_t wp_launch_nn_dist(int DP, bool hist, cudaStream_t s, const NNArgs& a) {
-    const int qblocks = (a.R + NN_QPB - 1) / NN_QPB;
+// DP: padded dimension, one of 16, 32, 48, 64, of which the first TC are in
+// use.  Grid: query blocks x the args' entry slices.
+cudaError_t wp_launch_nn_dist(int DP, int TC, bool hist, cudaStream_t s, const NNArgs& a) {
+    const int qblocks = (a.R + NN_THREADS - 1) / NN_THREADS;
     if (qblocks == 0) return cudaSuccess;
     const dim3 grid(qblocks, a.slices * (hist && a.sub > 1 ? a.sub : 1));
     switch (DP) {
-        case 16: return launch_dist<16>(hist, grid, s, a);
-        case 32: return launch_dist<32>(hist, grid, s, a);
-        case 48: return launch_dist<48>(hist, grid, s, a);
-        case 64: return launch_dist<64>(hist, grid, s, a);
+        case 16: return TC <= 8 ? launch_dist<16, 2>(hist, grid, s, a) : launch_dist<16, 4>(hist, grid, s, a);
+        case 32: return TC <= 24 ? launch_dist<32, 6>(hist, grid, s, a) : launch_dist<32, 8>(hist, grid, s, a);
+        case 48: return TC <= 36 ? launch_dist<48, 9>(hist, grid, s, a) : launch_dist<48, 12>(hist, grid, s, a);
+        case 64: return TC <= 56 ? launch_dist<64, 14>(hist, grid, s, a) : launch_dist<64, 16>(hist, grid, s, a);
         default: return cudaErrorInvalidValue;
     }
 }
 
-template <int DP>
+template <int DP, int DQ>
 static cudaError_t launch_estimate(dim3 grid, cudaStream_t s, const NNArgs& a) {
     const size_t smem = wp_nn_dist_smem_bytes(DP, true);
-    cudaError_t e = cudaFuncSetAttribute(wp_nn_estimate_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e =
+        cudaFuncSetAttribute(wp_nn_estimate_kernel<DP, DQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    wp_nn_estimate_kernel<DP><<<grid, NN_THREADS, smem, s>>>(a);
+    wp_nn_estimate_kernel<DP, DQ><<<grid, NN_THREADS, smem, s>>>(a);
     return cudaGetLastError();
 }
 
 // The per-query bin origins (a.qbase) from a.sample_n sampled entries;
 // a.coarse: [R][bins] scratch.  `ctas`: CTAs to spread the work over.
-cudaError_t wp_launch_nn_estimate(int DP, int ctas, cudaStream_t s, const NNArgs& a) {
-    const int qblocks = (a.R + NN_QPB - 1) / NN_QPB;
+cudaError_t wp_launch_nn_estimate(int DP, int TC, int ctas, cudaStream_t s, const NNArgs& a) {
+    const int qblocks = (a.R + NN_THREADS - 1) / NN_THREADS;
     if (qblocks == 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(a.coarse + (long)a.q0 * NN_NB, 0, sizeof(unsigned) * (size_t)a.R * NN_NB, s);
     if (e != cudaSuccess) return e;
     // at least 256 sample points per part (the read's own set-up costs as much as some tens)
     const dim3 grid(qblocks, std::max(1, std::min((ctas + qblocks - 1) / qblocks, a.sample_n / 256)));
     switch (DP) {
-        case 16: e = launch_estimate<16>(grid, s, a); break;
-        case 32: e = launch_estimate<32>(grid, s, a); break;
-        case 48: e = launch_estimate<48>(grid, s, a); break;
-        case 64: e = launch_estimate<64>(grid, s, a); break;
+        case 16: e = TC <= 8 ? launch_estimate<16, 2>(grid, s, a) : launch_estimate<16, 4>(grid, s, a); break;
+        case 32: e = TC <= 24 ? launch_estimate<32, 6>(grid, s, a) : launch_estimate<32, 8>(grid, s, a); break;
+        case 48: e = TC <= 36 ? launch_estimate<48, 9>(grid, s, a) : launch_estimate<48, 12>(grid, s, a); break;
+        case 64: e = TC <= 56 ? launch_estimate<64, 14>(grid, s, a) : launch_estimate<64, 16>(grid, s, a); break;
         default: return cudaErrorInvalidValue;
     }
     if (e != cudaSuccess) return e;
