@@ -45,13 +45,14 @@ __global__ void wp_count_flops_kernel(BatchArgs, double*);
 cudaError_t wp_launch_engine(int C, bool has_block, int threads, size_t smem, cudaStream_t s,
                              const BatchArgs& a, const int2* in, const int* in_count, int* in_head,
                              int2* out, int* out_count, int slab_half, int scr_floats,
-                             int spill_error, int* grid_out);
+                             int spill_error, long pairs, int* grid_out);
 size_t wp_engine_smem_bytes(int slab_half, int scr_floats, bool has_block, int threads);
+cudaError_t wp_launch_shape(const void* kernel, int threads, size_t smem, int* per_sm, int* sms);
 cudaError_t wp_launch_coop(int C, bool has_block, int lanes, cudaStream_t s, const BatchArgs& a, const int2* in,
                            const int* in_count, int* in_head, int2* out, int* out_count, int slab_half,
-                           int spill_error);
+                           int spill_error, long pairs);
 cudaError_t wp_launch_dense(bool has_block, int T, int C, size_t smem_optin, cudaStream_t stream,
-                            const BatchArgs& a);
+                            const BatchArgs& a, long pairs);
 bool wp_dense_fits(int T, int S_cap, int C, bool has_block, size_t smem_optin);
 cudaError_t wp_launch_fma_probe(int blocks, int threads, int iters, cudaStream_t stream, float* sink);
 cudaError_t wp_launch_fit_estep(bool has_block, int grid, int threads, cudaStream_t s, const FitArgs& a);
@@ -194,12 +195,15 @@ struct EngineReplay {
     BatchArgs a;
     int C = 0, T = 0, nt = 0;
     bool hb = false, dense = false;
+    long pairs = 0;  // the batch's slots
     int threads[WP_MAX_TIERS], half[WP_MAX_TIERS], lanes[WP_MAX_TIERS];
     int2* list[WP_MAX_TIERS];
     int* cnt = nullptr;
 };
 
 struct wp_ctx {
+    DevBuf d_small;            // a small classify call's outputs
+    void* h_small = nullptr;   // and their page-locked copy
     int device = 0;
     cudaStream_t stream = nullptr;
     EngineReplay replay;
@@ -604,8 +608,9 @@ wp_status run_batch(wp_ctx* ctx, const double* d_rads, int R, double dist_cutoff
         WP_CUDA(cudaGetLastError(), "summary launch");
         if (window_factors) {
             const size_t wsm = wp_window_smem_bytes(C, W, 128);
-            WP_CUDA(cudaFuncSetAttribute(wp_window_factors_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)wsm), "window factors attribute");
+            int per_sm = 0, sms = 0;
+            WP_CUDA(wp_launch_shape(reinterpret_cast<const void*>(wp_window_factors_kernel), 128, wsm, &per_sm, &sms),
+                    "window factors shape");
             wp_window_factors_kernel<<<(int)((n + 127) / 128), 128, wsm, ctx->stream>>>(a);
             ctx->launches++;
             WP_CUDA(cudaGetLastError(), "window factors launch");
@@ -731,13 +736,9 @@ wp_status run_batch(wp_ctx* ctx, const double* d_rads, int R, double dist_cutoff
             if (groups) {
                 // persistent: as many CTAs as are resident, at most one warp per read
                 const size_t gsm = wp_compact_groups_smem_bytes(a.n_grp, a.P);
-                WP_CUDA(cudaFuncSetAttribute(wp_compact_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)gsm), "compact attribute");
-                int per_sm = 0;
-                WP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wp_compact_groups_kernel,
-                                                                      WP_GROUP_WARPS * 32, gsm), "compact occupancy");
-                int sms = 1;
-                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+                int per_sm = 0, sms = 1;
+                WP_CUDA(wp_launch_shape(reinterpret_cast<const void*>(wp_compact_groups_kernel), WP_GROUP_WARPS * 32,
+                                        gsm, &per_sm, &sms), "compact shape");
                 const int grid = std::max(1, std::min(sms * std::max(per_sm, 1),
                                                       (R + WP_GROUP_WARPS - 1) / WP_GROUP_WARPS));
                 wp_compact_groups_kernel<<<grid, WP_GROUP_WARPS * 32, gsm, ctx->stream>>>(a);
@@ -755,18 +756,18 @@ wp_status run_batch(wp_ctx* ctx, const double* d_rads, int R, double dist_cutoff
             const int spill_error = last && !dense ? 1 : 0;
             WP_CUDA(tiers[k].lanes > 0
                             ? wp_launch_coop(C, hb, tiers[k].lanes, ctx->stream, a, lists[k]->as<int2>(), cnt + 2 * k,
-                                             cnt + 2 * k + 1, next, next_count, tiers[k].half, spill_error)
+                                             cnt + 2 * k + 1, next, next_count, tiers[k].half, spill_error, n_slots)
                             : wp_launch_engine(C, hb, tiers[k].threads,
                                                wp_engine_smem_bytes(tiers[k].half, 0, hb, tiers[k].threads),
                                                ctx->stream, a, lists[k]->as<int2>(), cnt + 2 * k, cnt + 2 * k + 1,
-                                               next, next_count, tiers[k].half, 0, spill_error,
+                                               next, next_count, tiers[k].half, 0, spill_error, n_slots,
                                                k == 0 ? &ctx->last_engine_grid : nullptr),
                     "engine pass");
             ctx->launches++;
         }
         if (dense) {
             TimedLaunch tl(ctx, 0);
-            WP_CUDA(wp_launch_dense(hb, T, C, (size_t)ctx->smem_optin, ctx->stream, a), "dense launch");
+            WP_CUDA(wp_launch_dense(hb, T, C, (size_t)ctx->smem_optin, ctx->stream, a, n_slots), "dense launch");
             ctx->launches++;
         }
         if (mode == MODE_CLASSIFY) {
@@ -777,6 +778,7 @@ wp_status run_batch(wp_ctx* ctx, const double* d_rads, int R, double dist_cutoff
             rp.hb = hb;
             rp.nt = nt;
             rp.dense = dense;
+            rp.pairs = n_slots;
             for (int k = 0; k < nt; k++) {
                 rp.threads[k] = tiers[k].threads;
                 rp.half[k] = tiers[k].half;
@@ -810,14 +812,21 @@ wp_status check_ready(wp_ctx* ctx) {
     return WP_OK;
 }
 
+// The status for a batch's nonzero error word.
+wp_status batch_error(wp_ctx* ctx, int err) {
+    if (err == 2) return fail(ctx, WP_ERR_UNSUPPORTED, "a pair's state exceeds every shared-memory shape");
+    return fail(ctx, WP_ERR_CUDA, "internal: peptide state exceeded its shape");
+}
+
 wp_status finish(wp_ctx* ctx) {
     WP_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
     int err = 0;
     WP_CUDA(cudaMemcpy(&err, ctx->d_err.p, sizeof(int), cudaMemcpyDeviceToHost), "read err");
-    if (err == 2) return fail(ctx, WP_ERR_UNSUPPORTED, "a pair's state exceeds every shared-memory shape");
-    if (err) return fail(ctx, WP_ERR_CUDA, "internal: peptide state exceeded its shape");
-    return WP_OK;
+    return err ? batch_error(ctx, err) : WP_OK;
 }
+
+// Reads up to which a classify call's outputs go through page-locked memory.
+constexpr int SMALL_READS = 4096;
 
 // ChannelModel::adjusted_mu (parameterization/model/channel-model.h:35-54)
 // on the host, for the kNN entry coordinates.
@@ -1830,6 +1839,7 @@ void wp_ctx_destroy(wp_ctx* ctx) {
     if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
     collect_timing(ctx);
     cudaStreamDestroy(ctx->stream);
+    if (ctx->h_small) cudaFreeHost(ctx->h_small);
     delete ctx;
 }
 
@@ -1904,16 +1914,16 @@ wp_status wp_engine_replay(wp_ctx* ctx, int reps, double* ms) {
             int* next_count = last ? rp.cnt + WP_CNT_DENSE : rp.cnt + 2 * (k + 1);
             WP_CUDA(rp.lanes[k] > 0
                             ? wp_launch_coop(rp.C, rp.hb, rp.lanes[k], ctx->stream, a, rp.list[k], rp.cnt + 2 * k,
-                                             rp.cnt + 2 * k + 1, next, next_count, rp.half[k], 1)
+                                             rp.cnt + 2 * k + 1, next, next_count, rp.half[k], 1, rp.pairs)
                             : wp_launch_engine(rp.C, rp.hb, rp.threads[k],
                                                wp_engine_smem_bytes(rp.half[k], 0, rp.hb, rp.threads[k]), ctx->stream,
                                                a, rp.list[k], rp.cnt + 2 * k, rp.cnt + 2 * k + 1, next, next_count,
-                                               rp.half[k], 0, 1, nullptr),
+                                               rp.half[k], 0, 1, rp.pairs, nullptr),
                     "engine pass");
             ctx->launches++;
         }
         if (rp.dense) {
-            WP_CUDA(wp_launch_dense(rp.hb, rp.T, rp.C, (size_t)ctx->smem_optin, ctx->stream, a), "dense launch");
+            WP_CUDA(wp_launch_dense(rp.hb, rp.T, rp.C, (size_t)ctx->smem_optin, ctx->stream, a, rp.pairs), "dense launch");
             ctx->launches++;
         }
     }
@@ -2033,6 +2043,30 @@ wp_status wp_hmm_classify(wp_ctx* ctx, const double* rads, int R, double dist_cu
     }
     st = upload_reads(ctx, rads, R);
     if (st != WP_OK) return st;
+    if (R <= SMALL_READS) {
+        // a small batch: the outputs side by side and through page-locked memory
+        // (a copy to pageable memory takes some 9 us of its own, and there were
+        // five): score, total, log score, id, then the error word
+        const size_t r = (size_t)R;
+        WP_CUDA(ctx->d_small.ensure(28 * (size_t)SMALL_READS), "alloc out");
+        if (!ctx->h_small)
+            WP_CUDA(cudaHostAlloc(&ctx->h_small, 28 * (size_t)SMALL_READS + sizeof(int), cudaHostAllocDefault), "alloc out");
+        double* d = ctx->d_small.as<double>();
+        st = run_batch(ctx, ctx->d_rads.as<double>(), R, dist_cutoff, cand, cand_off, MODE_CLASSIFY, nullptr,
+                       reinterpret_cast<int32_t*>(d + 3 * r), d, d + r, d + 2 * r, nullptr);
+        if (st != WP_OK) return st;
+        char* h = static_cast<char*>(ctx->h_small);
+        WP_CUDA(cudaMemcpyAsync(h + 28 * r, ctx->d_err.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "copy out");
+        WP_CUDA(cudaMemcpyAsync(h, d, 28 * r, cudaMemcpyDeviceToHost, ctx->stream), "copy out");
+        WP_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
+        memcpy(out_score, h, 8 * r);
+        memcpy(out_total, h + 8 * r, 8 * r);
+        if (out_log_score) memcpy(out_log_score, h + 16 * r, 8 * r);
+        memcpy(out_id, h + 24 * r, 4 * r);
+        int err = 0;
+        memcpy(&err, h + 28 * r, sizeof(int));
+        return err ? batch_error(ctx, err) : WP_OK;
+    }
     WP_CUDA(ctx->d_out_id.ensure(sizeof(int32_t) * R), "alloc out");
     WP_CUDA(ctx->d_out_score.ensure(sizeof(double) * R), "alloc out");
     WP_CUDA(ctx->d_out_total.ensure(sizeof(double) * R), "alloc out");

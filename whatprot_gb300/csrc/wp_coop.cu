@@ -30,6 +30,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "wp_common.cuh"
 #include "wp_engine.cuh"
 
@@ -584,45 +586,45 @@ size_t wp_coop_smem_bytes(int slab_half, bool has_block, int lanes) {
 int wp_coop_max_half() { return WP_COOP_IDX; }
 
 template <int C, bool HB, int G>
-static cudaError_t launch_coop(cudaStream_t s, const BatchArgs& a, const EngineLists& L) {
+static cudaError_t launch_coop(cudaStream_t s, const BatchArgs& a, const EngineLists& L, long pairs) {
     const size_t smem = wp_coop_smem_bytes(L.slab_half, HB, G);
-    cudaError_t e = cudaFuncSetAttribute(wp_coop_kernel<C, HB, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wp_coop_kernel<C, HB, G>, WP_COOP_THREADS, smem);
+    int sms = 0, per_sm = 0;
+    const cudaError_t e = wp_launch_shape(reinterpret_cast<const void*>(wp_coop_kernel<C, HB, G>), WP_COOP_THREADS,
+                                          smem, &per_sm, &sms);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    wp_coop_kernel<C, HB, G><<<sms * per_sm, WP_COOP_THREADS, smem, s>>>(a, L);
+    constexpr int in_hand = WP_COOP_THREADS / G;  // pairs of a CTA
+    const int grid = std::max(1, (int)std::min<long>((long)sms * per_sm, (pairs + in_hand - 1) / in_hand));
+    wp_coop_kernel<C, HB, G><<<grid, WP_COOP_THREADS, smem, s>>>(a, L);
     return cudaGetLastError();
 }
 
 template <int C, bool HB>
-static cudaError_t launch_coop_lanes(int lanes, cudaStream_t s, const BatchArgs& a, const EngineLists& L) {
+static cudaError_t launch_coop_lanes(int lanes, cudaStream_t s, const BatchArgs& a, const EngineLists& L,
+                                     long pairs) {
     switch (lanes) {
-        case 8: return launch_coop<C, HB, 8>(s, a, L);
-        case 16: return launch_coop<C, HB, 16>(s, a, L);
+        case 8: return launch_coop<C, HB, 8>(s, a, L, pairs);
+        case 16: return launch_coop<C, HB, 16>(s, a, L, pairs);
         default: return cudaErrorInvalidValue;
     }
 }
 
-// One pass over a work list, `lanes` lanes per pair (persistent grid).
+// One pass over a work list of at most `pairs`, `lanes` lanes per pair (persistent
+// grid).
 cudaError_t wp_launch_coop(int C, bool has_block, int lanes, cudaStream_t s, const BatchArgs& a, const int2* in,
                            const int* in_count, int* in_head, int2* out, int* out_count, int slab_half,
-                           int spill_error) {
+                           int spill_error, long pairs) {
     if (slab_half > WP_COOP_IDX) return cudaErrorInvalidValue;
     EngineLists L{in, in_count, in_head, out, out_count, slab_half, 0, spill_error};
     switch (C * 2 + (has_block ? 1 : 0)) {
-        case 2: return launch_coop_lanes<1, false>(lanes, s, a, L);
-        case 3: return launch_coop_lanes<1, true>(lanes, s, a, L);
-        case 4: return launch_coop_lanes<2, false>(lanes, s, a, L);
-        case 5: return launch_coop_lanes<2, true>(lanes, s, a, L);
-        case 6: return launch_coop_lanes<3, false>(lanes, s, a, L);
-        case 7: return launch_coop_lanes<3, true>(lanes, s, a, L);
-        case 8: return launch_coop_lanes<4, false>(lanes, s, a, L);
-        case 9: return launch_coop_lanes<4, true>(lanes, s, a, L);
+        case 2: return launch_coop_lanes<1, false>(lanes, s, a, L, pairs);
+        case 3: return launch_coop_lanes<1, true>(lanes, s, a, L, pairs);
+        case 4: return launch_coop_lanes<2, false>(lanes, s, a, L, pairs);
+        case 5: return launch_coop_lanes<2, true>(lanes, s, a, L, pairs);
+        case 6: return launch_coop_lanes<3, false>(lanes, s, a, L, pairs);
+        case 7: return launch_coop_lanes<3, true>(lanes, s, a, L, pairs);
+        case 8: return launch_coop_lanes<4, false>(lanes, s, a, L, pairs);
+        case 9: return launch_coop_lanes<4, true>(lanes, s, a, L, pairs);
         default: return cudaErrorInvalidValue;
     }
 }

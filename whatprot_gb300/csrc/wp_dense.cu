@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "wp_common.cuh"
+#include "wp_engine.cuh"
 
 #define WP_DENSE_WARPS 8
 
@@ -493,7 +494,7 @@ bool wp_dense_fits(int T, int S_cap, int C, bool has_block, size_t smem_optin) {
 }
 
 template <int C, bool HAS_BLOCK>
-static cudaError_t launch_dense(int T, size_t smem_optin, cudaStream_t stream, const BatchArgs& a) {
+static cudaError_t launch_dense(int T, size_t smem_optin, cudaStream_t stream, const BatchArgs& a, long pairs) {
     // Small class: as many states as let 4 CTAs share an SM (228 KB, 1 KB of
     // it per CTA the system's).
     const size_t fixed = dense_fixed_bytes();
@@ -511,31 +512,29 @@ static cudaError_t launch_dense(int T, size_t smem_optin, cudaStream_t stream, c
     }
     const size_t smem = fixed + arena;
     if (smem > smem_optin) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(wp_dense_kernel<C, HAS_BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wp_dense_kernel<C, HAS_BLOCK>, WP_DENSE_WARPS * 32, smem);
+    int sms = 0, per_sm = 0;
+    const cudaError_t e = wp_launch_shape(reinterpret_cast<const void*>(wp_dense_kernel<C, HAS_BLOCK>),
+                                          WP_DENSE_WARPS * 32, smem, &per_sm, &sms);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    wp_dense_kernel<C, HAS_BLOCK><<<sms * per_sm, WP_DENSE_WARPS * 32, smem, stream>>>(a, ps);
+    const int grid =
+            std::max(1, (int)std::min<long>((long)sms * per_sm, (pairs + WP_DENSE_WARPS - 1) / WP_DENSE_WARPS));
+    wp_dense_kernel<C, HAS_BLOCK><<<grid, WP_DENSE_WARPS * 32, smem, stream>>>(a, ps);
     return cudaGetLastError();
 }
 
-// Persistent grid over the dense list (BatchArgs::ovf).
+// Persistent grid over the dense list (BatchArgs::ovf, at most `pairs`).
 cudaError_t wp_launch_dense(bool has_block, int T, int C, size_t smem_optin, cudaStream_t stream,
-                            const BatchArgs& a) {
+                            const BatchArgs& a, long pairs) {
     switch (C * 2 + (has_block ? 1 : 0)) {
-        case 2: return launch_dense<1, false>(T, smem_optin, stream, a);
-        case 3: return launch_dense<1, true>(T, smem_optin, stream, a);
-        case 4: return launch_dense<2, false>(T, smem_optin, stream, a);
-        case 5: return launch_dense<2, true>(T, smem_optin, stream, a);
-        case 6: return launch_dense<3, false>(T, smem_optin, stream, a);
-        case 7: return launch_dense<3, true>(T, smem_optin, stream, a);
-        case 8: return launch_dense<4, false>(T, smem_optin, stream, a);
-        case 9: return launch_dense<4, true>(T, smem_optin, stream, a);
+        case 2: return launch_dense<1, false>(T, smem_optin, stream, a, pairs);
+        case 3: return launch_dense<1, true>(T, smem_optin, stream, a, pairs);
+        case 4: return launch_dense<2, false>(T, smem_optin, stream, a, pairs);
+        case 5: return launch_dense<2, true>(T, smem_optin, stream, a, pairs);
+        case 6: return launch_dense<3, false>(T, smem_optin, stream, a, pairs);
+        case 7: return launch_dense<3, true>(T, smem_optin, stream, a, pairs);
+        case 8: return launch_dense<4, false>(T, smem_optin, stream, a, pairs);
+        case 9: return launch_dense<4, true>(T, smem_optin, stream, a, pairs);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -51,6 +51,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "wp_common.cuh"
 #include "wp_engine.cuh"
 
@@ -990,37 +992,35 @@ size_t wp_engine_smem_bytes(int slab_half, int scr_floats, bool has_block, int t
 
 template <int C, bool HB>
 static cudaError_t launch_engine(int threads, size_t smem, cudaStream_t s, const BatchArgs& a,
-                                 const EngineLists& L, int* grid_out) {
-    cudaError_t e = cudaFuncSetAttribute(wp_engine_kernel<C, HB>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wp_engine_kernel<C, HB>, threads, smem);
+                                 const EngineLists& L, long pairs, int* grid_out) {
+    int sms = 0, per_sm = 0;
+    const cudaError_t e =
+            wp_launch_shape(reinterpret_cast<const void*>(wp_engine_kernel<C, HB>), threads, smem, &per_sm, &sms);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    int grid = sms * per_sm;
+    // no more CTAs than pairs that could come
+    const int grid = std::max(1, (int)std::min<long>((long)sms * per_sm, (pairs + threads - 1) / threads));
     if (grid_out) *grid_out = grid;
     wp_engine_kernel<C, HB><<<grid, threads, smem, s>>>(a, L);
     return cudaGetLastError();
 }
 
-// One engine pass over a work list (persistent grid: SMs x resident CTAs).
+// One engine pass over a work list of at most `pairs` (persistent grid: SMs x
+// resident CTAs).
 cudaError_t wp_launch_engine(int C, bool has_block, int threads, size_t smem, cudaStream_t s,
                              const BatchArgs& a, const int2* in, const int* in_count, int* in_head,
                              int2* out, int* out_count, int slab_half, int scr_floats,
-                             int spill_error, int* grid_out) {
+                             int spill_error, long pairs, int* grid_out) {
     EngineLists L{in, in_count, in_head, out, out_count, slab_half, scr_floats, spill_error};
     switch (C * 2 + (has_block ? 1 : 0)) {
-        case 2: return launch_engine<1, false>(threads, smem, s, a, L, grid_out);
-        case 3: return launch_engine<1, true>(threads, smem, s, a, L, grid_out);
-        case 4: return launch_engine<2, false>(threads, smem, s, a, L, grid_out);
-        case 5: return launch_engine<2, true>(threads, smem, s, a, L, grid_out);
-        case 6: return launch_engine<3, false>(threads, smem, s, a, L, grid_out);
-        case 7: return launch_engine<3, true>(threads, smem, s, a, L, grid_out);
-        case 8: return launch_engine<4, false>(threads, smem, s, a, L, grid_out);
-        case 9: return launch_engine<4, true>(threads, smem, s, a, L, grid_out);
+        case 2: return launch_engine<1, false>(threads, smem, s, a, L, pairs, grid_out);
+        case 3: return launch_engine<1, true>(threads, smem, s, a, L, pairs, grid_out);
+        case 4: return launch_engine<2, false>(threads, smem, s, a, L, pairs, grid_out);
+        case 5: return launch_engine<2, true>(threads, smem, s, a, L, pairs, grid_out);
+        case 6: return launch_engine<3, false>(threads, smem, s, a, L, pairs, grid_out);
+        case 7: return launch_engine<3, true>(threads, smem, s, a, L, pairs, grid_out);
+        case 8: return launch_engine<4, false>(threads, smem, s, a, L, pairs, grid_out);
+        case 9: return launch_engine<4, true>(threads, smem, s, a, L, pairs, grid_out);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -40,10 +40,10 @@ __global__ void wp_reduce_kernel(BatchArgs, int32_t*, double*, double*, double*,
 cudaError_t wp_launch_engine(int C, bool has_block, int threads, size_t smem, cudaStream_t s,
                              const BatchArgs& a, const int2* in, const int* in_count, int* in_head,
                              int2* out, int* out_count, int slab_half, int scr_floats,
-                             int spill_error, int* grid_out);
+                             int spill_error, long pairs, int* grid_out);
 size_t wp_engine_smem_bytes(int slab_half, int scr_floats, bool has_block, int threads);
 cudaError_t wp_launch_dense(bool has_block, int T, int C, size_t smem_optin, cudaStream_t stream,
-                            const BatchArgs& a);
+                            const BatchArgs& a, long pairs);
 bool wp_dense_fits(int T, int S_cap, int C, bool has_block, size_t smem_optin);
 
 namespace {
@@ -242,12 +242,12 @@ extern "C" wp_status wp_hmm_classify_noalloc(int device, const wp_seq_model* m, 
     wp_compact_kernel<<<R, 256, 0, s>>>(a);
     WP_NA(cudaGetLastError());
     WP_NA(wp_launch_engine(C, hb, 256, wp_engine_smem_bytes(half1, 0, hb, 256), s, a, a.work, cnt + 0,
-                           cnt + 1, reinterpret_cast<int2*>(base + o_ovf1), cnt + 2, half1, 0, 0, nullptr));
+                           cnt + 1, reinterpret_cast<int2*>(base + o_ovf1), cnt + 2, half1, 0, 0, (long)R * P, nullptr));
     WP_NA(wp_launch_engine(C, hb, 128, wp_engine_smem_bytes(half2, 0, hb, 128), s, a,
                            reinterpret_cast<int2*>(base + o_ovf1), cnt + 2, cnt + 3,
                            reinterpret_cast<int2*>(base + o_ovf2), cnt + 4, half2, 0,
-                           dense ? 0 : 1, nullptr));
-    if (dense) WP_NA(wp_launch_dense(hb, T, C, smem_optin, s, a));
+                           dense ? 0 : 1, (long)R * P, nullptr));
+    if (dense) WP_NA(wp_launch_dense(hb, T, C, smem_optin, s, a, (long)R * P));
     wp_reduce_kernel<<<(R + 3) / 4, 128, 0, s>>>(a, reinterpret_cast<int32_t*>(base + o_id),
                                                  reinterpret_cast<double*>(base + o_sc),
                                                  reinterpret_cast<double*>(base + o_tot), nullptr,
