@@ -60,3 +60,32 @@ def test_dense_slab_classes_vs_oracle(gpu_ctx, oracle, block):
     assert gpu_ctx.last_batch_stats()["dense"] > 0
     o = oracle.loglik_all(sm, 16, ds, rads, DBL_MAX, threads=8)
     assert_logp_close(g, o, "dense classes")
+
+
+@pytest.mark.parametrize("block,cut", [(False, DBL_MAX), (True, 4.0)])
+def test_passes_side_by_side(gpu_ctx, block, cut):
+    """A batch large enough for its passes to run side by side (65,536 pairs):
+    read by read the numbers of smaller batches, run directly and as a replayed
+    graph."""
+    import torch
+    sm = _model(3, block)
+    ds = random_dye_seqs(110, 3, 8, 26, max_per_channel=4, min_total=1, seed=11)
+    rads, _ = simulate_radiometries(sm, ds, 12, 700, seed=12)
+    R = len(rads)  # some reads are not detectable
+    assert R * 110 >= 65536
+    gpu_ctx.upload_model(sm, 12)
+    gpu_ctx.upload_peptides(ds)
+    whole = gpu_ctx.classify(rads, cut)
+    for lo in (0, 350):
+        for a, b in zip(gpu_ctx.classify(rads[lo:lo + 350], cut), whole):
+            assert np.array_equal(a, b[lo:lo + 350])
+    d = torch.from_numpy(rads).cuda()
+    oid = torch.zeros(R, dtype=torch.int32, device="cuda")
+    osc, otot = (torch.zeros(R, dtype=torch.float64, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    for _ in range(4):
+        oid.zero_()
+        osc.zero_()
+        torch.cuda.synchronize()
+        gpu_ctx.classify_device(d.data_ptr(), R, cut, oid.data_ptr(), osc.data_ptr(), otot.data_ptr(), async_=False)
+        assert np.array_equal(oid.cpu().numpy(), whole[0]) and np.array_equal(osc.cpu().numpy(), whole[1])
