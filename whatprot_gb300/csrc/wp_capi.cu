@@ -3168,6 +3168,14 @@ struct wp_mlp {
     DevBuf W1b, W2b, W3b;  // BF16 copies
     DevBuf X, Z1, H1, Z2, H2, dL, dZ2, dZ1, L, dH2, dH1, loss, labels, xsim, err;
     DevBuf topi, topp, mass, counts, loss_sum, tkfail;
+    // a training step's small reductions beside its large products
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+    ~wp_mlp() {
+        for (cudaEvent_t e : ev)
+            if (e) cudaEventDestroy(e);
+        if (side) cudaStreamDestroy(side);
+    }
 };
 
 namespace {
@@ -3182,9 +3190,10 @@ typedef __nv_bfloat16 bf16;
 
 // a_mn, b_mn: the operand is stored with K as its rows (wp_gemm_bf16).
 wp_status mlp_gemm(wp_ctx* ctx, wp_mlp* m, const void* A, int lda, bool a_mn, const void* B, int ldb, bool b_mn,
-                   int M, int N, int K, void* C, int ldc, int c_fp32, const float* bias, int act, void* Z) {
+                   int M, int N, int K, void* C, int ldc, int c_fp32, const float* bias, int act, void* Z,
+                   cudaStream_t s = nullptr) {
     cudaError_t e = wp_gemm_bf16(A, lda, a_mn, B, ldb, b_mn, M, N, K, C, ldc, c_fp32, bias, act, Z,
-                                 m->err.as<int>(), ctx->stream);
+                                 m->err.as<int>(), s ? s : ctx->stream);
     ctx->launches++;
     if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor-core GEMM launch");
     return WP_OK;
@@ -3236,24 +3245,40 @@ wp_status mlp_step(wp_ctx* ctx, wp_mlp* m, const int* labels, int B, float lr) {
     MLP_CUDA(wp_mlp_launch_softmax_ce(m->L.as<float>(), B, m->P, Pp, labels, 1.0f / (float)B,
                                       m->dL.as<bf16>(), m->loss.as<double>(), s), "softmax");
     ctx->launches++;
-    st = mlp_gemm(ctx, m, m->dL.p, Pp, true, m->H2.p, H, true, Pp, H, B, m->g[4].p, H, 1, nullptr, 0, nullptr);  // dW3
-    if (st != WP_OK) return st;
-    MLP_CUDA(wp_mlp_launch_colsum(m->dL.as<bf16>(), B, Pp, Pp, m->g[5].as<float>(), s), "colsum");
+    // The bias gradients (column sums) and dW1 take few SMs; they run on a second
+    // stream, on the SMs that the large products leave (128 and 126 of 152), dW3
+    // last so that there is something to run beside it.  4,096 x 20,000, 1,024
+    // wide: 1,007 us a step on one stream, 905 so.
+    if (!m->side) MLP_CUDA(cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking), "side stream");
+    for (cudaEvent_t& e : m->ev)
+        if (!e) MLP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "side event");
+    cudaStream_t side = m->side;
+    auto fork = [&](int i) {
+        cudaError_t e = cudaEventRecord(m->ev[i], s);
+        return e != cudaSuccess ? e : cudaStreamWaitEvent(side, m->ev[i], 0);
+    };
+    MLP_CUDA(fork(0), "fork");
+    MLP_CUDA(wp_mlp_launch_colsum(m->dL.as<bf16>(), B, Pp, Pp, m->g[5].as<float>(), side), "colsum");
     st = mlp_gemm(ctx, m, m->dL.p, Pp, false, m->W3b.p, H, true, B, H, Pp, m->dH2.p, H, 1, nullptr, 0, nullptr);  // dH2
     if (st != WP_OK) return st;
     MLP_CUDA(wp_mlp_launch_gelu_bwd(m->dH2.as<float>(), m->Z2.as<bf16>(), (long)B * H, m->dZ2.as<bf16>(), s), "gelu'");
-    ctx->launches += 2;
-    st = mlp_gemm(ctx, m, m->dZ2.p, H, true, m->H1.p, H, true, H, H, B, m->g[2].p, H, 1, nullptr, 0, nullptr);  // dW2
-    if (st != WP_OK) return st;
-    MLP_CUDA(wp_mlp_launch_colsum(m->dZ2.as<bf16>(), B, H, H, m->g[3].as<float>(), s), "colsum");
+    MLP_CUDA(fork(1), "fork");
+    MLP_CUDA(wp_mlp_launch_colsum(m->dZ2.as<bf16>(), B, H, H, m->g[3].as<float>(), side), "colsum");
     st = mlp_gemm(ctx, m, m->dZ2.p, H, false, m->W2b.p, H, true, B, H, H, m->dH1.p, H, 1, nullptr, 0, nullptr);  // dH1
     if (st != WP_OK) return st;
     MLP_CUDA(wp_mlp_launch_gelu_bwd(m->dH1.as<float>(), m->Z1.as<bf16>(), (long)B * H, m->dZ1.as<bf16>(), s), "gelu'");
-    ctx->launches += 2;
-    st = mlp_gemm(ctx, m, m->dZ1.p, H, true, m->X.p, 64, true, H, 64, B, m->g[0].p, 64, 1, nullptr, 0, nullptr);  // dW1
+    MLP_CUDA(fork(2), "fork");
+    st = mlp_gemm(ctx, m, m->dZ1.p, H, true, m->X.p, 64, true, H, 64, B, m->g[0].p, 64, 1, nullptr, 0, nullptr,
+                  side);  // dW1
     if (st != WP_OK) return st;
-    MLP_CUDA(wp_mlp_launch_colsum(m->dZ1.as<bf16>(), B, H, H, m->g[1].as<float>(), s), "colsum");
-    ctx->launches++;
+    MLP_CUDA(wp_mlp_launch_colsum(m->dZ1.as<bf16>(), B, H, H, m->g[1].as<float>(), side), "colsum");
+    MLP_CUDA(cudaEventRecord(m->ev[3], side), "join");
+    st = mlp_gemm(ctx, m, m->dZ2.p, H, true, m->H1.p, H, true, H, H, B, m->g[2].p, H, 1, nullptr, 0, nullptr);  // dW2
+    if (st != WP_OK) return st;
+    st = mlp_gemm(ctx, m, m->dL.p, Pp, true, m->H2.p, H, true, Pp, H, B, m->g[4].p, H, 1, nullptr, 0, nullptr);  // dW3
+    if (st != WP_OK) return st;
+    MLP_CUDA(cudaStreamWaitEvent(s, m->ev[3], 0), "join");
+    ctx->launches += 5;
     if (lr > 0.0f) {
         m->steps++;
         const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;

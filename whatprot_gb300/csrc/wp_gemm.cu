@@ -500,7 +500,10 @@ static cudaError_t gemm_launch(const CUtensorMap& ma, const CUtensorMap& mb, con
     cudaError_t e = cudaFuncSetAttribute(wp_gemm_tn_kernel<AMN, BMN, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    const int grid = std::min(gemm_tiles(p.M, p.N, BN), gemm_sms());
+    // as few CTAs as take the same number of tiles in turn: the SMs left over are
+    // free for kernels on other streams
+    const int tiles = gemm_tiles(p.M, p.N, BN), turns = (tiles + gemm_sms() - 1) / gemm_sms();
+    const int grid = (tiles + turns - 1) / turns;
     wp_gemm_tn_kernel<AMN, BMN, BN><<<grid, GEMM_THREADS, smem, s>>>(ma, mb, p);
     return cudaGetLastError();
 }
