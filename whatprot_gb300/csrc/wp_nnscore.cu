@@ -17,9 +17,10 @@
 // above 1e-8 of the largest weight) come from FP64 distances, as the reference
 // forms them, the far ones' from FP32 (their error is below 1e-8 of the largest
 // weight).  FP64 distances are summed from a per-read table of squared
-// differences; that and FP64 exp are what bounds the kernel: 108 FP64
-// instructions per 32 near tracks at 16 cycles each on this GPU's FP64 pipe.
-// 4,000 reads with 5,600 kept tracks, 20,000 ids: 9.7 ms, against 22.1 ms for a
+// differences, for the near tracks of a chunk side by side; that and FP64 exp (108
+// FP64 instructions per 32 near tracks at 16 cycles each on this GPU's FP64 pipe)
+// and the chain of barriers are what bounds the kernel.  4,000 reads with 5,600
+// kept tracks, 20,000 ids: 8.7 ms, 9.7 with near and far places mixed, against 22.1 ms for a
 // warp per read with its scores in global memory (780 MB of scattered
 // accumulators over the resident warps, beyond L2).
 #include <cuda_runtime.h>
@@ -35,7 +36,7 @@
 
 // Shared memory after the U scores and their bits.
 struct SCSmem {
-    double val[SC_SLAB];     // then the selected scores
+    double val[SC_SLAB];     // before them a chunk's near tracks (place, track), then the selected scores
     int id[SC_SLAB];         // then their ids
     double w[SC_THREADS];    // weights of the tracks in hand
     int s0[SC_THREADS];      // their first sources
@@ -45,7 +46,7 @@ struct SCSmem {
     unsigned hist[256];
     double red[SC_WARPS];
     int redi[SC_WARPS];
-    int item, digit, before, nsel;
+    int item, digit, before, nsel, nnear;
 };
 
 __device__ __forceinline__ int sc_scan_incl(int v, int* redi) {
@@ -164,31 +165,48 @@ __global__ void __launch_bounds__(SC_THREADS, 2) wp_nn_score_kernel(NNScoreArgs 
 
         // ---- the tracks' contributions
         double total_part = 0.0;
+        int2* near_list = reinterpret_cast<int2*>(s.val);
+        if (tid == 0) s.nnear = 0;
+        __syncthreads();
         for (int c0 = 0; c0 < n; c0 += SC_THREADS) {
             const int i = c0 + tid;
             int ns = 0;
             const int e = i < n ? a.kept_pos[base + i] : -1;
+            bool near = false;
             if (e >= 0) {
                 const float d2 = a.kept_d2[base + i];
-                double w;
-                if (q64 && (double)d2 < wlim) {
-                    const double d64 = a.table ? sc_d64(a.cnt + (long)e * a.DP, sq, a.NC, a.TC)
-                                               : wp_nn_exact_d2(q64, e, a.TC, a.C, a.DP, a.cnt, a.ctab, a.NC, a.ecoord);
-                    w = exp(-d64 / a.two_sig_sq);
-                } else {
+                near = q64 && (double)d2 < wlim;
+                if (!near) {
                     // 2^x: exp2f of the fraction, the integer part applied in FP64 so
                     // far entries keep a non-zero weight
                     const float x = -d2 * a.inv_two_sig_sq * 1.4426950408889634f;
                     const float fl = floorf(x);
-                    w = ldexp((double)exp2f(x - fl), (int)fl);
+                    s.w[tid] = ldexp((double)exp2f(x - fl), (int)fl);
                 }
                 const int f = a.src_off[e];
-                s.w[tid] = w;
                 s.s0[tid] = f;
                 ns = a.src_off[e + 1] - f;
             }
+            // the near tracks in hand side by side, so that the FP64 work fills warps
+            // (a list has gaps, and near and far places mixed)
+            {
+                const unsigned nm = __ballot_sync(0xffffffffu, near);
+                int at = 0;
+                if (lane == 0 && nm) at = atomicAdd(&s.nnear, __popc(nm));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (near) near_list[at + __popc(nm & ((1u << lane) - 1u))] = make_int2(tid, e);
+            }
+            __syncthreads();
+            const int nnear = s.nnear;
+            if (tid < nnear) {
+                const int2 t = near_list[tid];
+                const double d64 = a.table ? sc_d64(a.cnt + (long)t.y * a.DP, sq, a.NC, a.TC)
+                                           : wp_nn_exact_d2(q64, t.y, a.TC, a.C, a.DP, a.cnt, a.ctab, a.NC, a.ecoord);
+                s.w[t.x] = exp(-d64 / a.two_sig_sq);
+            }
             const int incl = sc_scan_incl(ns, s.redi);
             s.pre[tid] = incl;
+            if (tid == 0) s.nnear = 0;  // everyone has read it (the scan's barriers)
             __syncthreads();
             if (wid == 0) {
                 // batches of up to 32 sources, those of each 32 list places apart
