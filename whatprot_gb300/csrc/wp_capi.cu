@@ -608,15 +608,19 @@ wp_status run_batch(wp_ctx* ctx, const double* d_rads, int R, double dist_cutoff
                 ctx->d_hi.as<uint8_t>(), ctx->d_table.as<EmitEntry>(), entries);
         ctx->launches++;
         WP_CUDA(cudaGetLastError(), "prep launch");
-        wp_read_summary_kernel<<<(R + 127) / 128, 128, 0, ctx->stream>>>(a);
-        ctx->launches++;
-        WP_CUDA(cudaGetLastError(), "summary launch");
+        if (!window_factors) {
+            wp_read_summary_kernel<<<(R + 127) / 128, 128, 0, ctx->stream>>>(a);
+            ctx->launches++;
+            WP_CUDA(cudaGetLastError(), "summary launch");
+        }
         if (window_factors) {
-            const size_t wsm = wp_window_smem_bytes(C, W, 128);
+            // with the boxes' summary: whole reads per CTA
+            const int rpc = WP_WINDOW_THREADS / T;
+            const size_t wsm = wp_window_smem_bytes(C, W, WP_WINDOW_THREADS);
             int per_sm = 0, sms = 0;
-            WP_CUDA(wp_launch_shape(reinterpret_cast<const void*>(wp_window_factors_kernel), 128, wsm, &per_sm, &sms),
+            WP_CUDA(wp_launch_shape(reinterpret_cast<const void*>(wp_window_factors_kernel), WP_WINDOW_THREADS, wsm, &per_sm, &sms),
                     "window factors shape");
-            wp_window_factors_kernel<<<(int)((n + 127) / 128), 128, wsm, ctx->stream>>>(a);
+            wp_window_factors_kernel<<<(R + rpc - 1) / rpc, WP_WINDOW_THREADS, wsm, ctx->stream>>>(a);
             ctx->launches++;
             WP_CUDA(cudaGetLastError(), "window factors launch");
         }

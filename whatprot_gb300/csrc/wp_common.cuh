@@ -27,6 +27,7 @@
 #define WP_CNT_DENSE (2 * WP_MAX_TIERS)
 #define WP_CNT_LIVE (2 * WP_MAX_TIERS + 3)
 #define WP_CNT_N (2 * WP_MAX_TIERS + 4)
+#define WP_WINDOW_THREADS 128  // threads (read, timestep) per CTA of wp_window_factors_kernel, at least WP_MAX_TIMESTEPS
 #define WP_GROUP_WARPS 8      // warps per CTA of wp_compact_groups_kernel (one read at a time each)
 #define WP_GROUP_MAX 512      // dye-count vectors (groups) that kernel takes
 #define WP_GROUP_PERM_SMEM 8192  // peptides up to which it stages the shape order in shared memory
