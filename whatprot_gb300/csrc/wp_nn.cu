@@ -202,7 +202,7 @@ __device__ __forceinline__ void nn_load_tile(const NNArgs& a, int e0, int e_end,
 // tracks of 5,000 peptides x 60, 36 coordinates: 3.5 ms, 6.0 with a query per
 // lane and all 48 padded coordinates.
 template <int DP, int DQ>
-__global__ void __launch_bounds__(NN_THREADS, DQ > 12 ? 1 : 2) wp_nn_hist_kernel(NNArgs a) {
+__global__ void __launch_bounds__(NN_THREADS, DQ > 9 ? 1 : 2) wp_nn_hist_kernel(NNArgs a) {
     extern __shared__ __align__(16) unsigned char nn_smem[];
     float* tile = reinterpret_cast<float*>(nn_smem);
     int* thits = reinterpret_cast<int*>(tile + NN_TE * DP);
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(NN_THREADS, DQ > 12 ? 1 : 2) wp_nn_hist_kernel
 // the GPU (4,000 reads: 0.34 ms, against 3.6 ms with a CTA per 256 reads; two
 // queries per lane: 10,007 reads of 36 coordinates 0.75 -> 0.49 ms).
 template <int DP, int DQ>
-__global__ void __launch_bounds__(NN_THREADS, DQ > 12 ? 1 : 2) wp_nn_estimate_kernel(NNArgs a) {
+__global__ void __launch_bounds__(NN_THREADS, DQ > 9 ? 1 : 2) wp_nn_estimate_kernel(NNArgs a) {
     extern __shared__ __align__(16) unsigned char nn_smem[];
     float* tile = reinterpret_cast<float*>(nn_smem);
     int* thits = reinterpret_cast<int*>(tile + NN_TE * DP);
@@ -455,7 +455,7 @@ __global__ void wp_nn_threshold_kernel(NNArgs a) {
 // alike and write them in entry order.  The reads above: 4.8 ms, 6.1 with a query
 // per lane (45 million candidates written one by one).
 template <int DP, int DQ>
-__global__ void __launch_bounds__(NN_THREADS, DQ > 12 ? 1 : 2) wp_nn_collect_kernel(NNArgs a) {
+__global__ void __launch_bounds__(NN_THREADS, DQ > 9 ? 1 : 2) wp_nn_collect_kernel(NNArgs a) {
     extern __shared__ __align__(16) unsigned char nn_smem[];
     float* tile = reinterpret_cast<float*>(nn_smem);
     int* thits = reinterpret_cast<int*>(tile + NN_TE * DP);
