@@ -39,7 +39,8 @@
 
 #define NN_NB WP_NN_BINS    // distance bins per query
 #define NN_TE 32           // entries per shared-memory tile
-#define NN_THREADS 256     // threads per CTA in the distance kernels
+#define NN_THREADS 128     // threads (and reads) per CTA in the distance kernels
+#define NN_QBLOCK 256      // reads by which the entries are cut into slices
 #define NN_SEL_WARPS 4     // warps per CTA in the select kernel
 #define NN_HMAX 1024       // largest h
 
@@ -191,7 +192,7 @@ __device__ __forceinline__ void nn_load_tile(const NNArgs& a, int e0, int e_end,
     }
 }
 
-// A CTA's 256 queries are consecutive (sorted) slots, so a warp holds 32 similar
+// A CTA's 128 queries are consecutive (sorted) slots, so a warp holds 32 similar
 // reads; query i's histogram is row i (bank-conflict free).  Per tile of 32
 // entries, each query first bounds its distance to the tile's box (its two
 // lanes take every other tile): a tile beyond the start of the query's last bin
@@ -199,10 +200,14 @@ __device__ __forceinline__ void nn_load_tile(const NNArgs& a, int e0, int e_end,
 // the CTA loads the tile only if some query needs it, and a warp whose queries
 // all clear it skips the distances.  Bound by the shared-memory loads of the
 // entries' coordinates and the histogram atomics.  10,007 reads against the
-// tracks of 5,000 peptides x 60, 36 coordinates: 3.5 ms, 6.0 with a query per
-// lane and all 48 padded coordinates.
+// tracks of 5,000 peptides x 60, 36 coordinates: 3.2 ms, 6.0 with a query per
+// lane and all 48 padded coordinates.  CTAs of 128 threads: two queries of 37 to
+// 48 coordinates need some 170 registers, so three such CTAs fit an SM where one
+// of 256 does (4,000 reads, 48 coordinates, k = 10,000, all distance passes: 24.5
+// ms; one CTA of 256 30.7, two with spills 40.9, CTAs of 64 27.1, a query per lane
+// 33.6).
 template <int DP, int DQ>
-__global__ void __launch_bounds__(NN_THREADS, DQ > 9 ? 1 : 2) wp_nn_hist_kernel(NNArgs a) {
+__global__ void __launch_bounds__(NN_THREADS, DQ > 12 ? 2 : DQ > 9 ? 3 : 4) wp_nn_hist_kernel(NNArgs a) {
     extern __shared__ __align__(16) unsigned char nn_smem[];
     float* tile = reinterpret_cast<float*>(nn_smem);
     int* thits = reinterpret_cast<int*>(tile + NN_TE * DP);
@@ -331,9 +336,9 @@ __global__ void __launch_bounds__(NN_THREADS, DQ > 9 ? 1 : 2) wp_nn_hist_kernel(
 // selection stays exact whatever it says (a poor estimate only leaves more
 // candidates).  The sample is split over blockIdx.y so that small batches fill
 // the GPU (4,000 reads: 0.34 ms, against 3.6 ms with a CTA per 256 reads; two
-// queries per lane: 10,007 reads of 36 coordinates 0.75 -> 0.49 ms).
+// queries per lane: 10,007 reads of 36 coordinates 0.75 -> 0.57 ms).
 template <int DP, int DQ>
-__global__ void __launch_bounds__(NN_THREADS, DQ > 9 ? 1 : 2) wp_nn_estimate_kernel(NNArgs a) {
+__global__ void __launch_bounds__(NN_THREADS, DQ > 12 ? 2 : DQ > 9 ? 3 : 4) wp_nn_estimate_kernel(NNArgs a) {
     extern __shared__ __align__(16) unsigned char nn_smem[];
     float* tile = reinterpret_cast<float*>(nn_smem);
     int* thits = reinterpret_cast<int*>(tile + NN_TE * DP);
@@ -452,10 +457,10 @@ __global__ void wp_nn_threshold_kernel(NNArgs a) {
 }
 
 // The second pass, in the same shape: both lanes of a query count its candidates
-// alike and write them in entry order.  The reads above: 4.8 ms, 6.1 with a query
+// alike and write them in entry order.  The reads above: 4.3 ms, 6.1 with a query
 // per lane (45 million candidates written one by one).
 template <int DP, int DQ>
-__global__ void __launch_bounds__(NN_THREADS, DQ > 9 ? 1 : 2) wp_nn_collect_kernel(NNArgs a) {
+__global__ void __launch_bounds__(NN_THREADS, DQ > 12 ? 2 : DQ > 9 ? 3 : 4) wp_nn_collect_kernel(NNArgs a) {
     extern __shared__ __align__(16) unsigned char nn_smem[];
     float* tile = reinterpret_cast<float*>(nn_smem);
     int* thits = reinterpret_cast<int*>(tile + NN_TE * DP);
@@ -1069,7 +1074,7 @@ size_t wp_nn_dist_smem_bytes(int DP, bool with_hist) {
 
 int wp_nn_bins() { return NN_NB; }
 
-int wp_nn_queries_per_block() { return NN_THREADS; }
+int wp_nn_queries_per_block() { return NN_QBLOCK; }
 int wp_nn_select_warps() { return NN_SEL_WARPS; }
 int wp_nn_hmax() { return NN_HMAX; }
 
