@@ -34,7 +34,7 @@
 __global__ void wp_prep_reads_kernel(const DevModel*, const double*, int, unsigned, double,
                                      uint8_t*, uint8_t*, EmitEntry*, int);
 __global__ void wp_read_summary_kernel(BatchArgs);
-__global__ void wp_window_factors_kernel(BatchArgs);
+__global__ void wp_prep_window_kernel(BatchArgs, const double*, unsigned, double, uint8_t*, uint8_t*, EmitEntry*);
 size_t wp_window_smem_bytes(int C, int W, int threads);
 __global__ void wp_compact_kernel(BatchArgs);
 __global__ void wp_compact_groups_kernel(BatchArgs);
@@ -603,26 +603,26 @@ wp_status run_batch(wp_ctx* ctx, const double* d_rads, int R, double dist_cutoff
     {
         long n = (long)R * T;
         TimedLaunch tl(ctx, 1);
-        wp_prep_reads_kernel<<<(int)((n + 127) / 128), 128, 0, ctx->stream>>>(
-                a.model, d_rads, R, (unsigned)ctx->dmax, dist_cutoff, ctx->d_lo.as<uint8_t>(),
-                ctx->d_hi.as<uint8_t>(), ctx->d_table.as<EmitEntry>(), entries);
-        ctx->launches++;
-        WP_CUDA(cudaGetLastError(), "prep launch");
-        if (!window_factors) {
+        if (window_factors) {
+            const int rpc = WP_WINDOW_THREADS / T;  // whole reads per CTA
+            const size_t wsm = wp_window_smem_bytes(C, W, WP_WINDOW_THREADS);
+            int per_sm = 0, sms = 0;
+            WP_CUDA(wp_launch_shape(reinterpret_cast<const void*>(wp_prep_window_kernel), WP_WINDOW_THREADS, wsm,
+                                    &per_sm, &sms), "prep shape");
+            wp_prep_window_kernel<<<(R + rpc - 1) / rpc, WP_WINDOW_THREADS, wsm, ctx->stream>>>(
+                    a, d_rads, (unsigned)ctx->dmax, dist_cutoff, ctx->d_lo.as<uint8_t>(), ctx->d_hi.as<uint8_t>(),
+                    ctx->d_table.as<EmitEntry>());
+            ctx->launches++;
+            WP_CUDA(cudaGetLastError(), "prep launch");
+        } else {
+            wp_prep_reads_kernel<<<(int)((n + 127) / 128), 128, 0, ctx->stream>>>(
+                    a.model, d_rads, R, (unsigned)ctx->dmax, dist_cutoff, ctx->d_lo.as<uint8_t>(),
+                    ctx->d_hi.as<uint8_t>(), ctx->d_table.as<EmitEntry>(), entries);
+            ctx->launches++;
+            WP_CUDA(cudaGetLastError(), "prep launch");
             wp_read_summary_kernel<<<(R + 127) / 128, 128, 0, ctx->stream>>>(a);
             ctx->launches++;
             WP_CUDA(cudaGetLastError(), "summary launch");
-        }
-        if (window_factors) {
-            // with the boxes' summary: whole reads per CTA
-            const int rpc = WP_WINDOW_THREADS / T;
-            const size_t wsm = wp_window_smem_bytes(C, W, WP_WINDOW_THREADS);
-            int per_sm = 0, sms = 0;
-            WP_CUDA(wp_launch_shape(reinterpret_cast<const void*>(wp_window_factors_kernel), WP_WINDOW_THREADS, wsm, &per_sm, &sms),
-                    "window factors shape");
-            wp_window_factors_kernel<<<(R + rpc - 1) / rpc, WP_WINDOW_THREADS, wsm, ctx->stream>>>(a);
-            ctx->launches++;
-            WP_CUDA(cudaGetLastError(), "window factors launch");
         }
     }
     if (mode == MODE_FLOPS) {

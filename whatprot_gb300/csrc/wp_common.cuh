@@ -27,7 +27,7 @@
 #define WP_CNT_DENSE (2 * WP_MAX_TIERS)
 #define WP_CNT_LIVE (2 * WP_MAX_TIERS + 3)
 #define WP_CNT_N (2 * WP_MAX_TIERS + 4)
-#define WP_WINDOW_THREADS 128  // threads (read, timestep) per CTA of wp_window_factors_kernel, at least WP_MAX_TIMESTEPS
+#define WP_WINDOW_THREADS 128  // threads (read, timestep) per CTA of wp_prep_window_kernel, at least WP_MAX_TIMESTEPS
 #define WP_GROUP_WARPS 8      // warps per CTA of wp_compact_groups_kernel (one read at a time each)
 #define WP_GROUP_MAX 512      // dye-count vectors (groups) that kernel takes
 #define WP_GROUP_PERM_SMEM 8192  // peptides up to which it stages the shape order in shared memory
@@ -242,7 +242,7 @@ struct BatchArgs {
     // when some factor lies more than 2^100 below its window's largest; per
     // (r, t, c) and box [L_t, u), u in (L_t, U_t], the window's exponent
     // minus the box's at byte u - 1 (gdelta).  Written by
-    // wp_window_factors_kernel; the engine scales them instead of
+    // wp_prep_window_kernel; the engine scales them instead of
     // normalising each pair's box itself.
     float* gtab;
     uint8_t* gdelta;

@@ -64,7 +64,7 @@ __device__ __forceinline__ int bvol(uint32_t w) {
 
 // A read's emission factors as the engine reads them: the (mant, expo)
 // table, and where present the window-normalised FP32 factors with their
-// per-box exponent corrections (wp_window_factors_kernel).
+// per-box exponent corrections (wp_prep_window_kernel).
 struct ReadEmit {
     const EmitEntry* tab;  // [(t C + c) W + n]
     const float* gt;       // same layout, null when absent

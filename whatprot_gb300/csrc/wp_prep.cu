@@ -14,10 +14,11 @@
 //                           cmin_{t'} and min_{t'<=t} cmax_{t'}, the
 //                           allow-detached flag of each emission and whether
 //                           the read prunes every pair.
-//   wp_window_factors_kernel  one thread per (read, timestep): the emission
-//                           factors normalised over the pruning window, for
-//                           the engine (non-interacting models); the CTA's
-//                           rows staged through shared memory.
+//   wp_prep_window_kernel   one thread per (read, timestep), without
+//                           interactions: the two kernels above in one, and
+//                           the emission factors normalised over the
+//                           pruning window, for the engine; the CTA's rows
+//                           stay in shared memory.
 //   wp_compact_kernel       one CTA per read (candidate lists, loglik):
 //                           pairs whose pruned range is empty get
 //                           probability 0 (PeptideHMM::probability,
@@ -108,52 +109,50 @@ __device__ EmitEntry make_entry(double v) {
 
 // One thread per (read, t).  Writes box_lo/box_hi[r][t][c] and the
 // emission entries of timestep t.
-__global__ void wp_prep_reads_kernel(const DevModel* __restrict__ model,
-                                     const double* __restrict__ rads, int R,
-                                     unsigned max_num_dyes, double dist_cutoff,
-                                     uint8_t* __restrict__ box_lo,
-                                     uint8_t* __restrict__ box_hi,
-                                     EmitEntry* __restrict__ table, int entries_per_read) {
-    const DevModel& m = *model;
-    const int T = m.T, C = m.C;
-    const bool tabled = !m.interacting;  // per-count quantities from the model's tables
-    // Non-interacting models: the pruning thresholds mu_d + s_d and mu_d -
-    // s_d (s_d = dist_cutoff * sigma_d) per (channel, count), once per CTA,
-    // each rounded as the reference's separate multiply and add round it.
-    // And the pdf's normalisation 1 / (sigma sqrt(2 pi)) as an FP32
-    // mantissa in [0.5, 1) and an exponent.
-    // The thresholds also rounded to FP32 (rounding is monotone, so FP32
-    // order decides every comparison but ties, which go to FP64), and
-    // log2(e) / (2 sigma^2) times 2^40 (exact) for the exponent's fixed point.
-    __shared__ double s_thi[WP_MAX_CHANNELS][WP_W + 1], s_tlo[WP_MAX_CHANNELS][WP_W + 1];
-    __shared__ double s_l2d40[WP_MAX_CHANNELS][WP_W + 1];
-    __shared__ float s_thi_f[WP_MAX_CHANNELS][WP_W + 1], s_tlo_f[WP_MAX_CHANNELS][WP_W + 1];
-    __shared__ float s_nm[WP_MAX_CHANNELS][WP_W + 1];
-    __shared__ int s_ne[WP_MAX_CHANNELS][WP_W + 1];
-    if (tabled) {
-        for (int k = threadIdx.x; k < C * (WP_W + 1); k += blockDim.x) {
-            const int c = k / (WP_W + 1), d = k % (WP_W + 1);
-            const double sd = __dmul_rn(dist_cutoff, m.e_sig[c][d]);
-            s_thi[c][d] = __dadd_rn(m.e_amu[c][d], sd);
-            s_tlo[c][d] = __dsub_rn(m.e_amu[c][d], sd);
-            s_thi_f[c][d] = (float)s_thi[c][d];
-            s_tlo_f[c][d] = (float)s_tlo[c][d];
-            s_l2d40[c][d] = m.e_l2den[c][d] * 0x1p40;
-            int ne;
-            float nm = (float)frexp(m.e_norm[c][d], &ne);
-            if (nm >= 1.0f) {  // rounding up to 1.0
-                nm = 0.5f;
-                ne += 1;
-            }
-            s_nm[c][d] = nm;
-            s_ne[c][d] = ne;
+// Non-interacting models: the pruning thresholds mu_d + s_d and mu_d -
+// s_d (s_d = dist_cutoff * sigma_d) per (channel, count), once per CTA,
+// each rounded as the reference's separate multiply and add round it.
+// And the pdf's normalisation 1 / (sigma sqrt(2 pi)) as an FP32
+// mantissa in [0.5, 1) and an exponent.
+// The thresholds also rounded to FP32 (rounding is monotone, so FP32
+// order decides every comparison but ties, which go to FP64), and
+// log2(e) / (2 sigma^2) times 2^40 (exact) for the exponent's fixed point.
+struct PrepTables {
+    double thi[WP_MAX_CHANNELS][WP_W + 1], tlo[WP_MAX_CHANNELS][WP_W + 1];
+    double l2d40[WP_MAX_CHANNELS][WP_W + 1];
+    float thi_f[WP_MAX_CHANNELS][WP_W + 1], tlo_f[WP_MAX_CHANNELS][WP_W + 1];
+    float nm[WP_MAX_CHANNELS][WP_W + 1];
+    int ne[WP_MAX_CHANNELS][WP_W + 1];
+};
+
+__device__ __forceinline__ void prep_tables(PrepTables& s, const DevModel& m, double dist_cutoff) {
+    for (int k = threadIdx.x; k < m.C * (WP_W + 1); k += blockDim.x) {
+        const int c = k / (WP_W + 1), d = k % (WP_W + 1);
+        const double sd = __dmul_rn(dist_cutoff, m.e_sig[c][d]);
+        s.thi[c][d] = __dadd_rn(m.e_amu[c][d], sd);
+        s.tlo[c][d] = __dsub_rn(m.e_amu[c][d], sd);
+        s.thi_f[c][d] = (float)s.thi[c][d];
+        s.tlo_f[c][d] = (float)s.tlo[c][d];
+        s.l2d40[c][d] = m.e_l2den[c][d] * 0x1p40;
+        int ne;
+        float nm = (float)frexp(m.e_norm[c][d], &ne);
+        if (nm >= 1.0f) {  // rounding up to 1.0
+            nm = 0.5f;
+            ne += 1;
         }
-        __syncthreads();
+        s.nm[c][d] = nm;
+        s.ne[c][d] = ne;
     }
-    long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= (long)R * T) return;
-    int r = (int)(gid / T), t = (int)(gid % T);
-    const double* rad = rads + (long)r * T * C;
+}
+
+// One read's timestep: emission range and factors.  rad: its C intensities;
+// box_lo, box_hi: its C bounds; out: its table row (C W entries, or W^C with
+// interactions).
+__device__ __forceinline__ void prep_step(const DevModel& m, const PrepTables& s, const double* __restrict__ rad,
+                                          unsigned max_num_dyes, double dist_cutoff, uint8_t* box_lo, uint8_t* box_hi,
+                                          EmitEntry* out) {
+    const int C = m.C;
+    const bool tabled = !m.interacting;  // per-count quantities from the model's tables
     unsigned lo[WP_MAX_CHANNELS], hi[WP_MAX_CHANNELS];
     // PeptideEmission ctor pruned_range (peptide-emission.cc:50-163).
     if (dist_cutoff == DBL_MAX) {
@@ -168,20 +167,20 @@ __global__ void wp_prep_reads_kernel(const DevModel* __restrict__ model,
         // for the first count with mu + s > x and, from there, the first
         // with mu - s > x compare x with the thresholds.
         for (int c = 0; c < C; c++) {
-            const double x = rad[t * C + c];
+            const double x = rad[c];
             const float xf = (float)x;
             unsigned cmin = max_num_dyes + 1;
             for (unsigned d = 0; d < max_num_dyes + 1; d++) {
-                const float tf = s_thi_f[c][d];
-                if (tf > xf || (tf == xf && s_thi[c][d] > x)) {
+                const float tf = s.thi_f[c][d];
+                if (tf > xf || (tf == xf && s.thi[c][d] > x)) {
                     cmin = d;
                     break;
                 }
             }
             unsigned cmax = max_num_dyes + 1;
             for (unsigned d = cmin; d < max_num_dyes + 1; d++) {
-                const float tf = s_tlo_f[c][d];
-                if (tf > xf || (tf == xf && s_tlo[c][d] > x)) {
+                const float tf = s.tlo_f[c][d];
+                if (tf > xf || (tf == xf && s.tlo[c][d] > x)) {
                     cmax = d;
                     break;
                 }
@@ -214,7 +213,7 @@ __global__ void wp_prep_reads_kernel(const DevModel* __restrict__ model,
                     s = dist_cutoff * dev_sigma(m, c, mu);
                 }
                 // x / 1.0 == x exactly: the division (slow in FP64) only where mu != 1
-                const double q = mu1 == 1.0 ? rad[t * C + c] + s : (rad[t * C + c] + s) / mu1;
+                const double q = mu1 == 1.0 ? rad[c] + s : (rad[c] + s) / mu1;
                 unsigned new_cts = (unsigned)lround(q);
                 if (new_cts > max_num_dyes + 1) new_cts = max_num_dyes + 1;
                 if (new_cts != counts_hi[c]) {
@@ -235,7 +234,7 @@ __global__ void wp_prep_reads_kernel(const DevModel* __restrict__ model,
                     mu = dev_adjusted_mu(m, c, counts_lo);
                     s = dist_cutoff * dev_sigma(m, c, mu);
                 }
-                if (mu + s > rad[t * C + c]) {
+                if (mu + s > rad[c]) {
                     cmin = d;
                     break;
                 }
@@ -253,7 +252,7 @@ __global__ void wp_prep_reads_kernel(const DevModel* __restrict__ model,
                     mu = dev_adjusted_mu(m, c, counts_hi);
                     s = dist_cutoff * dev_sigma(m, c, mu);
                 }
-                if (mu - s > rad[t * C + c]) {
+                if (mu - s > rad[c]) {
                     cmax = d;
                     break;
                 }
@@ -264,13 +263,12 @@ __global__ void wp_prep_reads_kernel(const DevModel* __restrict__ model,
         }
     }
     for (int c = 0; c < C; c++) {
-        box_lo[((long)r * T + t) * C + c] = (uint8_t)lo[c];
-        box_hi[((long)r * T + t) * C + c] = (uint8_t)hi[c];
+        box_lo[c] = (uint8_t)lo[c];
+        box_hi[c] = (uint8_t)hi[c];
     }
     // Emission factors (peptide-emission.cc:167-180): the product over
     // channels of the Gaussian pdf, zero outside the box.
     const int W = (int)max_num_dyes + 1;
-    EmitEntry* out = table + (long)r * entries_per_read;
     if (!m.interacting) {
         // pdf of channel c depends on n_c only: store per (t, c, n).
         for (int c = 0; c < C; c++) {
@@ -291,17 +289,17 @@ __global__ void wp_prep_reads_kernel(const DevModel* __restrict__ model,
                     // FP32 rate on this GPU).  Far tails (y <= -1000, where
                     // FP64 itself nears underflow) take the FP64 exp so
                     // that zeros fall where the reference's do.
-                    const double offset = rad[t * C + c] - m.e_amu[c][n];
-                    const double y40 = -(offset * offset) * s_l2d40[c][n];
+                    const double offset = rad[c] - m.e_amu[c][n];
+                    const double y40 = -(offset * offset) * s.l2d40[c][n];
                     if (y40 > -1000.0 * 0x1p40) {
                         // round(y * 2^24): floor(y * 2^40), then to nearest
                         const long long q24 = (__double2ll_rd(y40) + (1ll << 15)) >> 16;
                         const int fl = (int)(q24 >> 24);
                         const float fr = exp2f((float)(int)(q24 & 0xffffff) * 0x1p-24f);
-                        const float pm = s_nm[c][n] * fr;  // in [0.5, 2]
+                        const float pm = s.nm[c][n] * fr;  // in [0.5, 2]
                         const bool up = pm >= 1.0f;
                         en.mant = up ? 0.5f * pm : pm;
-                        en.expo = s_ne[c][n] + (up ? 1 : 0) + fl;
+                        en.expo = s.ne[c][n] + (up ? 1 : 0) + fl;
                         if (en.mant >= 1.0f) {  // rounding up to 1.0
                             en.mant = 0.5f;
                             en.expo += 1;
@@ -310,7 +308,7 @@ __global__ void wp_prep_reads_kernel(const DevModel* __restrict__ model,
                         en = make_entry(m.e_norm[c][n] * exp(-offset * offset / m.e_den[c][n]));
                     }
                 }
-                out[(t * C + c) * W + n] = en;
+                out[c * W + n] = en;
             }
         }
     } else {
@@ -327,11 +325,31 @@ __global__ void wp_prep_reads_kernel(const DevModel* __restrict__ model,
             double v = 0.0;
             if (in_box) {
                 v = 1.0;
-                for (int c = 0; c < C; c++) v *= dev_pdf(m, c, rad[t * C + c], counts);
+                for (int c = 0; c < C; c++) v *= dev_pdf(m, c, rad[c], counts);
             }
-            out[t * G + g] = make_entry(v);
+            out[g] = make_entry(v);
         }
     }
+}
+
+__global__ void wp_prep_reads_kernel(const DevModel* __restrict__ model,
+                                     const double* __restrict__ rads, int R,
+                                     unsigned max_num_dyes, double dist_cutoff,
+                                     uint8_t* __restrict__ box_lo,
+                                     uint8_t* __restrict__ box_hi,
+                                     EmitEntry* __restrict__ table, int entries_per_read) {
+    const DevModel& m = *model;
+    const int T = m.T, C = m.C;
+    __shared__ PrepTables s;
+    if (!m.interacting) {
+        prep_tables(s, m, dist_cutoff);
+        __syncthreads();
+    }
+    const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (gid >= (long)R * T) return;
+    const int r = (int)(gid / T), t = (int)(gid % T);
+    prep_step(m, s, rads + gid * C, max_num_dyes, dist_cutoff, box_lo + gid * C, box_hi + gid * C,
+              table + (long)r * entries_per_read + (long)t * (entries_per_read / T));
 }
 
 
@@ -375,10 +393,13 @@ __global__ void wp_read_summary_kernel(BatchArgs a) {
     a.flags[r] = (uint8_t)empty;
 }
 
-// One thread per (read, t), non-interacting models: the read's boxes as in
-// wp_read_summary_kernel (a CTA holds whole reads, each thread goes over its
-// read's bounds in shared memory: one launch less, and no chain of byte loads per
-// read; 11.9 -> 6.3 us for one read, 72 -> 54 for 20,000) and
+// One thread per (read, t), non-interacting models, whole reads per CTA: the
+// emission ranges and factors (prep_step), the read's boxes as in
+// wp_read_summary_kernel (each thread goes over its read's bounds in shared
+// memory) and the window-normalised factors, in one kernel: the rows stay in
+// shared memory between them and go out coalesced.  20,000 reads 87 us, 129 as two
+// kernels and 149 as three; 3,001 reads 20 us, 33 and 42.
+// Window factors:
 // the window-normalised emission factors the engine reads (BatchArgs::gtab, gK,
 // gdelta).  For a pair's box [L_t, u) of channel c the engine multiplies the
 // window factors by 2^gdelta, which gives exactly mant * 2^(expo - k_box), k_box
@@ -388,13 +409,17 @@ __global__ void wp_read_summary_kernel(BatchArgs a) {
 // normalising exponent: the same numbers the engine's own normalisation of
 // the box gives.  Where a factor lies further below, gK = WP_GK_NONE and the
 // engine normalises that (read, t) itself.
-// Shared memory of wp_window_factors_kernel: per item its table row and its
+// Shared memory of wp_prep_window_kernel: per item its table row and its
 // outputs (C W entries, floats and bytes).
 size_t wp_window_smem_bytes(int C, int W, int threads) {
     return (size_t)threads * C * W * (sizeof(EmitEntry) + sizeof(float) + 1);
 }
 
-__global__ void wp_window_factors_kernel(BatchArgs a) {
+__global__ void __launch_bounds__(WP_WINDOW_THREADS) wp_prep_window_kernel(BatchArgs a, const double* __restrict__ rads,
+                                                                           unsigned max_num_dyes, double dist_cutoff,
+                                                                           uint8_t* __restrict__ box_lo,
+                                                                           uint8_t* __restrict__ box_hi,
+                                                                           EmitEntry* __restrict__ table) {
     const DevModel& m = *a.model;
     const int T = m.T, C = m.C, W = a.W;
     const int CW = C * W;
@@ -412,16 +437,20 @@ __global__ void wp_window_factors_kernel(BatchArgs a) {
     __shared__ uint8_t s_lo[WP_WINDOW_THREADS * WP_MAX_CHANNELS], s_hi[WP_WINDOW_THREADS * WP_MAX_CHANNELS];
     __shared__ int s_empty[WP_WINDOW_THREADS];
     const int n_ent = n_items * CW;
-    {
-        const EmitEntry* src = a.tab + item0 * CW;  // [r][t][c][n]: item (r, t) at (r T + t) C W
-        for (int k = threadIdx.x; k < n_ent; k += blockDim.x) s_tab[k] = src[k];
-        for (int k = threadIdx.x; k < n_items * C; k += blockDim.x) {
-            s_lo[k] = a.lo[item0 * C + k];
-            s_hi[k] = a.hi[item0 * C + k];
-        }
-        s_empty[threadIdx.x] = 0;
-    }
+    __shared__ PrepTables s_prep;
+    prep_tables(s_prep, m, dist_cutoff);
+    s_empty[threadIdx.x] = 0;
     __syncthreads();
+    if ((int)threadIdx.x < n_items)
+        prep_step(m, s_prep, rads + (item0 + threadIdx.x) * C, max_num_dyes, dist_cutoff, s_lo + threadIdx.x * C,
+                  s_hi + threadIdx.x * C, s_tab + threadIdx.x * CW);
+    __syncthreads();
+    for (int k = threadIdx.x; k < n_ent; k += blockDim.x)
+        table[item0 * CW + k] = s_tab[k];  // [r][t][c][n]: item (r, t) at (r T + t) C W
+    for (int k = threadIdx.x; k < n_items * C; k += blockDim.x) {
+        box_lo[item0 * C + k] = s_lo[k];
+        box_hi[item0 * C + k] = s_hi[k];
+    }
     const int item = threadIdx.x, rl = item / T, t = item - rl * T;  // read of the CTA, timestep
     int Lt[WP_MAX_CHANNELS] = {0, 0, 0, 0}, Ut[WP_MAX_CHANNELS] = {255, 255, 255, 255};
     if (item < n_items) {
