@@ -1,0 +1,97 @@
+"""E-steps with a read whose dyes of one channel go dark for some cycles and come
+back: an ordinary fault of a real run (a missed registration, a blinking dye)
+that the model gives a small, positive probability.  The forward vector then
+holds the read's only path at 2^-33 or so per dark dye and cycle, and the frame
+factor of its counts is the inverse.
+
+Every sum has to be finite, alone and among clean reads, with the warp kernel and
+with the thread-per-read one; while dark dyes times cycles are at most two
+(2^-66) FP32 vectors lose nothing, and every sum lies within 1e-5 of its
+parameter's denominator of the oracle's (the tolerance of test_gpu_fit.py)."""
+import numpy as np
+import pytest
+
+from oracle_lib import WpoFitSums
+from whatprot_gb300.model import DyeSeqSet, parse_dye_seq
+from whatprot_gb300.simulate import paper_model, simulate_radiometries
+
+pytestmark = pytest.mark.gpu
+
+CONTROL = "..0.1.2.0.0.1.2.1.02"  # 4 / 3 / 3 dyes
+CASES = [
+    # C, T, dye-seq, dark channel, dark cycles, blocking, emission
+    (3, 16, CONTROL, 0, 1, False, True),
+    (3, 16, CONTROL, 0, 2, False, True),
+    (3, 16, CONTROL, 2, 2, True, False),
+    (3, 16, CONTROL, 1, 3, True, True),
+    (3, 16, CONTROL, 2, 5, False, False),
+    (1, 9, ".......0", 0, 1, False, True),
+    (1, 9, ".......0", 0, 3, False, True),
+    (2, 10, "......0.0.1", 0, 2, False, True),
+    (2, 10, "......0.0.01", 0, 2, True, True),
+    (2, 10, "......0.0.0.01", 0, 1, False, False),
+    (2, 10, "......0.0.0.0.01", 0, 1, True, False),
+]
+
+
+def _blinking(sm, C, T, seq, channel, dark):
+    """A read without losses but the cut's, channel `channel` dark from cycle 1."""
+    x = np.zeros((1, T, C))
+    for t in range(T):
+        for c in range(C):
+            n = int((seq[t:] == c).sum())
+            x[0, t, c] = n + 0.02 * n * (-1) ** (t + c) + 0.002
+    x[0, 1:1 + dark, channel] = 0.003
+    return x
+
+
+@pytest.mark.parametrize("clean", [0, 200])
+@pytest.mark.parametrize("case", CASES, ids=[f"C{c[0]}T{c[1]}n{len(c[2])}c{c[3]}x{c[4]}{'B' if c[5] else ''}{'E' if c[6] else ''}" for c in CASES])
+def test_blinking_read(gpu_ctx, oracle, case, clean):
+    C, T, s, channel, dark, block, emission = case
+    sm = paper_model(C)
+    if block:
+        sm.p_initial_block, sm.p_cyclic_block = 0.04, 0.03
+    seq = parse_dye_seq(s)
+    bad = _blinking(sm, C, T, np.asarray(seq), channel, dark)
+    ds = DyeSeqSet(C, [seq], np.array([0], np.int32), np.array([1], np.int32))
+    good, _ = simulate_radiometries(sm, ds, T, 2 * clean + 20, seed=T + dark)
+    rads = np.concatenate([good[:clean // 2], bad, good[clean // 2:clean]])
+    gpu_ctx.upload_model(sm, T)
+    gpu_ctx.fit_begin(seq, rads)
+    gpu_ctx.fit_set_emission(emission)
+    got = []
+    try:
+        for kind in (0, 1):
+            gpu_ctx.fit_set_kernel(kind)
+            sums, lp, nz = gpu_ctx.fit_estep()
+            d = sums.as_dict(T, C)
+            if emission:
+                d.update(zip(("emis_w", "emis_x", "emis_xx"), gpu_ctx.fit_emission_sums().arrays(C)))
+            assert np.isfinite(lp) or nz == len(rads)
+            for k, v in d.items():
+                assert np.all(np.isfinite(v)), (kind, k, v)
+            got.append(d)
+    finally:
+        gpu_ctx.fit_set_kernel(0)
+        gpu_ctx.fit_set_emission(False)
+    if int((np.asarray(seq)[1:] == channel).sum()) * dark > 2:
+        return
+    o = WpoFitSums()
+    for r in rads:
+        oracle.improve_fit(sm, T, seq, r, max(int((seq == c).sum()) for c in range(C)), sums=o)
+    e = o.as_dict(T, C)
+
+    def near(key, want, den):
+        for d in got:
+            x, w = np.asarray(d[key], np.float64), np.asarray(want, np.float64)
+            assert np.all(np.abs(x - w) <= 1e-5 * np.maximum(np.asarray(den, np.float64), 1e-3)), (key, x, w)
+
+    for k in ("edman", "bleach", "dud", "init_block", "cyc_block"):
+        near(k + "_num", e[k][0], e[k][1])
+        near(k + "_den", e[k][1], e[k][1])
+    near("detach_n", e["detach_n"], e["detach_n"])
+    near("detach_x", e["detach_x"], e["detach_n"])
+    if emission:
+        for k in ("emis_w", "emis_x", "emis_xx"):
+            near(k, e[k], np.full_like(e[k], e["emis_w"].sum() / C))

@@ -43,8 +43,7 @@ struct DevModel {
     float p_det[WP_MAX_TIMESTEPS];      // p_detach[t]
     float dud[WP_MAX_CHANNELS][WP_TRI];    // prob(from, to) at from*(from+1)/2+to
     float bleach[WP_MAX_CHANNELS][WP_TRI];
-    double q_dud[WP_MAX_CHANNELS];      // p_dud and p_bleach as given (factors of the fit's counts)
-    double q_bleach[WP_MAX_CHANNELS];
+    double q_bleach[WP_MAX_CHANNELS];   // p_bleach as given (a factor of the fit's counts)
     // Emission model (FP64: the emission factors are computed as the
     // reference does, then rounded once).
     double bg_sig[WP_MAX_CHANNELS];
@@ -124,7 +123,6 @@ inline wp_status wp_fill_dev_model(const wp_seq_model* m, int T, DevModel* hp) {
     for (int c = 0; c < C; c++) {
         wp_binomial_table(m->p_dud[c], WP_MAX_DYES_PER_CHANNEL, h.dud[c]);
         wp_binomial_table(m->p_bleach[c], WP_MAX_DYES_PER_CHANNEL, h.bleach[c]);
-        h.q_dud[c] = m->p_dud[c];
         h.q_bleach[c] = m->p_bleach[c];
         h.bg_sig[c] = m->bg_sig[c];
         h.sig[c] = m->sig[c];

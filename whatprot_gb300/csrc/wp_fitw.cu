@@ -16,8 +16,9 @@
 //   * Detach: sums of f and f x over the non-zero states.
 //   * Edman: f behind the bleach steps against the backward vectors on both
 //     sides of the cut, recomputed from x_{t+1} (two multiply-adds).
-//   * Dud: the start is one state, so P and the dud counts are dot products of
-//     the emission-weighted vector at t = 0 with 1 + C fixed vectors.
+//   * Dud: the start is one state, so P is the dot product of the emission-weighted
+//     vector at t = 0 with one fixed vector, and a channel's dud count the same
+//     weighted by the dyes a state has lost, D_c - n_c.
 //   * Emission statistics at t: column sums of f b at the next chain's input.
 //
 // Layout: rows of S = prod (D_c + 1) dye-count states per Edman cut.  Lanes own
@@ -30,8 +31,9 @@
 // timesteps: the resident warps' slabs stay in L2).
 //
 // Vectors are FP32 with powers of two carried as integers (backward after each
-// step, forward in the next step's weights); sums over states are FP32, their
-// frame factor 2^(exponents) / P and the sums over reads FP64, in a fixed order.
+// step, forward in the next step's weights); sums over the states of one timestep
+// are FP32, their frame factor 2^(exponents) / P and the sums over timesteps and
+// reads FP64, in a fixed order.
 //
 // Bound by instruction issue and shared-memory bandwidth (about 150 issue slots
 // per 32 states and timestep).  50,000 reads, 3 channels (4/3/3 dyes), 16
@@ -60,6 +62,21 @@ __device__ __forceinline__ float fw_sum(float v) {
     return v;
 }
 
+// The lanes' sums of N values (a power of two): lane l gets that of value l mod N.
+template <int N>
+__device__ __forceinline__ float fw_sums(float (&v)[N], int lane) {
+#pragma unroll
+    for (int w = N / 2; w >= 1; w >>= 1) {
+        const bool up = (lane & w) != 0;
+#pragma unroll
+        for (int i = 0; i < w; i++)
+            v[i] = (up ? v[i + w] : v[i]) + __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + w], w);
+    }
+#pragma unroll
+    for (int o = N; o < 32; o <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
 // Largest of the lanes' non-negative floats.
 __device__ __forceinline__ float fw_max(float v) {
     return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
@@ -69,6 +86,12 @@ __device__ __forceinline__ float fw_max(float v) {
 __device__ __forceinline__ float fw_exp2(float v, int e) {
     const int a = max(-126, min(126, e)), b = max(-126, min(126, e - a));
     return v * __int_as_float((a + 127) << 23) * __int_as_float((b + 127) << 23);
+}
+
+// 2^e, the frame of sums whose truth is a count: where e passes 1000 they have long
+// underflowed to zero, and zero they stay.
+__device__ __forceinline__ double fw_exp2d(int e) {
+    return __hiloint2double((max(-1000, min(1000, e)) + 1023) << 20, 0);
 }
 
 // Exponent k with v = m 2^k, m in [0.5, 1); 0 for v = 0.
@@ -148,7 +171,7 @@ __device__ float fw_binomial(float* v, int n, int W, int st, unsigned magic, con
 }
 
 // Shared memory of a CTA (floats): per e the Edman cut, the columns' dye
-// counts, the dud vectors, the binomial tables; then per warp its vectors.
+// counts, the dud vector, the binomial tables; then per warp its vectors.
 struct FWLayout {
     int S, T, C, wsum;
     int tri;        // entries of the channels' binomial tables
@@ -176,18 +199,18 @@ __host__ __device__ inline FWLayout fw_layout(int T, int C, const int* D, bool h
     w += 2 * L.S + 32;          // front pad and weights of one timestep
     w += T * L.wsum;            // weights per (t, c, n)
     w += emission ? L.S : 0;    // column products (emission statistics)
-    w += 6 * (T + 1);           // per timestep: kmx, exponents, pd, detach sums
+    w += 7 * (T + 1);           // per timestep: kmx, exponents, pd, detach sums and their frame
     w = (w + 3) / 4 * 4;
     w += 2 * nslots;            // FP64 sums
     L.per_warp = (w + 3) / 4 * 4;
     L.cuts = 2;
     for (int c = 0; c < C; c++) L.cuts = D[c] + 2 > L.cuts ? D[c] + 2 : L.cuts;
-    L.shared = (2 * T * L.cuts + T + L.S + (1 + C) * L.S + L.tri + 3) / 4 * 4;
+    L.shared = (2 * T * L.cuts + T + L.S + L.S + L.tri + 3) / 4 * 4;
     return L;
 }
 
 template <int C, bool HB>
-__global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, float* slab, long slab_stride) {
+__global__ void __launch_bounds__(FW_WARPS * 32, 2) wp_fit_warp_kernel(FitArgs a, float* slab, long slab_stride) {
     extern __shared__ __align__(16) float fw_smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpc = blockDim.x >> 5;
     const int inst = a.inst_ctas > 0 ? (int)(blockIdx.x / a.inst_ctas) : 0;
@@ -222,8 +245,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, f
     int* e_ch = reinterpret_cast<int*>(e_cut + T * L.cuts);
     uint32_t* coord = reinterpret_cast<uint32_t*>(e_ch + T);  // [S] dye counts, 4 bits per channel
     float* dud0 = reinterpret_cast<float*>(coord + S);        // [S] start through the duds
-    float* dudc = dud0 + S;                                   // [C][S] with one dye fewer on channel c
-    float* bleach = dudc + C * S;                             // the channels' binomial tables
+    float* bleach = dud0 + S;                                 // the channels' binomial tables
     int boff[C];
     {
         int o = 0;
@@ -248,23 +270,15 @@ __global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, f
     }
     for (int j = threadIdx.x; j < S; j += blockDim.x) {
         uint32_t pk = 0;
-        float full = 1.f, less[C];
-#pragma unroll
-        for (int c = 0; c < C; c++) less[c] = 1.f;
+        float full = 1.f;
 #pragma unroll
         for (int c = 0; c < C; c++) {
             const int n = (j / st[c]) % W[c], D = W[c] - 1;
             pk |= (uint32_t)n << (4 * c);
-            const float p = m.dud[c][D * (D + 1) / 2 + n];
-            const float q = n < D ? m.dud[c][(D - 1) * D / 2 + n] : 0.f;  // D >= 1 where n < D
-            full *= p;
-#pragma unroll
-            for (int k = 0; k < C; k++) less[k] *= k == c ? q : p;
+            full *= m.dud[c][D * (D + 1) / 2 + n];
         }
         coord[j] = pk;
         dud0[j] = full;
-#pragma unroll
-        for (int c = 0; c < C; c++) dudc[c * S + j] = less[c];
     }
 #pragma unroll
     for (int c = 0; c < C; c++)
@@ -284,6 +298,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, f
     float* pdx = reinterpret_cast<float*>(kx + T + 1);  // detached state's backward value beside x_t
     float* dx = pdx + T + 1;                     // detach sums per timestep
     float* dn = dx + T + 1;
+    int* dfr = reinterpret_cast<int*>(dn + T + 1);  // their frame's exponent
     double* acc = reinterpret_cast<double*>(mine + L.per_warp - 2 * a.nslots);
     for (int i = lane; i < L.per_warp; i += 32) mine[i] = 0.f;
     float* xs = slab + ((long)blockIdx.x * wpc + wib) * slab_stride;  // x_t at the sum of the earlier ones' sizes
@@ -302,6 +317,15 @@ __global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, f
         }
         __syncwarp();
     };
+
+    // The timesteps' sums, value i of every timestep in lane i, FP64 over timesteps
+    // and reads: a term's frame factor passes FP32's range where a read's earlier
+    // and later timesteps favour different states, and an FP32 sum over timesteps
+    // would add terms of different frames.  0, 1: the detach sums (FP64 at the read's
+    // end); 2: the cyclic block's denominator; 3: the forward vector's sum; 4, 5:
+    // Edman; from 6: bleach; then the block's numerator.
+    constexpr int NV = 6 + 2 * C + (HB ? 1 : 0), NR = NV <= 8 ? 8 : 16;
+    double all_reads = 0.0;
 
     double lp_m = 0.0;  // of the lane's read among the last 32: P = lp_m 2^lp_e
     int lp_e = 0;
@@ -449,9 +473,12 @@ __global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, f
                     } else {
                         b *= 1.f - m.p_ib;
                     }
-                    Ps = fmaf(dud0[j], b, Ps);
+                    const float v = dud0[j] * b;
+                    Ps += v;
+                    const uint32_t pk = coord[j];
 #pragma unroll
-                    for (int c = 0; c < C; c++) dudn[c] = fmaf(dudc[c * S + j], b, dudn[c]);
+                    for (int c = 0; c < C; c++)
+                        dudn[c] = fmaf((float)(a.D[c] - (int)((pk >> (4 * c)) & 15u)), v, dudn[c]);
                 }
             }
             Ps = fw_sum(Ps);
@@ -473,13 +500,10 @@ __global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, f
             if (++lp_n == 32) flush_logp();
         }
         if (!live) continue;
-        const float invP = 1.0f / Pm;
-        const double dinvP = a.emission ? 1.0 / (double)Pm : 0.0;
+        const double invP = 1.0 / (double)Pm;
+        double tsum = 0.0;  // times P
 
         // ---- forward sweep with the expected counts
-        float edn = 0.f, edd = 0.f, bn[C], bd[C], cbn = 0.f, cbd = 0.f;
-#pragma unroll
-        for (int c = 0; c < C; c++) bn[c] = bd[c] = 0.f;
         float fpd = 0.f;
         int Ea = kmx[0], kf;
         {
@@ -496,7 +520,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, f
         // detached state's gd, both in the frame 2^e / P
         auto emission = [&](int t, float gd, int e) {
             __syncwarp();
-            const double sc = ldexp(dinvP, e - EP);
+            const double sc = invP * fw_exp2d(e - EP);
             for (int b = lane; b < L.wsum; b += 32) {
                 int c = 0, n = b;
 #pragma unroll
@@ -534,7 +558,9 @@ __global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, f
             const float p = m.p_det[t - 1], keep = 1.f - p;
             const float pdt = pdx[t];
             const int fr = Ea + Ebr[t] - EP;  // frame of f times backward values here
-            const float sf = fw_exp2(invP, fr);
+            float sum[NR];
+#pragma unroll
+            for (int i = 0; i < NR; i++) sum[i] = 0.f;
             // detachment, block and bleach sums, column by column
             float Fnz = 0.f, F0 = 0.f, Gnz = 0.f, G0 = 0.f, Fa = 0.f, Gaa = 0.f, Gab = 0.f;
             for (int h = 0; h < NC; h++) {
@@ -569,9 +595,9 @@ __global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, f
                     const uint32_t pk = coord[j];
 #pragma unroll
                     for (int c = 0; c < C; c++) {
-                        const float n = (float)((pk >> (4 * c)) & 15u) * keep * sf;
-                        bd[c] = fmaf(n, H, bd[c]);
-                        bn[c] = fmaf(n, n != 0.f ? K[c] : 0.f, bn[c]);
+                        const float n = (float)((pk >> (4 * c)) & 15u);
+                        sum[6 + 2 * c] = fmaf(n, n != 0.f ? K[c] : 0.f, sum[6 + 2 * c]);
+                        sum[7 + 2 * c] = fmaf(n, H, sum[7 + 2 * c]);
                     }
                     if (j == 0) {
                         F0 = fs;
@@ -584,23 +610,20 @@ __global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, f
                 }
             }
             if (a.emission) emission(t - 1, fpd * pdt, Ea + Ebr[t]);
-            Fnz = fw_sum(Fnz);
-            Gnz = fw_sum(Gnz);
-            F0 = __shfl_sync(0xffffffffu, F0, 0);
-            const float Fall = Fnz + F0;
-            if (lane == 0) {
-                const float x = p * pdt * Fnz;
-                dx[t - 1] = x * sf;
-                dn[t - 1] = fmaf(keep, Gnz, x) * sf;
-                if (!HB) {
-                    const float G = Gnz + G0;
-                    cbd += fmaf(keep, G, p * pdt * Fall) * sf * (1.f - m.p_cb);
-                }
-            }
+            // a timestep's constants are multiplied into the sums one by one: folded
+            // into one FP32 factor they would bias every term alike
+#pragma unroll
+            for (int c = 0; c < 2 * C; c++) sum[6 + c] *= keep;
+            // (F0, G0: lane 0's, zero in the others)
+            sum[0] = p * pdt * Fnz;
+            sum[1] = fmaf(keep, Gnz, sum[0]);
+            sum[3] = Fnz + F0;
             if (HB) {
                 const float gb = fmaf(keep, Gab, p * pdt * Fa), ga = fmaf(keep, Gaa, p * pdt * Fa);
-                cbn = fmaf(m.p_cb * sf, gb, cbn);
-                cbd = fmaf(sf, fmaf(1.f - m.p_cb, ga, m.p_cb * gb), cbd);
+                sum[2] = fmaf(1.f - m.p_cb, ga, m.p_cb * gb);
+                sum[NV - 1] = m.p_cb * gb;
+            } else {
+                sum[2] = (1.f - m.p_cb) * fmaf(keep, Gnz + G0, p * pdt * sum[3]);
             }
             __syncwarp();
             // the next chain's backward vector
@@ -679,10 +702,13 @@ __global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, f
                 }
                 __syncwarp();
             }
-            en *= pf * keep * sf;
-            edn += en;
-            edd = fmaf(keep * sf, ed, edd) + en;
-            fpd = wv[0] * sc * fmaf(p, Fall, fpd);
+            sum[4] = pf * (keep * en);
+            sum[5] = fmaf(keep, ed, sum[4]);
+            const float mine_v = fw_sums<NR>(sum, lane);
+            if (lane < 2) (lane == 0 ? dx : dn)[t - 1] = mine_v;
+            if (lane == 0) dfr[t - 1] = fr;
+            tsum = fma((double)mine_v, fw_exp2d(fr), tsum);
+            fpd = wv[0] * sc * fmaf(p, __shfl_sync(0xffffffffu, mine_v, 3), fpd);
             Ea += kf + kmx[t];
             kf = fw_expo(fw_max(fmaxf(mx, fpd)));
         }
@@ -707,29 +733,35 @@ __global__ void __launch_bounds__(FW_WARPS * 32) wp_fit_warp_kernel(FitArgs a, f
                     slot = s;
                 }
             };
-            const float fp = fw_exp2(invP, Eb + kmx[0] - EP);  // frame of P
-            put(0, 0, fw_sum(edn));
-            put(1, 1, fw_sum(edd));
-            if (HB) put(2, 2, m.p_ib * ib * fp);
+            const double fp = invP * fw_exp2d(Eb + kmx[0] - EP);  // frame of P
+            if (HB) put(2, 2, m.p_ib * ib, fp);
             put(3, 3, 1.f);
-            if (HB) put(4, 4, fw_sum(cbn));
-            put(5, 5, fw_sum(cbd));
 #pragma unroll
             for (int c = 0; c < C; c++) {
-                put(6 + 4 * c, fw_rate(T, c), fw_sum(bn[c]), m.q_bleach[c]);
-                put(7 + 4 * c, fw_rate(T, c) + 1, fw_sum(bd[c]));
-                put(8 + 4 * c, fw_rate(T, c) + 2, (float)a.D[c] * fw_sum(dudn[c]) * fp, m.q_dud[c]);
+                put(8 + 4 * c, fw_rate(T, c) + 2, fw_sum(dudn[c]), fp);
                 put(9 + 4 * c, fw_rate(T, c) + 3, (float)a.D[c]);
             }
             if (slot >= 0) acc[slot] += (double)mine_v * mine_q;
+            all_reads = fma(tsum, invP, all_reads);
             for (int t = lane; t < T - 1; t += 32) {
-                acc[fw_det(t)] += (double)dx[t];
-                acc[fw_det(t) + 1] += (double)dn[t];
+                const double f = invP * fw_exp2d(dfr[t]);
+                acc[fw_det(t)] += (double)dx[t] * f;
+                acc[fw_det(t) + 1] += (double)dn[t] * f;
             }
             __syncwarp();
         }
     }
     flush_logp();
+    {
+        const int i = lane;
+        if (i == 2) acc[5] += all_reads;
+        if (i == 4 || i == 5) acc[i - 4] += all_reads;
+        if (i >= 6 && i < 6 + 2 * C) {
+            const int c = (i - 6) >> 1;
+            acc[fw_rate(T, c) + (i & 1)] += (i & 1) ? all_reads : all_reads * m.q_bleach[c];
+        }
+        if (HB && i == NV - 1) acc[4] += all_reads;
+    }
     __syncthreads();
     // the CTA's sums, its warps in order
     for (int k = threadIdx.x; k < a.nslots; k += blockDim.x) {
