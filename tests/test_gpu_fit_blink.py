@@ -4,10 +4,12 @@ that the model gives a small, positive probability.  The forward vector then
 holds the read's only path at 2^-33 or so per dark dye and cycle, and the frame
 factor of its counts is the inverse.
 
-Every sum has to be finite, alone and among clean reads, with the warp kernel and
-with the thread-per-read one; while dark dyes times cycles are at most two
-(2^-66) FP32 vectors lose nothing, and every sum lies within 1e-5 of its
-parameter's denominator of the oracle's (the tolerance of test_gpu_fit.py)."""
+Every sum has to be finite, alone and among clean reads, and with the warp
+kernel no further from the oracle than with the thread-per-read kernel, up to
+the 1e-5 of the parameter's denominator that test_gpu_fit.py allows any E-step
+(both hold the vectors in FP32: a path far enough below the largest entry is lost
+to both, below 2^-149 to the thread kernel).  While dark dyes times cycles are at
+most two (2^-66), nothing is lost: 1e-5."""
 import numpy as np
 import pytest
 
@@ -22,11 +24,15 @@ CASES = [
     # C, T, dye-seq, dark channel, dark cycles, blocking, emission
     (3, 16, CONTROL, 0, 1, False, True),
     (3, 16, CONTROL, 0, 2, False, True),
+    (3, 16, CONTROL, 1, 2, False, False),
     (3, 16, CONTROL, 2, 2, True, False),
     (3, 16, CONTROL, 1, 3, True, True),
     (3, 16, CONTROL, 2, 5, False, False),
     (1, 9, ".......0", 0, 1, False, True),
     (1, 9, ".......0", 0, 3, False, True),
+    (1, 9, ".......0", 0, 4, False, True),   # the largest entry is subnormal afterwards
+    (1, 9, ".......0", 0, 4, True, False),
+    (1, 12, "........0", 0, 5, False, True),
     (2, 10, "......0.0.1", 0, 2, False, True),
     (2, 10, "......0.0.01", 0, 2, True, True),
     (2, 10, "......0.0.0.01", 0, 1, False, False),
@@ -71,21 +77,22 @@ def test_blinking_read(gpu_ctx, oracle, case, clean):
             assert np.isfinite(lp) or nz == len(rads)
             for k, v in d.items():
                 assert np.all(np.isfinite(v)), (kind, k, v)
-            got.append(d)
+            got.append((d, nz))
     finally:
         gpu_ctx.fit_set_kernel(0)
         gpu_ctx.fit_set_emission(False)
-    if int((np.asarray(seq)[1:] == channel).sum()) * dark > 2:
-        return
+    (a, nza), (b, nzb) = got
+    assert nza <= nzb
     o = WpoFitSums()
     for r in rads:
         oracle.improve_fit(sm, T, seq, r, max(int((seq == c).sum()) for c in range(C)), sums=o)
     e = o.as_dict(T, C)
+    lost = int((np.asarray(seq)[1:] == channel).sum()) * dark > 2
 
     def near(key, want, den):
-        for d in got:
-            x, w = np.asarray(d[key], np.float64), np.asarray(want, np.float64)
-            assert np.all(np.abs(x - w) <= 1e-5 * np.maximum(np.asarray(den, np.float64), 1e-3)), (key, x, w)
+        x, y, w = (np.asarray(v, np.float64) for v in (a[key], b[key], want))
+        tol = 1e-5 * np.maximum(np.asarray(den, np.float64), 1e-3)
+        assert np.all(np.abs(x - w) <= (np.abs(y - w) if lost else 0.0) + tol), (key, x, y, w)
 
     for k in ("edman", "bleach", "dud", "init_block", "cyc_block"):
         near(k + "_num", e[k][0], e[k][1])

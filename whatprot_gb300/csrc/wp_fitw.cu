@@ -47,6 +47,10 @@
 
 #define FW_WARPS 8    // most warps per CTA
 #define FW_MAXW 6     // fibres of up to this length are processed in registers
+#define FW_LOW (-8)   // vectors 2^8 and more below their place are brought up at once
+#define FW_TOP 96     // the forward vector's largest entry is kept near 2^96: where later
+                      // timesteps contradict earlier ones the read's path can lie far below
+                      // it (2^-33 per dark dye and cycle), and FP32 ends at 2^-149
 #define FW_EMIS_N (WP_MAX_DYES_PER_CHANNEL + 1)
 
 // The slots of wp_fit.cu.
@@ -448,10 +452,22 @@ __global__ void __launch_bounds__(FW_WARPS * 32, 2) wp_fit_warp_kernel(FitArgs a
                     }
                     __syncwarp();
                 }
-                const int k = fw_expo(fw_max(mx));
+                int k = fw_expo(fw_max(mx)), up = 0;
+                if (k < FW_LOW) {
+                    // left to the weights of the next step, so small a vector would
+                    // cost its terms their low bits, and below 2^-127 the scale
+                    // that undoes it would be infinite
+                    up = k;
+                    k = 0;
+                    for (int i = lane; i < t * S; i += 32) {
+                        out[i] = XA[i] = fw_exp2(XA[i], -up);
+                        if (HB) out[t * S + i] = XB[i] = fw_exp2(XB[i], -up);
+                    }
+                    pd = fw_exp2(pd, -up);
+                }
                 if (lane == 0) {
                     pdx[t] = pd;
-                    Ebr[t] = Eb + kmx[t];
+                    Ebr[t] = Eb + kmx[t] + up;
                     kx[t] = k;
                 }
                 __syncwarp();
@@ -505,17 +521,31 @@ __global__ void __launch_bounds__(FW_WARPS * 32, 2) wp_fit_warp_kernel(FitArgs a
 
         // ---- forward sweep with the expected counts
         float fpd = 0.f;
-        int Ea = kmx[0], kf;
+        int Ea = kmx[0] - FW_TOP, kf;
         {
             float mx = 0.f;
             for (int j = lane; j < S; j += 32) {
-                const float v = wv[j] * dud0[j];
+                const float v = wv[j] * (dud0[j] * 0x1p96f);
                 FA[j] = (1.f - m.p_ib) * v;
                 if (HB) FB[j] = m.p_ib * v;
                 mx = fmaxf(mx, v);
             }
-            kf = fw_expo(fw_max(mx));
+            kf = fw_expo(fw_max(mx)) - FW_TOP;
         }
+        // the same as above for the forward vector of n states
+        auto bring_up = [&](int n) {
+            if (kf >= FW_LOW) return;
+            __syncwarp();
+            for (int i = lane; i < n; i += 32) {
+                FA[i] = fw_exp2(FA[i], -kf);
+                if (HB) FB[i] = fw_exp2(FB[i], -kf);
+            }
+            __syncwarp();
+            fpd = fw_exp2(fpd, -kf);
+            Ea += kf;
+            kf = 0;
+        };
+        bring_up(S);
         // emission statistics at t from the column products g in colv and the
         // detached state's gd, both in the frame 2^e / P
         auto emission = [&](int t, float gd, int e) {
@@ -707,10 +737,13 @@ __global__ void __launch_bounds__(FW_WARPS * 32, 2) wp_fit_warp_kernel(FitArgs a
             const float mine_v = fw_sums<NR>(sum, lane);
             if (lane < 2) (lane == 0 ? dx : dn)[t - 1] = mine_v;
             if (lane == 0) dfr[t - 1] = fr;
-            tsum = fma((double)mine_v, fw_exp2d(fr), tsum);
+            // (the Edman sums' backward vectors are those before x_t was brought up)
+            const int fe = Ea + kmx[t] - EP + (t + 1 < T ? Ebr[t + 1] + kx[t + 1] : 0);
+            tsum = fma((double)mine_v, fw_exp2d((lane & ~1) == 4 ? fe : fr), tsum);
             fpd = wv[0] * sc * fmaf(p, __shfl_sync(0xffffffffu, mine_v, 3), fpd);
             Ea += kf + kmx[t];
-            kf = fw_expo(fw_max(fmaxf(mx, fpd)));
+            kf = fw_expo(fw_max(fmaxf(mx, fpd))) - FW_TOP;
+            bring_up((t + 1) * S);
         }
         if (a.emission) {
             __syncwarp();
