@@ -102,3 +102,30 @@ def test_blinking_read(gpu_ctx, oracle, case, clean):
     if emission:
         for k in ("emis_w", "emis_x", "emis_xx"):
             near(k, e[k], np.full_like(e[k], e["emis_w"].sum() / C))
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+def test_subnormal_largest_entry(gpu_ctx, oracle, kind):
+    """One dye dark for four cycles and nearly so for a fifth: the vector left has its
+    largest entry near 2^-138, beyond 2^-127 which one FP32 factor undoes, and with 11
+    bits there (the warp kernel holds it higher).  Some ten roundings of 2^-12 in a row:
+    2.5e-3 of a count; 1e-2 allowed."""
+    C, T = 1, 10
+    sm = paper_model(C)
+    seq = np.asarray(parse_dye_seq("........0"))
+    x = _blinking(sm, C, T, seq, 0, 4)
+    x[0, 5, 0] = 0.038
+    gpu_ctx.upload_model(sm, T)
+    gpu_ctx.fit_begin(seq, x)
+    gpu_ctx.fit_set_kernel(kind)
+    try:
+        sums, _, _ = gpu_ctx.fit_estep()
+    finally:
+        gpu_ctx.fit_set_kernel(0)
+    a = sums.as_dict(T, C)
+    _, _, o = oracle.improve_fit(sm, T, seq, x[0], 1)
+    e = o.as_dict(T, C)
+    for k in ("edman", "bleach", "dud", "cyc_block"):
+        for j, w in enumerate(("_num", "_den")):
+            assert np.all(np.abs(a[k + w] - np.asarray(e[k][j])) <= 1e-2 * np.maximum(e[k][1], 1e-3)), (k + w, a[k + w], e[k][j])
+    assert np.all(np.abs(a["detach_n"] - e["detach_n"]) <= 1e-2), (a["detach_n"], e["detach_n"])

@@ -85,6 +85,14 @@ __device__ void vec_scale_pow2(const Vec& v, long n, int k) {
     v.pd() *= f;
 }
 
+// The exponent that a vector of largest entry mx is normalised by: at least -126,
+// as exp2i ends at 2^127 (a subnormal largest entry then stays below 1/2).
+__device__ __forceinline__ int fit_norm_expo(float mx) {
+    int k = 0;
+    if (mx > 0.0f) frexpf(mx, &k);
+    return max(k, -126);
+}
+
 struct Shape {
     int C, S;
     int W[WP_MAX_CHANNELS];   // D_c + 1
@@ -317,8 +325,7 @@ __device__ double fit_read(const FitArgs& a, const SmemModel& M, int r, const Sh
                 mx = fmaxf(mx, bv[0].A(i));
                 if (HB) mx = fmaxf(mx, bv[0].B(i));
             }
-            int k = 0;
-            if (mx > 0.0f) frexpf(mx, &k);
+            const int k = fit_norm_expo(mx);
             Vec cp = vec(CP0 + t);
             for (long i = 0; i < n0; i++) {
                 cp.A(i) = bv[0].A(i);
@@ -426,8 +433,7 @@ __device__ double fit_read(const FitArgs& a, const SmemModel& M, int r, const Sh
         al.pd() *= emit_at(a, tab, sh, 0, 0, kmax);
         tot += al.pd();
         Ea += kmax;
-        int k = 0;
-        if (tot > 0.0f) frexpf(tot, &k);
+        const int k = fit_norm_expo(tot);
         vec_scale_pow2<HB>(al, S, k);
         Ea += k;
     }
@@ -555,8 +561,7 @@ __device__ double fit_read(const FitArgs& a, const SmemModel& M, int r, const Sh
             al.pd() *= emit_at(a, tab, sh, t, 0, kmax);
             tot += al.pd();
             Ea += kmax;
-            int k = 0;
-            if (tot > 0.0f) frexpf(tot, &k);
+            const int k = fit_norm_expo(tot);
             vec_scale_pow2<HB>(al, n1, k);
             Ea += k;
         }
@@ -941,8 +946,7 @@ __global__ void __launch_bounds__(FIT_NT) wp_fit_cta_kernel(FitArgs a, float* ck
                 }
                 if (threadIdx.x == 0) mx = fmaxf(mx, *b0.pd);
                 cta_reduce<true>(&mx, 1, red, rout);
-                int k = 0;
-                if (rout[0] > 0.f) frexpf(rout[0], &k);
+                const int k = fit_norm_expo(rout[0]);
                 const float sc = exp2i(-k);
                 copy_vec(b0, gvec(t), n0, sc);
                 copy_vec(b0, vec(CUR), n0, sc);
@@ -1055,8 +1059,7 @@ __global__ void __launch_bounds__(FIT_NT) wp_fit_cta_kernel(FitArgs a, float* ck
             }
             if (threadIdx.x == 0) tot += *al2.pd;
             cta_reduce<false>(&tot, 1, red, rout);
-            int k = 0;
-            if (rout[0] > 0.f) frexpf(rout[0], &k);
+            const int k = fit_norm_expo(rout[0]);
             Ea += kmx[0];
             copy_vec(al2, al2, S, exp2i(-k));
             Ea += k;
@@ -1240,8 +1243,7 @@ __global__ void __launch_bounds__(FIT_NT) wp_fit_cta_kernel(FitArgs a, float* ck
                 }
                 if (threadIdx.x == 0) tot += *al.pd;
                 cta_reduce<false>(&tot, 1, red, rout);
-                int k = 0;
-                if (rout[0] > 0.f) frexpf(rout[0], &k);
+                const int k = fit_norm_expo(rout[0]);
                 Ea += kmx[t];
                 copy_vec(al, al, n1, exp2i(-k));
                 Ea += k;
