@@ -104,6 +104,41 @@ def test_blinking_read(gpu_ctx, oracle, case, clean):
             near(k, e[k], np.full_like(e[k], e["emis_w"].sum() / C))
 
 
+FAR = [
+    # C, T, dye-seq, dark channel, from cycle, dark cycles.  Kernel 0 is the warp kernel, and
+    # for the second shape (110 states, 44 timesteps) the CTA kernel.
+    (1, 60, "." * 56 + "0", 0, 1, 40),
+    (2, 44, "0" * 8 + "1" * 10 + "." * 30 + "0", 0, 8, 35),
+]
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("case", FAR, ids=["C1T60", "C2T44"])
+def test_frame_beyond_fp64(gpu_ctx, case, kind):
+    """Forward and backward vectors whose overlap is below 2^-1023, the end of an
+    FP64 factor: finite sums (the read's own counts have underflowed)."""
+    C, T, s, channel, start, dark = case
+    sm = paper_model(C)
+    seq = np.asarray(parse_dye_seq(s))
+    x = _blinking(sm, C, T, seq, channel, 0)
+    x[0, start:start + dark, channel] = 0.003
+    gpu_ctx.upload_model(sm, T)
+    gpu_ctx.fit_begin(seq, x)
+    gpu_ctx.fit_set_emission(True)
+    gpu_ctx.fit_set_kernel(kind)
+    try:
+        sums, lp, nz = gpu_ctx.fit_estep()
+        em = gpu_ctx.fit_emission_sums().arrays(C)
+    finally:
+        gpu_ctx.fit_set_kernel(0)
+        gpu_ctx.fit_set_emission(False)
+    assert nz == 0 and np.isfinite(lp)
+    for k, v in sums.as_dict(T, C).items():
+        assert np.all(np.isfinite(v)), (k, v)
+    for v in em:
+        assert np.all(np.isfinite(v))
+
+
 @pytest.mark.parametrize("kind", [0, 1])
 def test_subnormal_largest_entry(gpu_ctx, oracle, kind):
     """One dye dark for four cycles and nearly so for a fifth: the vector left has its

@@ -93,6 +93,10 @@ __device__ __forceinline__ int fit_norm_expo(float mx) {
     return max(k, -126);
 }
 
+// 2^e / Pm, the factor of sums over states.  Where e passes 1000 the sums have long
+// underflowed to zero, and zero they must stay.
+__device__ __forceinline__ double fit_frame(float Pm, int e) { return ldexp(1.0 / (double)Pm, min(e, 1000)); }
+
 struct Shape {
     int C, S;
     int W[WP_MAX_CHANNELS];   // D_c + 1
@@ -351,7 +355,7 @@ __device__ double fit_read(const FitArgs& a, const SmemModel& M, int r, const Sh
     const double logP = log((double)Pm) + (double)EP * 0.69314718055994530942;
     // scale(t) = 2^(Ea + Eb_chain - EP) / Pm, the factor turning f*b products of
     // the scaled vectors into f*b/P.
-    auto scale_of = [&](int Ea, int Ebc) { return ldexp(1.0 / (double)Pm, Ea + Ebc - EP); };
+    auto scale_of = [&](int Ea, int Ebc) { return fit_frame(Pm, Ea + Ebc - EP); };
 
     // Emission statistics at emission t (no reference counterpart): the
     // posterior f * b / P of each state (f the forward vector before the
@@ -967,7 +971,7 @@ __global__ void __launch_bounds__(FIT_NT) wp_fit_cta_kernel(FitArgs a, float* ck
         const float Pm = frexpf(Ps, &EP);
         EP += Eb[0];
         if (threadIdx.x == 0 && a.logp) a.logp[ro] = log((double)Pm) + (double)EP * 0.69314718055994530942;
-        auto scale_of = [&](int Ea, int Ebc) { return ldexp(1.0 / (double)Pm, Ea + Ebc - EP); };
+        auto scale_of = [&](int Ea, int Ebc) { return fit_frame(Pm, Ea + Ebc - EP); };
 
         // emission statistics of emission t from the buckets (thread 0, FP64)
         auto emis_add = [&](int t, const SVec& f, const SVec& b, double sc) {
