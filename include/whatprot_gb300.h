@@ -502,7 +502,8 @@ wp_status wp_mlp_train(wp_ctx* ctx, wp_mlp* mlp, long long num_reads, int batch,
                        float lr, unsigned long long seed, double* out_loss);
 
 /* One step on a device batch: d_x [B][T*C] FP32, d_labels [B] peptide
- * indices (-1: skip), B a multiple of 64.  lr 0 computes the gradients only
+ * indices (below 0: skip; of the set's size or more: WP_ERR_INVALID after a
+ * step that skips them and changes no weight), B a multiple of 64.  lr 0 computes the gradients only
  * (wp_mlp_get with grad = 1 reads them). */
 wp_status wp_mlp_train_step(wp_ctx* ctx, wp_mlp* mlp, const float* d_x,
                             const int32_t* d_labels, int B, float lr,

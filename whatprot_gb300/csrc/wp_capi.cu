@@ -93,10 +93,10 @@ cudaError_t wp_launch_dedup(const DedupArgs& a, cudaStream_t s, int* launches);
 cudaError_t wp_mlp_launch_input(const float* xf, const double* xd, int B, int TC, __nv_bfloat16* X, cudaStream_t s);
 cudaError_t wp_mlp_launch_colsum(const __nv_bfloat16* M, int rows, int cols, int ld, float* out, cudaStream_t s);
 cudaError_t wp_mlp_launch_softmax_ce(const float* logits, int B, int P, int ld, const int* labels, float scale,
-                                     __nv_bfloat16* dL, double* loss, cudaStream_t s);
+                                     __nv_bfloat16* dL, double* loss, int* bad, cudaStream_t s);
 cudaError_t wp_mlp_launch_gelu_bwd(const float* dH, const __nv_bfloat16* Z, long n, __nv_bfloat16* dZ, cudaStream_t s);
 cudaError_t wp_mlp_launch_adam(float* w, const float* g, float* m, float* v, long n, float lr, float b1, float b2,
-                               float eps, float bc1, float bc2, __nv_bfloat16* wb, cudaStream_t s);
+                               float eps, float bc1, float bc2, __nv_bfloat16* wb, const int* bad, cudaStream_t s);
 cudaError_t wp_mlp_launch_to_bf16(const float* in, long n, __nv_bfloat16* out, cudaStream_t s);
 cudaError_t wp_mlp_launch_init(float* w, long rows, long cols, long valid_rows, float std, unsigned long long seed,
                                cudaStream_t s);
@@ -3172,7 +3172,8 @@ struct wp_mlp {
     DevBuf w[6], g[6], m[6], v[6];
     long n[6] = {0, 0, 0, 0, 0, 0};
     DevBuf W1b, W2b, W3b;  // BF16 copies
-    DevBuf X, Z1, H1, Z2, H2, dL, dZ2, dZ1, L, dH2, dH1, loss, labels, xsim, err;
+    DevBuf X, Z1, H1, Z2, H2, dL, dZ2, dZ1, L, dH2, dH1, loss, labels, xsim;
+    DevBuf err;  // a pipeline wait that expired; a label without a class
     DevBuf topi, topp, mass, counts, loss_sum, tkfail;
     // a training step's small reductions beside its large products
     cudaStream_t side = nullptr;
@@ -3249,7 +3250,7 @@ wp_status mlp_step(wp_ctx* ctx, wp_mlp* m, const int* labels, int B, float lr) {
     wp_status st = mlp_forward(ctx, m, B);
     if (st != WP_OK) return st;
     MLP_CUDA(wp_mlp_launch_softmax_ce(m->L.as<float>(), B, m->P, Pp, labels, 1.0f / (float)B,
-                                      m->dL.as<bf16>(), m->loss.as<double>(), s), "softmax");
+                                      m->dL.as<bf16>(), m->loss.as<double>(), m->err.as<int>() + 1, s), "softmax");
     ctx->launches++;
     // The bias gradients (column sums) and dW1 take few SMs; they run on a second
     // stream, on the SMs that the large products leave (128 and 126 of 152), dW3
@@ -3292,7 +3293,8 @@ wp_status mlp_step(wp_ctx* ctx, wp_mlp* m, const int* labels, int B, float lr) {
         bf16* wb[6] = {m->W1b.as<bf16>(), nullptr, m->W2b.as<bf16>(), nullptr, m->W3b.as<bf16>(), nullptr};
         for (int i = 0; i < 6; i++) {
             MLP_CUDA(wp_mlp_launch_adam(m->w[i].as<float>(), m->g[i].as<float>(), m->m[i].as<float>(),
-                                        m->v[i].as<float>(), m->n[i], lr, b1, b2, eps, bc1, bc2, wb[i], s), "adam");
+                                        m->v[i].as<float>(), m->n[i], lr, b1, b2, eps, bc1, bc2, wb[i], m->err.as<int>() + 1, s),
+                     "adam");
             ctx->launches++;
         }
     }
@@ -3309,9 +3311,13 @@ wp_status mlp_check(wp_ctx* ctx, wp_mlp* m) {
 
 wp_status mlp_finish(wp_ctx* ctx, wp_mlp* m) {
     MLP_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
-    int err = 0;
-    MLP_CUDA(cudaMemcpy(&err, m->err.p, sizeof(int), cudaMemcpyDeviceToHost), "read err");
-    if (err) return fail(ctx, WP_ERR_TIMEOUT, "a tensor-core GEMM pipeline wait expired");
+    int err[2] = {0, 0};
+    MLP_CUDA(cudaMemcpy(err, m->err.p, sizeof(err), cudaMemcpyDeviceToHost), "read err");
+    if (err[0]) return fail(ctx, WP_ERR_TIMEOUT, "a tensor-core GEMM pipeline wait expired");
+    if (err[1]) {
+        MLP_CUDA(cudaMemsetAsync(m->err.as<int>() + 1, 0, sizeof(int), ctx->stream), "clear err");
+        return fail(ctx, WP_ERR_INVALID, "a label is not a class of the network");
+    }
     return WP_OK;
 }
 
@@ -3377,11 +3383,11 @@ wp_status wp_mlp_create(wp_ctx* ctx, int hidden, unsigned long long seed, wp_mlp
         }
     }
     if (m->W1b.ensure(sizeof(bf16) * H * 64) || m->W2b.ensure(sizeof(bf16) * H * H) ||
-        m->W3b.ensure(sizeof(bf16) * Pp * H) || m->err.ensure(sizeof(int)) || m->loss_sum.ensure(sizeof(double))) {
+        m->W3b.ensure(sizeof(bf16) * Pp * H) || m->err.ensure(2 * sizeof(int)) || m->loss_sum.ensure(sizeof(double))) {
         delete m;
         return fail(ctx, WP_ERR_OOM, "alloc network");
     }
-    cudaMemsetAsync(m->err.p, 0, sizeof(int), ctx->stream);
+    cudaMemsetAsync(m->err.p, 0, 2 * sizeof(int), ctx->stream);
     // He-style initialisation: N(0, 2 / fan_in) for the GELU layers,
     // N(0, 1 / fan_in) for the logits; biases zero; padded classes zero.
     cudaError_t e = wp_mlp_launch_init(m->w[0].as<float>(), H, 64, H, sqrtf(2.0f / (float)TC), seed, ctx->stream);
@@ -3477,6 +3483,7 @@ wp_status wp_mlp_train_step(wp_ctx* ctx, wp_mlp* m, const float* d_x, const int3
     st = mlp_step(ctx, m, m->labels.as<int>(), B, lr);
     if (st != WP_OK) return st;
     st = mlp_finish(ctx, m);
+    if (st == WP_ERR_INVALID && lr > 0.0f) m->steps--;  // no weight was changed
     if (st != WP_OK) return st;
     if (out_loss) {
         std::vector<double> hl(B);

@@ -74,7 +74,8 @@ __device__ float block_sum(float v, float* sh) {
 }
 
 // One CTA per row: softmax over the first P logits, cross-entropy against
-// the label (rows with label < 0 are skipped: loss 0, gradient 0), and the
+// the label (rows with label < 0 are skipped: loss 0, gradient 0; so are those
+// with a label of P or more, which set *bad), and the
 // logit gradient (softmax - onehot) * scale as BF16 (zero past P).  The row
 // (ld a multiple of 4, 16-byte aligned) stays in shared memory, so HBM sees
 // each logit once and each exponential is formed once.  Bound by issue slots and
@@ -84,12 +85,17 @@ __device__ float block_sum(float v, float* sh) {
 // again for each pass.
 __global__ void __launch_bounds__(256) wp_softmax_ce_kernel(const float* __restrict__ logits, int P, int ld,
                                                             const int* __restrict__ labels, float scale,
-                                                            bf16* __restrict__ dL, double* __restrict__ loss, int keep) {
+                                                            bf16* __restrict__ dL, double* __restrict__ loss, int keep,
+                                                            int* __restrict__ bad) {
     extern __shared__ __align__(16) float ce_row[];
     __shared__ float sh[32];
     const long row = blockIdx.x;
     const float* l = logits + row * ld;
-    const int y = labels[row];
+    int y = labels[row];
+    if (y >= P) {  // from the caller's memory: no class, and no index
+        y = -1;
+        if (threadIdx.x == 0) atomicExch(bad, 1);
+    }
     float mx = -INFINITY;
     if (keep) {
 #pragma unroll 4
@@ -220,13 +226,14 @@ __global__ void __launch_bounds__(256) wp_colsum_bf16_kernel(const bf16* __restr
 }
 
 // Adam (Kingma & Ba 2015) on FP32 master weights; refreshes the BF16 copy.
-// Four weights per thread (n a multiple of 4, 16-byte aligned).  Bound by HBM (30
+// Four weights per thread (n a multiple of 4, 16-byte aligned).  Nothing is
+// changed where *bad is set (a label without a class).  Bound by HBM (30
 // bytes per weight): 20.5 million in 84 us, 113 with one weight per thread.
 __global__ void wp_adam_kernel(float4* __restrict__ w, const float4* __restrict__ g, float4* __restrict__ m,
                                float4* __restrict__ v, long n4, float lr, float b1, float b2, float eps, float bc1,
-                               float bc2, uint2* __restrict__ wb) {
+                               float bc2, uint2* __restrict__ wb, const int* __restrict__ bad) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n4) return;
+    if (i >= n4 || *bad) return;
     const float4 g4 = g[i], m4 = m[i], v4 = v[i], w4 = w[i];
     const float gi[4] = {g4.x, g4.y, g4.z, g4.w};
     float mi[4] = {m4.x, m4.y, m4.z, m4.w}, vi[4] = {v4.x, v4.y, v4.z, v4.w}, wi[4] = {w4.x, w4.y, w4.z, w4.w};
@@ -684,7 +691,7 @@ cudaError_t wp_mlp_launch_colsum(const bf16* M, int rows, int cols, int ld, floa
 }
 
 cudaError_t wp_mlp_launch_softmax_ce(const float* logits, int B, int P, int ld, const int* labels, float scale,
-                                     bf16* dL, double* loss, cudaStream_t s) {
+                                     bf16* dL, double* loss, int* bad, cudaStream_t s) {
     // two CTAs per SM keep their rows up to 28,000 logits, one up to 56,000
     const size_t smem = sizeof(float) * ld;
     const bool keep = smem <= 220 * 1024;
@@ -693,7 +700,7 @@ cudaError_t wp_mlp_launch_softmax_ce(const float* logits, int B, int P, int ld, 
             cudaFuncSetAttribute(wp_softmax_ce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    wp_softmax_ce_kernel<<<B, 256, keep ? smem : 0, s>>>(logits, P, ld, labels, scale, dL, loss, keep ? 1 : 0);
+    wp_softmax_ce_kernel<<<B, 256, keep ? smem : 0, s>>>(logits, P, ld, labels, scale, dL, loss, keep ? 1 : 0, bad);
     return cudaGetLastError();
 }
 
@@ -707,12 +714,12 @@ cudaError_t wp_mlp_launch_gelu_bwd(const float* dH, const bf16* Z, long n, bf16*
 }
 
 cudaError_t wp_mlp_launch_adam(float* w, const float* g, float* m, float* v, long n, float lr, float b1, float b2,
-                               float eps, float bc1, float bc2, bf16* wb, cudaStream_t s) {
+                               float eps, float bc1, float bc2, bf16* wb, const int* bad, cudaStream_t s) {
     if (n % 4) return cudaErrorInvalidValue;
     const long n4 = n / 4;
     wp_adam_kernel<<<(int)((n4 + 255) / 256), 256, 0, s>>>(
             reinterpret_cast<float4*>(w), reinterpret_cast<const float4*>(g), reinterpret_cast<float4*>(m),
-            reinterpret_cast<float4*>(v), n4, lr, b1, b2, eps, bc1, bc2, reinterpret_cast<uint2*>(wb));
+            reinterpret_cast<float4*>(v), n4, lr, b1, b2, eps, bc1, bc2, reinterpret_cast<uint2*>(wb), bad);
     return cudaGetLastError();
 }
 
