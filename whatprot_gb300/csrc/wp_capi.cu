@@ -47,7 +47,6 @@ cudaError_t wp_launch_engine(int C, bool has_block, int threads, size_t smem, cu
                              int2* out, int* out_count, int slab_half, int scr_floats,
                              int spill_error, long pairs, int* grid_out);
 size_t wp_engine_smem_bytes(int slab_half, int scr_floats, bool has_block, int threads);
-cudaError_t wp_launch_shape(const void* kernel, int threads, size_t smem, int* per_sm, int* sms);
 void wp_launch_shape_forget();
 cudaError_t wp_launch_coop(int C, bool has_block, int lanes, cudaStream_t s, const BatchArgs& a, const int2* in,
                            const int* in_count, int* in_head, int2* out, int* out_count, int slab_half,

@@ -431,6 +431,10 @@ __device__ __forceinline__ void load_smem_model(SmemModel& S, const DevModel& m)
     }
 }
 
+// CTAs of a shape per SM and the device's SMs, the kernel ready to be launched so
+// (wp_shape.cu): for every kernel whose dynamic shared memory varies.
+cudaError_t wp_launch_shape(const void* kernel, int threads, size_t smem, int* per_sm, int* sms);
+
 // Arguments of one Baum-Welch E-step (wp_fit.cu).
 struct FitArgs {
     const DevModel* model;

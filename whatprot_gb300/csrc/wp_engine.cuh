@@ -150,6 +150,3 @@ struct EngineLists {
     int scr_floats;   // reserved per-thread scratch (floats), 0 when unused
     int spill_error;  // nonzero: nothing downstream takes spills; flag err
 };
-
-// wp_shape.cu
-cudaError_t wp_launch_shape(const void* kernel, int threads, size_t smem, int* per_sm, int* sms);

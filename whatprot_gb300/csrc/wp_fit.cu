@@ -1274,26 +1274,27 @@ long wp_fit_cta_ckpt_floats(int T, int S, bool has_block) {
     return (long)(T + 1) * VS;
 }
 
+static const void* fit_cta_kernel(bool has_block) {
+    return has_block ? reinterpret_cast<const void*>(wp_fit_cta_kernel<true>)
+                     : reinterpret_cast<const void*>(wp_fit_cta_kernel<false>);
+}
+
 cudaError_t wp_launch_fit_cta(bool has_block, int grid, size_t smem, cudaStream_t s, const FitArgs& a, float* ckpt,
                               long ck_stride) {
-    if (has_block) {
-        cudaFuncSetAttribute(wp_fit_cta_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        wp_fit_cta_kernel<true><<<grid, FIT_NT, smem, s>>>(a, ckpt, ck_stride);
-    } else {
-        cudaFuncSetAttribute(wp_fit_cta_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        wp_fit_cta_kernel<false><<<grid, FIT_NT, smem, s>>>(a, ckpt, ck_stride);
-    }
+    int per_sm = 0, sms = 0;
+    const cudaError_t e = wp_launch_shape(fit_cta_kernel(has_block), FIT_NT, smem, &per_sm, &sms);
+    if (e != cudaSuccess) return e;
+    if (has_block) wp_fit_cta_kernel<true><<<grid, FIT_NT, smem, s>>>(a, ckpt, ck_stride);
+    else wp_fit_cta_kernel<false><<<grid, FIT_NT, smem, s>>>(a, ckpt, ck_stride);
     return cudaGetLastError();
 }
 
+// Resident CTAs per SM (0: the shape does not fit).
 int wp_fit_cta_ctas_per_sm(bool has_block, size_t smem) {
-    int n = 0;
-    if (has_block) {
-        cudaFuncSetAttribute(wp_fit_cta_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wp_fit_cta_kernel<true>, FIT_NT, smem);
-    } else {
-        cudaFuncSetAttribute(wp_fit_cta_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wp_fit_cta_kernel<false>, FIT_NT, smem);
+    int n = 0, sms = 0;
+    if (wp_launch_shape(fit_cta_kernel(has_block), FIT_NT, smem, &n, &sms) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
     }
     return n;
 }

@@ -834,12 +834,8 @@ int wp_fit_warp_max_warps() { return FW_WARPS; }
 int wp_fit_warp_ctas_per_sm(int C, bool hb, size_t smem, int warps) {
     const void* k = fw_pick(C, hb);
     if (!k) return 0;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, warps * 32, smem) != cudaSuccess) {
+    int n = 0, sms = 0;
+    if (wp_launch_shape(k, warps * 32, smem, &n, &sms) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -852,7 +848,8 @@ cudaError_t wp_launch_fit_warp(int C, bool hb, int grid, int warps, size_t smem,
     if (!k) return cudaErrorInvalidValue;
     FitArgs args = a;
     void* p[] = {&args, &slab, &slab_stride};
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int per_sm = 0, sms = 0;
+    const cudaError_t e = wp_launch_shape(k, warps * 32, smem, &per_sm, &sms);
     if (e != cudaSuccess) return e;
     return cudaLaunchKernel(k, dim3(grid), dim3(warps * 32), p, smem, s);
 }

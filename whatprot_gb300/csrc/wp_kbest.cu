@@ -725,8 +725,9 @@ size_t wp_kbest_smem_bytes(int TC, int NC, int stack_cap, bool inter) {
 
 template <int DP, bool INTER>
 static cudaError_t kb_launch(int grid, size_t smem, cudaStream_t s, const KBArgs& a) {
-    cudaError_t e = cudaFuncSetAttribute(wp_kbest_kernel<DP, INTER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    int per_sm = 0, sms = 0;
+    const cudaError_t e = wp_launch_shape(reinterpret_cast<const void*>(wp_kbest_kernel<DP, INTER>), KB_WARPS * 32,
+                                          smem, &per_sm, &sms);
     if (e != cudaSuccess) return e;
     wp_kbest_kernel<DP, INTER><<<grid, KB_WARPS * 32, smem, s>>>(a);
     return cudaGetLastError();

@@ -1176,8 +1176,9 @@ size_t wp_khits_smem_bytes(int TC, int NC, int stack_cap) {
 
 template <int DP>
 static cudaError_t kh_launch(int grid, size_t smem, cudaStream_t s, const KHArgs& a) {
-    cudaError_t e =
-        cudaFuncSetAttribute(wp_khits_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int per_sm = 0, sms = 0;
+    const cudaError_t e = wp_launch_shape(reinterpret_cast<const void*>(wp_khits_kernel<DP>), KH_WARPS * 32, smem,
+                                          &per_sm, &sms);
     if (e != cudaSuccess) return e;
     wp_khits_kernel<DP><<<grid, KH_WARPS * 32, smem, s>>>(a);
     return cudaGetLastError();

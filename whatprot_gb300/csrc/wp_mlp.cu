@@ -28,6 +28,9 @@
 #include <math.h>
 #include <stdint.h>
 
+// wp_shape.cu
+cudaError_t wp_launch_shape(const void* kernel, int threads, size_t smem, int* per_sm, int* sms);
+
 typedef __nv_bfloat16 bf16;
 
 // Radiometries (FP32 or FP64, [B][TC]) to BF16 inputs [B][64] (zero padded).
@@ -696,8 +699,9 @@ cudaError_t wp_mlp_launch_softmax_ce(const float* logits, int B, int P, int ld, 
     const size_t smem = sizeof(float) * ld;
     const bool keep = smem <= 220 * 1024;
     if (keep) {
+        int per_sm = 0, sms = 0;
         const cudaError_t e =
-            cudaFuncSetAttribute(wp_softmax_ce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                wp_launch_shape(reinterpret_cast<const void*>(wp_softmax_ce_kernel), 256, smem, &per_sm, &sms);
         if (e != cudaSuccess) return e;
     }
     wp_softmax_ce_kernel<<<B, 256, keep ? smem : 0, s>>>(logits, P, ld, labels, scale, dL, loss, keep ? 1 : 0, bad);

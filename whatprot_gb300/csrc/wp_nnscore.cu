@@ -450,9 +450,8 @@ size_t wp_nn_score_smem_bytes(int U, int table_entries) {
 }
 
 int wp_nn_score_ctas_per_sm(size_t smem) {
-    int n = 0;
-    if (cudaFuncSetAttribute(wp_nn_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wp_nn_score_kernel, SC_THREADS, smem) != cudaSuccess) {
+    int n = 0, sms = 0;
+    if (wp_launch_shape(reinterpret_cast<const void*>(wp_nn_score_kernel), SC_THREADS, smem, &n, &sms) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -461,7 +460,10 @@ int wp_nn_score_ctas_per_sm(size_t smem) {
 
 cudaError_t wp_launch_nn_score(int grid, size_t smem, cudaStream_t s, const NNScoreArgs& a) {
     if (a.R == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(a.next, 0, sizeof(int), s);
+    int n = 0, sms = 0;
+    cudaError_t e =
+            wp_launch_shape(reinterpret_cast<const void*>(wp_nn_score_kernel), SC_THREADS, smem, &n, &sms);
+    if (e == cudaSuccess) e = cudaMemsetAsync(a.next, 0, sizeof(int), s);
     if (e != cudaSuccess) return e;
     wp_nn_score_kernel<<<grid, SC_THREADS, smem, s>>>(a);
     return cudaGetLastError();
