@@ -47,7 +47,7 @@ cudaError_t wp_launch_engine(int C, bool has_block, int threads, size_t smem, cu
                              int2* out, int* out_count, int slab_half, int scr_floats,
                              int spill_error, long pairs, int* grid_out);
 size_t wp_engine_smem_bytes(int slab_half, int scr_floats, bool has_block, int threads);
-void wp_launch_shape_forget();
+void wp_launch_shape_check();
 cudaError_t wp_launch_coop(int C, bool has_block, int lanes, cudaStream_t s, const BatchArgs& a, const int2* in,
                            const int* in_count, int* in_head, int2* out, int* out_count, int slab_half,
                            int spill_error, long pairs);
@@ -1852,13 +1852,13 @@ wp_status wp_ctx_create(wp_ctx** out, int device) {
     if (cudaGetDeviceCount(&n) != cudaSuccess || n == 0 || device < 0 || device >= n) return WP_ERR_CUDA;
     wp_ctx* ctx = new (std::nothrow) wp_ctx();
     if (!ctx) return WP_ERR_OOM;
-    wp_launch_shape_forget();
     ctx->device = device;
     if (cudaSetDevice(device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) {
         delete ctx;
         return WP_ERR_CUDA;
     }
+    wp_launch_shape_check();
     cudaDeviceGetAttribute(&ctx->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     if (ctx->d_model.ensure(sizeof(DevModel)) != cudaSuccess) {
         cudaStreamDestroy(ctx->stream);

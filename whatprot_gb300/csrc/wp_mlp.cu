@@ -23,7 +23,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <mutex>
 #include <curand_kernel.h>
 #include <math.h>
 #include <stdint.h>
@@ -748,24 +747,9 @@ cudaError_t wp_mlp_launch_topk(const float* logits, int R, int P, int ld, int h,
     cudaError_t e = cudaMemsetAsync(fail_count, 0, sizeof(int), s);
     if (e != cudaSuccess) return e;
     const size_t smem = sizeof(unsigned long long) * TK_WARPS * TK_CAP + sizeof(unsigned) * TK_WARPS * 256;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    // launch shape, once per device
-    static int shape_sms[64] = {0}, shape_per_sm[64] = {0};
-    static std::mutex shape_mu;
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> lk(shape_mu);
-    if (shape_sms[dev] == 0) {
-        e = cudaFuncSetAttribute(wp_topk_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        int sms0 = 0, per0 = 0;
-        cudaDeviceGetAttribute(&sms0, cudaDevAttrMultiProcessorCount, dev);
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per0, wp_topk_warp_kernel, TK_WARPS * 32, smem);
-        if (e != cudaSuccess) return e;
-        shape_per_sm[dev] = per0;
-        shape_sms[dev] = sms0;
-    }
-    const int sms = shape_sms[dev], per_sm = shape_per_sm[dev];
+    int sms = 0, per_sm = 0;
+    e = wp_launch_shape(reinterpret_cast<const void*>(wp_topk_warp_kernel), TK_WARPS * 32, smem, &per_sm, &sms);
+    if (e != cudaSuccess) return e;
     const int grid = std::max(1, std::min(sms * std::max(per_sm, 1), (R + TK_WARPS - 1) / TK_WARPS));
     const int vec4 = (ld % 4 == 0 && ((uintptr_t)logits & 15u) == 0) ? 1 : 0;
     wp_topk_warp_kernel<<<grid, TK_WARPS * 32, smem, s>>>(logits, R, P, ld, h, counts, idx, prob, mass, fail,

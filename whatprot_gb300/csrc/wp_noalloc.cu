@@ -37,7 +37,7 @@ __global__ void wp_prep_reads_kernel(const DevModel*, const double*, int, unsign
 __global__ void wp_read_summary_kernel(BatchArgs);
 __global__ void wp_compact_kernel(BatchArgs);
 __global__ void wp_reduce_kernel(BatchArgs, int32_t*, double*, double*, double*, const int*);
-void wp_launch_shape_forget();
+void wp_launch_shape_check();
 cudaError_t wp_launch_engine(int C, bool has_block, int threads, size_t smem, cudaStream_t s,
                              const BatchArgs& a, const int2* in, const int* in_count, int* in_head,
                              int2* out, int* out_count, int slab_half, int scr_floats,
@@ -88,7 +88,6 @@ extern "C" wp_status wp_hmm_classify_noalloc(int device, const wp_seq_model* m, 
     if (!m || R < 0 || P < 1 || !offsets || !ids || !counts) return WP_ERR_INVALID;
     if (R > 0 && (!rads || !out_id || !out_score || !out_total)) return WP_ERR_INVALID;
     if (device < 0 || device >= WP_NOALLOC_MAX_DEVICES) return WP_ERR_INVALID;
-    wp_launch_shape_forget();  // no context: the device may have been reset since the last call
     const int C = m->num_channels;
     if (C < 1 || C > WP_MAX_CHANNELS || T < 1 || T > WP_MAX_TIMESTEPS) return WP_ERR_UNSUPPORTED;
     if (!m->p_bleach || !m->p_dud || !m->bg_sig || !m->mu || !m->sig) return WP_ERR_INVALID;
@@ -149,6 +148,7 @@ extern "C" wp_status wp_hmm_classify_noalloc(int device, const wp_seq_model* m, 
 
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
     if (cudaSetDevice(device) != cudaSuccess) return WP_ERR_CUDA;
+    wp_launch_shape_check();
     // Set-up, once per device: the device address of the scratch array.
     // The first call on a device does this and must come before any stream
     // capture.

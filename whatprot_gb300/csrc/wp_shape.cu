@@ -2,59 +2,87 @@
 // device: how many CTAs share an SM, and the function attribute that allows the
 // shared memory.  A small classify call spent some 2 us of host time per launch
 // on asking again.
+//
+// The attribute belongs to the function on the device, whatever context asks: here
+// it only ever grows, so a launch finds what its thread was told.
 #include <cuda_runtime.h>
+#include <stdint.h>
 
-#include <map>
 #include <mutex>
-#include <tuple>
 
 namespace {
+
 struct Shape {
-    int per_sm, sms;
+    const void* kernel;  // null: free
+    size_t smem;
+    int dev, threads, per_sm, sms;
 };
-constexpr size_t MOST = 4096;  // shapes kept
+// A fixed table (callers that may not allocate come here too); a shape that finds its
+// places taken replaces the first of them and is asked for again by whoever lost it.
+constexpr int SETS = 256, WAYS = 4;
 std::mutex mu;
-std::map<std::tuple<const void*, int, int, size_t>, Shape> shapes;
+Shape shapes[SETS][WAYS];
+
+// Never launched: its attribute is MARK on a device whose function attributes are
+// as this file left them, and the default again after a reset of the device.
+__global__ void wp_shape_mark_kernel() {}
+constexpr int MARK = 40 * 1024;
+
+Shape* set_of(const void* kernel, int dev, int threads, size_t smem) {
+    uint64_t h = reinterpret_cast<uintptr_t>(kernel);
+    h = (h ^ (h >> 7)) * 0x9E3779B97F4A7C15ull;
+    h = (h ^ smem ^ ((uint64_t)threads << 32) ^ ((uint64_t)dev << 48)) * 0x9E3779B97F4A7C15ull;
+    return shapes[h >> 56];
+}
+
 }  // namespace
 
 // CTAs of `threads` threads and `smem` bytes of dynamic shared memory per SM of
 // the current device (*per_sm, 0 if none fits) and its SMs (*sms); the kernel may
-// be launched with that much shared memory afterwards.  Safe from several
-// threads: the attribute only ever grows.
+// be launched with that much shared memory afterwards.  Safe from several threads.
 cudaError_t wp_launch_shape(const void* kernel, int threads, size_t smem, int* per_sm, int* sms) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> lk(mu);
-    const auto key = std::make_tuple(kernel, dev, threads, smem);
-    const auto it = shapes.find(key);
-    if (it != shapes.end()) {
-        *per_sm = it->second.per_sm;
-        *sms = it->second.sms;
-        return cudaSuccess;
+    Shape* set = set_of(kernel, dev, threads, smem);
+    Shape* place = &set[0];
+    for (int i = WAYS - 1; i >= 0; i--) {
+        if (!set[i].kernel) {
+            place = &set[i];
+        } else if (set[i].kernel == kernel && set[i].smem == smem && set[i].dev == dev && set[i].threads == threads) {
+            *per_sm = set[i].per_sm;
+            *sms = set[i].sms;
+            return cudaSuccess;
+        }
     }
     cudaFuncAttributes attr;
     e = cudaFuncGetAttributes(&attr, kernel);
     if (e == cudaSuccess && (size_t)attr.maxDynamicSharedSizeBytes < smem)
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    Shape s = {0, 0};
+    Shape s = {kernel, smem, dev, threads, 0, 0};
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&s.sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s.per_sm, kernel, threads, smem);
     if (e != cudaSuccess) return e;
-    try {
-        if (shapes.size() >= MOST) shapes.clear();
-        shapes[key] = s;
-    } catch (...) {
-        // not kept: asked again next time
-    }
+    *place = s;
     *per_sm = s.per_sm;
     *sms = s.sms;
     return cudaSuccess;
 }
 
-// Forgets the shapes (a new context: the device may have been reset since, and
-// its function attributes with it).
-void wp_launch_shape_forget() {
+// At the start of a context's life, and of a call without one: if the current device
+// has been reset since its shapes were kept, its function attributes went with it,
+// and the shapes are forgotten.
+void wp_launch_shape_check() {
+    int dev = 0;
+    cudaFuncAttributes attr;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
     std::lock_guard<std::mutex> lk(mu);
-    shapes.clear();
+    const void* mark = reinterpret_cast<const void*>(wp_shape_mark_kernel);
+    if (cudaFuncGetAttributes(&attr, mark) == cudaSuccess && attr.maxDynamicSharedSizeBytes == MARK) return;
+    for (auto& set : shapes)
+        for (Shape& s : set)
+            if (s.dev == dev) s.kernel = nullptr;
+    cudaFuncSetAttribute(mark, cudaFuncAttributeMaxDynamicSharedMemorySize, MARK);
+    cudaGetLastError();  // not marked: asked again next time
 }
