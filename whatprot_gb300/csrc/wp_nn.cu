@@ -953,11 +953,12 @@ __global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelec
             nsel += __popc(sm);
         }
         __syncwarp();
-        // bitonic sort ascending by (score, id) over the next power of two
+        // bitonic sort ascending by (score, id) over the next power of two, by the
+        // scores' bits (wp_nnscore.cu)
         int n2 = 1;
         while (n2 < nsel) n2 <<= 1;
         for (int i = nsel + lane; i < n2; i += 32) {
-            s_key[wib][i] = INFINITY;
+            s_key[wib][i] = __longlong_as_double(-1ll);
             s_id[wib][i] = 0x7fffffff;
         }
         __syncwarp();
@@ -969,7 +970,8 @@ __global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelec
                         const bool up = (i & size) == 0;
                         const double ki = s_key[wib][i], kj = s_key[wib][j];
                         const int ii = s_id[wib][i], ij = s_id[wib][j];
-                        const bool gt = ki > kj || (ki == kj && ii > ij);
+                        const unsigned long long bi = nn_dbits(ki), bj = nn_dbits(kj);
+                        const bool gt = bi > bj || (bi == bj && ii > ij);
                         if (gt == up) {
                             s_key[wib][i] = kj;
                             s_key[wib][j] = ki;

@@ -391,12 +391,13 @@ __global__ void __launch_bounds__(SC_THREADS, 2) wp_nn_score_kernel(NNScoreArgs 
         int n2 = 1;
         while (n2 < nsel) n2 <<= 1;
         for (int i = nsel + tid; i < n2; i += SC_THREADS) {
-            s.val[i] = INFINITY;
+            s.val[i] = __longlong_as_double(-1ll);
             s.id[i] = 0x7fffffff;
         }
         __syncthreads();
         // bitonic sort ascending by (score, id); scores are never negative, so
-        // their bits order as they do
+        // their bits order as they do, and a NaN's (a read that is not finite) come
+        // after all but the padding's, whatever its sign
         for (int size = 2; size <= n2; size <<= 1)
             for (int stride = size >> 1; stride > 0; stride >>= 1) {
                 for (int i = tid; i < n2; i += SC_THREADS) {
@@ -404,7 +405,8 @@ __global__ void __launch_bounds__(SC_THREADS, 2) wp_nn_score_kernel(NNScoreArgs 
                     if (j > i) {
                         const double vi = s.val[i], vj = s.val[j];
                         const int ii = s.id[i], ij = s.id[j];
-                        const long long ki = __double_as_longlong(vi), kj = __double_as_longlong(vj);
+                        const unsigned long long ki = (unsigned long long)__double_as_longlong(vi),
+                                                 kj = (unsigned long long)__double_as_longlong(vj);
                         const bool gt = ki > kj || (ki == kj && ii > ij);
                         if (gt == ((i & size) == 0)) {
                             s.val[i] = vj;
