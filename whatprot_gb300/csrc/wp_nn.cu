@@ -991,6 +991,10 @@ __global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelec
             a.out_cand_score[(long)oq * h + i] = s_key[wib][i];
             if (a.out_cand_pep) a.out_cand_pep[(long)oq * h + i] = a.dense_pep[u];
         }
+        for (int i = nsel + lane; i < h; i += 32) {  // the places past them
+            a.out_cand_id[(long)oq * h + i] = -1;
+            a.out_cand_score[(long)oq * h + i] = 0.0;
+        }
         if (a.out_subfrac) {
             // HybridClassifier: sum of adjusted score x peptide count, in
             // candidate order (hybrid-classifier.cc:58-64); the terms formed
