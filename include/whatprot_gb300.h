@@ -553,6 +553,12 @@ long long wp_launch_count(const wp_ctx* ctx);
  * slab), [3] pairs run by the dense fallback.  No reference counterpart. */
 wp_status wp_last_batch_stats(wp_ctx* ctx, long long* stats4);
 
+/* Which kernels the last calls on this context took (tests, tuning):
+ * routes[0] reads of the last kNN batch whose k-hit set was found by levels,
+ * [1] reads whose search was replayed, [2] the last dedup's keys (0 no dedup
+ * yet, 1 words, 2 one key per instance).  No reference counterpart. */
+wp_status wp_last_routes(wp_ctx* ctx, long long* routes3);
+
 /* The context's CUDA stream (a cudaStream_t), for callers that order their
  * own work or events against it.  No reference counterpart. */
 void* wp_ctx_stream(const wp_ctx* ctx);

@@ -29,7 +29,7 @@ STATUS = {0: "WP_OK", 1: "WP_ERR_INVALID", 2: "WP_ERR_OOM", 3: "WP_ERR_CUDA",
 EXPORTS = ["wp_ctx_create", "wp_ctx_destroy", "wp_last_error", "wp_model_upload",
            "wp_peptides_upload", "wp_hmm_classify", "wp_hmm_classify_device",
            "wp_hmm_loglik_all", "wp_hmm_count_flops", "wp_launch_count", "wp_ctx_stream",
-           "wp_timing_enable", "wp_timing_read", "wp_probe_fp32_peak", "wp_last_batch_stats",
+           "wp_timing_enable", "wp_timing_read", "wp_probe_fp32_peak", "wp_last_batch_stats", "wp_last_routes",
            "wp_fit_begin", "wp_fit_estep", "wp_hmm_fit", "wp_fit_offset_exponential", "wp_fit_set_kernel",
            "wp_hmm_bootstrap_fit", "wp_fit_mstep", "wp_fit_set_emission", "wp_fit_emission_sums",
            "wp_fit_emission_mstep",
@@ -184,6 +184,8 @@ def load_library(path: Optional[str] = None):
     lib.wp_engine_replay.restype = I
     lib.wp_last_batch_stats.argtypes = [V, V]
     lib.wp_last_batch_stats.restype = I
+    lib.wp_last_routes.argtypes = [V, V]
+    lib.wp_last_routes.restype = I
     lib.wp_fit_set_kernel.argtypes = [V, I]
     lib.wp_fit_set_kernel.restype = I
     lib.wp_fit_begin.argtypes = [V, V, I, V, I]
@@ -769,6 +771,12 @@ class Context:
         out = np.zeros(4, np.int64)
         self._check(self.lib.wp_last_batch_stats(self.h, _ptr(out)))
         return {"slots": int(out[0]), "nonempty": int(out[1]), "pass2": int(out[2]), "dense": int(out[3])}
+
+    def last_routes(self) -> dict:
+        """wp_last_routes: reads of the last kNN batch by levels and replayed, the last dedup's keys."""
+        out = np.zeros(3, np.int64)
+        self._check(self.lib.wp_last_routes(self.h, _ptr(out)))
+        return {"levels": int(out[0]), "replayed": int(out[1]), "dedup": ("", "words", "rank")[int(out[2])]}
 
     def fp32_peak_tflops(self) -> float:
         out = ctypes.c_double()

@@ -310,6 +310,7 @@ struct wp_ctx {
     DevBuf d_nn_cnt8, d_nn_nodes, d_nn_ctab, d_nn_ecoord, d_nn_llo, d_nn_lhi;
     // the replay's scratch and results (wp_kbest.cu)
     DevBuf d_kb_reg, d_kb_prev, d_kb_stage, d_kb_next, d_kb_work, d_kb_tfd, d_kb_tfpos, d_kb_tfflag;
+    long long routes[3] = {0, 0, 0};  // wp_last_routes
     // the k-hit sets by levels (wp_khits.cu): counts as nibbles, scratch
     bool nn_nib_packed = false;
     DevBuf d_nn_nib, d_kh_ent, d_kh_d, d_kh_bin, d_kh_order, d_kh_rank, d_kh_state, d_kh_memd, d_kh_memk, d_kh_sorted, d_kh_seg, d_kh_kpos, d_kh_kd2,
@@ -1634,6 +1635,7 @@ wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, in
     WP_CUDA(ctx->d_nn_subfrac.ensure(sizeof(double) * Rz), "alloc");
     WP_CUDA(ctx->d_nn_err.ensure(sizeof(int)), "alloc");
     WP_CUDA(cudaMemsetAsync(ctx->d_nn_err.p, 0, sizeof(int), ctx->stream), "clear");
+    ctx->routes[0] = ctx->routes[1] = 0;
     if (R == 0) return WP_OK;
     if (N == 0) {
         WP_CUDA(cudaMemsetAsync(ctx->d_nn_ncand.p, 0, sizeof(int) * R, ctx->stream), "clear");
@@ -1705,6 +1707,8 @@ wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, in
             ctx->launches += 2;
         }
     }
+    ctx->routes[0] = R - left;
+    ctx->routes[1] = ctx->nn_selection == WP_NN_KDTREE ? left : 0;
     if (left > 0) {
         st = nn_run_slots(ctx, d_rads, left, R, k, sig, h, hybrid);
         if (st != WP_OK) return st;
@@ -1891,6 +1895,13 @@ const char* wp_last_error(const wp_ctx* ctx) { return ctx ? ctx->err.c_str() : "
 long long wp_launch_count(const wp_ctx* ctx) { return ctx ? ctx->launches : 0; }
 
 void* wp_ctx_stream(const wp_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
+
+wp_status wp_last_routes(wp_ctx* ctx, long long* routes) {
+    if (!ctx || !routes) return WP_ERR_INVALID;
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    for (int i = 0; i < 3; i++) routes[i] = ctx->routes[i];
+    return WP_OK;
+}
 
 wp_status wp_last_batch_stats(wp_ctx* ctx, long long* stats) {
     if (!ctx || !stats) return WP_ERR_INVALID;
@@ -2819,6 +2830,7 @@ wp_status dedup_run(wp_ctx* ctx, int n, int T, int C, int bits, const uint8_t* i
     const int most = ctx->sim_max_dyes;
     const int rank_bits = in_u8 && pep && most >= 1 && most <= 15 ? track_rank_bits(T, C, most) : 65;
     const bool ranked = rank_bits + id_bits <= 64;
+    ctx->routes[2] = ranked ? 2 : 1;
     const size_t nn = (size_t)std::max(n, 1);
     if (!ranked) WP_CUDA(ctx->d_dd_words.ensure(sizeof(uint64_t) * W * nn), "alloc dedup");
     WP_CUDA(ctx->d_dd_k0.ensure(sizeof(uint64_t) * nn), "alloc dedup");
