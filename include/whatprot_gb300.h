@@ -390,7 +390,7 @@ wp_status wp_nn_kd_tree_order(const double* coords, int N, int D, int k, int32_t
  * top h ids.  Writes per read out_ncand[r] <= h, out_cand_id /
  * out_cand_score [R][h] (ascending score, ties by ascending id; the
  * reference's heap leaves equal scores unordered) and out_total[r] =
- * sum(weight * hits).  Places past out_ncand[r]: id -1, score 0.  h <= 1024. */
+ * sum(weight * hits).  Places past out_ncand[r]: id 0, score 0.  h <= 1024. */
 wp_status wp_nn_classify(wp_ctx* ctx, const double* rads, int num_reads, int k,
                          double sig, int h, int32_t* out_ncand,
                          int32_t* out_cand_id, double* out_cand_score,

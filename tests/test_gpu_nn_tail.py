@@ -1,4 +1,4 @@
-"""Places of a read's candidate list past its candidates: id -1, score 0, whatever
+"""Places of a read's candidate list past its candidates: id 0, score 0, whatever
 the memory held before (a call with more candidates), in both vote kernels and with
 both selections."""
 import numpy as np
@@ -32,6 +32,6 @@ def test_places_past_the_candidates(gpu_ctx, selection, ids):
             assert n.min() < h
             for r in range(len(reads)):
                 assert np.all(cid[r, :n[r]] >= 0) and np.all(sc[r, :n[r]] > 0), r
-                assert np.all(cid[r, n[r]:] == -1) and np.all(sc[r, n[r]:] == 0), r
+                assert np.all(cid[r, n[r]:] == 0) and np.all(sc[r, n[r]:] == 0), r
     finally:
         gpu_ctx.set_nn_selection("kdtree")

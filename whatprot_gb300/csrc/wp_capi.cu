@@ -1641,7 +1641,7 @@ wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, in
         WP_CUDA(cudaMemsetAsync(ctx->d_nn_ncand.p, 0, sizeof(int) * R, ctx->stream), "clear");
         WP_CUDA(cudaMemsetAsync(ctx->d_nn_total.p, 0, sizeof(double) * R, ctx->stream), "clear");
         WP_CUDA(cudaMemsetAsync(ctx->d_nn_subfrac.p, 0, sizeof(double) * R, ctx->stream), "clear");
-        WP_CUDA(cudaMemsetAsync(ctx->d_nn_cand_id.p, 0xff, sizeof(int) * Rz * h, ctx->stream), "clear");
+        WP_CUDA(cudaMemsetAsync(ctx->d_nn_cand_id.p, 0, sizeof(int) * Rz * h, ctx->stream), "clear");
         WP_CUDA(cudaMemsetAsync(ctx->d_nn_cand_score.p, 0, sizeof(double) * Rz * h, ctx->stream), "clear");
         return WP_OK;
     }

@@ -992,7 +992,7 @@ __global__ void __launch_bounds__(NN_SEL_WARPS * 32) wp_nn_select_kernel(NNSelec
             if (a.out_cand_pep) a.out_cand_pep[(long)oq * h + i] = a.dense_pep[u];
         }
         for (int i = nsel + lane; i < h; i += 32) {  // the places past them
-            a.out_cand_id[(long)oq * h + i] = -1;
+            a.out_cand_id[(long)oq * h + i] = 0;
             a.out_cand_score[(long)oq * h + i] = 0.0;
         }
         if (a.out_subfrac) {

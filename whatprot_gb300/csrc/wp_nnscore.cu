@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) wp_nn_score_kernel(NNScoreArgs 
             if (a.out_subfrac) s.val[i] = (s.val[i] / tot) * (double)a.dense_count[u];
         }
         for (int i = nsel + tid; i < h; i += SC_THREADS) {  // the places past them
-            a.out_cand_id[(long)oq * h + i] = -1;
+            a.out_cand_id[(long)oq * h + i] = 0;
             a.out_cand_score[(long)oq * h + i] = 0.0;
         }
         if (a.out_subfrac) {
