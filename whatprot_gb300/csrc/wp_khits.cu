@@ -62,6 +62,9 @@
 // table look-ups of 48 coordinates for every entry met) and 41 ms for the
 // brute-force passes that then collected the entries (the list holds them all);
 // 2,000 reads against 70,000 tracks, k = 1,000: 0.83 ms against 4.1 and 4.0 ms.
+// Whole calls of 2,000 and of 100 reads against 470,000 tracks by k, with the replay
+// in brackets: 30,000 57 and 33 ms (230 and 173), 100,000 271 and 77 (535 and 409),
+// 400,000 761 and 123 (1,628 and 808): no k of this range is better off with it.
 // Tried and left out: integer sums in place of the FP64 ones in the groups, no
 // faster (39.9 against 41.4 ms for the whole call); warps that start from the
 // reads with the fewest dyes so as to help sooner, 1.55 against 1.67 ms in the
@@ -76,10 +79,11 @@
 #define KH_NB 1024     // distance bins: 16 octaves below the first leaf's farthest corner
 #define KH_SH 17       // float bits >> 17: exponent and 6 mantissa bits
 #define KH_WARPS 4     // warps per CTA
-#define KH_RANK 2048   // most entries of a group that are ranked
+#define KH_RANK 8192   // most entries of a group that are ranked (a power of two)
 #define KH_EPS 2e-6f   // bound of the FP32 distances' relative error (27 roundings, all terms >= 0)
 #define KH_GRP 96      // entries per group of bins, about
 #define KH_MAXG 1024   // groups
+#define KH_CROWD 9     // kh_group: the group cannot be taken in FP32 order
 #define KH_WAIT 4000000  // most turns of a wait (0.2 to 1 us each)
 
 struct KHSmem {
@@ -289,8 +293,11 @@ __device__ __forceinline__ KHList kh_list(const KHArgs& a, long gw, long own) {
 }
 
 // Looks inside group g of warp gw's list of n (its levels' n, from the state
-// above it): the larger of M and the largest found, or minus a fatal code.
-template <int DP>
+// above it): the larger of M and the largest found, or minus a fatal code; KH_CROWD
+// if more neighbours than a block takes lie within the FP32 error of one another.
+// EXACT: for a group that came to that, in the order of the FP64 distances (sets
+// dense at the top's distance: 9 of 150 reads at k = 200,000 of 470,000 tracks).
+template <int DP, bool EXACT>
 __device__ __noinline__ int kh_group(const KHArgs& a, long gw, long own, int n, int lane, int g, int tf, int k,
                                      const double* sq64, int M) {
     KHList L = kh_list(a, gw, own);
@@ -301,18 +308,23 @@ __device__ __noinline__ int kh_group(const KHArgs& a, long gw, long own, int n, 
     const int4 gr = L.group[g];
     const int m = gr.w - gr.z;
     if (m > KH_RANK) return -5;
-    // the group by FP32 distance (equal ones in any order)
-    for (int j = lane; j < m; j += 32)
-        L.mem_d[j] = ((long long)__float_as_uint(L.d[L.order[gr.z + j].x]) << 11) | j;
-    __syncwarp();
-    kh_rank(L, lane, m, [&](int j, int place) {
+    if constexpr (EXACT) {
+        kh_bin_d64<DP>(a, L, lane, gr.z, m, sq64);
+    } else {
+        // the group by FP32 distance (equal ones in any order)
+        for (int j = lane; j < m; j += 32)
+            L.mem_d[j] = (long long)__float_as_uint(L.d[L.order[gr.z + j].x]) * KH_RANK + j;
+        __syncwarp();
+    }
+    const bool distinct = kh_rank(L, lane, m, [&](int j, int place) {
         const int2 x = L.order[gr.z + j];
         L.sorted[place] = x;
         L.rank[x.x] = (uint16_t)place;
     });
+    if (EXACT && !distinct) return -6;
     __syncwarp();
     int Tx = st.x, cx = st.y, Hx = st.z;
-    // blocks of up to 32 levels, cut where neighbours differ by more
+    // blocks of up to 64 levels, cut where neighbours differ by more
     // than the FP32 error: n between the blocks and a bound inside,
     // as for the groups
     for (int j0 = 0; j0 < m && !fatal;) {
@@ -336,10 +348,10 @@ __device__ __noinline__ int kh_group(const KHArgs& a, long gw, long own, int n, 
                 cut[u] = __ballot_sync(0xffffffffu, j == m - 1 || (j < m - 1 && (u == 0 || lane < 31) &&
                                                                    d[u] * (1.f - KH_EPS) > next * (1.f + KH_EPS)));
             }
-            len = cut[0] ? 32 - __clz(cut[0]) : (cut[1] ? 32 + __ffs(cut[1]) : 0);
+            len = EXACT ? min(64, m - j0) : cut[0] ? 32 - __clz(cut[0]) : (cut[1] ? 32 + __ffs(cut[1]) : 0);
         }
-        if (len == 0) {
-            fatal = 9;
+        if (!EXACT && len == 0) {
+            fatal = KH_CROWD;
             break;
         }
 #pragma unroll
@@ -501,7 +513,8 @@ __device__ __forceinline__ void kh_help(const KHArgs& a, long own, int lane, KHS
         const int M = __shfl_sync(0xffffffffu, *(volatile int*)&sh->M, 0);
         g = pick[g];
         if (a.state[gw * 3 * KH_MAXG + g].w <= M) break;  // nor do the rest exceed it
-        const int found = kh_group<DP>(a, gw, own, n, lane, g, tf, k, sq64, M);
+        int found = kh_group<DP, false>(a, gw, own, n, lane, g, tf, k, sq64, M);
+        if (found == -KH_CROWD) found = kh_group<DP, true>(a, gw, own, n, lane, g, tf, k, sq64, M);
         if (lane == 0) {
             if (found > M) atomicMax(&sh->M, found);
             if (found < 0) atomicMax(&sh->fatal, -found);
