@@ -153,6 +153,12 @@ struct DevBuf {
         if (e == cudaSuccess) cap = want;
         return e;
     }
+    void release() {
+        if (p) cudaFree(p);
+        p = nullptr;
+        cap = 0;
+        g_alloc_epoch++;
+    }
     template <class T>
     T* as() const {
         return static_cast<T*>(p);
@@ -1145,17 +1151,28 @@ wp_status nn_khits(wp_ctx* ctx, const double* d_rads, int q0, int n, int slice_l
     long long grid = std::min<long long>((long long)sms * per_sm, (n + wpc - 1) / wpc);
     const size_t per_warp = (size_t)a.cap * 24 + (size_t)wp_khits_groups() * 56 + (size_t)wp_khits_rank() * 20;
     grid = std::max<long long>(1, std::min<long long>(grid, (long long)((6ull << 30) / (per_warp * wpc))));
-    const size_t warps = (size_t)grid * wpc, list = a.cap * warps;
-    WP_CUDA(ctx->d_kh_ent.ensure(sizeof(int2) * list), "alloc kNN lists");
-    WP_CUDA(ctx->d_kh_d.ensure(sizeof(float) * list), "alloc kNN lists");
-    WP_CUDA(ctx->d_kh_bin.ensure(sizeof(uint16_t) * list), "alloc kNN lists");
-    WP_CUDA(ctx->d_kh_order.ensure(sizeof(int2) * list), "alloc kNN lists");
-    WP_CUDA(ctx->d_kh_rank.ensure(sizeof(uint16_t) * list), "alloc kNN lists");
-    WP_CUDA(ctx->d_kh_state.ensure(sizeof(int4) * 3 * wp_khits_groups() * warps), "alloc kNN lists");
-    WP_CUDA(ctx->d_kh_seg.ensure(sizeof(int2) * wp_khits_groups() * warps), "alloc kNN lists");
-    WP_CUDA(ctx->d_kh_memd.ensure(sizeof(long long) * wp_khits_rank() * warps), "alloc kNN lists");
-    WP_CUDA(ctx->d_kh_memk.ensure(sizeof(unsigned) * wp_khits_rank() * warps), "alloc kNN lists");
-    WP_CUDA(ctx->d_kh_sorted.ensure(sizeof(int2) * wp_khits_rank() * warps), "alloc kNN lists");
+    // fewer warps where the device has not the memory left, down to one CTA; without
+    // even that the slots are left to the replay
+    const size_t list = a.cap, groups = wp_khits_groups(), ranked = wp_khits_rank();
+    const std::pair<DevBuf*, size_t> scratch[] = {
+            {&ctx->d_kh_ent, sizeof(int2) * list},        {&ctx->d_kh_d, sizeof(float) * list},
+            {&ctx->d_kh_bin, sizeof(uint16_t) * list},    {&ctx->d_kh_order, sizeof(int2) * list},
+            {&ctx->d_kh_rank, sizeof(uint16_t) * list},   {&ctx->d_kh_state, sizeof(int4) * 3 * groups},
+            {&ctx->d_kh_seg, sizeof(int2) * groups},      {&ctx->d_kh_memd, sizeof(long long) * ranked},
+            {&ctx->d_kh_memk, sizeof(unsigned) * ranked}, {&ctx->d_kh_sorted, sizeof(int2) * ranked}};
+    for (;; grid = (grid + 1) / 2) {
+        cudaError_t e = cudaSuccess;
+        for (const auto& b : scratch)
+            if (e == cudaSuccess) e = b.first->ensure(b.second * (size_t)grid * wpc);
+        if (e == cudaSuccess) break;
+        if (e != cudaErrorMemoryAllocation) return cuda_fail(ctx, e, "alloc kNN lists");
+        cudaGetLastError();
+        for (const auto& b : scratch) b.first->release();
+        if (grid == 1) {
+            WP_CUDA(cudaMemsetAsync(a.kept_n + q0, 0xff, sizeof(int) * n, ctx->stream), "clear");
+            return WP_OK;
+        }
+    }
     a.ent = ctx->d_kh_ent.as<int2>();
     a.d = ctx->d_kh_d.as<float>();
     a.bin = ctx->d_kh_bin.as<uint16_t>();
