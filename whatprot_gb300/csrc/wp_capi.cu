@@ -1092,9 +1092,14 @@ wp_status nn_prepare_peptides(wp_ctx* ctx) {
 
 // Whether the reference's k-hit sets can be found by levels (wp_khits.cu):
 // coordinates that are a channel's mean times the count, counts of at most 15,
-// hits that reach k and whose sums fit 31 bits.
+// hits that reach k and whose sums fit 31 bits.  From k = 3: the tree has a leaf per
+// k hits or so, and with leaves of one or two tracks most reads (at k = 1) or some (2)
+// have more leaves with tracks in them than the kernel notes, and are searched twice.
+// 2,000 reads, 470,000 tracks, with levels and without: k = 1 2,334 and 1,121 ms, 2
+// 475 and 254, 3 154 and 161, 4 114 and 126, 10 45 and 63; 70,000 tracks: 216 and
+// 116, 40 and 37, 21.6 and 26.8, 16.7 and 22.8 ms for 1 to 4.
 bool nn_by_levels(const wp_ctx* ctx, long long k) {
-    return ctx->nn_selection == WP_NN_KDTREE && !ctx->nn_inter && ctx->nn_NC >= 2 && ctx->nn_NC <= 16 &&
+    return k >= 3 && ctx->nn_selection == WP_NN_KDTREE && !ctx->nn_inter && ctx->nn_NC >= 2 && ctx->nn_NC <= 16 &&
            k <= ctx->nn_hits_total && ctx->nn_hits_total < (1ll << 31);
 }
 
