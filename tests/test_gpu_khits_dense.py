@@ -46,3 +46,34 @@ def test_dense(gpu_ctx):
             alone = (x - b2[:-2] > 1e-10 * x) & (b2[2:] - x > 1e-10 * x)
             alone[0] = alone[0] and n0[r] < 64
             assert np.array_equal(id0[r, :n0[r]][alone], id1[r, :n0[r]][alone]), r
+
+
+def test_distances_apart_in_64_bits_only(gpu_ctx):
+    """Reads a hair (1e-9) from equal distances to whole families of tracks: the order
+    within a family shows in the last bits of FP64, below FP32 and below the 32-bit keys
+    that entries are ranked by first."""
+    T, C, N, R, k = 6, 3, 5000, 60, 900
+    rng = np.random.default_rng(12)
+    tracks = rng.integers(0, 3, (2 * N, T, C)).astype(np.int16)
+    tracks[:, :, C - 1] = 0
+    tracks = np.unique(tracks.reshape(2 * N, -1), axis=0)
+    tracks = tracks[rng.permutation(len(tracks))[:N]].reshape(-1, T, C)
+    hits = np.minimum(rng.pareto(0.9, N) + 1, 50).astype(np.int32)
+    dts = DyeTrackSet(tracks, np.arange(N + 1, dtype=np.int32), rng.integers(0, N // 4, N).astype(np.int32),
+                      np.ones(N, np.int32), hits)
+    reads = 1.3 + 0.3 * rng.integers(0, 2, (R, 1, 1)) + rng.random((R, T, C)) * 1e-9
+    got = []
+    for interacting in (False, True):
+        sm = paper_model(C)
+        if interacting:
+            sm.channel_models[0].flat_interactions[C - 1] = 0.5
+        gpu_ctx.upload_model(sm, T)
+        gpu_ctx.upload_tracks(dts)
+        gpu_ctx.set_nn_selection("kdtree")
+        got.append(gpu_ctx.nn_classify(reads, k, 0.5, 64))
+        if not interacting:
+            assert gpu_ctx.last_routes()["levels"] >= R // 2
+    (n0, id0, sc0, tot0), (n1, id1, sc1, tot1) = got
+    assert np.array_equal(n0, n1)
+    assert np.allclose(tot0, tot1, rtol=1e-12, atol=0)
+    assert np.allclose(sc0, sc1, rtol=1e-12, atol=0)

@@ -693,7 +693,7 @@ struct KHArgs {
     uint16_t* bin;              // [warps][cap]
     int2* order;                // [warps][cap]
     uint16_t* rank;             // [warps][cap]
-    int4* state;                // [warps][2][groups]
+    int4* state;                // [warps][3][groups]
     long long* mem_d;           // [warps][rank limit]
     unsigned* mem_k;            // [warps][rank limit]
     int2* sorted;               // [warps][rank limit]

@@ -491,6 +491,21 @@ __device__ __noinline__ int kh_group(const KHArgs& a, long gw, long own, int n, 
     return fatal ? -fatal : M;
 }
 
+// The np groups picked of warp gw's list again, by itself and in FP64 order: the
+// largest n found, or minus a fatal code.
+template <int DP>
+__device__ __noinline__ int kh_exact_groups(const KHArgs& a, long gw, int lane, int np, int tf, int n, int k,
+                                            const double* sq64, int M) {
+    const int4* state = a.state + gw * 3 * KH_MAXG;
+    const int* pick = reinterpret_cast<const int*>(state + 2 * KH_MAXG);
+    for (int i = 0; i < np && state[pick[i]].w > M; i++) {
+        const int found = kh_group<DP, true>(a, gw, gw, n, lane, pick[i], tf, k, sq64, M);
+        if (found < 0) return found;
+        M = found;
+    }
+    return M;
+}
+
 // One warp's groups, for the CTA's warps to take (kh_help).
 struct KHShare {
     int open;   // groups can be taken
@@ -513,8 +528,7 @@ __device__ __forceinline__ void kh_help(const KHArgs& a, long own, int lane, KHS
         const int M = __shfl_sync(0xffffffffu, *(volatile int*)&sh->M, 0);
         g = pick[g];
         if (a.state[gw * 3 * KH_MAXG + g].w <= M) break;  // nor do the rest exceed it
-        int found = kh_group<DP, false>(a, gw, own, n, lane, g, tf, k, sq64, M);
-        if (found == -KH_CROWD) found = kh_group<DP, true>(a, gw, own, n, lane, g, tf, k, sq64, M);
+        const int found = kh_group<DP, false>(a, gw, own, n, lane, g, tf, k, sq64, M);
         if (lane == 0) {
             if (found > M) atomicMax(&sh->M, found);
             if (found < 0) atomicMax(&sh->fatal, -found);
@@ -1011,6 +1025,11 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(const __grid
             M = *(volatile int*)&sh->M;
             fatal = max(fatal, *(volatile int*)&sh->fatal);
             __syncwarp();
+            if (fatal == KH_CROWD) {
+                const int found = kh_exact_groups<DP>(a, gw, lane, np, tf, n, k, sq64, M);
+                fatal = max(-found, 0);
+                M = max(found, 0);
+            }
             // ---- 4. the M-th nearest entry
             if (!fatal) {
                 int b = -1;
@@ -1029,6 +1048,8 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(const __grid
                         L.rank[L.order[start + j].x] = (uint16_t)place;
                         if (place == want) at = j;
                     });
+                    // (ranked twice where 32-bit keys tie: the second time counts)
+                    if (at >= 0 && (int)L.rank[L.order[start + at].x] != want) at = -1;
                     const unsigned hit = __ballot_sync(0xffffffffu, at >= 0);
                     if (!distinct || !hit) fatal = 8;
                     __syncwarp();
