@@ -1712,7 +1712,8 @@ wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, in
         WP_CUDA(cudaMemcpyAsync(perm.data(), ctx->d_nn_qperm.p, sizeof(int) * R, cudaMemcpyDeviceToHost, ctx->stream), "copy");
         WP_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
         for (int r = 0; r < R; r++)
-            if (kept[r] < 0) rest.push_back(perm[r]);
+            if (kept[r] == WP_KH_LATE) return fail(ctx, WP_ERR_TIMEOUT, "kNN levels: a wait for another warp ran out");
+            else if (kept[r] < 0) rest.push_back(perm[r]);
         left = (int)rest.size();
         if (left > 0) {
             WP_CUDA(ctx->d_nn_subset.ensure(sizeof(int) * left), "alloc");

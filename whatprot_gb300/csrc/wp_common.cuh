@@ -711,6 +711,7 @@ struct KHArgs {
     float* kept_d2;             // [Rc][stride] FP32 squared distances as the collect pass forms them
     int* kept_n;                // [R]
 };
+#define WP_KH_LATE (-2)         // kept_n of a slot whose warp waited in vain: the call fails
 
 // FP64 squared distance from a query to entry p as LeafNode::consider sums
 // it (kd-tree/leaf-node.h:31-62): per coordinate x = q - e, x * x, summed in

@@ -83,6 +83,7 @@
 #define KH_EPS 2e-6f   // bound of the FP32 distances' relative error (27 roundings, all terms >= 0)
 #define KH_GRP 96      // entries per group of bins, about
 #define KH_MAXG 1024   // groups
+#define KH_LATE 15     // a wait ran out (the largest of a read's fatal codes)
 #define KH_CROWD 9     // kh_group: the group cannot be taken in FP32 order
 #define KH_WAIT 4000000  // most turns of a wait (0.2 to 1 us each)
 
@@ -536,6 +537,11 @@ __device__ __forceinline__ void kh_help(const KHArgs& a, long own, int lane, KHS
         __syncwarp();
         if (found < 0) break;
     }
+}
+
+// The slots nobody has taken yet: left to the replay.
+__device__ __noinline__ void kh_drain(const KHArgs& a) {
+    for (int i = atomicAdd(a.next, 1); i < a.Rc; i = atomicAdd(a.next, 1)) a.kept_n[a.q0 + a.Rc - 1 - i] = -1;
 }
 
 template <int DP>
@@ -1018,7 +1024,7 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(const __grid
                     __nanosleep(200);
                     wait++;
                 }
-                if (wait == KH_WAIT) sh->fatal = 14;
+                if (wait == KH_WAIT) sh->fatal = KH_LATE;
                 __threadfence_block();
             }
             __syncwarp();
@@ -1157,7 +1163,13 @@ __global__ void __launch_bounds__(KH_WARPS * 32, 4) wp_khits_kernel(const __grid
                 }
             }
         }
-        if (lane == 0) a.kept_n[slot] = fatal ? -1 : M;
+        if (lane == 0) a.kept_n[slot] = fatal ? (fatal == KH_LATE ? WP_KH_LATE : -1) : M;
+        if (fatal == KH_LATE) {
+            // a helper may still be using this warp's list and record: the warp looks
+            // into no more reads, and the call fails
+            if (lane == 0) kh_drain(a);
+            break;
+        }
         __syncwarp();
     }
     // no reads left: help until the CTA's other warps are through (or, past the
