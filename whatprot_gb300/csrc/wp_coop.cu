@@ -353,14 +353,12 @@ __global__ void __launch_bounds__(WP_COOP_THREADS) wp_coop_kernel(BatchArgs a, E
                 run = false;
             }
             const int nst = run ? vn : 0;  // states to go through
-            // strides of the bleached box, one byte per channel
-            uint32_t stpk = 0;
+            // strides of the bleached box
             int stb[C];
             int vb = 1;
 #pragma unroll
             for (int c = C - 1; c >= 0; c--) {
                 stb[c] = vb;
-                stpk = bset(stpk, c, vb);
                 vb *= bget(bx.w, c);
             }
             // failure plus success, rounded as edman_emit does (one rounding)
@@ -583,7 +581,6 @@ size_t wp_coop_smem_bytes(int slab_half, bool has_block, int lanes) {
     return ((sizeof(SmemModel) + 15) & ~(size_t)15) + sizeof(uint32_t) * ((WP_COOP_IDX + 1 + 3) & ~3) +
            pair * (WP_COOP_THREADS / lanes);
 }
-int wp_coop_max_half() { return WP_COOP_IDX; }
 
 template <int C, bool HB, int G>
 static cudaError_t launch_coop(cudaStream_t s, const BatchArgs& a, const EngineLists& L, long pairs) {

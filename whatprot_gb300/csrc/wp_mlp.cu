@@ -685,7 +685,7 @@ cudaError_t wp_mlp_launch_input(const float* xf, const double* xd, int B, int TC
     return cudaGetLastError();
 }
 
-// rows, cols multiples of 64; rows split so that every SM gets about eight CTAs.
+// rows, cols multiples of 64; a CTA takes CS_COLS columns and all rows.
 cudaError_t wp_mlp_launch_colsum(const bf16* M, int rows, int cols, int ld, float* out, cudaStream_t s) {
     if (rows % 64 || cols % 64) return cudaErrorInvalidValue;
     wp_colsum_bf16_kernel<<<cols / CS_COLS, 256, 0, s>>>(M, rows, ld, out);
