@@ -1357,7 +1357,7 @@ def run_fit(args):
             "config": {"workload": FIT_WORKLOAD, "reads": R, "timesteps": T, "channels": C,
                        "dye_seq": "".join("." if d < 0 else str(int(d)) for d in seq),
                        "l2": "flushed between steps (512 MB write)"},
-            "roofline": {"bound": "fp32", "kernel": "wp_fit_cta_kernel", "achieved": fit_achieved,
+            "roofline": {"bound": "fp32", "kernel": "wp_fit_warp_kernel", "achieved": fit_achieved,
                          "peak": fit_peak, "unit": "TFLOP/s",
                          "frac": (fit_achieved / fit_peak) if (fit_achieved and fit_peak) else None,
                          "traffic": None, "algorithmic_flops_per_step": fit_flops,
