@@ -1090,17 +1090,23 @@ wp_status nn_prepare_peptides(wp_ctx* ctx) {
     return WP_OK;
 }
 
-// Whether the reference's k-hit sets can be found by levels (wp_khits.cu):
-// coordinates that are a channel's mean times the count, counts of at most 15,
-// hits that reach k and whose sums fit 31 bits.  From k = 3: the tree has a leaf per
-// k hits or so, and with leaves of one or two tracks most reads (at k = 1) or some (2)
-// have more leaves with tracks in them than the kernel notes, and are searched twice.
-// 2,000 reads, 470,000 tracks, with levels and without: k = 1 2,334 and 1,121 ms, 2
-// 475 and 254, 3 154 and 161, 4 114 and 126, 10 45 and 63; 70,000 tracks: 216 and
-// 116, 40 and 37, 21.6 and 26.8, 16.7 and 22.8 ms for 1 to 4.
-bool nn_by_levels(const wp_ctx* ctx, long long k) {
-    return k >= 3 && ctx->nn_selection == WP_NN_KDTREE && !ctx->nn_inter && ctx->nn_NC >= 2 && ctx->nn_NC <= 16 &&
-           k <= ctx->nn_hits_total && ctx->nn_hits_total < (1ll << 31);
+// Whether R reads' k-hit sets are found by levels (wp_khits.cu): coordinates that
+// are a channel's mean times the count, counts of at most 15, hits that reach k and
+// whose sums fit 31 bits.  The tree has a leaf per k hits or so, and with few hits to
+// a leaf some reads (at k = 1 most) have more leaves with tracks in them than the
+// kernel notes and are searched twice, which shows where they are few.  Whole calls in
+// ms with levels, with the replay in brackets:
+// - 2 reads, 344,000 tracks: k = 24 3.4 (4.0), 16 4.4 (4.6), 8 8.6 (3.2), 4 13.2
+//   (3.3); one read of 12 against 1,016,000 tracks, levels' speed over the replay's:
+//   k = 48 0.82 to 1.61, 24 0.59 to 1.18, 16 0.49 to 1.82, 6 0.29 to 1.12;
+// - 16 reads, 36,000 / 344,000 / 1,016,000 tracks: k = 16 1.3 (2.1) / 13.6 (16.6) / 37
+//   (44), 4 3.1 (3.6) / 52 (54) / 157 (158), 3 4.0 (4.3) / 70 (71) / 222 (202);
+// - 2,000 reads, the same: k = 16 1.7 (3.5) / 15.8 (23.3) / 40 (57), 4 5.7 (5.7) / 58
+//   (60) / 166 (165), 3 7.2 (6.5) / 81 (78) / 247 (233); 470,000 tracks, k = 1 2,334
+//   (1,121).
+bool nn_by_levels(const wp_ctx* ctx, long long k, int R) {
+    return k >= (R >= 16 ? 4 : 24) && ctx->nn_selection == WP_NN_KDTREE && !ctx->nn_inter && ctx->nn_NC >= 2 &&
+           ctx->nn_NC <= 16 && k <= ctx->nn_hits_total && ctx->nn_hits_total < (1ll << 31);
 }
 
 // The k-hit sets by levels of the query slots q0 .. q0 + n: their candidate
@@ -1672,7 +1678,7 @@ wp_status nn_run(wp_ctx* ctx, const double* d_rads, int R, int k, double sig, in
     st = nn_sort_rows(ctx, ctx->d_nn_queries.as<float>(), R, DP, T * C);
     if (st != WP_OK) return st;
     int left = R;
-    if (nn_by_levels(ctx, k)) {
+    if (nn_by_levels(ctx, k, R)) {
         // the candidate lists of a chunk of reads, then their weights and scores.
         // A set has at most min(N, k) entries (each has a hit, and the set is some
         // walk prefix's shortest one); its bin's rest and the slices' gaps come on
