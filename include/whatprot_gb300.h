@@ -192,9 +192,10 @@ wp_status wp_fit_estep_batch(wp_ctx* ctx, const wp_seq_model* models, int B,
                              const int32_t* read_idx, int num_reads,
                              wp_fit_sums* out, double* sum_logp, int* num_zero);
 
-/* E-step kernel choice: 0 (default) by the shape: one warp per read with its
- * vectors in shared memory where enough of them fit, one CTA per read where
- * one fits, else one thread per read; 1 always one thread per read (tests
+/* E-step kernel choice: 0 (default) by the shape and the number of reads: one
+ * warp per read with its vectors in shared memory where enough of them fit, one
+ * CTA per read where one fits (and for few reads with long fibres or chains),
+ * else one thread per read; 1 always one thread per read (tests
  * compare them).  No reference counterpart. */
 wp_status wp_fit_set_kernel(wp_ctx* ctx, int kind);
 
@@ -556,8 +557,9 @@ wp_status wp_last_batch_stats(wp_ctx* ctx, long long* stats4);
 /* Which kernels the last calls on this context took (tests, tuning):
  * routes[0] reads of the last kNN batch whose k-hit set was found by levels,
  * [1] reads whose search was replayed, [2] the last dedup's keys (0 no dedup
- * yet, 1 words, 2 one key per instance).  No reference counterpart. */
-wp_status wp_last_routes(wp_ctx* ctx, long long* routes3);
+ * yet, 1 words, 2 one key per instance), [3] the last E-step's kernel (0 none
+ * yet, 1 a warp per read, 2 a CTA, 3 a thread).  No reference counterpart. */
+wp_status wp_last_routes(wp_ctx* ctx, long long* routes4);
 
 /* The context's CUDA stream (a cudaStream_t), for callers that order their
  * own work or events against it.  No reference counterpart. */

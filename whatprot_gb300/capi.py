@@ -773,10 +773,12 @@ class Context:
         return {"slots": int(out[0]), "nonempty": int(out[1]), "pass2": int(out[2]), "dense": int(out[3])}
 
     def last_routes(self) -> dict:
-        """wp_last_routes: reads of the last kNN batch by levels and replayed, the last dedup's keys."""
-        out = np.zeros(3, np.int64)
+        """wp_last_routes: reads of the last kNN batch by levels and replayed, the last dedup's keys,
+        the last E-step's kernel."""
+        out = np.zeros(4, np.int64)
         self._check(self.lib.wp_last_routes(self.h, _ptr(out)))
-        return {"levels": int(out[0]), "replayed": int(out[1]), "dedup": ("", "words", "rank")[int(out[2])]}
+        return {"levels": int(out[0]), "replayed": int(out[1]), "dedup": ("", "words", "rank")[int(out[2])],
+                "estep": ("", "warp", "cta", "thread")[int(out[3])]}
 
     def fp32_peak_tflops(self) -> float:
         out = ctypes.c_double()

@@ -122,6 +122,7 @@ cudaError_t wp_launch_fit_cta(bool has_block, int grid, size_t smem, cudaStream_
                               long ck_stride);
 int wp_fit_cta_ctas_per_sm(bool has_block, size_t smem);
 int wp_fit_warp_max_warps();
+int wp_fit_warp_register_dyes();
 size_t wp_fit_warp_smem_bytes(int T, int C, const int* D, bool hb, bool emission, int nslots, int warps);
 long wp_fit_warp_slab_floats(int T, int S, bool hb);
 int wp_fit_warp_ctas_per_sm(int C, bool hb, size_t smem, int warps);
@@ -316,7 +317,7 @@ struct wp_ctx {
     DevBuf d_nn_cnt8, d_nn_nodes, d_nn_ctab, d_nn_ecoord, d_nn_llo, d_nn_lhi;
     // the replay's scratch and results (wp_kbest.cu)
     DevBuf d_kb_reg, d_kb_prev, d_kb_stage, d_kb_next, d_kb_work, d_kb_tfd, d_kb_tfpos, d_kb_tfflag;
-    long long routes[3] = {0, 0, 0};  // wp_last_routes
+    long long routes[4] = {0, 0, 0, 0};  // wp_last_routes
     // the k-hit sets by levels (wp_khits.cu): counts as nibbles, scratch
     bool nn_nib_packed = false;
     DevBuf d_nn_nib, d_kh_ent, d_kh_d, d_kh_bin, d_kh_order, d_kh_rank, d_kh_state, d_kh_memd, d_kh_memk, d_kh_sorted, d_kh_seg, d_kh_kpos, d_kh_kd2,
@@ -1928,7 +1929,7 @@ void* wp_ctx_stream(const wp_ctx* ctx) { return ctx ? (void*)ctx->stream : nullp
 wp_status wp_last_routes(wp_ctx* ctx, long long* routes) {
     if (!ctx || !routes) return WP_ERR_INVALID;
     std::lock_guard<std::mutex> lk(ctx->mu);
-    for (int i = 0; i < 3; i++) routes[i] = ctx->routes[i];
+    for (int i = 0; i < 4; i++) routes[i] = ctx->routes[i];
     return WP_OK;
 }
 
@@ -2449,19 +2450,36 @@ wp_status wp_fit_begin(wp_ctx* ctx, const int16_t* dye_seq, int length, const do
     return WP_OK;
 }
 
-// Which E-step kernel takes a shape: a warp per read where at least eight
-// warps' vectors fit an SM's shared memory (60.3 against 5.6 ms for 50,000 reads
-// of 80 states and 16 timesteps; with fewer warps their latency shows and a
-// CTA per read is no slower), else a CTA per read where one read fits, else
-// none (the thread-per-read kernel).
+// Which E-step kernel takes B lists of R reads of a shape: a warp per read where at
+// least eight warps' vectors fit an SM's shared memory (60.3 against 5.6 ms for 50,000
+// reads of 80 states and 16 timesteps; with fewer warps their latency shows and a
+// CTA per read is no slower), else a CTA per read where one read fits, else none (the
+// thread-per-read kernel).
+//
+// A warp takes longer over a read than a CTA does where fibres are too long for
+// registers (a channel of 6 dyes or more), with blocking, several such channels, 13
+// dyes or long chains, and in long blocked chains of any dyes.  That shows while the
+// reads are no more than a turn of resident CTAs (some 304 reads); from the second
+// turn on the many warps win.  E-steps in ms, warp and (CTA): one channel of 10 dyes,
+// 64 timesteps, blocked, 300 reads 1.55 (0.92), 500 1.54 (1.73), 5,000 5.5 (15.3); 7 + 7
+// dyes, 12 timesteps, 8 reads 0.24 (0.22), blocked 0.39 (0.23); 6 dyes, 12 timesteps,
+// 300 reads 0.12 (0.14), blocked, 8 0.15 (0.14); 6 dyes, 64 timesteps, 8 reads 0.75
+// (0.64); 1 dye, 64 timesteps, blocked, 8 reads 0.65 (0.56), 500 0.67 (1.22).  The
+// longest fibres, blocked, need more turns: 15 dyes, 24 timesteps, 500 reads 0.73
+// (0.65), 700 0.74 (0.92); 64 timesteps, 300 3.7 (1.2), 1,500 7.3 (5.7), 2,400 7.3
+// (8.8).
 struct FitShape {
     int warps = 0;   // warps (reads at a time) per CTA of the warp kernel, 0: the CTA kernel
     int per_sm = 0;  // resident CTAs per SM
     size_t smem = 0;
     long stride = 0;  // scratch floats per CTA
 };
-static FitShape fit_shape(const wp_ctx* ctx, int T, int C, const int* D, int S, bool hb, bool emis) {
-    FitShape f;
+static FitShape fit_shape(const wp_ctx* ctx, int T, int C, const int* D, int S, bool hb, bool emis, long R, int B) {
+    FitShape f, cta;
+    cta.smem = wp_fit_cta_smem_bytes(T, C, S, hb, emis);
+    // (the kernel also holds the binomial tables in static shared memory)
+    cta.per_sm = (long)cta.smem + (long)sizeof(SmemModel) <= (long)ctx->smem_optin ? wp_fit_cta_ctas_per_sm(hb, cta.smem) : 0;
+    cta.stride = wp_fit_cta_ckpt_floats(T, S, hb);
     // the CTA size with the most resident warps
     for (int w = wp_fit_warp_max_warps(); w >= 1; w--) {
         const size_t smem = wp_fit_warp_smem_bytes(T, C, D, hb, emis, wp_fit_nslots(T, C, emis), w);
@@ -2472,15 +2490,18 @@ static FitShape fit_shape(const wp_ctx* ctx, int T, int C, const int* D, int S, 
             f.smem = smem;
         }
     }
-    if (f.per_sm * f.warps >= 8) {
-        f.stride = wp_fit_warp_slab_floats(T, S, hb) * f.warps;
-        return f;
+    if (f.per_sm * f.warps < 8) return cta;
+    f.stride = wp_fit_warp_slab_floats(T, S, hb) * f.warps;
+    int most = 0, wide = 0, turns = 0, sms = 0;
+    for (int c = 0; c < C; c++) {
+        most = std::max(most, D[c]);
+        wide += D[c] > wp_fit_warp_register_dyes() ? 1 : 0;
     }
-    f.warps = 0;
-    f.smem = wp_fit_cta_smem_bytes(T, C, S, hb, emis);
-    // (the kernel also holds the binomial tables in static shared memory)
-    f.per_sm = (long)f.smem + (long)sizeof(SmemModel) <= (long)ctx->smem_optin ? wp_fit_cta_ctas_per_sm(hb, f.smem) : 0;
-    f.stride = wp_fit_cta_ckpt_floats(T, S, hb);
+    if (wide > 0 && hb) turns = most < 13 || T < 20 ? 1 : (T <= 40 ? 2 : 5);
+    else if (wide > 0) turns = most >= 13 || wide > 1 || T > 32 ? 1 : 0;
+    else turns = hb && T > 40 ? 1 : 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    if (cta.per_sm > 0 && R <= turns * std::max<long>(1, (long)sms * cta.per_sm / B)) return cta;
     return f;
 }
 
@@ -2527,8 +2548,9 @@ wp_status wp_fit_estep(wp_ctx* ctx, wp_fit_sums* out, double* sum_logp, int* num
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     const bool emis = ctx->fit_emission;
     const int nslots = wp_fit_nslots(T, C, emis);
-    const FitShape shape = fit_shape(ctx, T, C, ctx->fit_D, S, hb, emis);
+    const FitShape shape = fit_shape(ctx, T, C, ctx->fit_D, S, hb, emis, R, 1);
     const bool use_cta = shape.per_sm > 0 && !ctx->fit_force_thread;
+    ctx->routes[3] = !use_cta ? 3 : shape.warps ? 1 : 2;
     const int threads = 128;
     int grid = 0;
     long nth = 0, per = 0;
@@ -2667,8 +2689,9 @@ wp_status wp_fit_estep_batch(wp_ctx* ctx, const wp_seq_model* models, int B, con
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     const int nslots = wp_fit_nslots(T, C, false);
-    const FitShape shape = fit_shape(ctx, T, C, ctx->fit_D, S, hb, false);
+    const FitShape shape = fit_shape(ctx, T, C, ctx->fit_D, S, hb, false, Rb, B);
     if (shape.per_sm <= 0) return fail(ctx, WP_ERR_UNSUPPORTED, "batched E-steps need the CTA-per-read kernel");
+    ctx->routes[3] = shape.warps ? 1 : 2;
     // CTAs per instance: the device's resident CTAs shared out (rounded down,
     // so that all CTAs are resident in one wave), at most one per read
     const long reads_per_cta = std::max(1, shape.warps);

@@ -830,6 +830,9 @@ static const void* fw_pick(int C, bool hb) {
 
 int wp_fit_warp_max_warps() { return FW_WARPS; }
 
+// Dyes of a channel up to which its fibres are processed in registers.
+int wp_fit_warp_register_dyes() { return FW_MAXW - 1; }
+
 // Resident CTAs per SM (0: the shape does not fit).
 int wp_fit_warp_ctas_per_sm(int C, bool hb, size_t smem, int warps) {
     const void* k = fw_pick(C, hb);
